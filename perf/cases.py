@@ -31,25 +31,25 @@ def listed():
         # The smallest call: one sequence of a small model, where launches and latency are what a token costs.
         dict(name="gpt2-small step", model="gpt2-small", mode="decode", weights="fp16", layers=12, rows=1, context=159),
         # The largest GPT-2 for sixteen sequences (four prompts with four hypotheses each have as many rows); 25 heads, width 1600.
-        dict(name="gpt2-xl step, 16 rows", model="gpt2-xl", mode="decode", weights="fp16", layers=48, rows=16, context=255),
+        dict(name="gpt2-xl step 16 rows", model="gpt2-xl", mode="decode", weights="fp16", layers=48, rows=16, context=255),
         # Chat with one user on a 7B model with INT4 weights: the headline workload.
         dict(name="llama-7b step", model="llama-7b", mode="decode", weights="int4", group=128, layers=32, rows=1, context=511),
         # The same model serving a batch ...
-        dict(name="llama-7b step, 16 rows", model="llama-7b", mode="decode", weights="int4", group=128, layers=32, rows=16, context=511),
+        dict(name="llama-7b step 16 rows", model="llama-7b", mode="decode", weights="int4", group=128, layers=32, rows=16, context=511),
         # ... and a larger one at a shorter context.
-        dict(name="llama-7b step, 32 rows", model="llama-7b", mode="decode", weights="int4", group=128, layers=32, rows=32, context=255),
+        dict(name="llama-7b step 32 rows", model="llama-7b", mode="decode", weights="int4", group=128, layers=32, rows=32, context=255),
         # Time to the first token: a prompt in one pass, then the step that reads its last token.
         dict(name="llama-7b prompt", model="llama-7b", mode="prompt", weights="int4", group=128, layers=32, rows=1, context=511),
         # fp16 weights (the reference's default precision), multi-query attention, a long context, a small batch.
-        dict(name="chatglm2 step, 8 rows", model="chatglm2-6b", mode="decode", weights="fp16", layers=28, rows=8, context=1151),
+        dict(name="chatglm2 step 8 rows", model="chatglm2-6b", mode="decode", weights="fp16", layers=28, rows=8, context=1151),
         # FP8 through the operator surface: the casts and products of the matrices of four blocks and the output layer.  (Not as whole
         # steps: casts whose input lies between two E4M3 values make two right implementations drift apart by several per cent within
         # one block.)
-        dict(name="chatglm2 fp8 products, 8 rows", model="chatglm2-6b", mode="products", weights="fp8", layers=4, rows=8, context=0),
+        dict(name="chatglm2 fp8 products 8 rows", model="chatglm2-6b", mode="products", weights="fp8", layers=4, rows=8, context=0),
         # A recurrent model takes a prompt token by token: eight iterations of the loop for 32 sequences.
-        dict(name="rwkv loop, 32 rows", model="rwkv4-1b5", mode="loop", weights="fp16", layers=24, rows=32, context=8),
+        dict(name="rwkv loop 32 rows", model="rwkv4-1b5", mode="loop", weights="fp16", layers=24, rows=32, context=8),
         # Hybrid decoder (attention and state-space layers), a step of a small batch behind long prompts.
-        dict(name="sabisun-2k step, 8 rows", model="sabisun-2k", mode="decode", weights="bf16", layers=16, rows=8, context=2047),
+        dict(name="sabisun-2k step 8 rows", model="sabisun-2k", mode="decode", weights="bf16", layers=16, rows=8, context=2047),
         # A long prompt of one sequence, logits of its last token.
         dict(name="sabisun-2k prompt", model="sabisun-2k", mode="serve", weights="bf16", layers=16, rows=1, context=2048, tokens=0),
         # Requests of unequal lengths: all prompts as one batch, then six more tokens each, then they end.
