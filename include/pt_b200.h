@@ -187,7 +187,8 @@ int pt_linear_static_scratch(const pt_linear_args *args, void *stream);
  *              (w_tiled = 1: one contiguous bulk copy per stage, the layout for a model's weights).
  *   PT_W_INT4: x = fp16 [m, k_in], w = pt_gemm_repack of the reference's int8 [n_out, k_in/2] rows (w_tiled = 1), scales fp16
  *              [n_out, k_in/group]; every weight becomes fp16(q) * scale with one rounding (Int4ToHalf,
- *              custom_ops/int4_to_half_codelets.cpp:18-38) on its way to the tensor core.
+ *              custom_ops/int4_to_half_codelets.cpp:18-38) on its way to the tensor core.  Also epilogue PT_EPI_SWIGLU: rows in the
+ *              interleaved order of pt_linear_repack (eight gate rows, the same eight up rows), out [m, n_out / 2].
  *   PT_W_BF16: x = bf16 [m, k_in], w = pt_gemm_repack of bf16 [n_out, k_in] (w_tiled = 1); out = bf16 or fp32 (out_dtype),
  *              epilogue PT_EPI_STORE, _RELU2, _GLU or _GELU_MUL on alpha * (x . w^T).  k_in a multiple of 64.
  * FP8 and INT4: k_in must be a multiple of 128.  Accumulation is fp32.  k-slices (ksplit, 0 = chosen by the library) are summed in a fixed
@@ -196,8 +197,8 @@ typedef struct pt_gemm_args {
   int wfmt;               /* PT_W_FP8, PT_W_INT4 or PT_W_BF16                       */
   int m, n_out, k_in;
   int group;              /* INT4: scale group along k (a multiple of 128)          */
-  int epilogue;           /* PT_EPI_STORE, PT_EPI_RESIDUAL or PT_EPI_BIAS            */
-  int ksplit;             /* 0 = let the library choose                             */
+  int epilogue;           /* PT_EPI_STORE, PT_EPI_RESIDUAL, PT_EPI_BIAS or (INT4) PT_EPI_SWIGLU */
+  int ksplit;             /* 0 = let the library choose (INT4: at most 8 are made of what is asked for) */
   int w_tiled;            /* 1: w was tiled by pt_gemm_repack; 0: row-major (FP8 only) */
   const void *x, *w;
   const void *scales;     /* INT4: fp16 [n_out, k_in / group]                        */
@@ -212,7 +213,7 @@ typedef struct pt_gemm_args {
   int out_dtype;          /* PT_W_BF16: PT_DT_BF16 or PT_DT_F32                      */
   float alpha;            /* PT_W_BF16: factor on the fp32 sum; 0 = 1                */
   const pt_dense_ext *ext; /* PT_W_BF16: further arguments, or NULL                  */
-  int pdl;                /* PT_W_BF16: 1: programmatic dependent launch (see pt_linear_args.pdl) */
+  int pdl;                /* PT_W_BF16, PT_W_INT4: 1: programmatic dependent launch (see pt_linear_args.pdl) */
 } pt_gemm_args;
 size_t pt_gemm_workspace_bytes(int m, int n_out, int max_ksplit);
 int pt_gemm(const pt_gemm_args *args, void *stream);

@@ -5,9 +5,9 @@
 //           in the E4M3 form): tcgen05.mma kind::f8f6f4, fp32 accumulation in tensor memory, scales applied in the epilogue.
 //   * BF16: W and X bfloat16, tcgen05.mma kind::f16, bf16 or fp32 output with the epilogues of dense_out.cuh: the same kernel as FP8
 //           with 64 elements of k per 128-byte operand row.  Grouped: every tile of activation rows names its weight matrix.
-//   * INT4: W is packed nibbles with fp16 group scales (utils/param_handler/precision_strategy.py:24-42,56-60).  A transform
-//           warpgroup turns every staged tile into fp16(q) * scale - one fp16 rounding per weight, exactly the reference's
-//           Int4ToHalf (custom_ops/int4_to_half_codelets.cpp:18-38) - in the shared-memory layout the tensor core reads;
+//   * INT4: W is packed nibbles with fp16 group scales (utils/param_handler/precision_strategy.py:24-42,56-60).  Transform
+//           warps turn every staged tile into fp16(q) * scale - one fp16 rounding per weight, exactly the reference's
+//           Int4ToHalf (custom_ops/int4_to_half_codelets.cpp:18-38) - in tensor memory, where the MMA takes its A operand from;
 //           tcgen05.mma kind::f16 multiplies it with the fp16 activations, fp32 accumulation.
 //
 // The weights are the big operand, so they take the 128-row M side of the instruction and the activation rows the N side
@@ -18,8 +18,9 @@
 // the row width, which caps an SM near 25 GB/s; contiguous bulk copies stream at the HBM rate).  The activations (few rows) and
 // the row-major weights of the plain FP8MatMul op come through tiled TMA (cp.async.bulk.tensor; this GPU's memory only, no
 // multicast).  One thread issues the MMAs and hands stages back with tcgen05.commit; the other warps convert (INT4: a deep ring
-// of raw nibble tiles feeds a short ring of fp16 operand tiles) and run the epilogue (tcgen05.ld, scale, fp16, coalesced stores
-// along n).  k-slices of one tile meet in a workspace and the last CTA to arrive sums them in slice order (deterministic).
+// of raw nibble tiles feeds a few slots of fp16 weights) and run the epilogue (tcgen05.ld, scale, fp16, coalesced stores
+// along n).  k-slices of one tile are summed in slice order (deterministic): INT4 by the blocks of a cluster, FP8 and BF16 in a
+// workspace by the last CTA to arrive.
 // Every wait is bounded: on a time-out the CTA raises the error flag, skips its remaining waits and still frees its tensor
 // memory.
 #include <cuda.h>
@@ -38,9 +39,10 @@ namespace tc {
 constexpr int BM = 128;            // weight rows per CTA
 constexpr int BKB = 128;           // bytes of k per stage and operand row (one 128-byte swizzle atom)
 constexpr int THREADS_F8 = 192;    // warp 0: producer, warp 1: MMA + tensor-memory allocation, warps 2-5: epilogue
-constexpr int THREADS_I4 = 352;    // warp 0: raw-tile producer, warp 1: MMA, warps 2-9: transform + epilogue, warp 10: activation producer
+constexpr int MAX_CLUSTER = 8;     // k-slices of a tile (one cluster)
 constexpr int A_TILE = BM * BKB;   // 16 KB: 128 rows x 128 bytes of k, 128-byte swizzle
 constexpr int RAW_TILE = BM * 32;  // 4 KB: 128 rows x 64 k of packed nibbles
+constexpr int RAW_STEP = 2 * RAW_TILE;   // a step of the INT4 kernel: 128 k
 
 struct GemmParams {
   int M, N, K;
@@ -71,6 +73,13 @@ struct GemmParams {
 
 // ------------------------------------------------------------------------------------------ PTX
 __device__ __forceinline__ uint32_t sa(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// One lane of the (whole) warp.  The single-thread roles go by it: the compiler then knows that one lane runs, and gives the instructions
+// that take uniform registers (bulk copies, MMAs, commits) their operands without a loop over the lanes.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+  return pred != 0;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(map),
                "r"(bar), "r"(x), "r"(y)
@@ -96,6 +105,35 @@ __device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t b
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d_tmem),
                  "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
                  : "memory");
+}
+// The same with A in tensor memory (lane = row, a column holds two consecutive k), fp16.
+__device__ __forceinline__ void umma_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d_tmem),
+               "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+               "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+               "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+               "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]),
+               "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// Distributed shared memory of a cluster: a local address in block `rank`, and all threads of all its blocks meeting.
+__device__ __forceinline__ uint32_t in_block(uint32_t local, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float4 load_cluster4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // The mbarrier gets one arrival once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -158,16 +196,160 @@ __device__ __forceinline__ void give_up(SharedCtl &ctl, int *error_flag, int cod
   ctl.abort = 1;
 }
 
-// One finished sum of the FP8 / INT4 kernels (fp16 output) or of the BF16 kernel.
+// A wait inside a hot loop: the first look is inline, the rest a call.
+__device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return mbar_wait(bar, parity, abort_flag); }
+__device__ __forceinline__ bool wait_fast(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return mbar_test(bar, parity) || wait_on(bar, parity, abort_flag); }
+// The same for a whole warp: every lane gets the same answer.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return __all_sync(0xffffffffu, wait_fast(bar, parity, abort_flag)); }
+
+// One finished sum of the FP8 / INT4 kernels (fp16 output) or of the BF16 kernel.  (SWIGLU, whose sums come in pairs: store_swiglu.)
+__device__ __forceinline__ __half fp16_out(const GemmParams &p, float acc, int m, int n) {
+  __half y = __float2half_rn(acc * p.out_scale);
+  if (p.epilogue == PT_EPI_RESIDUAL) return h_add(__ldcg(p.residual + (size_t)m * p.N + n), y);
+  if (p.epilogue == PT_EPI_BIAS) return h_add(y, p.bias[n]);
+  return y;
+}
 template <bool BF16, bool EXT> __device__ __forceinline__ void store_out(const GemmParams &p, float acc, int m, int n) {
-  if constexpr (BF16) {
-    dense_store<EXT>(p.dense, m, n, acc);
+  if constexpr (BF16) dense_store<EXT>(p.dense, m, n, acc);
+  else p.out[(size_t)m * p.out_ld + n] = fp16_out(p, acc, m, n);
+}
+// Sums of the gate row n (n % 16 < 8) and of the up row n + 8.
+__device__ __forceinline__ __half swiglu_h(const GemmParams &p, float gate, float up) {
+  return h_mul(__float2half_rn(up * p.out_scale), swish_h(__float2half_rn(gate * p.out_scale)));
+}
+// Sixteen rows m .. m + 15 of a warp's 32 weight rows (lane = n), all inside the output, fp16.  Neighbouring lanes trade values so that a
+// lane writes two consecutive n (SWIGLU: lanes n and n + 8, and each computes every other row of the pair's feature).
+template <int EPI> __device__ __forceinline__ void fp16_rows16(const GemmParams &p, const float (&sum)[16], int m, int n, int lane) {
+  if constexpr (EPI == PT_EPI_SWIGLU) {
+    const bool up = lane & 8;
+    __half *o = p.out + (size_t)(m + (up ? 1 : 0)) * p.out_ld + n / 16 * 8 + n % 8;
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      const float t = __shfl_xor_sync(0xffffffffu, up ? sum[j] : sum[j + 1], 8);
+      *o = up ? swiglu_h(p, t, sum[j + 1]) : swiglu_h(p, sum[j], t);
+      o += 2 * (size_t)p.out_ld;
+    }
   } else {
-    __half y = __float2half_rn(acc * p.out_scale);
-    if (p.epilogue == PT_EPI_RESIDUAL) y = h_add(__ldcg(p.residual + (size_t)m * p.N + n), y);
-    else if (p.epilogue == PT_EPI_BIAS) y = h_add(y, p.bias[n]);
-    p.out[(size_t)m * p.out_ld + n] = y;
+    const int odd = lane & 1;
+    __half2 *o = reinterpret_cast<__half2 *>(p.out + (size_t)(m + odd) * p.out_ld + (n - odd));
+    __half2 res[EPI == PT_EPI_RESIDUAL ? 8 : 1], bias = __half2half2(__half(0));
+    if constexpr (EPI == PT_EPI_RESIDUAL) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) res[j] = __ldcg(reinterpret_cast<const __half2 *>(p.residual + (size_t)(m + odd + 2 * j) * p.N + (n - odd)));
+    }
+    if constexpr (EPI == PT_EPI_BIAS) bias = *reinterpret_cast<const __half2 *>(p.bias + (n - odd));
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      const float t = __shfl_xor_sync(0xffffffffu, odd ? sum[j] : sum[j + 1], 1);   // even lane: row j of n + 1; odd lane: row j + 1 of n - 1
+      __half2 y = odd ? __floats2half2_rn(t * p.out_scale, sum[j + 1] * p.out_scale) : __floats2half2_rn(sum[j] * p.out_scale, t * p.out_scale);
+      if constexpr (EPI == PT_EPI_RESIDUAL) y = __hadd2_rn(res[j / 2], y);
+      if constexpr (EPI == PT_EPI_BIAS) y = __hadd2_rn(y, bias);
+      *o = y;
+      o += p.out_ld;   // (two rows, in units of two)
+    }
   }
+}
+// The epilogue of a tile without k-slices, fp16 outputs: `part` of `parts` warps share a quarter of the rows and take alternate 16 columns.
+__device__ __forceinline__ void epilogue_fp16(const GemmParams &p, uint32_t tmem, int q, int lane, int part, int parts, int n0, int m0) {
+  const int nq = n0 + q * 32, n = nq + lane, rows = min(p.mb, p.M - m0);
+  const bool pairs = nq + 32 <= p.N && p.out_ld % 2 == 0 && ((uintptr_t)p.out & 3) == 0 && (p.epilogue != PT_EPI_RESIDUAL || (p.N % 2 == 0 && ((uintptr_t)p.residual & 3) == 0)) &&
+                     (p.epilogue != PT_EPI_BIAS || ((uintptr_t)p.bias & 3) == 0);   // (uniform over the warp)
+  for (int c0 = part * 16; c0 < rows; c0 += 16 * parts) {
+    uint32_t v[16];
+    float sum[16];
+    tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) sum[j] = __uint_as_float(v[j]);
+    const int m = m0 + c0;
+    if (pairs && c0 + 16 <= rows) {
+      if (p.epilogue == PT_EPI_SWIGLU) fp16_rows16<PT_EPI_SWIGLU>(p, sum, m, n, lane);
+      else if (p.epilogue == PT_EPI_RESIDUAL) fp16_rows16<PT_EPI_RESIDUAL>(p, sum, m, n, lane);
+      else if (p.epilogue == PT_EPI_BIAS) fp16_rows16<PT_EPI_BIAS>(p, sum, m, n, lane);
+      else fp16_rows16<PT_EPI_STORE>(p, sum, m, n, lane);
+      continue;
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (c0 + j >= rows) break;
+      if (p.epilogue == PT_EPI_SWIGLU) {
+        const float up = __shfl_xor_sync(0xffffffffu, sum[j], 8);
+        if (n < p.N && !(lane & 8)) p.out[(size_t)(m + j) * p.out_ld + n / 16 * 8 + n % 8] = swiglu_h(p, sum[j], up);
+      } else if (n < p.N) {
+        store_out<false, false>(p, sum[j], m + j, n);
+      }
+    }
+  }
+}
+// Four consecutive fp16 outputs n .. n + 3 < N (n a multiple of four).
+__device__ __forceinline__ void fp16_store4(const GemmParams &p, int m, int n, const float4 &acc) {
+  const float a[4] = {acc.x, acc.y, acc.z, acc.w};
+  __half y[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) y[j] = fp16_out(p, a[j], m, n + j);
+  __half *o = p.out + (size_t)m * p.out_ld + n;
+  if (((uintptr_t)o & 7) == 0) *reinterpret_cast<uint2 *>(o) = *reinterpret_cast<const uint2 *>(y);
+  else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = y[j];
+  }
+}
+
+// k-slices of a tile: the blocks of a cluster, slice = rank.  Every block leaves its sums in its own shared memory as [mb][128] floats
+// (`part`: the operand ring, which nobody reads any more), the blocks meet, each sums its share of the tile over all of them in slice
+// order (deterministic) and writes it, and they meet again before their shared memory goes.  On B200 this replaces sums that went
+// through global memory to the last block to arrive, which then summed the whole tile alone.
+__device__ __forceinline__ void leave_sums(const GemmParams &p, uint32_t tmem, int q, int lane, int part, int parts, float *dst) {
+  for (int c0 = part * 16; c0 < p.mb; c0 += 16 * parts) {
+    uint32_t v[16];
+    tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) dst[(c0 + j) * BM + q * 32 + lane] = __uint_as_float(v[j]);
+  }
+}
+template <bool BF16, bool EXT>
+__device__ __forceinline__ void sum_cluster(const GemmParams &p, const SharedCtl &ctl, uint32_t part, int rank, int n0, int m0, int m_end, int threads) {
+  cluster_meet();
+  if (!ctl.abort) {
+    const int units = min(p.mb, m_end - m0) * (BM / 4), share = (units + p.ksplit - 1) / p.ksplit, last = min(units, (rank + 1) * share);
+    for (int i = rank * share + (int)threadIdx.x; i < last; i += threads) {
+      const int m = m0 + i / (BM / 4), n = n0 + (i % (BM / 4)) * 4;
+      if (n >= p.N) continue;
+      auto sum4 = [&](int unit) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int s0 = 0; s0 < p.ksplit; s0 += 4) {   // four loads in flight
+          float4 v[4];
+#pragma unroll
+          for (int s = 0; s < 4; ++s) v[s] = s0 + s < p.ksplit ? load_cluster4(in_block(part + unit * 16, s0 + s)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int s = 0; s < 4; ++s) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
+        }
+        return acc;
+      };
+      const bool glu = BF16 ? p.dense.epilogue == PT_EPI_GLU && n < p.dense.split_n : p.epilogue == PT_EPI_SWIGLU;
+      if (glu) {   // gate rows n % 16 < 8, their up rows eight further
+        if (n & 8) continue;
+        const float4 g = sum4(i), u = sum4(i + 2);
+        if constexpr (BF16) {
+          dense_store_glu4<EXT>(p.dense, m, n, g, u);
+        } else {
+          __half *o = p.out + (size_t)m * p.out_ld + n / 16 * 8 + n % 8;
+          o[0] = swiglu_h(p, g.x, u.x); o[1] = swiglu_h(p, g.y, u.y); o[2] = swiglu_h(p, g.z, u.z); o[3] = swiglu_h(p, g.w, u.w);
+        }
+        continue;
+      }
+      const float4 acc = sum4(i);
+      if (n + 4 <= p.N) {
+        if constexpr (BF16) dense_store4<EXT>(p.dense, m, n, acc);
+        else fp16_store4(p, m, n, acc);
+      } else {
+        store_out<BF16, EXT>(p, acc.x, m, n);
+        if (n + 1 < p.N) store_out<BF16, EXT>(p, acc.y, m, n + 1);
+        if (n + 2 < p.N) store_out<BF16, EXT>(p, acc.z, m, n + 2);
+      }
+    }
+  }
+  cluster_meet();
 }
 
 // Sixteen rows of one weight row per lane, gated: lanes n and n + 8 hold a feature's two sums.
@@ -523,37 +705,45 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
 }
 
 // ------------------------------------------------------------------------------------------ INT4
-// Dynamic shared memory: [operand stage][A tile 16 KB | B tile mb * 128 B] then [raw stage][4 KB of packed nibbles].
-// The raw ring is deep (it is what keeps HBM busy: up to 24 x 4 KB in flight per SM), the operand ring short.
-__global__ void __launch_bounds__(THREADS_I4, 1) gemm_int4_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
+// Weights go through the tensor memory: a transform warp turns a thread's row of a raw tile (128 nibbles) into 64 registers of fp16 pairs and
+// stores them to 64 tensor-memory columns, where the MMA reads its A operand (lane = weight row); shared memory holds only the raw ring
+// and the activations.  NG groups of four transform warps (one warp per quarter of the lanes) take the steps of 128 k in turn, so that the
+// chain of a step - raw tile, nibbles, slot free, tensor memory, MMA - overlaps with that of its neighbours.
+// What bounds it: up to about 100 activation rows the instructions of the single-thread roles and of the transform, beyond it the MMAs
+// (8 x mb / 2 cycles a step).  A wait costs a single thread a hundred cycles or more even when nothing is left to wait for, so a step has ONE
+// barrier in front of the MMAs (activations and weights arrive on the same one) and is 128 k deep.  The form before this one (64 k a
+// step, fp16 tiles through shared memory, eight warps in step) took 1500 cycles per 64 k whatever the number of rows.  Measured on B200,
+// 12288 x 4096 / 4096 x 11008, before and after: 16 rows 35 / 39 and 14.5 / 13 us, 511 rows 105 / 164 and 44.5 / 41 us (1150 TFLOP/s).
+// The groups run apart, and a wait tells only odd from even uses of a barrier.  A group that has done step i waits next for use (i + NG) / S of
+// slot (i + NG) % S; that the use before it is over follows from step i - S being over (which step i waited for) only if NG <= S.  The
+// same for a raw stage, whose copies may land in any order: R >= NG + S.
+// Dynamic shared memory: [slot][activations: two halves of 64 k, mb * 128 B each][raw stage][8 KB of packed nibbles].
+template <int NG>
+__global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
+  constexpr int THREADS = (3 + 4 * NG) * 32;   // warp 0: raw tiles, warp 1: MMA, then 4 NG transform + epilogue, last: activations
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ SharedCtl ctl;
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int n0 = blockIdx.x * BM, m0 = blockIdx.z * p.mb, ks = blockIdx.y;
-  const int kb0 = ks * p.kb_per_split, kb1 = min(p.n_kb, kb0 + p.kb_per_split);
-  const int n_it = kb1 - kb0;
+  const int st0 = ks * p.kb_per_split, n_it = min(p.n_kb, st0 + p.kb_per_split) - st0;   // (in steps)
   const int S = p.stages, R = p.raw_stages;
-  const uint32_t b_bytes = (uint32_t)p.mb * BKB;
-  const uint32_t stage_bytes = A_TILE + ((b_bytes + 1023u) & ~1023u);
-  unsigned char *raw_ring = smem + (size_t)S * stage_bytes;
+  const uint32_t half_bytes = (uint32_t)p.mb * BKB, slot_bytes = 2 * half_bytes;          // (half: a multiple of 2 KB)
+  unsigned char *raw_ring = smem + (size_t)S * slot_bytes;
   const uint32_t smem_s = sa(smem);
-  uint32_t tmem_cols = 32;
-  while ((int)tmem_cols < p.mb) tmem_cols <<= 1;
+  const uint32_t a_col = (uint32_t)(p.mb + 31) & ~31u, tmem_cols = a_col + 64 * S <= 256 ? 256 : 512;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(sa(&ctl.full[s]), 1);    // the activation tile of the stage has landed
-      mbar_init(sa(&ctl.ready[s]), 8);   // one arrival per transform warp: the fp16 weight tile is written
-      mbar_init(sa(&ctl.empty[s]), 1);   // the MMAs that read the stage have completed
+      mbar_init(sa(&ctl.full[s]), 5);    // the activations of the slot have landed; one arrival per warp of a group: its fp16 weights are in tensor memory
+      mbar_init(sa(&ctl.empty[s]), 1);   // the MMAs that read the slot have completed
     }
     for (int r = 0; r < R; ++r) {
       mbar_init(sa(&ctl.raw_full[r]), 1);
-      mbar_init(sa(&ctl.raw_empty[r]), 8);
+      mbar_init(sa(&ctl.raw_empty[r]), 4);
     }
     mbar_init(sa(&ctl.accum), 1);
     ctl.abort = 0;
-    ctl.last = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(sa(&ctl.tmem_base), tmem_cols);
@@ -561,58 +751,61 @@ __global__ void __launch_bounds__(THREADS_I4, 1) gemm_int4_kernel(const __grid_c
   __syncthreads();
   fence_after();
   const uint32_t tmem = ctl.tmem_base;
+  if (p.pdl) launch_dependents();   // not before the tensor memory is ours: a block of the next GEMM would keep it while it waits for this kernel
 
   if (warp == 0) {
-    // ---- raw nibble tiles: one contiguous 4 KB bulk copy per k block
-    if (lane == 0) {
-      const unsigned char *wt = p.w + ((size_t)blockIdx.x * p.n_kb + kb0) * RAW_TILE;
+    // ---- raw nibble tiles: one contiguous bulk copy per step (weights: nobody before has written them)
+    if (elect_one()) {
+      const unsigned char *wt = p.w + ((size_t)blockIdx.x * p.n_kb + st0) * RAW_STEP;
       const uint32_t raw0 = sa(raw_ring), full0 = sa(&ctl.raw_full[0]), empty0 = sa(&ctl.raw_empty[0]);
       int r = 0;
       uint32_t par = 1;
-      bool first_round = true;
       for (int it = 0; it < n_it; ++it) {
-        if (!first_round && !mbar_wait(empty0 + r * 8, par, &ctl.abort)) give_up(ctl, p.error_flag, 21);
-        if (ctl.abort) break;
+        if (it >= R && !wait_fast(empty0 + r * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
         const uint32_t fb = full0 + r * 8;
-        mbar_expect_tx(fb, RAW_TILE);
-        bulk_g2s(raw0 + r * RAW_TILE, wt, RAW_TILE, fb);
-        wt += RAW_TILE;
-        if (++r == R) { r = 0; par ^= 1u; first_round = false; }
+        mbar_expect_tx(fb, RAW_STEP);
+        bulk_g2s(raw0 + r * RAW_STEP, wt, RAW_STEP, fb);
+        wt += RAW_STEP;
+        if (++r == R) { r = 0; par ^= 1u; }
       }
     }
-  } else if (warp == 10) {
-    // ---- activation tiles (64 fp16 of k per row)
-    if (lane == 0) {
+  } else if (warp == 2 + 4 * NG) {
+    // ---- activation tiles (two boxes of 64 fp16 of k per row)
+    if (elect_one()) {
+      if (p.pdl) wait_for_prerequisites();
       const uint32_t full0 = sa(&ctl.full[0]), empty0 = sa(&ctl.empty[0]);
-      int s = 0, kx = kb0 * 64;
+      int s = 0, kx = st0 * 128;
       uint32_t par = 1;
-      bool first_round = true;
       for (int it = 0; it < n_it; ++it) {
-        if (!first_round && !mbar_wait(empty0 + s * 8, par, &ctl.abort)) give_up(ctl, p.error_flag, 25);
-        if (ctl.abort) break;
-        const uint32_t fb = full0 + s * 8;
-        mbar_expect_tx(fb, b_bytes);
-        tma_load_2d(smem_s + s * stage_bytes + A_TILE, &map_x, kx, m0, fb);
-        kx += 64;
-        if (++s == S) { s = 0; par ^= 1u; first_round = false; }
+        if (it >= S && !wait_fast(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 25); break; }
+        const uint32_t fb = full0 + s * 8, dst = smem_s + s * slot_bytes;
+        mbar_expect_tx(fb, slot_bytes);
+        tma_load_2d(dst, &map_x, kx, m0, fb);
+        tma_load_2d(dst + half_bytes, &map_x, kx + 64, m0, fb);
+        kx += 128;
+        if (++s == S) { s = 0; par ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc(false, p.mb);
-      const uint64_t adesc0 = smem_desc_sw128(smem_s), bdesc0 = smem_desc_sw128(smem_s + A_TILE);
-      const uint32_t ready0 = sa(&ctl.ready[0]), full0 = sa(&ctl.full[0]), empty0 = sa(&ctl.empty[0]), stage16 = stage_bytes >> 4;
+      const uint64_t bdesc0 = smem_desc_sw128(smem_s);
+      const uint32_t full0 = sa(&ctl.full[0]), empty0 = sa(&ctl.empty[0]), slot16 = slot_bytes >> 4, half16 = half_bytes >> 4;
       int s = 0;
       uint32_t par = 0, acc = 0;
       for (int it = 0; it < n_it; ++it) {
-        if (!mbar_wait(ready0 + s * 8, par, &ctl.abort) || !mbar_wait(full0 + s * 8, par, &ctl.abort)) give_up(ctl, p.error_flag, 22);
-        if (ctl.abort) break;
+        if (!wait_fast(full0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 22); break; }
         fence_after();
-        const uint64_t adesc = adesc0 + (uint64_t)(s * stage16), bdesc = bdesc0 + (uint64_t)(s * stage16);
-        umma<false>(tmem, adesc, bdesc, idesc, acc);   // four MMAs of 16 k (32 bytes) each
-        umma<false>(tmem, adesc + 2, bdesc + 2, idesc, 1u);
-        umma<false>(tmem, adesc + 4, bdesc + 4, idesc, 1u);
-        umma<false>(tmem, adesc + 6, bdesc + 6, idesc, 1u);
+        const uint64_t b0 = bdesc0 + (uint64_t)(s * slot16), b1 = b0 + half16;
+        const uint32_t at = tmem + a_col + s * 64;
+        umma_ta(tmem, at, b0, idesc, acc);   // eight MMAs of 16 k each: 32 bytes of an activation row, eight columns of weights
+        umma_ta(tmem, at + 8, b0 + 2, idesc, 1u);
+        umma_ta(tmem, at + 16, b0 + 4, idesc, 1u);
+        umma_ta(tmem, at + 24, b0 + 6, idesc, 1u);
+        umma_ta(tmem, at + 32, b1, idesc, 1u);
+        umma_ta(tmem, at + 40, b1 + 2, idesc, 1u);
+        umma_ta(tmem, at + 48, b1 + 4, idesc, 1u);
+        umma_ta(tmem, at + 56, b1 + 6, idesc, 1u);
         umma_commit(empty0 + s * 8);
         acc = 1u;
         if (++s == S) { s = 0; par ^= 1u; }
@@ -620,67 +813,83 @@ __global__ void __launch_bounds__(THREADS_I4, 1) gemm_int4_kernel(const __grid_c
       umma_commit(sa(&ctl.accum));
     }
   } else {
-    // ---- transform + epilogue: warps 2-9.  A warp reads tensor-memory lanes [32 (warp % 4), +32), so thread (warp, lane) owns row
-    // 32 (warp % 4) + lane of the tile; the two warps of a row share its k (transform) and its activation columns (epilogue).
-    const int q = warp & 3, half = (warp - 2) >> 2;
+    // ---- transform + epilogue.  A warp reaches tensor-memory lanes [32 (warp % 4), +32): thread (warp, lane) owns row 32 (warp % 4) + lane.
+    const int q = warp & 3, group = (warp - 2) >> 2;
     const int row = q * 32 + lane;
-    const int n = n0 + row;
     const int ngroups = p.K / p.group;
-    const __half *srow = p.scales + (size_t)min(n, p.N - 1) * ngroups;
-    __half sc_next = (n_it > 0) ? __ldg(srow + (kb0 * 64) / p.group) : __half(0);
+    const __half *srow = p.scales + (size_t)min(n0 + row, p.N - 1) * ngroups;
     const __half2 offA = __float2half2_rn(1032.0f), offB = __float2half2_rn(72.0f);
-    const uint32_t raw_full0 = sa(&ctl.raw_full[0]), raw_empty0 = sa(&ctl.raw_empty[0]), empty0 = sa(&ctl.empty[0]), ready0 = sa(&ctl.ready[0]);
-    const unsigned char *raw_mine = raw_ring + row * 32 + half * 16;
-    unsigned char *arow0 = smem + (row >> 3) * 1024 + (row & 7) * 128;
-    // scale index of a k block: blocks of 64 k, groups of p.group k -> the index moves on every (group / 64) blocks
-    const int blocks_per_group = p.group / 64;
-    int gidx = (kb0 * 64) / p.group, gleft = blocks_per_group - (kb0 % blocks_per_group);
-    int r = 0, s = 0;
-    uint32_t rpar = 0, spar = 1;
-    bool first_round = true;
-    for (int it = 0; it < n_it; ++it) {
+    const uint32_t raw_full0 = sa(&ctl.raw_full[0]), raw_empty0 = sa(&ctl.raw_empty[0]), empty0 = sa(&ctl.empty[0]), full0 = sa(&ctl.full[0]);
+    const unsigned char *raw_mine = raw_ring + row * 32;
+    const uint32_t a_lane = tmem + ((uint32_t)(q * 32) << 16) + a_col;
+    // scale index of a step: it moves on every (group / 128) steps
+    const int steps_per_group = p.group / 128;
+    int gidx = (st0 + group) / steps_per_group, gpos = (st0 + group) % steps_per_group;
+    int r = group % R, s = group % S;
+    uint32_t rpar = (group / R) & 1, spar = ((group / S) & 1) ^ 1;
+    __half sc_next = group < n_it ? __ldg(srow + gidx) : __half(0);
+    for (int it = group; it < n_it; it += NG) {
       const __half2 s2 = __half2half2(sc_next);
-      if (--gleft == 0) { ++gidx; gleft = blocks_per_group; }
-      if (it + 1 < n_it) sc_next = __ldg(srow + gidx);   // next block's scale: its latency hides behind this block
-      if (!mbar_wait(raw_full0 + r * 8, rpar, &ctl.abort)) give_up(ctl, p.error_flag, 23);
-      if (ctl.abort) break;
-      const uint4 w4 = *reinterpret_cast<const uint4 *>(raw_mine + (size_t)r * RAW_TILE);
-      const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
-      __syncwarp();
-      if (lane == 0) mbar_arrive(raw_empty0 + r * 8);   // the nibbles are in registers: the raw stage may be refilled
-      if (!first_round && !mbar_wait(empty0 + s * 8, spar, &ctl.abort)) give_up(ctl, p.error_flag, 26);
-      if (ctl.abort) break;
-      unsigned char *arow = arow0 + (size_t)s * stage_bytes;
+      gpos += NG;
+      while (gpos >= steps_per_group) { gpos -= steps_per_group; ++gidx; }
+      if (it + NG < n_it) sc_next = __ldg(srow + gidx);   // the next step's scale: its latency hides behind this step
+      if (!warp_wait(raw_full0 + r * 8, rpar, &ctl.abort)) { give_up(ctl, p.error_flag, 23); break; }
+      uint32_t words[16];
 #pragma unroll
-      for (int c4 = 0; c4 < 4; ++c4) {
-        // a word holds eight consecutive k as offset-binary nibbles u = q + 8: bits [0,4) k0, [16,20) k1, [4,8) k2, [20,24) k3, and the
-        // same again one byte up for k4..k7.  (1024 + u) and (64 + u) are exact in fp16; subtracting the offsets is exact; the
-        // product with the scale is the one fp16 rounding of the reference's Int4ToHalf.
-        const int c = half * 4 + c4;
-        const uint32_t w = words[c4], w8 = w >> 8;
-        __half2 h[4];
-        *reinterpret_cast<uint32_t *>(&h[0]) = (w & 0x000F000Fu) | 0x64006400u;
-        *reinterpret_cast<uint32_t *>(&h[1]) = (w & 0x00F000F0u) | 0x54005400u;
-        *reinterpret_cast<uint32_t *>(&h[2]) = (w8 & 0x000F000Fu) | 0x64006400u;
-        *reinterpret_cast<uint32_t *>(&h[3]) = (w8 & 0x00F000F0u) | 0x54005400u;
-        h[0] = __hmul2(__hsub2(h[0], offA), s2);
-        h[1] = __hmul2(__hsub2(h[1], offB), s2);
-        h[2] = __hmul2(__hsub2(h[2], offA), s2);
-        h[3] = __hmul2(__hsub2(h[3], offB), s2);
-        *reinterpret_cast<uint4 *>(arow + ((c ^ (row & 7)) << 4)) = *reinterpret_cast<const uint4 *>(h);
+      for (int h = 0; h < 4; ++h)
+        *reinterpret_cast<uint4 *>(&words[4 * h]) = *reinterpret_cast<const uint4 *>(raw_mine + (size_t)r * RAW_STEP + (h >> 1) * RAW_TILE + (h & 1) * 16);
+      if (it >= S && !warp_wait(empty0 + s * 8, spar, &ctl.abort)) { give_up(ctl, p.error_flag, 26); break; }
+      fence_after();
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t v[32];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          // a word holds eight consecutive k as offset-binary nibbles u = q + 8: bits [0,4) k0, [16,20) k1, [4,8) k2, [20,24) k3, and the
+          // same again one byte up for k4..k7.  (1024 + u) and (64 + u) are exact in fp16; subtracting the offsets is exact; the
+          // product with the scale is the one fp16 rounding of the reference's Int4ToHalf.
+          const uint32_t w = words[8 * half + c], w8 = w >> 8;
+          __half2 h[4];
+          *reinterpret_cast<uint32_t *>(&h[0]) = (w & 0x000F000Fu) | 0x64006400u;
+          *reinterpret_cast<uint32_t *>(&h[1]) = (w & 0x00F000F0u) | 0x54005400u;
+          *reinterpret_cast<uint32_t *>(&h[2]) = (w8 & 0x000F000Fu) | 0x64006400u;
+          *reinterpret_cast<uint32_t *>(&h[3]) = (w8 & 0x00F000F0u) | 0x54005400u;
+          h[0] = __hmul2(__hsub2(h[0], offA), s2);
+          h[1] = __hmul2(__hsub2(h[1], offB), s2);
+          h[2] = __hmul2(__hsub2(h[2], offA), s2);
+          h[3] = __hmul2(__hsub2(h[3], offB), s2);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[4 * c + j] = *reinterpret_cast<const uint32_t *>(&h[j]);
+        }
+        tmem_st32(a_lane + s * 64 + half * 32, v);
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the tensor core
+      tmem_wait_st();
+      fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ready0 + s * 8);
-      if (++r == R) { r = 0; rpar ^= 1u; }
-      if (++s == S) { s = 0; spar ^= 1u; first_round = false; }
+      if (lane == 0) {
+        mbar_arrive(full0 + s * 8);
+        mbar_arrive(raw_empty0 + r * 8);   // the nibbles have been used (not merely asked for): the raw stage may be refilled
+      }
+      r += NG;
+      while (r >= R) { r -= R; rpar ^= 1u; }
+      s += NG;
+      while (s >= S) { s -= S; spar ^= 1u; }
     }
-    if (!mbar_wait(sa(&ctl.accum), 0, &ctl.abort)) give_up(ctl, p.error_flag, 24);
+    if (p.pdl) wait_for_prerequisites();                // the residual and the output are others' until here
+    const bool done = warp_wait(sa(&ctl.accum), 0, &ctl.abort);
+    if (!done) give_up(ctl, p.error_flag, 24);
     fence_after();
-    if (!ctl.abort && n_it > 0) epilogue<false, false>(p, tmem, q, lane, half, 2, n0, m0, p.M, ks);
+    if (done) {
+      if (p.ksplit > 1) leave_sums(p, tmem, q, lane, group, NG, reinterpret_cast<float *>(smem));
+      else epilogue_fp16(p, tmem, q, lane, group, NG, n0, m0);
+    }
     fence_before();
   }
-  if (p.ksplit > 1) reduce_slices<false, false>(p, ctl, n0, m0, p.M, THREADS_I4);
+  if (p.ksplit > 1) {
+    if (p.pdl) wait_for_prerequisites();
+    __syncwarp();
+    sum_cluster<false, false>(p, ctl, smem_s, ks, n0, m0, p.M, THREADS);
+  }
   __syncthreads();
   fence_after();
   if (warp == 1) tmem_dealloc(tmem, tmem_cols);
@@ -754,6 +963,26 @@ static int make_map(CUtensorMap *map, const void *base, CUtensorMapDataType dt, 
   return PT_OK;
 }
 
+// Tiles of the INT4 kernel.  A CTA spends on a step (128 k) the longer of transform and single-thread roles (about 350 cycles) and MMAs (4 mb
+// cycles), then its epilogue, and the CTAs run in rounds over the SMs: of all row counts per tile (steps of 16) and k-slices the pair with
+// the least time by this count is taken.
+struct Int4Plan { int mb, ksplit; };
+static Int4Plan plan_int4(int m, int n_tiles, int n_steps, int ksplit_req) {
+  Int4Plan best{16, 1};
+  double least = 1e30;
+  for (int mb = 16; mb <= 256; mb += 16) {
+    const int m_tiles = ceil_div(m, mb);
+    if (mb > 16 && m_tiles == ceil_div(m, mb - 16)) continue;    // fewer rows per tile do as well
+    for (int ks = 1; ks <= MAX_CLUSTER; ++ks) {
+      if (ksplit_req > 0 ? ks != std::min(std::min(ksplit_req, MAX_CLUSTER), n_steps) : ks > 1 && n_steps / ks < 4) continue;
+      const long long ctas = (long long)n_tiles * m_tiles * ks, rounds = (ctas + sm_count() - 1) / sm_count();
+      const double t = (double)rounds * (ceil_div(n_steps, ks) * (double)std::max(350, 4 * mb) + 1500 + 8 * mb) + (ks > 1 ? 2500 + 6 * mb : 0);
+      if (t < least) { least = t; best = {mb, ks}; }
+    }
+  }
+  return best;
+}
+
 }  // namespace tc
 }  // namespace pt
 
@@ -810,8 +1039,9 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     PT_REQUIRE(!bad, "pt_gemm: %s", bad);
     PT_REQUIRE(a->out_dtype == PT_DT_BF16 || a->out_dtype == PT_DT_F32, "pt_gemm: BF16 weights write bf16 or fp32, got type %d", a->out_dtype);
   } else {
-    PT_REQUIRE(a->epilogue == PT_EPI_STORE || a->epilogue == PT_EPI_RESIDUAL || a->epilogue == PT_EPI_BIAS, "pt_gemm: epilogue %d (store, residual or bias)",
-               a->epilogue);
+    PT_REQUIRE(a->epilogue == PT_EPI_STORE || a->epilogue == PT_EPI_RESIDUAL || a->epilogue == PT_EPI_BIAS || (int4 && a->epilogue == PT_EPI_SWIGLU),
+               "pt_gemm: epilogue %d (store, residual, bias or, INT4, swiglu)", a->epilogue);
+    PT_REQUIRE(a->epilogue != PT_EPI_SWIGLU || a->n_out % 16 == 0, "pt_gemm: SwiGLU epilogue needs n_out %% 16 == 0, got %d", a->n_out);
   }
   PT_REQUIRE(a->epilogue != PT_EPI_RESIDUAL || a->residual, "pt_gemm: residual epilogue needs residual");
   PT_REQUIRE(a->epilogue != PT_EPI_BIAS || a->bias, "pt_gemm: bias epilogue needs bias");
@@ -839,14 +1069,18 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     p.group_stride = pt_gemm_packed_bytes(a->wfmt, a->n_out, a->k_in);
   } else if (bf16)
     while (p.mb > 64 && n_tiles * ceil_div(a->m, p.mb) * 4 < sm_count() * 3) p.mb = ceil_div(p.mb, 32) * 16;
-  const int m_tiles = ceil_div(a->m, p.mb);
-  p.n_kb = (int4 || bf16) ? a->k_in / 64 : a->k_in / 128;
+  int m_tiles = ceil_div(a->m, p.mb);
+  p.n_kb = bf16 ? a->k_in / 64 : a->k_in / 128;
   // k-slices: fill the GPU when there are few tiles, but keep at least PT_TC_MIN_KB k-blocks per CTA
 #ifndef PT_TC_MIN_KB
 #define PT_TC_MIN_KB 8
 #endif
   int ksplit = a->ksplit;
-  if (ksplit <= 0) {
+  if (int4) {
+    const tc::Int4Plan plan = tc::plan_int4(a->m, n_tiles, p.n_kb, a->ksplit);
+    p.mb = plan.mb;
+    ksplit = plan.ksplit;
+  } else if (ksplit <= 0) {
     ksplit = std::max(1, (p.mb <= 64 ? 2 : 1) * sm_count() / (n_tiles * m_tiles));   // two CTAs fit an SM up to 64 activation rows
     // (with several blocks of activation rows a slice's sums cost more than its share of a short k saves: 128 x 2048 at 512 .. 8192
     // rows takes 19 - 21 us whole and 27 - 41 us in slices)
@@ -855,6 +1089,7 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     while (ksplit > 1 && pt_gemm_workspace_bytes(a->m, a->n_out, ksplit) > a->workspace_bytes) --ksplit;   // ... and never more than the caller's workspace holds
     if ((size_t)n_tiles * m_tiles > kGemmMaxCounters) ksplit = 1;
   }
+  m_tiles = ceil_div(a->m, p.mb);
   ksplit = std::max(1, std::min(ksplit, p.n_kb));
   p.kb_per_split = ceil_div(p.n_kb, ksplit);
   p.ksplit = ceil_div(p.n_kb, p.kb_per_split);
@@ -864,11 +1099,11 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   p.residual = (const __half *)a->residual;
   p.bias = (const __half *)a->bias;
   p.out = (__half *)a->out;
-  p.out_ld = a->out_ld > 0 ? a->out_ld : a->n_out;
+  p.out_ld = a->out_ld > 0 ? a->out_ld : (a->epilogue == PT_EPI_SWIGLU ? a->n_out / 2 : a->n_out);
   if (bf16) p.dense = make_dense_out(a->out, p.out_ld, a->out_dtype, a->epilogue, a->alpha, a->ext);
   p.error_flag = a->error_flag;
-  if (p.ksplit > 1) {
-    const size_t need = pt_gemm_workspace_bytes(a->m, a->n_out, p.ksplit);
+  if (int4 ? a->ksplit > 1 : p.ksplit > 1) {   // (INT4: slices that the caller asked for; the kernel itself needs no workspace)
+    const size_t need = pt_gemm_workspace_bytes(a->m, a->n_out, int4 ? a->ksplit : p.ksplit);
     PT_REQUIRE(a->workspace && a->workspace_bytes >= need, "pt_gemm: %d k-slices need %zu workspace bytes, got %zu", p.ksplit, need, a->workspace_bytes);
     PT_REQUIRE((size_t)n_tiles * m_tiles <= kGemmMaxCounters, "pt_gemm: %d x %d tiles exceed the %zu arrival counters of a k-slice workspace", n_tiles,
                m_tiles, kGemmMaxCounters);
@@ -883,7 +1118,7 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   const bool pair = PT_TC_PAIR && bf16 && p.ksplit == 1 && p.mb >= 128 && n_tiles >= 2 && (long long)ceil_div(n_tiles, 2) * m_tiles >= sm_count();
   const int na = pair ? 2 : 1;
   p.n_tiles = n_tiles;
-  p.pdl = bf16 && a->pdl ? 1 : 0;
+  p.pdl = (bf16 || int4) && a->pdl ? 1 : 0;
   const uint32_t b_bytes = (uint32_t)p.mb * tc::BKB;
   const uint32_t stage_bytes = na * tc::A_TILE + ((b_bytes + 1023u) & ~1023u);
   // Up to 64 activation rows a stage is small, and what limits the kernel is the one thread per CTA that issues the MMAs (about
@@ -897,11 +1132,16 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   const bool small = p.mb <= 64 || (bf16 && na * p.mb <= 256 && (long long)n_tiles * m_tiles * p.ksplit > sm_count());
   const uint32_t budget = (small ? PT_TC_BUDGET_SMALL_KB : 200) * 1024u;
   size_t smem;
+  const bool two_int4 = int4 && p.mb <= 128 && n_tiles * m_tiles * p.ksplit > sm_count();   // two CTAs per SM (each has half the tensor memory)
+  const int int4_groups = !two_int4 && p.mb <= 128 ? 4 : 2;   // above 128 rows a step's MMAs take longer than half a transform
   if (int4) {
-    p.stages = (int)std::min<uint32_t>(4, (budget - 8 * tc::RAW_TILE) / stage_bytes);
-    PT_REQUIRE(p.stages >= 2, "pt_gemm: tile does not fit shared memory");
-    p.raw_stages = (int)std::min<uint32_t>(24, (budget - p.stages * stage_bytes) / tc::RAW_TILE);
-    smem = (size_t)p.stages * stage_bytes + (size_t)p.raw_stages * tc::RAW_TILE + 1024;
+    // slots: 64 tensor-memory columns beside the accumulator and 256 bytes of shared memory per row each
+    p.stages = two_int4 ? (p.mb <= 64 ? 3 : 2) : (p.mb <= 128 ? 4 : p.mb <= 208 ? 3 : 2);
+    const uint32_t slots = p.stages * 2 * b_bytes, room = (two_int4 ? 104 : 217) * 1024u;
+    p.raw_stages = (int)std::min<uint32_t>(12, (room - slots) / tc::RAW_STEP);
+    smem = slots + (size_t)p.raw_stages * tc::RAW_STEP + 1024;
+    PT_REQUIRE(p.stages >= int4_groups && p.raw_stages >= p.stages + int4_groups, "pt_gemm: tile does not fit shared memory");
+    if (!two_int4) smem = std::max<size_t>(smem, 120 * 1024);   // never more CTAs on an SM than its tensor memory serves
   } else {
     p.stages = (int)std::min<uint32_t>(8, budget / stage_bytes);
     PT_REQUIRE(p.stages >= 2, "pt_gemm: tile does not fit shared memory");
@@ -927,13 +1167,34 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<true, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_int4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    PT_CUDA(cudaFuncSetAttribute(tc::gemm_int4_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    PT_CUDA(cudaFuncSetAttribute(tc::gemm_int4_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     attr_set = true;
   }
   dim3 grid(ceil_div(n_tiles, na), p.ksplit, m_tiles);
-  if (int4)
-    tc::gemm_int4_kernel<<<grid, tc::THREADS_I4, smem, as_stream(stream)>>>(map_x, p);
-  else if (bf16) {
+  if (int4) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((3 + 4 * int4_groups) * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = as_stream(stream);
+    cudaLaunchAttribute attr[2];
+    int n_attr = 0;
+    if (p.ksplit > 1) {
+      attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+      attr[n_attr].val.clusterDim.x = 1;
+      attr[n_attr].val.clusterDim.y = p.ksplit;
+      attr[n_attr++].val.clusterDim.z = 1;
+    }
+    if (p.pdl) {
+      attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[n_attr++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n_attr;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, int4_groups == 2 ? tc::gemm_int4_kernel<2> : tc::gemm_int4_kernel<4>, map_x, p);
+    if (e != cudaSuccess) return pt::set_error(PT_ERR_CUDA, "pt_gemm: %s", cudaGetErrorString(e));
+  } else if (bf16) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(tc::THREADS_F8);

@@ -77,13 +77,14 @@ class LlamaDecoder(DecodeLoop):
         def t(key):
             return state_dict[key].to(dev)
 
-        # More than 16 rows on one GPU with INT4 weights: the transformer linears run on the tcgen05 GEMM, weights tiled once (beyond
-        # 32 rows it is the only path).  Measured on B200, 7B width, 8 blocks: 16 rows 1.54 ms with the skinny-matmul kernels against
-        # 1.74 ms with the GEMM; 24 rows 2.44 against 2.02 ms; 32 rows 2.87 against 2.25 ms.
+        # More than 8 rows on one GPU with INT4 weights: the transformer linears run on the tcgen05 GEMM, weights tiled once (beyond
+        # 32 rows it is the only path).  Measured on B200, 7B width, the four products of a block: 9 .. 16 rows 102 us with the
+        # skinny-matmul kernels against 60 us with the GEMM, 32 rows 175 against 63; at 8 rows they are level (61 against 60) and the
+        # skinny-matmul kernels take the norms with them (persistent=False asks for those up to 16 rows).
         first_w = state_dict["model.layers.0.self_attn.q_proj.weight"]
         grp0 = (first_w.shape[1] * 2) // max(1, state_dict["model.layers.0.self_attn.q_proj.weight_scale"].numel() // first_w.shape[0]) \
             if first_w.dtype == torch.int8 else 0
-        self.use_gemm = ((batch > 16 or use_gemm is True) and use_gemm is not False and tp_size == 1 and first_w.dtype == torch.int8 and grp0 % 128 == 0 and persistent is not True
+        self.use_gemm = ((batch > 16 or (batch > 8 and persistent is None) or use_gemm is True) and use_gemm is not False and tp_size == 1 and first_w.dtype == torch.int8 and grp0 % 128 == 0 and persistent is not True
                          and c.d_model % 128 == 0 and c.ffn % 128 == 0)
 
         def col_parallel(keys, interleave=False):
@@ -92,7 +93,7 @@ class LlamaDecoder(DecodeLoop):
                 sc = [_rows(t(k + "_scale").reshape(t(k).shape[0], -1), r, tp) for k in keys]
                 grp = (ws[0].shape[1] * 2) // sc[0].shape[1]
                 if self.use_gemm:
-                    return ops.GemmWeight(ops.W_INT4, torch.cat(ws, 0), torch.cat(sc, 0), group=grp)
+                    return ops.GemmWeight(ops.W_INT4, torch.cat(ws, 0), torch.cat(sc, 0), group=grp, interleave_gate_up=interleave)
                 return ops.PackedLinear(ops.W_INT4, torch.cat(ws, 0), torch.cat(sc, 0), group=grp, interleave_gate_up=interleave)
             return ops.PackedLinear(ops.W_FP16, torch.cat(ws, 0).to(torch.float16), interleave_gate_up=interleave)
 
@@ -107,10 +108,11 @@ class LlamaDecoder(DecodeLoop):
             loc, ks = row_parallel_fp16(w, k_total, r, tp)
             return ops.PackedLinear(ops.W_FP16, loc), ks
 
-        def gemm_weight(keys):
+        def gemm_weight(keys, interleave=False):
             ws = [t(k) for k in keys]
             sc = [t(k + "_scale").reshape(w.shape[0], -1) for k, w in zip(keys, ws)]
-            return ops.GemmWeight(ops.W_INT4, torch.cat(ws, 0), torch.cat(sc, 0), group=(ws[0].shape[1] * 2) // sc[0].shape[1])
+            return ops.GemmWeight(ops.W_INT4, torch.cat(ws, 0), torch.cat(sc, 0), group=(ws[0].shape[1] * 2) // sc[0].shape[1],
+                                  interleave_gate_up=interleave)
 
         self.emb = t("model.embed_tokens.weight").to(torch.float16).contiguous()   # replicated: one row is read per token
         self.layers = []
@@ -142,7 +144,7 @@ class LlamaDecoder(DecodeLoop):
                         "ln1": self.layers[i]["ln1"], "ln2": self.layers[i]["ln2"],
                         "qkv": gemm_weight([p + "self_attn.q_proj.weight", p + "self_attn.k_proj.weight", p + "self_attn.v_proj.weight"]),
                         "o": gemm_weight([p + "self_attn.o_proj.weight"]),
-                        "gu": gemm_weight([p + "mlp.gate_proj.weight", p + "mlp.up_proj.weight"]),
+                        "gu": gemm_weight([p + "mlp.gate_proj.weight", p + "mlp.up_proj.weight"], interleave=True),
                         "down": gemm_weight([p + "mlp.down_proj.weight"])})
             self._pf_bufs = {}
         self.norm = t("model.norm.weight").contiguous()
@@ -207,7 +209,6 @@ class LlamaDecoder(DecodeLoop):
         self.lin_ws = ops.linear_workspace(B, max(3 * self.d_loc, 2 * self.f_loc, d, self.logits.shape[1]), 16, dev)
         if self.use_gemm:
             self.gemm_ws = ops.gemm_workspace(B, max(3 * d, 2 * f), 8, dev)
-            self.gu_out = torch.empty((B, 2 * f), **f16)
         self.graph = None
         # The persistent whole-step kernel covers INT4, batch <= 2, on one GPU or tensor-parallel over up to 8 (the all-reduces are
         # then fused into the kernel as peer stores); everything else takes the per-op kernels and NCCL.
@@ -363,7 +364,7 @@ class LlamaDecoder(DecodeLoop):
         self._enqueue_head()
 
     def _enqueue_layers_gemm(self):
-        """The transformer blocks at 16 or more rows: RMSNorm kernel, tcgen05 GEMMs (residual adds in their epilogues), SwiGLU kernel."""
+        """The transformer blocks at 9 or more rows: RMSNorm kernel, tcgen05 GEMMs (residual adds and SwiGLU in their epilogues)."""
         c = self.cfg
         L_ = ops._lib.lib()
 
@@ -379,8 +380,7 @@ class LlamaDecoder(DecodeLoop):
             ops.check(L_.pt_kv_append_attn(ctypes.byref(a), ops._stream()), "pt_kv_append_attn")
             ops.gemm(self.attn, L["o"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, workspace=self.gemm_ws, error_flag=self.error_flag)
             norm(L["ln2"])
-            ops.gemm(self.h, L["gu"], out=self.gu_out, workspace=self.gemm_ws, error_flag=self.error_flag)
-            ops.check(L_.pt_swiglu(ops._ptr(self.gu_out), self.batch, c.ffn, ops._ptr(self.act), self.act.shape[1], ops._stream()), "pt_swiglu")
+            ops.gemm(self.h, L["gu"], out=self.act, out_ld=self.act.shape[1], epilogue=ops.EPI_SWIGLU, workspace=self.gemm_ws, error_flag=self.error_flag)
             ops.gemm(self.act, L["down"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, workspace=self.gemm_ws, error_flag=self.error_flag)
 
     def prefill(self, n_tokens=None, chunk=1024):
@@ -410,8 +410,7 @@ class LlamaDecoder(DecodeLoop):
             if rows not in self._pf_bufs:
                 f16 = dict(dtype=torch.float16, device=self.device)
                 self._pf_bufs = {rows: SimpleNamespace(x=torch.empty((rows, d), **f16), h=torch.empty((rows, d), **f16), qkv=torch.empty((rows, 3 * d), **f16),
-                                                       attn=torch.empty((rows, d), **f16), gu=torch.empty((rows, 2 * f), **f16),
-                                                       act=torch.empty((rows, f), **f16), ws=ops.gemm_workspace(rows, max(3 * d, 2 * f), 8, self.device))}
+                                                       attn=torch.empty((rows, d), **f16), act=torch.empty((rows, f), **f16), ws=ops.gemm_workspace(rows, max(3 * d, 2 * f), 8, self.device))}
             w = self._pf_bufs[rows]
             ops.check(L_.pt_prefill_embed(ops._ptr(self.emb), ops._ptr(self.ids), c.max_len, B, P, s0, d, c.vocab, self.eos_id, ops._ptr(self.stop_mask),
                                           ops._ptr(w.x), ops._stream()), "pt_prefill_embed")
@@ -425,8 +424,7 @@ class LlamaDecoder(DecodeLoop):
                 ops.prefill_attn(w.qkv, self.caches[li], B, P, s0, c.n_head, self.score_scale, self.sin, self.cos, out=w.attn)
                 ops.gemm(w.attn, L["o"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, workspace=w.ws, error_flag=self.error_flag)
                 norm(L["ln2"])
-                ops.gemm(w.h, L["gu"], out=w.gu, workspace=w.ws, error_flag=self.error_flag)
-                ops.check(L_.pt_swiglu(ops._ptr(w.gu), rows, f, ops._ptr(w.act), f, ops._stream()), "pt_swiglu")
+                ops.gemm(w.h, L["gu"], out=w.act, epilogue=ops.EPI_SWIGLU, workspace=w.ws, error_flag=self.error_flag)
                 ops.gemm(w.act, L["down"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, workspace=w.ws, error_flag=self.error_flag)
         self.step_t.fill_(n)
         return n
@@ -462,7 +460,7 @@ class LlamaDecoder(DecodeLoop):
             for L in self.layers:
                 ops.gemm(self.h, L["qkv"], out=self.qkv, workspace=self.gemm_ws)
                 ops.gemm(self.attn, L["o"], out=self.part, workspace=self.gemm_ws)
-                ops.gemm(self.h, L["gu"], out=self.gu_out, workspace=self.gemm_ws)
+                ops.gemm(self.h, L["gu"], out=self.act, out_ld=self.act.shape[1], epilogue=ops.EPI_SWIGLU, workspace=self.gemm_ws)
                 ops.gemm(self.act, L["down"], out=self.part, workspace=self.gemm_ws)
             return
         for L in self.layers:

@@ -144,9 +144,15 @@ class GemmWeight:
     """A weight matrix tiled once for pt_gemm (pt_gemm_repack): FP8 bytes [n_out, k], or INT4 rows in the reference's int8
     [n_out, k/2] format plus fp16 scales [n_out, k/group], or bfloat16 [n_out, k]."""
 
-    def __init__(self, wfmt, w, scale=None, group=0, w_scale=1.0):
+    def __init__(self, wfmt, w, scale=None, group=0, w_scale=1.0, interleave_gate_up=False):
+        """interleave_gate_up: rows [f gate features | f up features] in the order EPI_SWIGLU wants (eight and eight in turn)."""
         L = _lib.lib()
         self.wfmt, self.n_out, self.w_scale = wfmt, w.shape[0], float(w_scale)
+        if interleave_gate_up:
+            if self.n_out % 16:
+                raise PtError(f"GemmWeight: interleaved (gate|up) rows need n_out % 16 == 0, got {self.n_out}")
+            order = torch.arange(self.n_out, device=w.device).view(2, -1, 8).transpose(0, 1).reshape(-1)
+            w, scale = w[order], None if scale is None else scale.reshape(self.n_out, -1)[order]
         if wfmt == W_INT4:
             self.k_in = w.shape[1] * 2
             self.group = int(group) if group else self.k_in
@@ -177,7 +183,7 @@ def gemm(x, gw, out=None, x_scale=1.0, epilogue=EPI_STORE, residual=None, worksp
     if x.shape[1] != gw.k_in:
         raise PtError(f"gemm: x has k={x.shape[1]}, weight has k={gw.k_in}")
     if out is None:
-        out = torch.empty((m, gw.n_out), dtype=torch.float16, device=x.device)
+        out = torch.empty((m, gw.n_out // 2 if epilogue == EPI_SWIGLU else gw.n_out), dtype=torch.float16, device=x.device)
     a = GemmArgs()
     a.wfmt, a.m, a.n_out, a.k_in, a.group, a.epilogue, a.ksplit = gw.wfmt, m, gw.n_out, gw.k_in, gw.group, epilogue, ksplit
     a.w_tiled = 1
