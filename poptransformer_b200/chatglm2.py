@@ -83,7 +83,10 @@ class ChatGLM2Decoder(DecodeLoop):
                 pl = ops.PackedLinear(ops.W_FP8, torch.cat(ws, 0).contiguous(), w_scale=scales.pop(), interleave_gate_up=interleave)
                 pl.act_scale = acts.pop()
                 return pl
-            return ops.PackedLinear(ops.W_FP16, torch.cat(ws, 0).to(torch.float16).contiguous(), interleave_gate_up=interleave)
+            w = torch.cat(ws, 0).to(torch.float16).contiguous()
+            if tp == 1:
+                return ops.fp16_linear(w, batch, interleave_gate_up=interleave)
+            return ops.PackedLinear(ops.W_FP16, w, interleave_gate_up=interleave)
 
         self.emb = t("transformer.embedding.word_embeddings.weight").to(torch.float16).contiguous()
         self.h_loc, self.d_loc, self.f_loc = c.n_head // tp, c.d_model // tp, c.ffn // tp
@@ -110,7 +113,7 @@ class ChatGLM2Decoder(DecodeLoop):
         self.ids = torch.full((B, c.max_len), self.pad_id, dtype=torch.int32, device=dev)
         self.step_t = torch.zeros(1, dtype=torch.int32, device=dev)
         self.stop_mask = torch.zeros(B, dtype=torch.int32, device=dev)
-        self.x = torch.empty((B, d), **f16)
+        self.x, self.h = torch.empty((B, d), **f16), torch.empty((B, d), **f16)
         self.qkv = torch.empty((B, (self.h_loc + 2 * c.n_group) * c.head_dim), **f16)
         self.attn = torch.empty((B, self.d_loc), **f16)
         self.act = torch.empty((B, self.f_loc), **f16)
@@ -138,6 +141,13 @@ class ChatGLM2Decoder(DecodeLoop):
         torch.cuda.synchronize()
 
     def _linear(self, x, pl, out, site, gamma=None, epilogue=ops.EPI_STORE, bias=None, residual=None):
+        if isinstance(pl, ops.GemmWeight):       # (fp16)
+            if gamma is not None:
+                ops.check(ops._lib.lib().pt_rms_norm(ops._ptr(x), None, ops._ptr(gamma), self.batch, self.cfg.d_model, self.cfg.eps, ops._ptr(self.h), None,
+                                                     ops._stream()), "pt_rms_norm")
+                x = self.h
+            ops.gemm(x, pl, out=out, epilogue=epilogue, bias=bias, residual=residual, error_flag=self.error_flag)
+            return
         fp8 = pl.wfmt == ops.W_FP8
         pro = (ops.PRO_RMSNORM_CAST_FP8 if fp8 else ops.PRO_RMSNORM) if gamma is not None else (ops.PRO_CAST_FP8 if fp8 else ops.PRO_NONE)
         a = ops.linear_args(x, pl, out, prologue=pro, epilogue=epilogue, gamma=gamma, eps=self.cfg.eps,

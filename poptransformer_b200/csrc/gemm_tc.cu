@@ -60,8 +60,6 @@ struct GemmParams {
   const __half *bias;
   __half *out;
   int out_ld;
-  float *partial;         // [ksplit][M][N] (ksplit > 1)
-  int *counters;          // [n tiles * m tiles]
   int *error_flag;
   DenseOut dense;         // BF16: what becomes of a finished sum
   const int *group_of;    // BF16, grouped: the weight matrix of every tile of mb rows (negative: none)
@@ -187,7 +185,6 @@ struct SharedCtl {
   uint64_t raw_full[24], raw_empty[24];
   uint32_t tmem_base;
   volatile int abort;
-  int last;
 };
 
 // What every role does when one of its waits runs out.
@@ -207,6 +204,8 @@ __device__ __forceinline__ __half fp16_out(const GemmParams &p, float acc, int m
   __half y = __float2half_rn(acc * p.out_scale);
   if (p.epilogue == PT_EPI_RESIDUAL) return h_add(__ldcg(p.residual + (size_t)m * p.N + n), y);
   if (p.epilogue == PT_EPI_BIAS) return h_add(y, p.bias[n]);
+  if (p.epilogue == PT_EPI_BIAS_GELU) return gelu_h(h_add(y, p.bias[n]));
+  if (p.epilogue == PT_EPI_BIAS_RESIDUAL) return h_add(__ldcg(p.residual + (size_t)m * p.N + n), h_add(y, p.bias[n]));
   return y;
 }
 template <bool BF16, bool EXT> __device__ __forceinline__ void store_out(const GemmParams &p, float acc, int m, int n) {
@@ -232,18 +231,20 @@ template <int EPI> __device__ __forceinline__ void fp16_rows16(const GemmParams 
   } else {
     const int odd = lane & 1;
     __half2 *o = reinterpret_cast<__half2 *>(p.out + (size_t)(m + odd) * p.out_ld + (n - odd));
-    __half2 res[EPI == PT_EPI_RESIDUAL ? 8 : 1], bias = __half2half2(__half(0));
-    if constexpr (EPI == PT_EPI_RESIDUAL) {
+    constexpr bool RES = EPI == PT_EPI_RESIDUAL || EPI == PT_EPI_BIAS_RESIDUAL, BIAS = EPI == PT_EPI_BIAS || EPI == PT_EPI_BIAS_GELU || EPI == PT_EPI_BIAS_RESIDUAL;
+    __half2 res[RES ? 8 : 1], bias = __half2half2(__half(0));
+    if constexpr (RES) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) res[j] = __ldcg(reinterpret_cast<const __half2 *>(p.residual + (size_t)(m + odd + 2 * j) * p.N + (n - odd)));
     }
-    if constexpr (EPI == PT_EPI_BIAS) bias = *reinterpret_cast<const __half2 *>(p.bias + (n - odd));
+    if constexpr (BIAS) bias = *reinterpret_cast<const __half2 *>(p.bias + (n - odd));
 #pragma unroll
     for (int j = 0; j < 16; j += 2) {
       const float t = __shfl_xor_sync(0xffffffffu, odd ? sum[j] : sum[j + 1], 1);   // even lane: row j of n + 1; odd lane: row j + 1 of n - 1
       __half2 y = odd ? __floats2half2_rn(t * p.out_scale, sum[j + 1] * p.out_scale) : __floats2half2_rn(sum[j] * p.out_scale, t * p.out_scale);
-      if constexpr (EPI == PT_EPI_RESIDUAL) y = __hadd2_rn(res[j / 2], y);
-      if constexpr (EPI == PT_EPI_BIAS) y = __hadd2_rn(y, bias);
+      if constexpr (BIAS) y = __hadd2_rn(y, bias);
+      if constexpr (EPI == PT_EPI_BIAS_GELU) y = __halves2half2(gelu_h(__low2half(y)), gelu_h(__high2half(y)));
+      if constexpr (RES) y = __hadd2_rn(res[j / 2], y);
       *o = y;
       o += p.out_ld;   // (two rows, in units of two)
     }
@@ -252,8 +253,8 @@ template <int EPI> __device__ __forceinline__ void fp16_rows16(const GemmParams 
 // The epilogue of a tile without k-slices, fp16 outputs: `part` of `parts` warps share a quarter of the rows and take alternate 16 columns.
 __device__ __forceinline__ void epilogue_fp16(const GemmParams &p, uint32_t tmem, int q, int lane, int part, int parts, int n0, int m0) {
   const int nq = n0 + q * 32, n = nq + lane, rows = min(p.mb, p.M - m0);
-  const bool pairs = nq + 32 <= p.N && p.out_ld % 2 == 0 && ((uintptr_t)p.out & 3) == 0 && (p.epilogue != PT_EPI_RESIDUAL || (p.N % 2 == 0 && ((uintptr_t)p.residual & 3) == 0)) &&
-                     (p.epilogue != PT_EPI_BIAS || ((uintptr_t)p.bias & 3) == 0);   // (uniform over the warp)
+  const bool pairs = nq + 32 <= p.N && p.out_ld % 2 == 0 && ((uintptr_t)p.out & 3) == 0 && (!p.residual || (p.N % 2 == 0 && ((uintptr_t)p.residual & 3) == 0)) &&
+                     (!p.bias || ((uintptr_t)p.bias & 3) == 0);   // (uniform over the warp)
   for (int c0 = part * 16; c0 < rows; c0 += 16 * parts) {
     uint32_t v[16];
     float sum[16];
@@ -265,6 +266,8 @@ __device__ __forceinline__ void epilogue_fp16(const GemmParams &p, uint32_t tmem
       if (p.epilogue == PT_EPI_SWIGLU) fp16_rows16<PT_EPI_SWIGLU>(p, sum, m, n, lane);
       else if (p.epilogue == PT_EPI_RESIDUAL) fp16_rows16<PT_EPI_RESIDUAL>(p, sum, m, n, lane);
       else if (p.epilogue == PT_EPI_BIAS) fp16_rows16<PT_EPI_BIAS>(p, sum, m, n, lane);
+      else if (p.epilogue == PT_EPI_BIAS_GELU) fp16_rows16<PT_EPI_BIAS_GELU>(p, sum, m, n, lane);
+      else if (p.epilogue == PT_EPI_BIAS_RESIDUAL) fp16_rows16<PT_EPI_BIAS_RESIDUAL>(p, sum, m, n, lane);
       else fp16_rows16<PT_EPI_STORE>(p, sum, m, n, lane);
       continue;
     }
@@ -367,36 +370,27 @@ template <int GLU, bool EXT> __device__ __forceinline__ void glu_rows16(const Ge
   }
 }
 
-// Epilogue of the warps that own the tile's rows (tensor-memory lane quarter warp % 4): `part` of `parts` warps share a quarter
-// and take alternate 16-column chunks.
-template <bool BF16, bool EXT>
-__device__ __forceinline__ void epilogue(const GemmParams &p, uint32_t tmem, int q, int lane, int part, int parts, int n0, int m0, int m_end, int ks, int c_first = 0) {
+// The BF16 kernel's general epilogue: any sizes and alignment, 16 columns a step.
+template <bool EXT>
+__device__ __forceinline__ void epilogue_any(const GemmParams &p, uint32_t tmem, int q, int lane, int n0, int m0, int m_end, int c_first) {
   const int n = n0 + q * 32 + lane;
-  for (int c0 = c_first + part * 16; c0 < min(p.mb, m_end - m0); c0 += 16 * parts) {
+  for (int c0 = c_first; c0 < min(p.mb, m_end - m0); c0 += 16) {
     uint32_t v[16];
     float sum[16];
     tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
     for (int j = 0; j < 16; ++j) sum[j] = __uint_as_float(v[j]);
-    if constexpr (BF16) {
-      if (p.ksplit == 1 && p.dense.epilogue == PT_EPI_GLU && n0 + q * 32 < p.dense.split_n) {   // (uniform over the warp)
-        if (EXT && p.dense.glu == PT_GLU_SILU) glu_rows16<PT_GLU_SILU, EXT>(p, sum, m0 + c0, m_end, n, lane);
-        else if (EXT && p.dense.glu == PT_GLU_GELU) glu_rows16<PT_GLU_GELU, EXT>(p, sum, m0 + c0, m_end, n, lane);
-        else glu_rows16<PT_GLU_CLAMPED, EXT>(p, sum, m0 + c0, m_end, n, lane);
-        continue;
-      }
+    if (p.dense.epilogue == PT_EPI_GLU && n0 + q * 32 < p.dense.split_n) {   // (uniform over the warp)
+      if (EXT && p.dense.glu == PT_GLU_SILU) glu_rows16<PT_GLU_SILU, EXT>(p, sum, m0 + c0, m_end, n, lane);
+      else if (EXT && p.dense.glu == PT_GLU_GELU) glu_rows16<PT_GLU_GELU, EXT>(p, sum, m0 + c0, m_end, n, lane);
+      else glu_rows16<PT_GLU_CLAMPED, EXT>(p, sum, m0 + c0, m_end, n, lane);
+      continue;
     }
     if (n < p.N) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const int m = m0 + c0 + j;
-        if (m >= m_end) break;
-        const float acc = sum[j];
-        if (p.ksplit > 1) {
-          p.partial[((size_t)ks * p.M + m) * p.N + n] = acc;
-        } else {
-          store_out<BF16, EXT>(p, acc, m, n);
-        }
+        if (m0 + c0 + j >= m_end) break;
+        dense_store<EXT>(p.dense, m0 + c0 + j, n, sum[j]);
       }
     }
   }
@@ -459,13 +453,13 @@ __device__ __forceinline__ void epilogue_rows32(const DenseOut &d, void *out, in
     }
   }
 }
-template <bool EXT> __device__ __forceinline__ void epilogue_bf16(const GemmParams &p, uint32_t tmem, int q, int lane, int n0, int m0, int m_end, int ks) {
+template <bool EXT> __device__ __forceinline__ void epilogue_bf16(const GemmParams &p, uint32_t tmem, int q, int lane, int n0, int m0, int m_end) {
   const DenseOut &d = p.dense;
   const int nq = n0 + q * 32, n = nq + lane;
   // (warp-uniform) where this warp's 32 outputs go
   const bool second = nq >= d.split_n, glu = d.epilogue == PT_EPI_GLU && !second, f32 = second || d.out_dt == PT_DT_F32;
   // whole columns of 32 rows inside the output; 4-byte aligned pairs for bf16
-  const bool fast = p.ksplit == 1 && nq + 32 <= p.N && !(!second && d.epilogue == PT_EPI_GELU_MUL && f32) && !(glu && f32) && (!EXT || ((!d.row_scale || (glu && d.glu == PT_GLU_SILU)) && (second || (f32 ? d.epilogue != PT_EPI_XIELU : d.epilogue != PT_EPI_SOFTCAP)))) &&
+  const bool fast = nq + 32 <= p.N && !(!second && d.epilogue == PT_EPI_GELU_MUL && f32) && !(glu && f32) && (!EXT || ((!d.row_scale || (glu && d.glu == PT_GLU_SILU)) && (second || (f32 ? d.epilogue != PT_EPI_XIELU : d.epilogue != PT_EPI_SOFTCAP)))) &&
                     (f32 || glu || (d.out_ld % 2 == 0 && ((uintptr_t)d.out & 3) == 0));
   const int rows = min(p.mb, m_end - m0), whole = fast ? rows & ~31 : 0;
   for (int c0 = 0; c0 < whole; c0 += 32) {
@@ -489,89 +483,21 @@ template <bool EXT> __device__ __forceinline__ void epilogue_bf16(const GemmPara
       else epilogue_rows32<OUT_BF16, ACT_NONE>(d, d.out, d.out_ld, v, n, m0 + c0, lane);
     }
   }
-  if (whole < rows) epilogue<true, EXT>(p, tmem, q, lane, 0, 1, n0, m0, m_end, ks, whole);
-}
-
-// k-slices of this tile meet: the last CTA to arrive sums them in slice order.
-template <bool BF16, bool EXT>
-__device__ __forceinline__ void reduce_slices(const GemmParams &p, SharedCtl &ctl, int n0, int m0, int m_end, int threads) {
-  const int tid = threadIdx.x;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    const int tile = blockIdx.z * gridDim.x + blockIdx.x;
-    ctl.last = (atomicAdd(p.counters + tile, 1) == p.ksplit - 1);
-    if (ctl.last) p.counters[tile] = 0;   // ready for the next launch on this stream
-  }
-  __syncthreads();
-  if (ctl.last && !ctl.abort) {
-    __threadfence();
-    // every thread sums the slices of one output element at a time, all slices' loads in flight together (at most 8 per batch)
-    const int rows = min(p.mb, m_end - m0);
-    if constexpr (BF16) {
-      if (p.N % 4 == 0) {   // four outputs per thread and step: a quarter of the trips to L2
-        for (int i = tid; i < rows * (BM / 4); i += threads) {
-          const int m = m0 + i / (BM / 4), n = n0 + (i % (BM / 4)) * 4;
-          if (n >= p.N) continue;
-          auto sum4 = [&](int nn) {
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int s0 = 0; s0 < p.ksplit; s0 += 4) {
-              float4 part[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                part[j] = (s0 + j < p.ksplit) ? __ldcg(reinterpret_cast<const float4 *>(p.partial + ((size_t)(s0 + j) * p.M + m) * p.N + nn)) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) { acc.x += part[j].x; acc.y += part[j].y; acc.z += part[j].z; acc.w += part[j].w; }
-            }
-            return acc;
-          };
-          if (p.dense.epilogue == PT_EPI_GLU && n < p.dense.split_n) {   // gate features n % 16 < 8, their up features eight further
-            if (n & 8) continue;
-            const float4 gt = sum4(n), up = sum4(n + 8);
-            dense_store_glu4<EXT>(p.dense, m, n, gt, up);
-            continue;
-          }
-          dense_store4<EXT>(p.dense, m, n, sum4(n));
-        }
-        return;
-      }
-    }
-    for (int i = tid; i < rows * BM; i += threads) {
-      const int m = m0 + i / BM, n = n0 + (i % BM);
-      if (n >= p.N) continue;
-      auto sum1 = [&](int nn) {
-        float acc = 0.f;
-        for (int s0 = 0; s0 < p.ksplit; s0 += 8) {
-          float part[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) part[j] = (s0 + j < p.ksplit) ? __ldcg(p.partial + ((size_t)(s0 + j) * p.M + m) * p.N + nn) : 0.f;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc += part[j];
-        }
-        return acc;
-      };
-      if constexpr (BF16) {
-        if (p.dense.epilogue == PT_EPI_GLU && n < p.dense.split_n) {
-          if (!(n & 8)) dense_store_glu<EXT>(p.dense, m, n, sum1(n), sum1(n + 8));
-          continue;
-        }
-      }
-      store_out<BF16, EXT>(p, sum1(n), m, n);
-    }
-  }
+  if (whole < rows) epilogue_any<EXT>(p, tmem, q, lane, n0, m0, m_end, whole);
 }
 
 // ------------------------------------------------------------------------------------------ FP8 and BF16
 // Dynamic shared memory: [stage][NA A tiles of 16 KB | B tile mb * 128 B], every tile 1024-byte aligned.  NA = 2: a CTA takes 256 weight
 // rows (two accumulators), which fetches a third less per product than NA = 1; without k-slices.
-template <bool BF16, int NA, bool EXT>
+template <int FMT, int NA, bool EXT>
 __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                                    const GemmParams p) {
-  constexpr int KX = BF16 ? BKB / 2 : BKB;   // elements of k per stage
+  constexpr bool BF16 = FMT == PT_W_BF16, F8 = FMT == PT_W_FP8;
+  constexpr int KX = F8 ? BKB : BKB / 2;     // elements of k per stage
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ SharedCtl ctl;
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int n0 = blockIdx.x * (BM * NA), m0 = blockIdx.z * p.mb, ks = blockIdx.y;
   const int kb0 = ks * p.kb_per_split, kb1 = min(p.n_kb, kb0 + p.kb_per_split);
   const int n_it = kb1 - kb0, na = NA == 1 ? 1 : min(NA, p.n_tiles - (int)blockIdx.x * NA);
@@ -603,7 +529,6 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
     }
     mbar_init(sa(&ctl.accum), 1);
     ctl.abort = 0;
-    ctl.last = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(sa(&ctl.tmem_base), tmem_cols);
@@ -612,10 +537,10 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
   fence_after();
   const uint32_t tmem = ctl.tmem_base;
   // Not before: a CTA of the next GEMM that found the tensor memory free would keep it while it waits for this kernel to end.
-  if (BF16 && p.pdl) launch_dependents();
+  if (p.pdl) launch_dependents();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // (ring positions and parities are carried as counters: this thread's instruction count per stage is what limits a CTA)
       const unsigned char *wt = p.w + w_base + ((size_t)blockIdx.x * NA * p.n_kb + kb0) * A_TILE;
       const size_t next_tile = (size_t)p.n_kb * A_TILE;
@@ -634,7 +559,7 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
         wt += A_TILE;
       };
       int early = 0;                         // stages whose weights are already on their way
-      if (BF16 && p.pdl) {
+      if (p.pdl) {
         for (; early < min(p.stages, n_it); ++early) {
           mbar_expect_tx(full0 + early * 8, tx);
           load_w(smem_s + early * stage_bytes, full0 + early * 8);
@@ -642,8 +567,7 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
         wait_for_prerequisites();
       }
       for (int it = 0; it < n_it; ++it) {
-        if (!first_round && !mbar_wait(empty0 + s * 8, par, &ctl.abort)) give_up(ctl, p.error_flag, 21);
-        if (ctl.abort) break;
+        if (!first_round && !wait_fast(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
         const uint32_t st = smem_s + s * stage_bytes, fb = full0 + s * 8;
         if (it >= early) {
           mbar_expect_tx(fb, tx);
@@ -655,7 +579,7 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // One thread issues every MMA of the CTA, so its loop is kept to a few dozen instructions per stage: descriptors are one
       // 64-bit add away from the stage-0 descriptors (the start-address field counts 16-byte units), ring position and parity
       // are counters.  (Measured: with divisions and descriptor rebuilds in this loop a stage took 0.6 us whatever its size.)
@@ -665,20 +589,19 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
       int s = 0;
       uint32_t par = 0, acc = 0;
       for (int it = 0; it < n_it; ++it) {
-        if (!mbar_wait(full0 + s * 8, par, &ctl.abort)) give_up(ctl, p.error_flag, 22);
-        if (ctl.abort) break;
+        if (!wait_fast(full0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 22); break; }
         fence_after();
         const uint64_t adesc = adesc0 + (uint64_t)(s * stage16), bdesc = bdesc0 + (uint64_t)(s * stage16);
-        umma<!BF16>(tmem, adesc, bdesc, idesc, acc);   // four MMAs of 32 bytes of k each; inside the swizzle atom the start address moves by 32 bytes
-        umma<!BF16>(tmem, adesc + 2, bdesc + 2, idesc, 1u);
-        umma<!BF16>(tmem, adesc + 4, bdesc + 4, idesc, 1u);
-        umma<!BF16>(tmem, adesc + 6, bdesc + 6, idesc, 1u);
+        umma<F8>(tmem, adesc, bdesc, idesc, acc);   // four MMAs of 32 bytes of k each; inside the swizzle atom the start address moves by 32 bytes
+        umma<F8>(tmem, adesc + 2, bdesc + 2, idesc, 1u);
+        umma<F8>(tmem, adesc + 4, bdesc + 4, idesc, 1u);
+        umma<F8>(tmem, adesc + 6, bdesc + 6, idesc, 1u);
         if (NA == 2 && na == 2) {
           const uint64_t a2 = adesc + (A_TILE >> 4);
-          umma<!BF16>(tmem + acc_cols, a2, bdesc, idesc, acc);
-          umma<!BF16>(tmem + acc_cols, a2 + 2, bdesc + 2, idesc, 1u);
-          umma<!BF16>(tmem + acc_cols, a2 + 4, bdesc + 4, idesc, 1u);
-          umma<!BF16>(tmem + acc_cols, a2 + 6, bdesc + 6, idesc, 1u);
+          umma<F8>(tmem + acc_cols, a2, bdesc, idesc, acc);
+          umma<F8>(tmem + acc_cols, a2 + 2, bdesc + 2, idesc, 1u);
+          umma<F8>(tmem + acc_cols, a2 + 4, bdesc + 4, idesc, 1u);
+          umma<F8>(tmem + acc_cols, a2 + 6, bdesc + 6, idesc, 1u);
         }
         umma_commit(empty0 + s * 8);
         acc = 1u;
@@ -687,18 +610,26 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
       umma_commit(sa(&ctl.accum));   // fires when every MMA above has completed
     }
   } else {
-    if (!mbar_wait(sa(&ctl.accum), 0, &ctl.abort)) give_up(ctl, p.error_flag, 24);
+    if (p.pdl) wait_for_prerequisites();                // the residual and the output are others' until here
+    const bool done = warp_wait(sa(&ctl.accum), 0, &ctl.abort);
+    if (!done) give_up(ctl, p.error_flag, 24);
     fence_after();
-    if (!ctl.abort && n_it > 0) {
-      if constexpr (BF16) {
-        for (int a = 0; a < na; ++a) epilogue_bf16<EXT>(p, tmem + a * acc_cols, warp & 3, lane, n0 + a * BM, m0, m_end, ks);
+    if (done && n_it > 0) {
+      if (NA == 1 && p.ksplit > 1) {
+        leave_sums(p, tmem, warp & 3, lane, 0, 1, reinterpret_cast<float *>(smem));
+      } else if constexpr (BF16) {
+        for (int a = 0; a < na; ++a) epilogue_bf16<EXT>(p, tmem + a * acc_cols, warp & 3, lane, n0 + a * BM, m0, m_end);
       } else {
-        epilogue<false, false>(p, tmem, warp & 3, lane, 0, 1, n0, m0, m_end, ks);
+        epilogue_fp16(p, tmem, warp & 3, lane, 0, 1, n0, m0);
       }
     }
     fence_before();
   }
-  if (NA == 1 && p.ksplit > 1) reduce_slices<BF16, EXT>(p, ctl, n0, m0, m_end, THREADS_F8);
+  if (NA == 1 && p.ksplit > 1) {
+    if (p.pdl) wait_for_prerequisites();
+    __syncwarp();
+    sum_cluster<BF16, EXT>(p, ctl, smem_s, ks, n0, m0, m_end, THREADS_F8);
+  }
   __syncthreads();
   fence_after();
   if (warp == 1) tmem_dealloc(tmem, tmem_cols);
@@ -990,14 +921,14 @@ using namespace pt;
 
 extern "C" size_t pt_gemm_packed_bytes(int wfmt, int n_out, int k_in) {
   const size_t rows = (size_t)ceil_div(n_out, tc::BM) * tc::BM;
-  return wfmt == PT_W_INT4 ? rows * (size_t)(k_in / 2) : rows * (size_t)k_in * (wfmt == PT_W_BF16 ? 2 : 1);
+  return wfmt == PT_W_INT4 ? rows * (size_t)(k_in / 2) : rows * (size_t)k_in * (wfmt == PT_W_FP8 ? 1 : 2);
 }
 
 extern "C" int pt_gemm_repack(int wfmt, const void *w, int n_out, int k_in, void *packed, void *stream) {
-  PT_REQUIRE(wfmt == PT_W_INT4 || wfmt == PT_W_FP8 || wfmt == PT_W_BF16, "pt_gemm_repack: weight format %d (INT4, FP8 or BF16)", wfmt);
+  PT_REQUIRE(wfmt == PT_W_INT4 || wfmt == PT_W_FP8 || wfmt == PT_W_BF16 || wfmt == PT_W_FP16, "pt_gemm_repack: unknown weight format %d", wfmt);
   PT_REQUIRE(w && packed && w != packed, "pt_gemm_repack: needs distinct source and destination buffers");
   PT_REQUIRE(((uintptr_t)w & 15) == 0 && ((uintptr_t)packed & 15) == 0, "pt_gemm_repack: buffers must be 16-byte aligned");
-  const int k_step = wfmt == PT_W_BF16 ? 64 : 128;
+  const int k_step = wfmt == PT_W_BF16 || wfmt == PT_W_FP16 ? 64 : 128;
   PT_REQUIRE(n_out > 0 && k_in > 0 && k_in % k_step == 0, "pt_gemm_repack: k_in=%d must be a positive multiple of %d", k_in, k_step);
   const int n_tiles = ceil_div(n_out, tc::BM);
   if (wfmt == PT_W_INT4) {
@@ -1005,7 +936,7 @@ extern "C" int pt_gemm_repack(int wfmt, const void *w, int n_out, int k_in, void
     const size_t n_words = (size_t)n_tiles * n_kb * 1024;
     tc::int4_tile_kernel<<<sm_count() * 8, 256, 0, as_stream(stream)>>>((const uint32_t *)w, (uint32_t *)packed, n_out, k_in, n_kb, n_words);
   } else {
-    const int k_bytes = wfmt == PT_W_BF16 ? 2 * k_in : k_in, n_kb = k_bytes / 128;
+    const int k_bytes = wfmt == PT_W_FP8 ? k_in : 2 * k_in, n_kb = k_bytes / 128;
     const size_t n_units = (size_t)n_tiles * n_kb * 1024;
     tc::fp8_tile_kernel<<<sm_count() * 8, 256, 0, as_stream(stream)>>>((const uint4 *)w, (uint4 *)packed, n_out, k_bytes, n_kb, n_units);
   }
@@ -1013,10 +944,8 @@ extern "C" int pt_gemm_repack(int wfmt, const void *w, int n_out, int k_in, void
   return PT_OK;
 }
 
-// k-slice workspace layout: [arrival counters, kGemmCounterBytes][partial sums].  The counter region has ONE size for every
-// shape, so that GEMMs of different widths can share a workspace: with a shape-dependent offset the partial sums of a narrow
-// GEMM (o_proj) would land where a wide one (q|k|v) expects zeroed counters.  16384 counters: one per (128-row weight tile,
-// block of activation rows); a shape with more tiles than that runs without k-slices when the split is automatic.
+// What a caller hands over for k-slices that it asks for.  (The kernels sum the slices of a tile in the shared memory of a cluster and use no
+// workspace; the size is as it always was.)
 constexpr size_t kGemmCounterBytes = 65536;
 constexpr size_t kGemmMaxCounters = kGemmCounterBytes / sizeof(int);
 
@@ -1026,9 +955,9 @@ extern "C" size_t pt_gemm_workspace_bytes(int m, int n_out, int max_ksplit) {
 
 extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   PT_REQUIRE(a, "pt_gemm: null args");
-  PT_REQUIRE(a->wfmt == PT_W_INT4 || a->wfmt == PT_W_FP8 || a->wfmt == PT_W_BF16, "pt_gemm: weight format %d (INT4, FP8 or BF16)", a->wfmt);
-  const bool int4 = a->wfmt == PT_W_INT4, bf16 = a->wfmt == PT_W_BF16;
-  const int k_step = bf16 ? 64 : 128;
+  PT_REQUIRE(a->wfmt == PT_W_INT4 || a->wfmt == PT_W_FP8 || a->wfmt == PT_W_BF16 || a->wfmt == PT_W_FP16, "pt_gemm: unknown weight format %d", a->wfmt);
+  const bool int4 = a->wfmt == PT_W_INT4, bf16 = a->wfmt == PT_W_BF16, fp16 = a->wfmt == PT_W_FP16;
+  const int k_step = bf16 || fp16 ? 64 : 128;
   PT_REQUIRE(a->m >= 1 && a->n_out >= 1 && a->k_in >= k_step && a->k_in % k_step == 0, "pt_gemm: bad shape m=%d n_out=%d k_in=%d (k_in a multiple of %d)",
              a->m, a->n_out, a->k_in, k_step);
   PT_REQUIRE(a->x && a->w && a->out, "pt_gemm: null x / w / out");
@@ -1039,13 +968,16 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     PT_REQUIRE(!bad, "pt_gemm: %s", bad);
     PT_REQUIRE(a->out_dtype == PT_DT_BF16 || a->out_dtype == PT_DT_F32, "pt_gemm: BF16 weights write bf16 or fp32, got type %d", a->out_dtype);
   } else {
-    PT_REQUIRE(a->epilogue == PT_EPI_STORE || a->epilogue == PT_EPI_RESIDUAL || a->epilogue == PT_EPI_BIAS || (int4 && a->epilogue == PT_EPI_SWIGLU),
-               "pt_gemm: epilogue %d (store, residual, bias or, INT4, swiglu)", a->epilogue);
+    PT_REQUIRE(a->epilogue == PT_EPI_STORE || a->epilogue == PT_EPI_RESIDUAL || a->epilogue == PT_EPI_BIAS || ((int4 || fp16) && a->epilogue == PT_EPI_SWIGLU) ||
+                   (fp16 && (a->epilogue == PT_EPI_BIAS_GELU || a->epilogue == PT_EPI_BIAS_RESIDUAL)),
+               "pt_gemm: epilogue %d (store, residual or bias; INT4 and FP16: swiglu; FP16: bias with gelu or residual)", a->epilogue);
     PT_REQUIRE(a->epilogue != PT_EPI_SWIGLU || a->n_out % 16 == 0, "pt_gemm: SwiGLU epilogue needs n_out %% 16 == 0, got %d", a->n_out);
   }
-  PT_REQUIRE(a->epilogue != PT_EPI_RESIDUAL || a->residual, "pt_gemm: residual epilogue needs residual");
-  PT_REQUIRE(a->epilogue != PT_EPI_BIAS || a->bias, "pt_gemm: bias epilogue needs bias");
-  PT_REQUIRE(!(int4 || bf16) || a->w_tiled, "pt_gemm: INT4 and BF16 weights must be tiled with pt_gemm_repack");
+  const bool wants_bias = a->epilogue == PT_EPI_BIAS || a->epilogue == PT_EPI_BIAS_GELU || a->epilogue == PT_EPI_BIAS_RESIDUAL;
+  const bool wants_residual = a->epilogue == PT_EPI_RESIDUAL || a->epilogue == PT_EPI_BIAS_RESIDUAL;
+  PT_REQUIRE(!wants_residual || a->residual, "pt_gemm: residual epilogue needs residual");
+  PT_REQUIRE(!wants_bias || a->bias, "pt_gemm: bias epilogue needs bias");
+  PT_REQUIRE(a->wfmt == PT_W_FP8 || a->w_tiled, "pt_gemm: INT4, BF16 and FP16 weights must be tiled with pt_gemm_repack");
   if (int4)
     PT_REQUIRE(a->scales && a->group >= 128 && a->group % 128 == 0 && a->k_in % a->group == 0,
                "pt_gemm: INT4 needs scales and a group (%d) that is a multiple of 128 dividing k_in=%d", a->group, a->k_in);
@@ -1067,13 +999,15 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     p.group_of = a->ext->group_of;
     p.group_used = a->ext->group_used;
     p.group_stride = pt_gemm_packed_bytes(a->wfmt, a->n_out, a->k_in);
-  } else if (bf16)
+  } else if (bf16 || fp16)
     while (p.mb > 64 && n_tiles * ceil_div(a->m, p.mb) * 4 < sm_count() * 3) p.mb = ceil_div(p.mb, 32) * 16;
   int m_tiles = ceil_div(a->m, p.mb);
-  p.n_kb = bf16 ? a->k_in / 64 : a->k_in / 128;
-  // k-slices: fill the GPU when there are few tiles, but keep at least PT_TC_MIN_KB k-blocks per CTA
+  p.n_kb = bf16 || fp16 ? a->k_in / 64 : a->k_in / 128;
+  // k-slices: fill the GPU when there are few tiles, with at least PT_TC_MIN_KB k-blocks per CTA.  Not to the brim: the slices of a tile
+  // start together in one cluster, and 36 clusters of eight did not fit 148 SMs of two CTAs each at once (4608 x 4096 at 8 rows: 14.7 us
+  // with 8 slices, 11.1 with 7; 12288 x 4096: 26 us with 3 slices, 20 with 2).
 #ifndef PT_TC_MIN_KB
-#define PT_TC_MIN_KB 8
+#define PT_TC_MIN_KB 3
 #endif
   int ksplit = a->ksplit;
   if (int4) {
@@ -1081,14 +1015,12 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     p.mb = plan.mb;
     ksplit = plan.ksplit;
   } else if (ksplit <= 0) {
-    ksplit = std::max(1, (p.mb <= 64 ? 2 : 1) * sm_count() / (n_tiles * m_tiles));   // two CTAs fit an SM up to 64 activation rows
+    ksplit = std::max(1, (p.mb <= 64 ? 2 : 1) * sm_count() * 7 / 8 / (n_tiles * m_tiles));   // two CTAs fit an SM up to 64 activation rows
     // (with several blocks of activation rows a slice's sums cost more than its share of a short k saves: 128 x 2048 at 512 .. 8192
     // rows takes 19 - 21 us whole and 27 - 41 us in slices)
-    ksplit = std::max(1, std::min(ksplit, p.n_kb / (bf16 && m_tiles > 1 ? 32 : PT_TC_MIN_KB)));
-    ksplit = std::min(ksplit, 8);                                           // what pt_gemm_workspace_bytes is usually asked for ...
-    while (ksplit > 1 && pt_gemm_workspace_bytes(a->m, a->n_out, ksplit) > a->workspace_bytes) --ksplit;   // ... and never more than the caller's workspace holds
-    if ((size_t)n_tiles * m_tiles > kGemmMaxCounters) ksplit = 1;
+    ksplit = std::max(1, std::min(ksplit, p.n_kb / ((bf16 || fp16) && m_tiles > 1 ? 32 : PT_TC_MIN_KB)));
   }
+  ksplit = std::min(ksplit, tc::MAX_CLUSTER);
   m_tiles = ceil_div(a->m, p.mb);
   ksplit = std::max(1, std::min(ksplit, p.n_kb));
   p.kb_per_split = ceil_div(p.n_kb, ksplit);
@@ -1096,19 +1028,17 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   p.epilogue = a->epilogue;
   p.out_scale = int4 ? 1.0f : (a->x_scale > 0.f ? a->x_scale : 1.0f) * (a->w_scale > 0.f ? a->w_scale : 1.0f);
   p.scales = (const __half *)a->scales;
-  p.residual = (const __half *)a->residual;
-  p.bias = (const __half *)a->bias;
+  p.residual = wants_residual ? (const __half *)a->residual : nullptr;
+  p.bias = wants_bias ? (const __half *)a->bias : nullptr;
   p.out = (__half *)a->out;
   p.out_ld = a->out_ld > 0 ? a->out_ld : (a->epilogue == PT_EPI_SWIGLU ? a->n_out / 2 : a->n_out);
   if (bf16) p.dense = make_dense_out(a->out, p.out_ld, a->out_dtype, a->epilogue, a->alpha, a->ext);
   p.error_flag = a->error_flag;
-  if (int4 ? a->ksplit > 1 : p.ksplit > 1) {   // (INT4: slices that the caller asked for; the kernel itself needs no workspace)
-    const size_t need = pt_gemm_workspace_bytes(a->m, a->n_out, int4 ? a->ksplit : p.ksplit);
+  if (a->ksplit > 1 && p.ksplit > 1) {   // slices that the caller asked for
+    const size_t need = pt_gemm_workspace_bytes(a->m, a->n_out, p.ksplit);
     PT_REQUIRE(a->workspace && a->workspace_bytes >= need, "pt_gemm: %d k-slices need %zu workspace bytes, got %zu", p.ksplit, need, a->workspace_bytes);
     PT_REQUIRE((size_t)n_tiles * m_tiles <= kGemmMaxCounters, "pt_gemm: %d x %d tiles exceed the %zu arrival counters of a k-slice workspace", n_tiles,
                m_tiles, kGemmMaxCounters);
-    p.counters = (int *)a->workspace;
-    p.partial = (float *)((char *)a->workspace + kGemmCounterBytes);
   }
 
   // BF16 without k-slices: two weight tiles per CTA when half as many CTAs still fill the GPU
@@ -1118,7 +1048,7 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   const bool pair = PT_TC_PAIR && bf16 && p.ksplit == 1 && p.mb >= 128 && n_tiles >= 2 && (long long)ceil_div(n_tiles, 2) * m_tiles >= sm_count();
   const int na = pair ? 2 : 1;
   p.n_tiles = n_tiles;
-  p.pdl = (bf16 || int4) && a->pdl ? 1 : 0;
+  p.pdl = a->pdl ? 1 : 0;
   const uint32_t b_bytes = (uint32_t)p.mb * tc::BKB;
   const uint32_t stage_bytes = na * tc::A_TILE + ((b_bytes + 1023u) & ~1023u);
   // Up to 64 activation rows a stage is small, and what limits the kernel is the one thread per CTA that issues the MMAs (about
@@ -1129,7 +1059,8 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
 #endif
   // BF16 also with large tiles when there are more of them than SMs: the epilogue of one CTA then hides behind the products of the
   // other (two accumulators of 256 columns fill the tensor memory).
-  const bool small = p.mb <= 64 || (bf16 && na * p.mb <= 256 && (long long)n_tiles * m_tiles * p.ksplit > sm_count());
+  // (The sums of a slice take 512 bytes per row of the ring.)
+  const bool small = p.mb <= 64 || ((bf16 || fp16) && !(p.ksplit > 1 && p.mb > 128) && na * p.mb <= 256 && (long long)n_tiles * m_tiles * p.ksplit > sm_count());
   const uint32_t budget = (small ? PT_TC_BUDGET_SMALL_KB : 200) * 1024u;
   size_t smem;
   const bool two_int4 = int4 && p.mb <= 128 && n_tiles * m_tiles * p.ksplit > sm_count();   // two CTAs per SM (each has half the tensor memory)
@@ -1146,12 +1077,12 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     p.stages = (int)std::min<uint32_t>(8, budget / stage_bytes);
     PT_REQUIRE(p.stages >= 2, "pt_gemm: tile does not fit shared memory");
     smem = (size_t)p.stages * stage_bytes + 1024;
-    if (bf16 && p.mb > 64) smem = std::max<size_t>(smem, (na * p.mb > 256 ? 120 : 80) * 1024);   // never more CTAs on an SM than its tensor memory holds accumulators for
+    if (p.mb > 64) smem = std::max<size_t>(smem, (na * p.mb > 256 ? 120 : 80) * 1024);   // never more CTAs on an SM than its tensor memory holds accumulators for
   }
 
   CUtensorMap map_w, map_x;
   memset(&map_w, 0, sizeof(map_w));
-  if (int4) {
+  if (int4 || fp16) {
     if (int rc = tc::make_map(&map_x, a->x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)a->k_in, (uint64_t)a->m, 64, (uint32_t)p.mb, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
   } else if (bf16) {
     if (int rc = tc::make_map(&map_x, a->x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a->k_in, (uint64_t)a->m, 64, (uint32_t)p.mb, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
@@ -1162,56 +1093,48 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   }
   static bool attr_set = false;
   if (!attr_set) {
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<false, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<true, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<true, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_FP8, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_FP16, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_BF16, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_BF16, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_BF16, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_BF16, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     PT_CUDA(cudaFuncSetAttribute(tc::gemm_int4_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     PT_CUDA(cudaFuncSetAttribute(tc::gemm_int4_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     attr_set = true;
   }
   dim3 grid(ceil_div(n_tiles, na), p.ksplit, m_tiles);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(int4 ? (3 + 4 * int4_groups) * 32 : tc::THREADS_F8);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = as_stream(stream);
+  cudaLaunchAttribute attr[2];
+  int n_attr = 0;
+  if (p.ksplit > 1) {   // the k-slices of a tile: one cluster
+    attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+    attr[n_attr].val.clusterDim.x = 1;
+    attr[n_attr].val.clusterDim.y = p.ksplit;
+    attr[n_attr++].val.clusterDim.z = 1;
+  }
+  if (p.pdl) {
+    attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n_attr++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n_attr;
+  cudaError_t e;
   if (int4) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((3 + 4 * int4_groups) * 32);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = as_stream(stream);
-    cudaLaunchAttribute attr[2];
-    int n_attr = 0;
-    if (p.ksplit > 1) {
-      attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-      attr[n_attr].val.clusterDim.x = 1;
-      attr[n_attr].val.clusterDim.y = p.ksplit;
-      attr[n_attr++].val.clusterDim.z = 1;
-    }
-    if (p.pdl) {
-      attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[n_attr++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n_attr;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, int4_groups == 2 ? tc::gemm_int4_kernel<2> : tc::gemm_int4_kernel<4>, map_x, p);
-    if (e != cudaSuccess) return pt::set_error(PT_ERR_CUDA, "pt_gemm: %s", cudaGetErrorString(e));
-  } else if (bf16) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(tc::THREADS_F8);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = as_stream(stream);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = p.pdl ? 1 : 0;
-    const bool ext = dense_needs_ext(a->epilogue, a->ext);
-    const auto kernel = pair ? (ext ? tc::gemm_dense_kernel<true, 2, true> : tc::gemm_dense_kernel<true, 2, false>)
-                             : (ext ? tc::gemm_dense_kernel<true, 1, true> : tc::gemm_dense_kernel<true, 1, false>);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, p);
-    if (e != cudaSuccess) return pt::set_error(PT_ERR_CUDA, "pt_gemm: %s", cudaGetErrorString(e));
-  } else
-    tc::gemm_dense_kernel<false, 1, false><<<grid, tc::THREADS_F8, smem, as_stream(stream)>>>(map_w, map_x, p);
+    e = cudaLaunchKernelEx(&cfg, int4_groups == 2 ? tc::gemm_int4_kernel<2> : tc::gemm_int4_kernel<4>, map_x, p);
+  } else {
+    const bool ext = bf16 && dense_needs_ext(a->epilogue, a->ext);
+    const auto kernel = fp16 ? tc::gemm_dense_kernel<PT_W_FP16, 1, false>
+                       : !bf16 ? tc::gemm_dense_kernel<PT_W_FP8, 1, false>
+                       : pair ? (ext ? tc::gemm_dense_kernel<PT_W_BF16, 2, true> : tc::gemm_dense_kernel<PT_W_BF16, 2, false>)
+                              : (ext ? tc::gemm_dense_kernel<PT_W_BF16, 1, true> : tc::gemm_dense_kernel<PT_W_BF16, 1, false>);
+    e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, p);
+  }
+  if (e != cudaSuccess) return pt::set_error(PT_ERR_CUDA, "pt_gemm: %s", cudaGetErrorString(e));
   PT_LAUNCH_CHECK("pt_gemm");
   return PT_OK;
 }

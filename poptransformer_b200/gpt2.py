@@ -61,21 +61,22 @@ class GPT2Decoder(DecodeLoop):
         self.d_loc, self.h_loc = d // tp, c.n_head // tp
         cols = lambda w, k: w[:, r * (k // tp):(r + 1) * (k // tp)].contiguous()        # 'end': rank r's input features
         end_bias = lambda b: b if tp == 1 else b.repeat(B, 1).contiguous()           # added once, after the all-reduce
+        lin = (lambda w: ops.fp16_linear(w, B)) if tp == 1 else (lambda w: ops.PackedLinear(ops.W_FP16, w))
         self.layers = []
         for i in range(c.n_layer):
             p = f"transformer.h.{i}."
             self.layers.append({
                 "ln1": (t(p + "ln_1.weight"), t(p + "ln_1.bias")), "ln2": (t(p + "ln_2.weight"), t(p + "ln_2.bias")),
-                "c_attn": ops.PackedLinear(ops.W_FP16, fused_qkv_rows(t(p + "attn.c_attn.weight"), r, tp).contiguous()),
+                "c_attn": lin(fused_qkv_rows(t(p + "attn.c_attn.weight"), r, tp).contiguous()),
                 "b_attn": fused_qkv_rows(t(p + "attn.c_attn.bias"), r, tp).contiguous(),
-                "c_proj": ops.PackedLinear(ops.W_FP16, cols(t(p + "attn.c_proj.weight"), d)), "b_proj": end_bias(t(p + "attn.c_proj.bias")),
-                "c_fc": ops.PackedLinear(ops.W_FP16, rows(t(p + "mlp.c_fc.weight"), r, tp).contiguous()),
+                "c_proj": lin(cols(t(p + "attn.c_proj.weight"), d)), "b_proj": end_bias(t(p + "attn.c_proj.bias")),
+                "c_fc": lin(rows(t(p + "mlp.c_fc.weight"), r, tp).contiguous()),
                 "b_fc": rows(t(p + "mlp.c_fc.bias"), r, tp).contiguous(),
-                "m_proj": ops.PackedLinear(ops.W_FP16, cols(t(p + "mlp.c_proj.weight"), 4 * d)), "b_mproj": end_bias(t(p + "mlp.c_proj.bias")),
+                "m_proj": lin(cols(t(p + "mlp.c_proj.weight"), 4 * d)), "b_mproj": end_bias(t(p + "mlp.c_proj.bias")),
             })
         self.ln_f = (t("transformer.ln_f.weight"), t("transformer.ln_f.bias"))
         head, self.vocab_loc = vocab_rows(self.wte, r, tp) if tp > 1 else (self.wte, c.vocab)
-        self.head = ops.PackedLinear(ops.W_FP16, head)                           # tied: logits = h . wte^T
+        self.head = lin(head)                           # tied: logits = h . wte^T
         f16 = dict(dtype=torch.float16, device=dev)
         self.ids = torch.full((B, c.max_len), self.pad_id, dtype=torch.int32, device=dev)
         self.pos = torch.arange(c.max_len, dtype=torch.int32, device=dev).repeat(B, 1).contiguous()   # position ids = step
@@ -108,6 +109,12 @@ class GPT2Decoder(DecodeLoop):
         """norm = (gamma, beta): the LayerNorm in front of the linear (ops.layer_norm_ce, NormCE arithmetic) runs as the kernel's
         prologue instead of as a launch of its own."""
         pro = {}
+        if isinstance(pl, ops.GemmWeight):
+            if norm is not None:
+                self._norm(x, norm, self.h)
+                x = self.h
+            ops.gemm(x, pl, out=out, epilogue=epilogue, bias=bias, residual=residual, error_flag=self.error_flag)
+            return
         if norm is not None and self.batch <= 8:
             pro = dict(prologue=ops.PRO_NORMCE, gamma=norm[0], beta=norm[1], eps=self.cfg.eps)
         elif norm is not None:

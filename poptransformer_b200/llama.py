@@ -95,7 +95,12 @@ class LlamaDecoder(DecodeLoop):
                 if self.use_gemm:
                     return ops.GemmWeight(ops.W_INT4, torch.cat(ws, 0), torch.cat(sc, 0), group=grp, interleave_gate_up=interleave)
                 return ops.PackedLinear(ops.W_INT4, torch.cat(ws, 0), torch.cat(sc, 0), group=grp, interleave_gate_up=interleave)
-            return ops.PackedLinear(ops.W_FP16, torch.cat(ws, 0).to(torch.float16), interleave_gate_up=interleave)
+            return fp16(torch.cat(ws, 0).to(torch.float16), interleave)
+
+        def fp16(w, interleave=False):
+            if tp_size == 1 and persistent is None:
+                return ops.fp16_linear(w, batch, interleave_gate_up=interleave)
+            return ops.PackedLinear(ops.W_FP16, w, interleave_gate_up=interleave)
 
         def row_parallel(key, k_total):
             w = t(key)
@@ -106,7 +111,7 @@ class LlamaDecoder(DecodeLoop):
                 loc, loc_s, grp_loc, ks = row_parallel_int4(w, t(key + "_scale").reshape(w.shape[0], -1), k_total, r, tp)
                 return ops.PackedLinear(ops.W_INT4, loc, loc_s, group=grp_loc), ks
             loc, ks = row_parallel_fp16(w, k_total, r, tp)
-            return ops.PackedLinear(ops.W_FP16, loc), ks
+            return fp16(loc), ks
 
         def gemm_weight(keys, interleave=False):
             ws = [t(k) for k in keys]
@@ -155,7 +160,7 @@ class LlamaDecoder(DecodeLoop):
             if pad:
                 head = torch.cat([head, torch.zeros((pad, d), dtype=torch.float16, device=dev)], 0)   # shard() zero-pads
             head = head[r * self.vocab_loc:(r + 1) * self.vocab_loc]
-        self.head = ops.PackedLinear(ops.W_FP16, head.contiguous())
+        self.head = fp16(head.contiguous()) if batch > 2 else ops.PackedLinear(ops.W_FP16, head.contiguous())
         self.sin, self.cos = rope_tables(c.max_len, c.head_dim, dev)
         self.score_scale = float(np.float16(1 / math.sqrt(c.head_dim)))
         self._state_opts = dict(page_size=page_size, persistent=persistent, keep_logits=keep_logits, tp_buffers=tp_buffers, wait_limit=wait_limit)
@@ -310,6 +315,11 @@ class LlamaDecoder(DecodeLoop):
             torch.distributed.all_reduce(tns, group=self.group)
 
     def _norm_linear(self, x, gamma, pl, out, epilogue=ops.EPI_STORE, out_ld=0):
+        if isinstance(pl, ops.GemmWeight):
+            ops.check(ops._lib.lib().pt_rms_norm(ops._ptr(x), None, ops._ptr(gamma), x.shape[0], x.shape[1], self.cfg.eps, ops._ptr(self.h), None,
+                                                 ops._stream()), "pt_rms_norm")
+            ops.gemm(self.h, pl, out=out, epilogue=epilogue, out_ld=out_ld, error_flag=self.error_flag)
+            return
         if x.shape[0] > 32:
             # beyond the skinny-matmul kernels' 32 rows (the fp16 LM head of a large batch, whose transformer linears run on the
             # GEMM): normalise once, then the linear in blocks of 32 rows
@@ -331,7 +341,7 @@ class LlamaDecoder(DecodeLoop):
     def _row_parallel(self, x_in, pl):
         """x <- fp16(x + all_reduce(fp16(x_in . W_r^T)))  (Linear 'end' + ops.add, llama2/model.py:42,45)."""
         if self.tp == 1:
-            ops.linear(x_in, pl, self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, workspace=self.lin_ws, pdl=self.pdl)
+            ops.linear_fp16(x_in, pl, self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, workspace=self.lin_ws, pdl=self.pdl)
         else:
             ops.linear(x_in, pl, self.part, workspace=self.lin_ws, pdl=self.pdl)
             self._all_reduce(self.part)
@@ -443,6 +453,9 @@ class LlamaDecoder(DecodeLoop):
     def _norm_linear_raw(self, x, gamma, pl, out_ptr, out_ld):
         """gate|up linear with the SwiGLU epilogue writing at a column offset of the (zero-padded) activation buffer."""
         L_ = ops._lib.lib()
+        if isinstance(pl, ops.GemmWeight):
+            self._norm_linear(x, gamma, pl, self.act, epilogue=ops.EPI_SWIGLU, out_ld=out_ld)     # (one GPU: no column offset)
+            return
         src = x
         pro = ops.PRO_RMSNORM
         if not self.fuse_norm:

@@ -142,7 +142,7 @@ def linear(x, pl, out=None, **kw):
 # ------------------------------------------------------------------------------------------ tensor-core GEMMs (16+ rows)
 class GemmWeight:
     """A weight matrix tiled once for pt_gemm (pt_gemm_repack): FP8 bytes [n_out, k], or INT4 rows in the reference's int8
-    [n_out, k/2] format plus fp16 scales [n_out, k/group], or bfloat16 [n_out, k]."""
+    [n_out, k/2] format plus fp16 scales [n_out, k/group], or float16 or bfloat16 [n_out, k]."""
 
     def __init__(self, wfmt, w, scale=None, group=0, w_scale=1.0, interleave_gate_up=False):
         """interleave_gate_up: rows [f gate features | f up features] in the order EPI_SWIGLU wants (eight and eight in turn)."""
@@ -157,18 +157,37 @@ class GemmWeight:
             self.k_in = w.shape[1] * 2
             self.group = int(group) if group else self.k_in
             self.scales = scale.reshape(self.n_out, self.k_in // self.group).to(torch.float16).contiguous()
-        elif wfmt in (W_FP8, W_BF16):
+        elif wfmt in (W_FP8, W_BF16, W_FP16):
             self.k_in, self.group, self.scales = w.shape[1], 0, None
         else:
-            raise PtError("GemmWeight: INT4, FP8 or BF16")
+            raise PtError("GemmWeight: INT4, FP8, FP16 or BF16")
         self.w = torch.empty(L.pt_gemm_packed_bytes(wfmt, self.n_out, self.k_in), dtype=torch.uint8, device=w.device)
         check(L.pt_gemm_repack(wfmt, _ptr(w.contiguous()), self.n_out, self.k_in, _ptr(self.w), _stream()), "pt_gemm_repack")
 
     @property
     def nbytes(self):
         """Algorithmic bytes one launch streams from HBM."""
-        wb = self.n_out * self.k_in // 2 if self.wfmt == W_INT4 else self.n_out * self.k_in * (2 if self.wfmt == W_BF16 else 1)
+        wb = self.n_out * self.k_in // 2 if self.wfmt == W_INT4 else self.n_out * self.k_in * (1 if self.wfmt == W_FP8 else 2)
         return wb + (self.scales.numel() * 2 if self.scales is not None else 0)
+
+
+# fp16 weights: rows from which the tcgen05 GEMM is the faster kernel.
+GEMM_FP16_ROWS = 4
+
+
+def fp16_linear(w, rows, interleave_gate_up=False):
+    """fp16 weights [n_out, k] for a decoder of `rows` rows, laid out for the kernel that serves that many: the skinny-matmul kernel, or from
+    GEMM_FP16_ROWS rows on (k a multiple of 64) the GEMM.  Call with `linear_fp16`."""
+    if rows >= GEMM_FP16_ROWS and w.shape[1] % 64 == 0:
+        return GemmWeight(W_FP16, w, interleave_gate_up=interleave_gate_up)
+    return PackedLinear(W_FP16, w, interleave_gate_up=interleave_gate_up)
+
+
+def linear_fp16(x, weight, out, epilogue=EPI_STORE, bias=None, residual=None, workspace=None, error_flag=None, pdl=0, out_ld=0):
+    """One linear on either layout of `fp16_linear` (no prologue)."""
+    if isinstance(weight, GemmWeight):
+        return gemm(x, weight, out=out, epilogue=epilogue, bias=bias, residual=residual, error_flag=error_flag, pdl=pdl, out_ld=out_ld)
+    return linear(x, weight, out, epilogue=epilogue, bias=bias, residual=residual, workspace=workspace, error_flag=error_flag, pdl=pdl, out_ld=out_ld)
 
 
 def gemm_workspace(m, n_out_max, max_ksplit=8, device="cuda"):

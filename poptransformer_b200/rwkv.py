@@ -48,9 +48,9 @@ class RWKVDecoder(DecodeLoop):
         h = lambda k: state_dict[k].to(dev).to(torch.float16).reshape(-1).contiguous()
         f = lambda k: state_dict[k].to(dev).to(torch.float32).reshape(-1)[r * dl:(r + 1) * dl].contiguous()   # sharded with the channels
         w16 = lambda k: state_dict[k].to(dev).to(torch.float16)
-        lin = lambda k: ops.PackedLinear(ops.W_FP16, w16(k).contiguous())
-        start = lambda k: ops.PackedLinear(ops.W_FP16, rows(w16(k), r, tp).contiguous())
-        end = lambda k, kl: ops.PackedLinear(ops.W_FP16, w16(k)[:, r * kl:(r + 1) * kl].contiguous())
+        pack = (lambda w: ops.fp16_linear(w, batch)) if tp == 1 else (lambda w: ops.PackedLinear(ops.W_FP16, w))
+        start = lambda k: pack(rows(w16(k), r, tp).contiguous())
+        end = lambda k, kl: pack(w16(k)[:, r * kl:(r + 1) * kl].contiguous())
         ln = lambda p: (h(p + ".weight"), h(p + ".bias"))
         self.emb = state_dict["rwkv.embeddings.weight"].to(dev).to(torch.float16).contiguous()
         self.layers = []
@@ -68,7 +68,7 @@ class RWKVDecoder(DecodeLoop):
             })
         self.ln_out = ln("rwkv.ln_out")
         head, self.vocab_loc = vocab_rows(w16("head.weight"), r, tp) if tp > 1 else (w16("head.weight").contiguous(), c.vocab)
-        self.head = ops.PackedLinear(ops.W_FP16, head)
+        self.head = pack(head)
         B, d = batch, c.d_model
         f16 = dict(dtype=torch.float16, device=dev)
         self.ids = torch.full((B, c.max_len), self.pad_id, dtype=torch.int32, device=dev)
@@ -102,13 +102,13 @@ class RWKVDecoder(DecodeLoop):
 
     def _linear(self, x, pl, out, epilogue=ops.EPI_STORE, residual=None, side=None):
         """side = None: on the current stream; side = i: on side stream i (between _fork and _join), with that stream's workspace."""
-        ws = self.lin_ws if side is None else self.side_ws[side]
-        a = ops.linear_args(x, pl, out, epilogue=epilogue, residual=residual, workspace=ws, error_flag=self.error_flag, pdl=self.pdl_linear)
+        kw = dict(epilogue=epilogue, residual=residual, workspace=self.lin_ws if side is None else self.side_ws[side], error_flag=self.error_flag,
+                  pdl=self.pdl_linear)
         if side is None:
-            ops.check(ops._lib.lib().pt_linear(ctypes.byref(a), ops._stream()), "pt_linear")
+            ops.linear_fp16(x, pl, out, **kw)
         else:
             with torch.cuda.stream(self.side[side]):
-                ops.check(ops._lib.lib().pt_linear(ctypes.byref(a), ops._stream()), "pt_linear")
+                ops.linear_fp16(x, pl, out, **kw)
 
     def _fork(self):
         main = torch.cuda.current_stream()
