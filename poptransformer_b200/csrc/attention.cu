@@ -1,17 +1,21 @@
 // Paged KV cache: append of the new token fused with split flash-decode attention.
 //
-// One block handles one page (page_size cached tokens) of one (sequence, kv-head): its K and V tiles are contiguous in the
-// pool.  The block that owns the page holding position `step` writes the new k/v into the pool and takes them from shared
+// One block handles a run of pages (page_size cached tokens each) of one (sequence, kv-head): a page's K and V tiles are contiguous
+// in the pool.  The block that owns the page holding position `step` writes the new k/v into the pool and takes them from shared
 // memory itself, so the append costs no extra pass over the cache.  Scores and P.V run on the tensor cores (see the kernel),
-// the softmax statistics are warp-shuffle reductions.  Every block leaves (max, sum, partial output) in the workspace; the
-// last block to arrive for a (sequence, kv-head) combines the pages in a fixed order, which keeps the result deterministic.
+// the softmax statistics are warp-shuffle reductions.  A block whose run is the whole history writes the output; otherwise every block
+// leaves (max, sum, partial output) in the workspace and the last block to arrive for a (sequence, kv-head) combines the runs in a
+// fixed order, which keeps the result deterministic.
 //
 // HBM-bound: algorithmic bytes = 2 * (step + 1) * head_dim * 2 per (sequence, kv-head), read once.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace pt {
 
 struct AttnParams {
+  int ppb;         // pages per block
   int B, n_head, n_kv, qpk, qsplit, H, page, max_pages, max_len, rope_mode, softmax_mode, rot_half, out_ld, pdl;
   __half scale_h;
   int use_scale;
@@ -73,7 +77,11 @@ __device__ __forceinline__ uint32_t pack_f2h2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// One block = one page of one (sequence, kv head, part of the group's q heads).  Both products run on the tensor cores
+// One block = `ppb` consecutive pages of one (sequence, kv head, part of the group's q heads), one page after the other: while a page's
+// weights are formed and multiplied, the K rows of the next are on their way to registers and its V tile to the other of two buffers.
+// The host takes as many pages per block as still leave about four blocks per SM: with one page per block the fixed cost of a block
+// (table look-up, rotation, partial results through L2, arrival) was most of the kernel.  (Measured on B200: see pages_per_block.)
+// Both products run on the tensor cores
 // (mma.sync m16n8k16, fp32 accumulation of exact fp16 products):
 //   scores^T [keys x heads] = K [keys x H] . q^T: warp w takes keys 16 w .. 16 w + 15 of each 64-key pass.  Its K rows go from
 //     global memory STRAIGHT into the A fragments: a lane loads 16 bytes = channels 32 pp + 8 tig .. + 7 of its two key rows,
@@ -85,14 +93,14 @@ __device__ __forceinline__ uint32_t pack_f2h2(float lo, float hi) {
 // The new token's key / value are staged in shared memory by the block that owns the last page and appended to the pool by one
 // block per kv head.
 template <int H>
-__global__ void __launch_bounds__(kAttnThreads, 5) kv_append_attn_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(kAttnThreads, 4) kv_append_attn_kernel(const AttnParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int VLD = H + 8;                               // V rows padded: ldmatrix reads 8 rows in 8 different bank groups
   constexpr int QLD = H + 32;                              // q rows: two heads read in one shared-memory phase sit 16 banks apart
   const int PAGE = p.page, KP = (PAGE + 15) & ~15;         // keys padded to whole 16-key steps
   const int PSLD = KP + 8;                                 // row stride of the score / weight rows
-  __half *Vs = reinterpret_cast<__half *>(smem);           // [KP][VLD]
-  __half *qs = Vs + (size_t)KP * VLD;                      // [NQ_MAX][QLD], rows >= nq are zero
+  __half *Vs0 = reinterpret_cast<__half *>(smem);          // [two of them if a block takes more than one page][KP][VLD]
+  __half *qs = Vs0 + (size_t)(p.ppb > 1 ? 2 : 1) * KP * VLD;                      // [NQ_MAX][QLD], rows >= nq are zero
   __half *newk = qs + (size_t)NQ_MAX * QLD;                // [H]: the new token's rotated key (owner block)
   float *ps = reinterpret_cast<float *>(newk + H);         // [NQ_MAX][PSLD]
   float *ml = ps + (size_t)NQ_MAX * PSLD;                  // [NQ_MAX][2]
@@ -101,7 +109,7 @@ __global__ void __launch_bounds__(kAttnThreads, 5) kv_append_attn_kernel(const A
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
   // With many q heads per kv head (multi-query attention) the heads of a group are shared out over `qsplit` blocks: each
   // re-reads the group's K/V page (through L2) and handles nq of the group's heads.
-  const int pg = blockIdx.x, kvh = blockIdx.y / p.qsplit, qpart = blockIdx.y - kvh * p.qsplit, b = blockIdx.z;
+  const int pg0 = blockIdx.x * p.ppb, kvh = blockIdx.y / p.qsplit, qpart = blockIdx.y - kvh * p.qsplit, b = blockIdx.z;
   const int nq = p.qpk / p.qsplit, q_lo = qpart * nq;   // this block's heads of the group: q_lo .. q_lo + nq - 1
   if (p.pdl) {
     // let the next kernel start prefetching its weights; everything this kernel reads was produced upstream
@@ -109,25 +117,30 @@ __global__ void __launch_bounds__(kAttnThreads, 5) kv_append_attn_kernel(const A
     asm volatile("griddepcontrol.wait;" ::: "memory");
   }
   // the page-table entry does not depend on the step: both loads go out together (one round trip less before the K / V loads)
-  const int phys = p.page_table[(size_t)b * p.max_pages + pg];
+  int phys = p.page_table[(size_t)b * p.max_pages + pg0];
   const int step = *p.step;
   if (step < 0 || step >= p.max_len) {  // no page / no RoPE row for this position: report it and leave the counters untouched
     if (tid == 0 && p.error_flag) atomicExch(p.error_flag, 12);
     return;
   }
-  const int n_active = step / PAGE + 1;
-  if (pg >= n_active) return;
-  const int n_valid = min(PAGE, step + 1 - pg * PAGE);
-  const bool owner = (pg == n_active - 1);
-  const int n_load = owner ? n_valid - 1 : n_valid;  // the newest token is not in the pool yet
-  const int slot = n_valid - 1;                      // owner: where the new token goes
+  const int n_pages = step / PAGE + 1;
+  if (pg0 >= n_pages) return;
+  const int pg1 = min(n_pages, pg0 + p.ppb), n_active = (n_pages + p.ppb - 1) / p.ppb;   // (blocks of this (sequence, kv head) that have pages)
+  const bool has_last = pg1 == n_pages;
+  const int slot = step - (n_pages - 1) * PAGE;      // where the new token goes in the last page
+  const int row_elems = (p.n_head + 2 * p.n_kv) * H;
+  const __half *qrow = p.qkv + (size_t)b * row_elems;
+  const __half *vnew = qrow + (size_t)(p.n_head + p.n_kv + kvh) * H;
 
-  __half *gK = p.pool + (((size_t)phys * 2 + 0) * p.n_kv + kvh) * PAGE * H;
-  __half *gV = p.pool + (((size_t)phys * 2 + 1) * p.n_kv + kvh) * PAGE * H;
-
-  // ---- this warp's K rows of the first 64-key pass, requested before anything else (keys 16 warp + g and + 8)
+  __half *gK, *gV;            // the tiles of the page that is being requested
+  int n_load;                 // its rows in the pool (the newest token is not there yet)
+  auto page_at = [&](int pg) {
+    gK = p.pool + (((size_t)phys * 2 + 0) * p.n_kv + kvh) * PAGE * H;
+    gV = p.pool + (((size_t)phys * 2 + 1) * p.n_kv + kvh) * PAGE * H;
+    n_load = pg == n_pages - 1 ? slot : PAGE;
+  };
   uint4 kf[2][H / 32];
-  auto load_k = [&](int kbase) {
+  auto load_k = [&](int kbase) {   // this warp's K rows of a 64-key pass: keys kbase + g and + 8
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int key = kbase + g + 8 * r;
@@ -136,23 +149,24 @@ __global__ void __launch_bounds__(kAttnThreads, 5) kv_append_attn_kernel(const A
         kf[r][pp] = key < n_load ? __ldcg(reinterpret_cast<const uint4 *>(gK + (size_t)key * H + pp * 32 + tig * 8)) : make_uint4(0, 0, 0, 0);
     }
   };
-  load_k(warp * 16);
-  const int row_elems = (p.n_head + 2 * p.n_kv) * H;
-  const __half *qrow = p.qkv + (size_t)b * row_elems;
-  // ---- V page -> shared memory as asynchronous 16-byte copies (no registers, in flight together with the K loads above)
-  const __half *vnew = qrow + (size_t)(p.n_head + p.n_kv + kvh) * H;
-  for (int e = tid; e < KP * (H / 8); e += kAttnThreads) {
-    const int r = e / (H / 8), c8 = e - r * (H / 8);
-    __half *dst = Vs + (size_t)r * VLD + c8 * 8;
-    if (r < n_load) {
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(gV + (size_t)r * H + c8 * 8) : "memory");
-    } else {   // rows beyond the valid tokens multiply weights of zero: keep them finite; the new token's row comes from qkv
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (owner && r == slot) v = *reinterpret_cast<const uint4 *>(vnew + c8 * 8);
-      *reinterpret_cast<uint4 *>(dst) = v;
+  // V page -> shared memory as asynchronous 16-byte copies (no registers, in flight together with the K loads)
+  auto load_v = [&](__half *Vs, bool last) {
+    for (int e = tid; e < KP * (H / 8); e += kAttnThreads) {
+      const int r = e / (H / 8), c8 = e - r * (H / 8);
+      __half *dst = Vs + (size_t)r * VLD + c8 * 8;
+      if (r < n_load) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(gV + (size_t)r * H + c8 * 8) : "memory");
+      } else {   // rows beyond the valid tokens multiply weights of zero: keep them finite; the new token's row comes from qkv
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (last && r == slot) v = *reinterpret_cast<const uint4 *>(vnew + c8 * 8);
+        *reinterpret_cast<uint4 *>(dst) = v;
+      }
     }
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  page_at(pg0);
+  load_k(warp * 16);   // the first page's loads go out before anything else
+  load_v(Vs0, pg0 == n_pages - 1);
 
   // ---- RoPE on the block's q heads (and on the new k)
   const __half *sin_r = p.sin_t + (size_t)step * p.rot_half;
@@ -165,77 +179,90 @@ __global__ void __launch_bounds__(kAttnThreads, 5) kv_append_attn_kernel(const A
     const int qh = i / (H / 2), j = i - qh * (H / 2);
     rope_pair(p, qrow + (size_t)(kvh * p.qpk + q_lo + qh) * H, sin_r, cos_r, j, qs + (size_t)qh * QLD);
   }
-  if (owner) {
+  if (has_last) {
     const __half *knew = qrow + (size_t)(p.n_head + kvh) * H;
     for (int j = tid; j < H / 2; j += kAttnThreads) rope_pair(p, knew, sin_r, cos_r, j, newk);
   }
   for (int i = tid; i < NQ_MAX * PSLD; i += kAttnThreads) ps[i] = 0.f;   // weights of padded keys and unused heads
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();
-  if (owner && qpart == 0) {   // one block of the group appends to the pool
-    for (int j = tid; j < H; j += kAttnThreads) {
-      gK[(size_t)slot * H + j] = newk[j];
-      gV[(size_t)slot * H + j] = Vs[(size_t)slot * VLD + j];
-    }
-  }
 
-  // ---- scores: keys 16 warp .. + 15 of every 64-key pass against the block's heads
-  for (int kbase = warp * 16; kbase < n_valid; kbase += 64) {
-    if (kbase != warp * 16) load_k(kbase);
-    if (owner) {   // the new token's key row comes from shared memory
+  const size_t head0 = (size_t)b * p.n_head + (size_t)kvh * p.qpk + q_lo;
+  constexpr int NT = H / 32;                   // 8-channel tiles per warp: warp w owns channels [w H/4, (w + 1) H/4)
+  float O[NT][2], M = -INFINITY, L = 0.f;      // head g of the block: outputs of this warp's channels, running maximum and sum
 #pragma unroll
-      for (int r = 0; r < 2; ++r)
-        if (kbase + g + 8 * r == slot) {
-#pragma unroll
-          for (int pp = 0; pp < H / 32; ++pp) kf[r][pp] = *reinterpret_cast<const uint4 *>(newk + pp * 32 + tig * 8);
-        }
-    }
-    float sc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int pp = 0; pp < H / 32; ++pp) {
-      const uint4 qv = *reinterpret_cast<const uint4 *>(qs + (size_t)g * QLD + pp * 32 + tig * 8);
-      mma_f16(sc, kf[0][pp].x, kf[1][pp].x, kf[0][pp].y, kf[1][pp].y, qv.x, qv.y);
-      mma_f16(sc, kf[0][pp].z, kf[1][pp].z, kf[0][pp].w, kf[1][pp].w, qv.z, qv.w);
-    }
-    // lane (g, tig): keys kbase + g (sc[0], sc[1]) and kbase + g + 8 (sc[2], sc[3]) against heads 2 tig and 2 tig + 1
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int key = kbase + g + 8 * (e >> 1), qh = 2 * tig + (e & 1);
-      if (key < n_valid && qh < nq) {
-        __half s16 = __float2half_rn(sc[e]);           // fp16 matmul output
-        if (p.use_scale) s16 = h_mul(s16, p.scale_h);  // ops.mul by fp16(1/sqrt(H))
-        ps[(size_t)qh * PSLD + key] = __half2float(s16);
+  for (int j = 0; j < NT; ++j) O[j][0] = O[j][1] = 0.f;
+  for (int pg = pg0; pg < pg1; ++pg) {
+    __half *Vs = Vs0 + (size_t)((pg - pg0) & 1) * KP * VLD;
+    const bool owner = pg == n_pages - 1;
+    const int n_valid = owner ? slot + 1 : PAGE;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();             // V and (first page) q are there; the weights of the page before have been used
+    if (owner && qpart == 0) {   // one block of the group appends to the pool
+      for (int j = tid; j < H; j += kAttnThreads) {
+        gK[(size_t)slot * H + j] = newk[j];
+        gV[(size_t)slot * H + j] = Vs[(size_t)slot * VLD + j];
       }
     }
-  }
-  __syncthreads();
+    if (pg + 1 < pg1) phys = p.page_table[(size_t)b * p.max_pages + pg + 1];
 
-  // ---- per-head softmax statistics (one warp per q head, warp-shuffle reductions)
-  for (int qh = warp; qh < nq; qh += kAttnThreads / 32) {
-    float *pr = ps + (size_t)qh * PSLD;
-    float m = -INFINITY;
-    if (p.softmax_mode == PT_SOFTMAX_F32) {
-      for (int t = lane; t < n_valid; t += 32) m = fmaxf(m, pr[t]);
-      m = warp_max(m);
-    } else {
-      m = 0.f;  // the reference exponentiates fp16 scores without subtracting the maximum
+    // ---- scores: keys 16 warp .. + 15 of every 64-key pass against the block's heads
+    for (int kbase = warp * 16; kbase < n_valid; kbase += 64) {
+      if (kbase != warp * 16) load_k(kbase);
+      if (owner) {   // the new token's key row comes from shared memory
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          if (kbase + g + 8 * r == slot) {
+#pragma unroll
+            for (int pp = 0; pp < H / 32; ++pp) kf[r][pp] = *reinterpret_cast<const uint4 *>(newk + pp * 32 + tig * 8);
+          }
+      }
+      float sc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int pp = 0; pp < H / 32; ++pp) {
+        const uint4 qv = *reinterpret_cast<const uint4 *>(qs + (size_t)g * QLD + pp * 32 + tig * 8);
+        mma_f16(sc, kf[0][pp].x, kf[1][pp].x, kf[0][pp].y, kf[1][pp].y, qv.x, qv.y);
+        mma_f16(sc, kf[0][pp].z, kf[1][pp].z, kf[0][pp].w, kf[1][pp].w, qv.z, qv.w);
+      }
+      // lane (g, tig): keys kbase + g (sc[0], sc[1]) and kbase + g + 8 (sc[2], sc[3]) against heads 2 tig and 2 tig + 1
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int key = kbase + g + 8 * (e >> 1), qh = 2 * tig + (e & 1);
+        if (key < KP && qh < nq) {
+          __half s16 = __float2half_rn(sc[e]);           // fp16 matmul output
+          if (p.use_scale) s16 = h_mul(s16, p.scale_h);  // ops.mul by fp16(1/sqrt(H))
+          ps[(size_t)qh * PSLD + key] = key < n_valid ? __half2float(s16) : 0.f;   // (no weight behind the newest key)
+        }
+      }
     }
-    float l = 0.f;
-    for (int t = lane; t < n_valid; t += 32) {
-      float e = expf(pr[t] - m);
-      if (p.softmax_mode == PT_SOFTMAX_F16) e = __half2float(__float2half_rn(e));
-      pr[t] = e;
-      l += e;
+    if (pg + 1 < pg1) {   // (the other buffer was last read before the barrier above)
+      page_at(pg + 1);
+      load_k(warp * 16);
+      load_v(Vs0 + (size_t)((pg + 1 - pg0) & 1) * KP * VLD, pg + 1 == n_pages - 1);
     }
-    l = warp_sum(l);
-    if (lane == 0) { ml[2 * qh] = m; ml[2 * qh + 1] = l; }
-  }
-  __syncthreads();
+    __syncthreads();
 
-  // ---- P.V: warp w owns channels [w H/4, (w + 1) H/4); rows of the A operand = heads (8 .. 15 are zero)
-  const size_t head0 = (size_t)b * p.n_head + (size_t)kvh * p.qpk + q_lo;
-  {
-    constexpr int NT = H / 32;                 // 8-channel tiles per warp
+    // ---- per-head softmax statistics of the page (one warp per q head, warp-shuffle reductions)
+    for (int qh = warp; qh < nq; qh += kAttnThreads / 32) {
+      float *pr = ps + (size_t)qh * PSLD;
+      float m = -INFINITY;
+      if (p.softmax_mode == PT_SOFTMAX_F32) {
+        for (int t = lane; t < n_valid; t += 32) m = fmaxf(m, pr[t]);
+        m = warp_max(m);
+      } else {
+        m = 0.f;  // the reference exponentiates fp16 scores without subtracting the maximum
+      }
+      float l = 0.f;
+      for (int t = lane; t < n_valid; t += 32) {
+        float e = expf(pr[t] - m);
+        if (p.softmax_mode == PT_SOFTMAX_F16) e = __half2float(__float2half_rn(e));
+        pr[t] = e;
+        l += e;
+      }
+      l = warp_sum(l);
+      if (lane == 0) { ml[2 * qh] = m; ml[2 * qh + 1] = l; }
+    }
+    __syncthreads();
+
+    // ---- P.V: rows of the A operand = heads (8 .. 15 are zero)
     float o[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
@@ -254,15 +281,43 @@ __global__ void __launch_bounds__(kAttnThreads, 5) kv_append_attn_kernel(const A
         if (j + 1 < NT) mma_f16(o[j + 1], a0, 0u, a2, 0u, b2, b3);
       }
     }
+    // ---- the page joins the run
     if (g < nq) {
+      const float m = ml[2 * g], top = fmaxf(M, m), was = M == top ? 1.f : expf(M - top), is = m == top ? 1.f : expf(m - top);
+      M = top;
+      L = L * was + ml[2 * g + 1] * is;
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
-        *reinterpret_cast<float2 *>(&p.ws_o[((head0 + g) * p.max_pages + pg) * H + warp * (H / 4) + j * 8 + 2 * tig]) = make_float2(o[j][0], o[j][1]);
+      for (int j = 0; j < NT; ++j) {
+        O[j][0] = O[j][0] * was + o[j][0] * is;
+        O[j][1] = O[j][1] * was + o[j][1] * is;
+      }
     }
   }
-  if (tid < nq) p.ws_ml[(head0 + tid) * p.max_pages + pg] = make_float2(ml[2 * tid], ml[2 * tid + 1]);
+  const int run = blockIdx.x;
+  if (n_active == 1) {   // the whole history: the output
+    if (g < nq) {
+      const size_t col = ((size_t)kvh * p.qpk + q_lo + g) * H + warp * (H / 4) + 2 * tig;
+      __half *dst = p.out + (size_t)b * p.out_ld + col;
+      uint8_t *dst8 = p.out8 ? p.out8 + (size_t)b * p.n_head * H + col : nullptr;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const __half y = __float2half_rn(O[j][e] / L);
+          dst[j * 8 + e] = y;
+          if (dst8) dst8[j * 8 + e] = (uint8_t)__nv_cvt_float_to_fp8(__half2float(y) * p.inv_out_scale, __NV_SATFINITE, __NV_E4M3);
+        }
+    }
+    return;
+  }
+  if (g < nq) {
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+      *reinterpret_cast<float2 *>(&p.ws_o[((head0 + g) * p.max_pages + run) * H + warp * (H / 4) + j * 8 + 2 * tig]) = make_float2(O[j][0], O[j][1]);
+    if (warp == 0 && tig == 0) p.ws_ml[(head0 + g) * p.max_pages + run] = make_float2(M, L);
+  }
 
-  // ---- last block to arrive for this (sequence, kv-head) combines the pages in page order
+  // ---- last block to arrive for this (sequence, kv-head) combines the runs in order
   __threadfence();
   __syncthreads();
   int *ctr = p.counters + ((size_t)b * p.n_kv + kvh) * p.qsplit + qpart;
@@ -274,7 +329,7 @@ __global__ void __launch_bounds__(kAttnThreads, 5) kv_append_attn_kernel(const A
   // The V tile is no longer needed: its shared memory takes the pages' (max, sum) pairs, then their weights.  All loads of a
   // stage are issued before the first is used, so the combine costs a handful of L2 round trips whatever the number of pages
   // and heads (a loop of dependent-looking loads per head and page made it the longest part of the kernel at 17 pages).
-  float *cw = reinterpret_cast<float *>(Vs);           // [nq][n_active] weights exp(m_i - M)
+  float *cw = reinterpret_cast<float *>(Vs0);          // [nq][n_active] weights exp(m_i - M)
   float *cl = cw + (size_t)nq * n_active;              // [nq][n_active] page sums, then cl[qh * n_active] = L of the head
   // (worth its two extra barriers from about sixteen (head, page) pairs on: measured 1 % slower than the plain loop at 1 head x 6 pages)
   const bool staged = nq * n_active >= 16 && (size_t)2 * nq * n_active * sizeof(float) <= (size_t)KP * VLD * sizeof(__half);
@@ -421,6 +476,13 @@ extern "C" size_t pt_attn_workspace_bytes(int batch, int n_head, int head_dim, i
   return align256(heads * sizeof(int)) + align256(heads * max_pages * sizeof(float2)) + heads * max_pages * head_dim * sizeof(float);
 }
 
+// Pages of one block: as many as leave four blocks per SM if the whole table is in use (what the shared memory and registers of a block of
+// two V buffers admit at a time).  Measured on B200 as whole steps, one page per block and this: Llama 7B, 512 (row, kv head) pairs of 8 pages 3.58
+// and 3.38 ms, 1024 of 4 pages 3.73 and 3.52, GPT-2 XL, 400 of 4 pages 2.63 and 2.52, ChatGLM2, 64 of 18 pages level at 3.47.
+static int pages_per_block(int units, int max_pages) {
+  return std::max(1, std::min(max_pages, (int)((long long)units * max_pages / (4 * sm_count()))));
+}
+
 extern "C" int pt_kv_append_attn(const pt_attn_args *a, void *stream) {
   PT_REQUIRE(a, "pt_kv_append_attn: null args");
   PT_REQUIRE(a->batch > 0 && a->n_head > 0 && a->n_kv > 0 && a->n_head % a->n_kv == 0,
@@ -466,14 +528,13 @@ extern "C" int pt_kv_append_attn(const pt_attn_args *a, void *stream) {
              a->max_len, a->page_size * a->max_pages);
   p.max_len = a->max_len > 0 ? a->max_len : a->page_size * a->max_pages;
 
-  const int nq = p.qpk / p.qsplit;
-  (void)nq;
+  p.ppb = pages_per_block(a->batch * a->n_kv * p.qsplit, a->max_pages);
   const int kp = (p.page + 15) & ~15;
-  const size_t smem = ((size_t)kp * (p.H + 8) + (size_t)NQ_MAX * (p.H + 32) + p.H) * sizeof(__half) +
+  const size_t smem = ((size_t)(p.ppb > 1 ? 2 : 1) * kp * (p.H + 8) + (size_t)NQ_MAX * (p.H + 32) + p.H) * sizeof(__half) +
                       ((size_t)NQ_MAX * (kp + 8) + (size_t)NQ_MAX * 2) * sizeof(float);
   PT_REQUIRE(smem <= 200 * 1024, "pt_kv_append_attn: tile needs %zu bytes of shared memory", smem);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(a->max_pages, a->n_kv * p.qsplit, a->batch);
+  cfg.gridDim = dim3(ceil_div(a->max_pages, p.ppb), a->n_kv * p.qsplit, a->batch);
   cfg.blockDim = dim3(kAttnThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = as_stream(stream);
