@@ -146,7 +146,7 @@ class ChatGLM2Decoder(DecodeLoop):
                 ops.check(ops._lib.lib().pt_rms_norm(ops._ptr(x), None, ops._ptr(gamma), self.batch, self.cfg.d_model, self.cfg.eps, ops._ptr(self.h), None,
                                                      ops._stream()), "pt_rms_norm")
                 x = self.h
-            ops.gemm(x, pl, out=out, epilogue=epilogue, bias=bias, residual=residual, error_flag=self.error_flag)
+            ops.gemm(x, pl, out=out, epilogue=epilogue, bias=bias, residual=residual, error_flag=self.error_flag, pdl=1)
             return
         fp8 = pl.wfmt == ops.W_FP8
         pro = (ops.PRO_RMSNORM_CAST_FP8 if fp8 else ops.PRO_RMSNORM) if gamma is not None else (ops.PRO_CAST_FP8 if fp8 else ops.PRO_NONE)
@@ -176,14 +176,14 @@ class ChatGLM2Decoder(DecodeLoop):
             return self.x8.view(-1)[:B * d].view(B, d)
 
         def gemm(x8, pl, out, **kw):
-            ops.gemm(x8, pl, out=out, x_scale=pl.act_scale, workspace=self.gemm_ws, error_flag=self.error_flag, **kw)
+            ops.gemm(x8, pl, out=out, x_scale=pl.act_scale, workspace=self.gemm_ws, error_flag=self.error_flag, pdl=1, **kw)
 
         ops.embedding(self.emb, self.ids, self.step_t, out=self.x)
         for li, L in enumerate(self.layers):
             gemm(norm_cast(L["ln1"], L["qkv"]), L["qkv"], self.qkv, epilogue=ops.EPI_BIAS, bias=L["b_qkv"])
             a8 = self.x8.view(-1)[:B * self.d_loc].view(B, self.d_loc)      # the attention kernel writes dense's E4M3 input itself
             a = ops.attn_args(self.qkv, self.step_t, self.caches[li], self.attn, self.h_loc, ops.ROPE_CHATGLM2, ops.SOFTMAX_F16, self.score_scale,
-                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=self.pdl_attn, out_fp8=a8, out_fp8_scale=L["dense"].act_scale)
+                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=self.pdl_attn or isinstance(L["dense"], ops.GemmWeight), out_fp8=a8, out_fp8_scale=L["dense"].act_scale)
             ops.check(L_.pt_kv_append_attn(ctypes.byref(a), st()), "pt_kv_append_attn")
             gemm(a8, L["dense"], self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x)
             gemm(norm_cast(L["ln2"], L["gu"]), L["gu"], self.gu_out)
@@ -202,7 +202,7 @@ class ChatGLM2Decoder(DecodeLoop):
         for li, L in enumerate(self.layers):
             self._linear(self.x, L["qkv"], self.qkv, "norm", gamma=L["ln1"], epilogue=ops.EPI_BIAS, bias=L["b_qkv"])
             a = ops.attn_args(self.qkv, self.step_t, self.caches[li], self.attn, self.h_loc, ops.ROPE_CHATGLM2, ops.SOFTMAX_F16, self.score_scale,
-                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=self.pdl_attn)
+                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=self.pdl_attn or isinstance(L["dense"], ops.GemmWeight))
             ops.check(L_.pt_kv_append_attn(ctypes.byref(a), ops._stream()), "pt_kv_append_attn")
             self._row_parallel(self.attn, L["dense"], "attn")
             self._linear(self.x, L["gu"], self.act, "norm", gamma=L["ln2"], epilogue=ops.EPI_SWIGLU)

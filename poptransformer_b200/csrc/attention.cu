@@ -111,11 +111,7 @@ __global__ void __launch_bounds__(kAttnThreads, 4) kv_append_attn_kernel(const A
   // re-reads the group's K/V page (through L2) and handles nq of the group's heads.
   const int pg0 = blockIdx.x * p.ppb, kvh = blockIdx.y / p.qsplit, qpart = blockIdx.y - kvh * p.qsplit, b = blockIdx.z;
   const int nq = p.qpk / p.qsplit, q_lo = qpart * nq;   // this block's heads of the group: q_lo .. q_lo + nq - 1
-  if (p.pdl) {
-    // let the next kernel start prefetching its weights; everything this kernel reads was produced upstream
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-  }
+  early_start();   // (the next kernel may fetch its weights meanwhile; everything this one reads was produced upstream)
   // the page-table entry does not depend on the step: both loads go out together (one round trip less before the K / V loads)
   int phys = p.page_table[(size_t)b * p.max_pages + pg0];
   const int step = *p.step;

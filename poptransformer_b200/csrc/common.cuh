@@ -45,6 +45,28 @@ static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// A launch whose blocks may become resident while the kernel before it in the stream still runs (if that one lets them: launch_dependents).  For
+// kernels that begin with early_start(): the launch and the start of the blocks then overlap with the kernel before.  Measured on
+// B200 in a graph: about 1.3 us a launch.
+__device__ __forceinline__ void early_start() {
+  launch_dependents();
+  wait_for_prerequisites();
+}
+template <typename... P, typename... A>
+static inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- fp16 arithmetic with the reference's "one rounding per op" semantics -------------
 __device__ __forceinline__ __half h_mul(__half a, __half b) { return __hmul_rn(a, b); }
 __device__ __forceinline__ __half h_add(__half a, __half b) { return __hadd_rn(a, b); }

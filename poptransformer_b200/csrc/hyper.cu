@@ -44,6 +44,7 @@ template <int VEC> __device__ __forceinline__ void st(float *p, const Vec<VEC> &
 
 // S > 0: that many streams, unrolled.  S == 0: p.streams (at most kMaxStreams).
 template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params p) {
+  early_start();
   constexpr int SM = S > 0 ? S : kMaxStreams;
   extern __shared__ __align__(16) float u_row[];   // [width]
   __shared__ float c_mix[SM * SM], c_out[SM], c_in[SM], red[32];
@@ -131,7 +132,7 @@ template <typename T, int S, int VEC> static int launch(const Params &p, cudaStr
   }
   const int want = ceil_div(ceil_div(p.width, VEC), 32) * 32, cap = p.rows <= 2 * sm_count() ? 1024 : 256;
   const int regs_cap = S == 0 ? 256 : 1024;
-  hyper_kernel<T, S, VEC><<<p.rows, std::min(std::min(want, cap), regs_cap), smem, st>>>(p);
+  launch_early(hyper_kernel<T, S, VEC>, p.rows, std::min(std::min(want, cap), regs_cap), smem, st, p);
   PT_LAUNCH_CHECK("pt_hyper");
   return PT_OK;
 }

@@ -50,6 +50,7 @@ __global__ void int4_to_half_axis0_kernel(const int8_t *__restrict__ w, const __
 // normInfKernel's (fp16-rounded mean inside the variance, clamp at 0, 1/sqrt).
 __global__ void norm_ce_kernel(const __half *__restrict__ x, const __half *__restrict__ gamma, const __half *__restrict__ beta,
                                int dim, float eps, int single_row, __half *__restrict__ out) {
+  early_start();
   __shared__ float red[32];
   const __half *xr = x + (size_t)blockIdx.x * dim;
   float s = 0.f, sq = 0.f;
@@ -83,6 +84,7 @@ __global__ void norm_ce_kernel(const __half *__restrict__ x, const __half *__res
 // units instead of single elements.
 __global__ void norm_ce_vec_kernel(const __half *__restrict__ x, const __half *__restrict__ gamma, const __half *__restrict__ beta,
                                    int dim, float eps, int single_row, __half *__restrict__ out) {
+  early_start();
   __shared__ float red[32];
   const size_t base = (size_t)blockIdx.x * dim;
   const int units = dim / 8;
@@ -137,6 +139,7 @@ __global__ void norm_ce_vec_kernel(const __half *__restrict__ x, const __half *_
 // at most 8 * 8 * 256).  The scalar two-pass kernel below took 15 us for 16 rows of 4096, all of it load latency.
 __global__ void rms_norm_vec_kernel(const __half *__restrict__ x, const __half *__restrict__ residual, const __half *__restrict__ gamma,
                                     int dim, float eps, __half *__restrict__ out, __half *__restrict__ sum_out) {
+  early_start();
   __shared__ float red[32];
   const size_t base = (size_t)blockIdx.x * dim;
   const int units = dim / 8;
@@ -182,6 +185,7 @@ __global__ void rms_norm_vec_kernel(const __half *__restrict__ x, const __half *
 
 __global__ void rms_norm_kernel(const __half *__restrict__ x, const __half *__restrict__ residual, const __half *__restrict__ gamma,
                                 int dim, float eps, __half *__restrict__ out, __half *__restrict__ sum_out) {
+  early_start();
   __shared__ float red[32];
   const size_t base = (size_t)blockIdx.x * dim;
   float sq = 0.f;
@@ -529,6 +533,7 @@ __global__ void copy_i32_kernel(const int *__restrict__ src, int *__restrict__ d
 
 // ------------------------------------------------------------------------------------------ FP8
 __global__ void cast_fp8_kernel(const __half *__restrict__ x, float inv_scale, size_t n, uint8_t *__restrict__ out) {
+  early_start();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = __nv_cvt_float_to_fp8(__half2float(x[i]) * inv_scale, __NV_SATFINITE, __NV_E4M3);
 }
@@ -575,6 +580,7 @@ __global__ void fp8_matmul_kernel(const uint8_t *__restrict__ a, const uint8_t *
 __global__ void wkv_kernel(const __half *__restrict__ k, const __half *__restrict__ v, const float *__restrict__ tf,
                            const float *__restrict__ td, float *__restrict__ num, float *__restrict__ den, float *__restrict__ mx,
                            int b, int c, __half *__restrict__ out) {
+  early_start();
   const size_t total = (size_t)b * c;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int ch = i % c;
@@ -599,6 +605,7 @@ __global__ void wkv_kernel(const __half *__restrict__ k, const __half *__restric
 __global__ void rwkv_mix_kernel(const __half *__restrict__ hidden, __half *__restrict__ state, const __half *__restrict__ wa,
                                 const __half *__restrict__ wb, const __half *__restrict__ wc, __half *__restrict__ oa, __half *__restrict__ ob,
                                 __half *__restrict__ oc, int rows, int dim) {
+  early_start();
   const size_t total = (size_t)rows * dim;
   const __half one = __float2half_rn(1.0f);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -614,6 +621,7 @@ __global__ void rwkv_mix_kernel(const __half *__restrict__ hidden, __half *__res
 //                          1: out = relu(a)^2              (ffn.py:53-54)
 //                          2: out = a / 2                  (rescale_every, rwkv/model.py:115-116)
 __global__ void rwkv_act_kernel(int mode, const __half *__restrict__ a, const __half *__restrict__ b, __half *__restrict__ out, size_t n) {
+  early_start();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const __half x = a[i];
     if (mode == 0) {
@@ -631,6 +639,7 @@ __global__ void rwkv_act_kernel(int mode, const __half *__restrict__ a, const __
 // ------------------------------------------------------------------------------------------ loop carry
 __global__ void embedding_kernel(const uint4 *__restrict__ table, const int *__restrict__ ids, int ids_stride, const int *step_dev,
                                  int dim8, int vocab, uint4 *__restrict__ out) {
+  early_start();
   const int b = blockIdx.x;
   const int step = step_dev ? min(max(*step_dev, 0), ids_stride - 1) : 0;  // a step past the container reads its last column
   int id = ids[(size_t)b * ids_stride + step];
@@ -639,6 +648,7 @@ __global__ void embedding_kernel(const uint4 *__restrict__ table, const int *__r
 }
 __global__ void step_containers_kernel(int *ids, int batch, int max_len, int *step_dev, const int *next_ids, int pad_id, int eos_id,
                                        int *stop_mask, int *done_flag) {
+  early_start();
   __shared__ int s_running;
   if (done_flag) {
     if (*done_flag) return;   // uniform: every thread reads the same word
@@ -665,11 +675,13 @@ __global__ void step_containers_kernel(int *ids, int batch, int max_len, int *st
   }
 }
 __global__ void add_f16_kernel(const __half *__restrict__ a, const __half *__restrict__ b, size_t n, __half *__restrict__ out) {
+  early_start();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) out[i] = h_add(a[i], b[i]);
 }
 
 // SwiGLU on the output of a fused gate|up linear whose rows are [gate features | up features]: out = fp16(up * swish(gate)).
 __global__ void swiglu_kernel(const __half *__restrict__ gu, int rows, int f, __half *__restrict__ out, int out_ld) {
+  early_start();
   const size_t total = (size_t)rows * f;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t b = i / f, j = i - b * f;
@@ -681,6 +693,7 @@ __global__ void swiglu_kernel(const __half *__restrict__ gu, int rows, int f, __
 // into registers (dim <= 8 * 8 * 256), bytes out.
 __global__ void rms_norm_fp8_kernel(const __half *__restrict__ x, const __half *__restrict__ gamma, int dim, float eps, float inv_scale,
                                     uint8_t *__restrict__ out) {
+  early_start();
   __shared__ float red[32];
   const size_t base = (size_t)blockIdx.x * dim;
   const int units = dim / 8;
@@ -720,6 +733,7 @@ __global__ void rms_norm_fp8_kernel(const __half *__restrict__ x, const __half *
 }
 // SwiGLU of [gate features | up features] rows, cast to E4M3 for the FP8 linear that follows.
 __global__ void swiglu_fp8_kernel(const __half *__restrict__ gu, int rows, int f, float inv_scale, uint8_t *__restrict__ out, int out_ld) {
+  early_start();
   const size_t total = (size_t)rows * f;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t b = i / f, j = i - b * f;
@@ -761,10 +775,10 @@ extern "C" int pt_norm_ce(const void *x, const void *gamma, const void *beta, in
   PT_REQUIRE((dim & 3) == 0, "our normCEOp require 4x a last dim, and current is: %d", dim);
   PT_REQUIRE(dim < 8192, "normalize_ce, last_dim_size should be <= 8192, and current is: %d", dim);
   if (dim % 8 == 0 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0)
-    norm_ce_vec_kernel<<<rows, 256, 0, as_stream(stream)>>>((const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
+    launch_early(norm_ce_vec_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
                                                            rows == 1 ? 1 : 0, (__half *)out);
   else
-    norm_ce_kernel<<<rows, 256, 0, as_stream(stream)>>>((const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
+    launch_early(norm_ce_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
                                                        rows == 1 ? 1 : 0, (__half *)out);
   PT_LAUNCH_CHECK("pt_norm_ce");
   return PT_OK;
@@ -777,10 +791,10 @@ extern "C" int pt_rms_norm(const void *x, const void *residual, const void *gamm
   PT_REQUIRE(!residual || sum_out, "pt_rms_norm: residual given without sum_out");
   const bool vec = dim % 8 == 0 && dim <= 8 * 8 * 256 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)residual | (uintptr_t)sum_out) & 15) == 0;
   if (vec)
-    rms_norm_vec_kernel<<<rows, 256, 0, as_stream(stream)>>>((const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
+    launch_early(rms_norm_vec_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
                                                             (__half *)out, (__half *)sum_out);
   else
-    rms_norm_kernel<<<rows, 256, 0, as_stream(stream)>>>((const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
+    launch_early(rms_norm_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
                                                         (__half *)out, (__half *)sum_out);
   PT_LAUNCH_CHECK("pt_rms_norm");
   return PT_OK;
@@ -919,7 +933,7 @@ extern "C" int pt_beam_search(const void *logits, int32_t *hyp, void *prob, cons
 extern "C" int pt_cast_fp8(const void *x, float scale, int64_t n, void *out, void *stream) {
   PT_REQUIRE(x && out && n > 0, "pt_cast_fp8: bad arguments");
   PT_REQUIRE(scale > 0.f, "pt_cast_fp8: scale must be > 0");
-  cast_fp8_kernel<<<grid_for((size_t)n), 256, 0, as_stream(stream)>>>((const __half *)x, 1.0f / scale, (size_t)n, (uint8_t *)out);
+  launch_early(cast_fp8_kernel, grid_for((size_t)n), 256, 0, as_stream(stream), (const __half *)x, 1.0f / scale, (size_t)n, (uint8_t *)out);
   PT_LAUNCH_CHECK("pt_cast_fp8");
   return PT_OK;
 }
@@ -945,7 +959,7 @@ extern "C" int pt_wkv(const void *k, const void *v, const float *time_first, con
                       float *max_state, int b, int c, void *out, void *stream) {
   PT_REQUIRE(k && v && time_first && time_decay && num && den && max_state && out, "pt_wkv: null pointer argument");
   PT_REQUIRE(b > 0 && c > 0, "pt_wkv: bad shape [%d, %d]", b, c);
-  wkv_kernel<<<grid_for((size_t)b * c), 256, 0, as_stream(stream)>>>((const __half *)k, (const __half *)v, time_first, time_decay, num, den,
+  launch_early(wkv_kernel, grid_for((size_t)b * c), 256, 0, as_stream(stream), (const __half *)k, (const __half *)v, time_first, time_decay, num, den,
                                                                      max_state, b, c, (__half *)out);
   PT_LAUNCH_CHECK("pt_wkv");
   return PT_OK;
@@ -955,7 +969,7 @@ extern "C" int pt_rwkv_mix(const void *hidden, void *state, const void *mix_a, c
                            void *out_c, int rows, int dim, void *stream) {
   PT_REQUIRE(hidden && state && mix_a && out_a && (!out_b || mix_b) && (!out_c || mix_c), "pt_rwkv_mix: null pointer argument");
   PT_REQUIRE(rows > 0 && dim > 0, "pt_rwkv_mix: bad shape [%d, %d]", rows, dim);
-  rwkv_mix_kernel<<<grid_for((size_t)rows * dim), 256, 0, as_stream(stream)>>>((const __half *)hidden, (__half *)state, (const __half *)mix_a,
+  launch_early(rwkv_mix_kernel, grid_for((size_t)rows * dim), 256, 0, as_stream(stream), (const __half *)hidden, (__half *)state, (const __half *)mix_a,
                                                                               (const __half *)mix_b, (const __half *)mix_c, (__half *)out_a,
                                                                               (__half *)out_b, (__half *)out_c, rows, dim);
   PT_LAUNCH_CHECK("pt_rwkv_mix");
@@ -964,7 +978,7 @@ extern "C" int pt_rwkv_mix(const void *hidden, void *state, const void *mix_a, c
 
 extern "C" int pt_rwkv_act(int mode, const void *a, const void *b, void *out, int64_t n, void *stream) {
   PT_REQUIRE(a && out && n > 0 && mode >= 0 && mode <= 2 && (mode != 0 || b), "pt_rwkv_act: bad arguments (mode %d)", mode);
-  rwkv_act_kernel<<<grid_for((size_t)n), 256, 0, as_stream(stream)>>>(mode, (const __half *)a, (const __half *)b, (__half *)out, (size_t)n);
+  launch_early(rwkv_act_kernel, grid_for((size_t)n), 256, 0, as_stream(stream), mode, (const __half *)a, (const __half *)b, (__half *)out, (size_t)n);
   PT_LAUNCH_CHECK("pt_rwkv_act");
   return PT_OK;
 }
@@ -973,7 +987,7 @@ extern "C" int pt_embedding(const void *table, const int32_t *ids, int ids_strid
                             void *out, void *stream) {
   PT_REQUIRE(table && ids && out, "pt_embedding: null pointer argument");
   PT_REQUIRE(batch > 0 && dim > 0 && dim % 8 == 0 && vocab > 0, "pt_embedding: bad shape batch=%d dim=%d (dim %% 8 == 0)", batch, dim);
-  embedding_kernel<<<batch, 128, 0, as_stream(stream)>>>((const uint4 *)table, ids, ids_stride, step_dev, dim / 8, vocab, (uint4 *)out);
+  launch_early(embedding_kernel, batch, 128, 0, as_stream(stream), (const uint4 *)table, ids, ids_stride, step_dev, dim / 8, vocab, (uint4 *)out);
   PT_LAUNCH_CHECK("pt_embedding");
   return PT_OK;
 }
@@ -982,7 +996,7 @@ extern "C" int pt_step_containers(int32_t *ids, int batch, int max_len, int32_t 
                                   int32_t *stop_mask, void *stream) {
   PT_REQUIRE(ids && step_dev && next_ids, "pt_step_containers: null pointer argument");
   PT_REQUIRE(batch > 0 && max_len > 0, "pt_step_containers: bad shape");
-  step_containers_kernel<<<1, 128, 0, as_stream(stream)>>>(ids, batch, max_len, step_dev, next_ids, pad_id, eos_id, stop_mask, nullptr);
+  launch_early(step_containers_kernel, 1, 128, 0, as_stream(stream), ids, batch, max_len, step_dev, next_ids, pad_id, eos_id, stop_mask, nullptr);
   PT_LAUNCH_CHECK("pt_step_containers");
   return PT_OK;
 }
@@ -991,14 +1005,14 @@ extern "C" int pt_step_containers_early_stop(int32_t *ids, int batch, int max_le
                                              int eos_id, int32_t *stop_mask, int32_t *done_flag, void *stream) {
   PT_REQUIRE(ids && step_dev && next_ids && stop_mask && done_flag, "pt_step_containers_early_stop: null pointer argument");
   PT_REQUIRE(batch > 0 && max_len > 0, "pt_step_containers_early_stop: bad shape");
-  step_containers_kernel<<<1, 128, 0, as_stream(stream)>>>(ids, batch, max_len, step_dev, next_ids, pad_id, eos_id, stop_mask, done_flag);
+  launch_early(step_containers_kernel, 1, 128, 0, as_stream(stream), ids, batch, max_len, step_dev, next_ids, pad_id, eos_id, stop_mask, done_flag);
   PT_LAUNCH_CHECK("pt_step_containers_early_stop");
   return PT_OK;
 }
 
 extern "C" int pt_swiglu(const void *gate_up, int rows, int f, void *out, int out_ld, void *stream) {
   PT_REQUIRE(gate_up && out && rows > 0 && f > 0, "pt_swiglu: bad arguments");
-  swiglu_kernel<<<grid_for((size_t)rows * f), 256, 0, as_stream(stream)>>>((const __half *)gate_up, rows, f, (__half *)out, out_ld > 0 ? out_ld : f);
+  launch_early(swiglu_kernel, grid_for((size_t)rows * f), 256, 0, as_stream(stream), (const __half *)gate_up, rows, f, (__half *)out, out_ld > 0 ? out_ld : f);
   PT_LAUNCH_CHECK("pt_swiglu");
   return PT_OK;
 }
@@ -1007,7 +1021,7 @@ extern "C" int pt_rms_norm_fp8(const void *x, const void *gamma, int rows, int d
   PT_REQUIRE(x && gamma && out, "pt_rms_norm_fp8: null pointer argument");
   PT_REQUIRE(rows > 0 && dim > 0 && dim % 8 == 0 && dim <= 8 * 8 * 256, "pt_rms_norm_fp8: bad shape [%d, %d] (dim a multiple of 8, at most 16384)", rows, dim);
   PT_REQUIRE(act_scale > 0.f, "pt_rms_norm_fp8: act_scale must be > 0");
-  rms_norm_fp8_kernel<<<rows, 256, 0, as_stream(stream)>>>((const __half *)x, (const __half *)gamma, dim, eps, 1.0f / act_scale, (uint8_t *)out);
+  launch_early(rms_norm_fp8_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, dim, eps, 1.0f / act_scale, (uint8_t *)out);
   PT_LAUNCH_CHECK("pt_rms_norm_fp8");
   return PT_OK;
 }
@@ -1015,7 +1029,7 @@ extern "C" int pt_rms_norm_fp8(const void *x, const void *gamma, int rows, int d
 extern "C" int pt_swiglu_fp8(const void *gate_up, int rows, int f, float act_scale, void *out, int out_ld, void *stream) {
   PT_REQUIRE(gate_up && out && rows > 0 && f > 0, "pt_swiglu_fp8: bad arguments");
   PT_REQUIRE(act_scale > 0.f, "pt_swiglu_fp8: act_scale must be > 0");
-  swiglu_fp8_kernel<<<grid_for((size_t)rows * f), 256, 0, as_stream(stream)>>>((const __half *)gate_up, rows, f, 1.0f / act_scale, (uint8_t *)out,
+  launch_early(swiglu_fp8_kernel, grid_for((size_t)rows * f), 256, 0, as_stream(stream), (const __half *)gate_up, rows, f, 1.0f / act_scale, (uint8_t *)out,
                                                                                  out_ld > 0 ? out_ld : f);
   PT_LAUNCH_CHECK("pt_swiglu_fp8");
   return PT_OK;
@@ -1023,7 +1037,7 @@ extern "C" int pt_swiglu_fp8(const void *gate_up, int rows, int f, float act_sca
 
 extern "C" int pt_add_f16(const void *a, const void *b, int64_t n, void *out, void *stream) {
   PT_REQUIRE(a && b && out && n > 0, "pt_add_f16: bad arguments");
-  add_f16_kernel<<<grid_for((size_t)n), 256, 0, as_stream(stream)>>>((const __half *)a, (const __half *)b, (size_t)n, (__half *)out);
+  launch_early(add_f16_kernel, grid_for((size_t)n), 256, 0, as_stream(stream), (const __half *)a, (const __half *)b, (size_t)n, (__half *)out);
   PT_LAUNCH_CHECK("pt_add_f16");
   return PT_OK;
 }

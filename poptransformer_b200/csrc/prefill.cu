@@ -32,6 +32,7 @@ struct Params {
 // have built over them: its step s marks a sequence whose id at position s + 1 is the eos id (models/base_model.py:313-346).
 __global__ void prefill_embed_kernel(const uint4 *__restrict__ table, const int *__restrict__ ids, int ids_stride, int n_tokens, int start, int dim8,
                                      int vocab, int eos_id, int *stop_mask, uint4 *__restrict__ out) {
+  early_start();
   const int row = blockIdx.x, b = row / n_tokens, t = row - b * n_tokens;
   int id = ids[(size_t)b * ids_stride + start + t];
   id = min(max(id, 0), vocab - 1);
@@ -40,6 +41,7 @@ __global__ void prefill_embed_kernel(const uint4 *__restrict__ table, const int 
 }
 
 __global__ void __launch_bounds__(64) prefill_rope_kv_kernel(const Params p) {
+  early_start();
   const int row = blockIdx.x, head = blockIdx.y, i = threadIdx.x;     // i: pair (i, i + 64)
   const int b = row / p.P, t = row - b * p.P, pos = p.start + t;
   const int dq = p.n_head * H;
@@ -73,6 +75,7 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
 // (running max / sum per query, fp32), the probabilities rounded to fp16 (the reference's softmax output is fp16) and used as
 // the A operand of O += P V (4 x 16 steps), fp32 accumulators.
 __global__ void __launch_bounds__(THREADS) prefill_attn_kernel(const Params p) {
+  early_start();
   __shared__ __align__(16) __half Ks[PAGE][KPAD];
   __shared__ __align__(16) __half Vs[PAGE][KPAD];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
@@ -199,7 +202,7 @@ extern "C" int pt_prefill_embed(const void *table, const int32_t *ids, int ids_s
   PT_REQUIRE(table && ids && out, "pt_prefill_embed: null pointer argument");
   PT_REQUIRE(batch > 0 && n_tokens > 0 && start >= 0 && start + n_tokens <= ids_stride && dim > 0 && dim % 8 == 0 && vocab > 0,
              "pt_prefill_embed: bad shape batch=%d n_tokens=%d start=%d ids_stride=%d dim=%d", batch, n_tokens, start, ids_stride, dim);
-  pf::prefill_embed_kernel<<<batch * n_tokens, 128, 0, as_stream(stream)>>>((const uint4 *)table, ids, ids_stride, n_tokens, start, dim / 8, vocab, eos_id,
+  launch_early(pf::prefill_embed_kernel, batch * n_tokens, 128, 0, as_stream(stream), (const uint4 *)table, ids, ids_stride, n_tokens, start, dim / 8, vocab, eos_id,
                                                                             stop_mask, (uint4 *)out);
   PT_LAUNCH_CHECK("pt_prefill_embed");
   return PT_OK;
@@ -219,9 +222,9 @@ extern "C" int pt_prefill_attn(const pt_prefill_attn_args *a, void *stream) {
   p.sin_t = (const __half *)a->rope_sin; p.cos_t = (const __half *)a->rope_cos;
   p.qkv = (__half *)a->qkv; p.pool = (__half *)a->pool; p.page_table = a->page_table; p.out = (__half *)a->out;
   p.scale_h = __float2half_rn(a->score_scale);
-  pf::prefill_rope_kv_kernel<<<dim3(a->batch * a->n_tokens, a->n_head), 64, 0, as_stream(stream)>>>(p);
+  launch_early(pf::prefill_rope_kv_kernel, dim3(a->batch * a->n_tokens, a->n_head), 64, 0, as_stream(stream), p);
   PT_LAUNCH_CHECK("pt_prefill_attn");
-  pf::prefill_attn_kernel<<<dim3(ceil_div(a->n_tokens, pf::BQ), a->n_head, a->batch), pf::THREADS, 0, as_stream(stream)>>>(p);
+  launch_early(pf::prefill_attn_kernel, dim3(ceil_div(a->n_tokens, pf::BQ), a->n_head, a->batch), pf::THREADS, 0, as_stream(stream), p);
   PT_LAUNCH_CHECK("pt_prefill_attn");
   return PT_OK;
 }

@@ -62,6 +62,7 @@ template <typename T> __global__ void ssm_conv_kernel(const Params p) {
 // window in registers; the last column of blocks computes the step sizes.
 constexpr int CONV_TOKENS = 16, CONV_THREADS = 128;
 template <int TAPS> __global__ void __launch_bounds__(CONV_THREADS) ssm_conv8_kernel(const Params p) {
+  early_start();
   typedef __nv_bfloat16 T;
   const T *zx = reinterpret_cast<const T *>(p.zx);
   const int ta = blockIdx.y * CONV_TOKENS, tb = min(p.n_tok, ta + CONV_TOKENS);
@@ -230,6 +231,7 @@ __device__ __forceinline__ void scan_decays(const Params &p, int row0, int valid
   if (lane == 0) d.keep = expf((float)last);
 }
 __global__ void ssm_decay_kernel(const Params p) {   // one warp per (chunk, head)
+  early_start();
   const int slot = blockIdx.y, h = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int s, t0;
   if (h >= p.heads || !chunk_of_slot(p.cu, p.n_seq, slot, s, t0)) return;
@@ -247,6 +249,7 @@ template <int NP, int CP> struct StateSmem {
 };
 // Block: one chunk, one head, CP columns.  The warps share the 16-row tiles of the state (and the columns when there are fewer tiles).
 template <int NP, int CP> __global__ void __launch_bounds__(CHUNK_THREADS) ssm_chunk_state_kernel(const Params p) {
+  early_start();
   typedef __nv_bfloat16 T;
   constexpr int XLD = CP + 8, MTILES = NP / 16, WPT = MTILES >= 8 ? 1 : 8 / MTILES;      // warps per row tile
   constexpr int MT = MTILES >= 8 ? MTILES / 8 : 1, NJ = CP / 8 / WPT;
@@ -324,6 +327,7 @@ template <int NP, int CP> __global__ void __launch_bounds__(CHUNK_THREADS) ssm_c
 // Thread: eight consecutive elements of one head's state, along the chunks of its sequence.  In place: sum of the chunk -> state
 // before the chunk, as eight bf16 hi parts and eight lo parts.
 __global__ void ssm_carry_kernel(const Params p) {
+  early_start();
   const int s = blockIdx.z, h = blockIdx.y, i = (blockIdx.x * blockDim.x + threadIdx.x) * 8, n = p.N * p.P;
   if (i >= n) return;
   const int chunks = (p.cu[s + 1] - p.cu[s] + CHUNK - 1) / CHUNK;
@@ -378,6 +382,7 @@ template <int NP, int CP> struct OutSmem {
 // Block: one chunk, one head, CP columns.  Two warps share 16 output rows, each with every other 16 state rows (first product) and
 // every other 16 tokens s (second product).
 template <int NP, int CP> __global__ void __launch_bounds__(CHUNK_THREADS) ssm_chunk_out_kernel(const Params p) {
+  early_start();
   typedef __nv_bfloat16 T;
   constexpr int XLD = CP + 8, BLD = NP + 8;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -510,6 +515,7 @@ constexpr int STEP_THREADS = 256;
 // Block: one sequence and one head.  Thread (n group, column quad) walks state rows n group, + n groups, ...; every state element is
 // read and written once, coalesced along the columns.
 template <typename T, int VEC> __global__ void __launch_bounds__(STEP_THREADS) ssm_step_kernel(const Params p) {
+  early_start();
   extern __shared__ __align__(16) float sm[];
   const int s = blockIdx.y, h = blockIdx.x, tid = threadIdx.x, g = h / (p.heads / p.groups);
   const int pos = p.start[s], slot = p.slot[s], t = p.cu[s];
@@ -582,6 +588,7 @@ template <typename T, int VEC> __global__ void __launch_bounds__(STEP_THREADS) s
 
 // ------------------------------------------------------------------------------------------ gate + group norm + ring
 template <typename T, int VEC> __global__ void ssm_norm_kernel(const Params p) {
+  early_start();
   extern __shared__ __align__(16) float sm[];
   float *gbuf = sm, *sums = sm + (p.inner + 3) / 4 * 4;     // gated row, then [norm_groups][warps per group]
   const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
@@ -644,13 +651,13 @@ template <int NP, int CP> static int launch_chunks(const Params &p, cudaStream_t
     set = true;
   }
   const dim3 grid(ceil_div(p.P, CP), p.heads, p.n_tok / CHUNK + p.n_seq);
-  ssm_decay_kernel<<<dim3(ceil_div(p.heads, 4), grid.z), 128, 0, st>>>(p);
+  launch_early(ssm_decay_kernel, dim3(ceil_div(p.heads, 4), grid.z), 128, 0, st, p);
   PT_LAUNCH_CHECK("pt_ssm");
-  ssm_chunk_state_kernel<NP, CP><<<grid, CHUNK_THREADS, sizeof(StateSmem<NP, CP>), st>>>(p);
+  launch_early(ssm_chunk_state_kernel<NP, CP>, grid, CHUNK_THREADS, sizeof(StateSmem<NP, CP>), st, p);
   PT_LAUNCH_CHECK("pt_ssm");
-  ssm_carry_kernel<<<dim3(ceil_div(p.N * p.P / 8, 64), p.heads, p.n_seq), 64, 0, st>>>(p);
+  launch_early(ssm_carry_kernel, dim3(ceil_div(p.N * p.P / 8, 64), p.heads, p.n_seq), 64, 0, st, p);
   PT_LAUNCH_CHECK("pt_ssm");
-  ssm_chunk_out_kernel<NP, CP><<<grid, CHUNK_THREADS, sizeof(OutSmem<NP, CP>), st>>>(p);
+  launch_early(ssm_chunk_out_kernel<NP, CP>, grid, CHUNK_THREADS, sizeof(OutSmem<NP, CP>), st, p);
   PT_LAUNCH_CHECK("pt_ssm");
   return PT_OK;
 }
@@ -665,17 +672,17 @@ template <typename T> static int run(const Params &p, bool plain, cudaStream_t s
     const size_t smem = ((size_t)(p.P + 2 * p.N + 3) / 4 * 4 + (size_t)ng * p.P) * sizeof(float);
     PT_REQUIRE(smem <= 48 * 1024, "pt_ssm: head width %d and state %d need %zu bytes of shared memory", p.P, p.N, smem);
     const dim3 grid(p.heads, p.n_seq);
-    if (v4) ssm_step_kernel<T, 4><<<grid, STEP_THREADS, smem, st>>>(p);
-    else ssm_step_kernel<T, 1><<<grid, STEP_THREADS, smem, st>>>(p);
+    if (v4) launch_early(ssm_step_kernel<T, 4>, grid, STEP_THREADS, smem, st, p);
+    else launch_early(ssm_step_kernel<T, 1>, grid, STEP_THREADS, smem, st, p);
     PT_LAUNCH_CHECK("pt_ssm");
   } else {
     if (!plain && sizeof(T) == 2 && p.taps <= 4 && p.C % 8 == 0 && p.inner % 8 == 0 && p.zx_ld % 8 == 0 && aligned_to(p.zx, 16) && aligned_to(p.xbc, 16) && aligned_to(p.ring, 16) && aligned_to(p.conv_w, 16)) {
       const dim3 grid(ceil_div(p.C / 8, CONV_THREADS) + 1, ceil_div(p.n_tok, CONV_TOKENS));
       switch (p.taps) {
-        case 1: ssm_conv8_kernel<1><<<grid, CONV_THREADS, 0, st>>>(p); break;
-        case 2: ssm_conv8_kernel<2><<<grid, CONV_THREADS, 0, st>>>(p); break;
-        case 3: ssm_conv8_kernel<3><<<grid, CONV_THREADS, 0, st>>>(p); break;
-        default: ssm_conv8_kernel<4><<<grid, CONV_THREADS, 0, st>>>(p); break;
+        case 1: launch_early(ssm_conv8_kernel<1>, grid, CONV_THREADS, 0, st, p); break;
+        case 2: launch_early(ssm_conv8_kernel<2>, grid, CONV_THREADS, 0, st, p); break;
+        case 3: launch_early(ssm_conv8_kernel<3>, grid, CONV_THREADS, 0, st, p); break;
+        default: launch_early(ssm_conv8_kernel<4>, grid, CONV_THREADS, 0, st, p); break;
       }
     } else {
       ssm_conv_kernel<T><<<dim3(ceil_div(p.C + p.heads, 256), p.n_tok), 256, 0, st>>>(p);
@@ -704,8 +711,8 @@ template <typename T> static int run(const Params &p, bool plain, cudaStream_t s
     PT_CUDA(cudaFuncSetAttribute(ssm_norm_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     PT_CUDA(cudaFuncSetAttribute(ssm_norm_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   }
-  if (v4) ssm_norm_kernel<T, 4><<<p.n_tok, threads, smem, st>>>(p);
-  else ssm_norm_kernel<T, 1><<<p.n_tok, threads, smem, st>>>(p);
+  if (v4) launch_early(ssm_norm_kernel<T, 4>, p.n_tok, threads, smem, st, p);
+  else launch_early(ssm_norm_kernel<T, 1>, p.n_tok, threads, smem, st, p);
   PT_LAUNCH_CHECK("pt_ssm");
   return PT_OK;
 }

@@ -214,6 +214,7 @@ __global__ void attn_rotate_kernel(const Params p) {
 }
 
 template <typename T> __global__ void kv_append_kernel(const Params p) {
+  early_start();
   const int t = blockIdx.x, s = p.tok_seq[t], pos = p.start[s] + t - p.cu[s];
   if (pos < 0 || pos >= p.max_len) {
     if (threadIdx.x == 0 && p.error_flag) atomicExch(p.error_flag, 12);
@@ -306,6 +307,7 @@ constexpr int TC_THREADS = 128, TILE = 64;   // TILE = the page size the tensor-
 // the warp sees completely take no mask.  DK / DV: dim / vdim rounded up to 32, 64, 128 .. (the padding holds zeros).  CTX: keys and
 // values are rows of the context; the first shared_dim dimensions of a key belong to all heads.
 template <int DK, int DV, bool CTX, bool EXT> __global__ void __launch_bounds__(TC_THREADS, DK > 128 ? 2 : 3) attn_prompt_kernel(const Params p) {
+  early_start();
   constexpr int KLD = DK + 8, VLD = DV + 8;
   extern __shared__ __align__(16) __nv_bfloat16 smb[];
   __nv_bfloat16 *Ks = smb, *Vs = smb + 2 * TILE * KLD;      // [2][TILE][KLD], [2][TILE][VLD]
@@ -522,6 +524,7 @@ template <int DK, int DV, bool CTX, bool EXT> __global__ void __launch_bounds__(
 // appends them.
 constexpr int NQ = 8;
 template <int DK, int DV, bool EXT> __global__ void __launch_bounds__(TC_THREADS) attn_decode_kernel(const Params p) {
+  early_start();
   constexpr int VLD = DV + 8, QLD = DK + 32, PSLD = TILE + 8;
   typedef __nv_bfloat16 T;
   extern __shared__ __align__(16) unsigned char smd[];

@@ -113,7 +113,7 @@ class GPT2Decoder(DecodeLoop):
             if norm is not None:
                 self._norm(x, norm, self.h)
                 x = self.h
-            ops.gemm(x, pl, out=out, epilogue=epilogue, bias=bias, residual=residual, error_flag=self.error_flag)
+            ops.gemm(x, pl, out=out, epilogue=epilogue, bias=bias, residual=residual, error_flag=self.error_flag, pdl=1)
             return
         if norm is not None and self.batch <= 8:
             pro = dict(prologue=ops.PRO_NORMCE, gamma=norm[0], beta=norm[1], eps=self.cfg.eps)
@@ -154,7 +154,7 @@ class GPT2Decoder(DecodeLoop):
         for li, L in enumerate(self.layers):
             self._linear(self.x, L["c_attn"], self.qkv, ops.EPI_BIAS, L["b_attn"], norm=L["ln1"])
             a = ops.attn_args(self.qkv, self.step_t, self.caches[li], self.attn, self.h_loc, ops.ROPE_NONE, ops.SOFTMAX_F16, 1.0, None, None,
-                              self.attn_ws, self.error_flag, pdl=self.pdl_attn)
+                              self.attn_ws, self.error_flag, pdl=self.pdl_attn or isinstance(L["c_proj"], ops.GemmWeight))
             ops.check(L_.pt_kv_append_attn(ctypes.byref(a), ops._stream()), "pt_kv_append_attn")
             self._row_parallel(self.attn, L["c_proj"], L["b_proj"])
             self._linear(self.x, L["c_fc"], self.act, ops.EPI_BIAS_GELU, L["b_fc"], norm=L["ln2"])

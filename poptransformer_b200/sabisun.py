@@ -162,10 +162,10 @@ class SabisunDecoder(SequenceDecoder):
                 ops.hyper(r.xs, n, c.eps, norm_w=s.norm, h=r.h, h_ld=s.proj.ld, w_in=s.hc.w_in, y=r.y, y_ld=c.width, mix=prev.hc.mix, w_out=prev.hc.w_out,
                           mult=c.residual_mult, sum_out=sums)
             if s.kind == "dense":
-                self._linear(s.proj, r.h, r.a, n, s.ld, r, epilogue=ops.EPI_RELU2)
-                self._linear(s.out, r.a, r.y, n, c.width, r)
+                self._linear(s.proj, r.h, r.a, n, s.ld, r, epilogue=ops.EPI_RELU2, pdl=1)
+                self._linear(s.out, r.a, r.y, n, c.width, r, pdl=1)
                 continue
-            self._linear(s.proj, r.h, r.a, n, s.ld, r)
+            self._linear(s.proj, r.h, r.a, n, s.ld, r, pdl=1)
             if s.kind == "attention":
                 m = s.m
                 ops.window_attn(view, r.a, s.ld, self.caches[s.layer], r.b, s.out.ld, m.heads, m.scale, m.window, m.keep_first, s.sink,
@@ -173,7 +173,7 @@ class SabisunDecoder(SequenceDecoder):
             else:
                 ops.ssm(view, r.a, s.ld, r.b, s.out.ld, s.w, self.rings[s.layer], self.states[s.layer], r.yin, r.xbc, r.dt, r.ssm_ws,
                         plain=self.plain)
-            self._linear(s.out, r.b, r.y, n, c.width, r)
+            self._linear(s.out, r.b, r.y, n, c.width, r, pdl=1)
 
     def _head(self, r, n, out, row_index=None, layer_sums=None, n_tok=0):
         """Logits of `n` rows (all of them, or the ones row_index names) after `_layers`."""
@@ -184,4 +184,4 @@ class SabisunDecoder(SequenceDecoder):
             ops.hyper(r.xs, n_tok, c.eps, sum_out=layer_sums[-1], **kw)
         if n:
             ops.hyper(r.xs, n, c.eps, norm_w=self.final_norm, h=r.h, h_ld=self.head.ld, row_index=row_index, **kw)
-            self._linear(self.head, r.h, out, n, c.vocab, r, alpha=c.logit_scale)
+            self._linear(self.head, r.h, out, n, c.vocab, r, alpha=c.logit_scale, pdl=1)
