@@ -221,5 +221,8 @@ class ChatGLM2Decoder(DecodeLoop):
         self.stop_mask.zero_()
 
     def step(self):
-        self.enqueue_step()
+        if self.graph is not None:
+            self.graph.replay()
+        else:
+            self.enqueue_step()
 

@@ -98,6 +98,7 @@ class RWKVDecoder(DecodeLoop):
         # split-k workspace, so three short waves share the SMs instead of running back to back.
         self.side = [torch.cuda.Stream(device=dev) for _ in range(2)] if tp == 1 else []
         self.side_ws = [ops.linear_workspace(B, d, 16, dev) for _ in self.side]
+        self.graph = None
         torch.cuda.synchronize()
 
     def _linear(self, x, pl, out, epilogue=ops.EPI_STORE, residual=None, side=None):
@@ -191,6 +192,18 @@ class RWKVDecoder(DecodeLoop):
         for i in range(self.cfg.n_layer):
             self.st_ffn[i].zero_(); self.st_att[i].zero_(); self.st_num[i].zero_(); self.st_den[i].zero_(); self.st_max[i].fill_(-1e30)
 
+    def capture(self):
+        """Captures one loop iteration in a CUDA graph; ids, step and recurrent states stay as they are."""
+        states = [t for ts in (self.st_ffn, self.st_att, self.st_num, self.st_den, self.st_max) for t in ts]
+        saved = [t.clone() for t in states]
+        super().capture()
+        for t, s in zip(states, saved):
+            t.copy_(s)
+
     def step(self):
-        self.enqueue_step()
+        # (the launches of a step take the host 5.8 ms at 24 layers, the device a third of it)
+        if self.graph is not None:
+            self.graph.replay()
+        else:
+            self.enqueue_step()
 
