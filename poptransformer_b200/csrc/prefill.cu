@@ -40,29 +40,74 @@ __global__ void prefill_embed_kernel(const uint4 *__restrict__ table, const int 
   if (threadIdx.x == 0 && stop_mask && start + t + 1 < ids_stride && ids[(size_t)b * ids_stride + start + t + 1] == eos_id) atomicOr(stop_mask + b, 1);
 }
 
-__global__ void __launch_bounds__(64) prefill_rope_kv_kernel(const Params p) {
-  early_start();
-  const int row = blockIdx.x, head = blockIdx.y, i = threadIdx.x;     // i: pair (i, i + 64)
-  const int b = row / p.P, t = row - b * p.P, pos = p.start + t;
+// One block per token, a thread takes eight channels of both halves of a head (16-byte accesses; a head per block with 2-byte accesses took
+// 12.4 us for 511 tokens of 32 heads).
+constexpr int ROPE_THREADS = 256;
+union Half8 { uint4 u; __half h[8]; };
+// VEC: all rows on 16-byte boundaries.
+template <bool VEC> __device__ __forceinline__ uint4 load8(const __half *x) {
+  if constexpr (VEC) {
+    return *reinterpret_cast<const uint4 *>(x);
+  } else {
+    Half8 r;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) r.h[j] = x[j];
+    return r.u;
+  }
+}
+template <bool VEC> __device__ __forceinline__ void store8(__half *x, const uint4 &v) {
+  if constexpr (VEC) {
+    *reinterpret_cast<uint4 *>(x) = v;
+  } else {
+    Half8 r;
+    r.u = v;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = r.h[j];
+  }
+}
+template <bool VEC> __global__ void __launch_bounds__(ROPE_THREADS) prefill_rope_kv_kernel(const Params p) {
+  const int row = blockIdx.x, b = row / p.P, t = row - b * p.P, pos = p.start + t;
   const int dq = p.n_head * H;
-  __half *q = p.qkv + (size_t)row * 3 * dq + (size_t)head * H, *k = q + dq, *v = k + dq;
-  const __half s = p.sin_t[(size_t)pos * (H / 2) + i], c = p.cos_t[(size_t)pos * (H / 2) + i];
-  const __half q1 = q[i], q2 = q[i + 64], k1 = k[i], k2 = k[i + 64];
-  q[i] = h_add(h_mul(q1, c), h_mul(__hneg(q2), s));
-  q[i + 64] = h_add(h_mul(q2, c), h_mul(q1, s));
   const int phys = p.page_table[(size_t)b * p.max_pages + pos / PAGE], slot = pos % PAGE;
-  __half *gK = p.pool + (((size_t)phys * 2 + 0) * p.n_head + head) * PAGE * H + (size_t)slot * H;
-  __half *gV = p.pool + (((size_t)phys * 2 + 1) * p.n_head + head) * PAGE * H + (size_t)slot * H;
-  gK[i] = h_add(h_mul(k1, c), h_mul(__hneg(k2), s));
-  gK[i + 64] = h_add(h_mul(k2, c), h_mul(k1, s));
-  gV[i] = v[i];
-  gV[i + 64] = v[i + 64];
+  for (int u = threadIdx.x; u < p.n_head * (H / 16); u += ROPE_THREADS) {
+    const int head = u / (H / 16), i = u % (H / 16) * 8;     // pairs (i .. i + 7, i + 64 .. i + 71)
+    __half *q = p.qkv + (size_t)row * 3 * dq + (size_t)head * H + i;
+    const __half *k = q + dq, *v = k + dq;
+    Half8 s, c, q1, q2, k1, k2, o1, o2;
+    s.u = load8<VEC>(p.sin_t + (size_t)pos * (H / 2) + i);
+    c.u = load8<VEC>(p.cos_t + (size_t)pos * (H / 2) + i);
+    q1.u = load8<VEC>(q); q2.u = load8<VEC>(q + 64);
+    k1.u = load8<VEC>(k); k2.u = load8<VEC>(k + 64);
+    const uint4 v1 = load8<VEC>(v), v2 = load8<VEC>(v + 64);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      o1.h[j] = h_add(h_mul(q1.h[j], c.h[j]), h_mul(__hneg(q2.h[j]), s.h[j]));
+      o2.h[j] = h_add(h_mul(q2.h[j], c.h[j]), h_mul(q1.h[j], s.h[j]));
+    }
+    store8<VEC>(q, o1.u);
+    store8<VEC>(q + 64, o2.u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      o1.h[j] = h_add(h_mul(k1.h[j], c.h[j]), h_mul(__hneg(k2.h[j]), s.h[j]));
+      o2.h[j] = h_add(h_mul(k2.h[j], c.h[j]), h_mul(k1.h[j], s.h[j]));
+    }
+    __half *gK = p.pool + (((size_t)phys * 2 + 0) * p.n_head + head) * PAGE * H + (size_t)slot * H + i;
+    __half *gV = p.pool + (((size_t)phys * 2 + 1) * p.n_head + head) * PAGE * H + (size_t)slot * H + i;
+    store8<VEC>(gK, o1.u);
+    store8<VEC>(gK + 64, o2.u);
+    store8<VEC>(gV, v1);
+    store8<VEC>(gV + 64, v2);
+  }
 }
 
 // ldmatrix of four 8x8 b16 matrices, transposed on the way: from a row-major [key][channel] tile this yields the B fragments
 // (k = key, n = channel) of two adjacent channel tiles for one 16-key step.
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
+}
+// The same without transposing: B fragments (k = channel, n = key) of a row-major [key][channel] tile.
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
 __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
   const __half2 h = __floats2half2_rn(lo, hi);
@@ -73,13 +118,15 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
 // registers.  Per page of 64 keys: S = Q K^T as 8 x 8 m16n8k16 tensor-core steps per warp (fp32 sums of exact fp16 products,
 // rounded to fp16 and scaled in fp16 like the reference's matmul output times its fp16 constant), causal mask, online softmax
 // (running max / sum per query, fp32), the probabilities rounded to fp16 (the reference's softmax output is fp16) and used as
-// the A operand of O += P V (4 x 16 steps), fp32 accumulators.
+// the A operand of O += P V (4 x 16 steps), fp32 accumulators.  A block is one chain of pages, so the next page's tiles are on their way
+// (cp.async, two buffers) while this one is used, and the tiles with the most pages start first.
+struct Tile { __half K[PAGE][KPAD], V[PAGE][KPAD]; };
 __global__ void __launch_bounds__(THREADS) prefill_attn_kernel(const Params p) {
   early_start();
-  __shared__ __align__(16) __half Ks[PAGE][KPAD];
-  __shared__ __align__(16) __half Vs[PAGE][KPAD];
+  extern __shared__ __align__(16) unsigned char pf_smem[];
+  Tile *tiles = reinterpret_cast<Tile *>(pf_smem);                    // [2]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
-  const int t0 = blockIdx.x * BQ, head = blockIdx.y, b = blockIdx.z;
+  const int t0 = (gridDim.x - 1 - blockIdx.x) * BQ, head = blockIdx.y, b = blockIdx.z;
   const int dq = p.n_head * H;
   const int q0 = t0 + warp * 16 + g, q1 = q0 + 8;                     // this lane's two query tokens (rows g and g + 8 of the warp's tile)
   const bool ok0 = q0 < p.P, ok1 = q1 < p.P;
@@ -103,28 +150,37 @@ __global__ void __launch_bounds__(THREADS) prefill_attn_kernel(const Params p) {
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
   const int last_pos = p.start + min(p.P, t0 + BQ) - 1;               // newest key any query of the tile may see
   const int warp_last = p.start + min(p.P, t0 + warp * 16 + 16) - 1;  // ... and any query of this warp
-  for (int pg = 0; pg * PAGE <= last_pos; ++pg) {
-    __syncthreads();                                                 // previous tiles consumed
+  auto request = [&](int pg) {
     const int phys = p.page_table[(size_t)b * p.max_pages + pg];
     const __half *gK = p.pool + (((size_t)phys * 2 + 0) * p.n_head + head) * PAGE * H;
     const __half *gV = p.pool + (((size_t)phys * 2 + 1) * p.n_head + head) * PAGE * H;
+    Tile &t = tiles[pg & 1];
     for (int e = tid; e < PAGE * (H / 8); e += THREADS) {
       const int r = e / (H / 8), c8 = e - r * (H / 8);
-      *reinterpret_cast<uint4 *>(&Ks[r][c8 * 8]) = *reinterpret_cast<const uint4 *>(gK + (size_t)r * H + c8 * 8);
-      *reinterpret_cast<uint4 *>(&Vs[r][c8 * 8]) = *reinterpret_cast<const uint4 *>(gV + (size_t)r * H + c8 * 8);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(&t.K[r][c8 * 8])), "l"(gK + (size_t)r * H + c8 * 8) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(&t.V[r][c8 * 8])), "l"(gV + (size_t)r * H + c8 * 8) : "memory");
     }
-    __syncthreads();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  request(0);
+  for (int pg = 0; pg * PAGE <= last_pos; ++pg) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();                                                 // this page is there, the one before is used up
+    if ((pg + 1) * PAGE <= last_pos) request(pg + 1);
     if (pg * PAGE > warp_last) continue;                             // nothing of this page is visible to this warp's queries (uniform per warp)
     // ---- scores of the warp's 16 queries against the page's 64 keys
     float sc[PAGE / 8][4];
+    const uint32_t k_lane = smem_addr(&tiles[pg & 1].K[lane & 7][(lane >> 3) * 8]);
 #pragma unroll
     for (int j = 0; j < PAGE / 8; ++j) {
       sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
-      const __half *kr = &Ks[j * 8 + g][2 * tig];
 #pragma unroll
-      for (int kk = 0; kk < H / 16; ++kk)
-        mma16816(sc[j], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], *reinterpret_cast<const uint32_t *>(kr + kk * 16),
-                 *reinterpret_cast<const uint32_t *>(kr + kk * 16 + 8));
+      for (int kk = 0; kk < H / 16; kk += 2) {
+        uint32_t b0, b1, b2, b3;   // keys 8 j .. +7: channels 16 kk .. +15 (b0, b1) and 16 kk + 16 .. +31 (b2, b3)
+        ldmatrix_x4(k_lane + (uint32_t)(j * 8 * KPAD + kk * 16) * 2u, b0, b1, b2, b3);
+        mma16816(sc[j], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b0, b1);
+        mma16816(sc[j], qa[kk + 1][0], qa[kk + 1][1], qa[kk + 1][2], qa[kk + 1][3], b2, b3);
+      }
     }
     float m_tile[2] = {-INFINITY, -INFINITY};
 #pragma unroll
@@ -168,7 +224,7 @@ __global__ void __launch_bounds__(THREADS) prefill_attn_kernel(const Params p) {
       o[j][2] *= corr[1]; o[j][3] *= corr[1];
     }
     // ---- O += P V: the score accumulators of two adjacent key tiles are the A fragment of one 16-key step
-    const uint32_t v_lane = smem_addr(&Vs[lane & 15][(lane >> 4) * 8]);
+    const uint32_t v_lane = smem_addr(&tiles[pg & 1].V[lane & 15][(lane >> 4) * 8]);
 #pragma unroll
     for (int k2 = 0; k2 < PAGE / 16; ++k2) {
       const uint32_t a0 = pack_h2(sc[2 * k2][0], sc[2 * k2][1]), a1 = pack_h2(sc[2 * k2][2], sc[2 * k2][3]);
@@ -222,9 +278,15 @@ extern "C" int pt_prefill_attn(const pt_prefill_attn_args *a, void *stream) {
   p.sin_t = (const __half *)a->rope_sin; p.cos_t = (const __half *)a->rope_cos;
   p.qkv = (__half *)a->qkv; p.pool = (__half *)a->pool; p.page_table = a->page_table; p.out = (__half *)a->out;
   p.scale_h = __float2half_rn(a->score_scale);
-  launch_early(pf::prefill_rope_kv_kernel, dim3(a->batch * a->n_tokens, a->n_head), 64, 0, as_stream(stream), p);
+  const bool vec = (((uintptr_t)a->qkv | (uintptr_t)a->rope_sin | (uintptr_t)a->rope_cos | (uintptr_t)a->pool) & 15) == 0;
+  launch_early(vec ? pf::prefill_rope_kv_kernel<true> : pf::prefill_rope_kv_kernel<false>, a->batch * a->n_tokens, pf::ROPE_THREADS, 0, as_stream(stream), p);
   PT_LAUNCH_CHECK("pt_prefill_attn");
-  launch_early(pf::prefill_attn_kernel, dim3(ceil_div(a->n_tokens, pf::BQ), a->n_head, a->batch), pf::THREADS, 0, as_stream(stream), p);
+  static bool set = false;
+  if (!set) {
+    PT_CUDA(cudaFuncSetAttribute(pf::prefill_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)sizeof(pf::Tile)));
+    set = true;
+  }
+  launch_early(pf::prefill_attn_kernel, dim3(ceil_div(a->n_tokens, pf::BQ), a->n_head, a->batch), pf::THREADS, 2 * sizeof(pf::Tile), as_stream(stream), p);
   PT_LAUNCH_CHECK("pt_prefill_attn");
   return PT_OK;
 }
