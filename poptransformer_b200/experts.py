@@ -41,7 +41,7 @@ class Experts:
         """Rows of a tile of the grouped products for n tokens: 1 for the skinny-matmul kernel, else about an expert's share."""
         if self.dtype == torch.float32:
             return 64
-        if n <= ops.DenseLinear.SKINNY_ROWS:
+        if n <= ops.GroupedLinear.SKINNY_ROWS:
             return 1
         share, tile = n * self.top / self.logits, 16
         while tile < 128 and tile < share:
@@ -65,7 +65,7 @@ class Experts:
         r.act = torch.empty(max(p * g.ff for p, g in zip(padded, groups)), dtype=dt, device=device)
         r.pair_y = torch.empty((max(padded), groups[0].width), dtype=dt, device=device)
         if dt == torch.bfloat16:
-            pairs = min(rows, ops.DenseLinear.SKINNY_ROWS) * top
+            pairs = min(rows, ops.GroupedLinear.SKINNY_ROWS) * top
             n = max(ops._lib.lib().pt_linear_workspace_bytes(pairs, x.n_out, 4) for g in groups for x in (g.up, g.back))
             if ws.lin_ws is None or n > ws.lin_ws.numel():
                 ws.lin_ws = torch.zeros(n, dtype=torch.uint8, device=device)

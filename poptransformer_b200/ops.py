@@ -34,7 +34,8 @@ SOFTMAX_F32, SOFTMAX_F16 = 0, 1
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream's handle.  (Called for every launch: torch.cuda.current_stream() builds a stream object each time, 2 us.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t):
@@ -44,11 +45,14 @@ def _ptr(t):
         raise PtError("libpt_b200 ops need CUDA tensors (there is no CPU path)")
     if not t.is_contiguous():
         raise PtError("libpt_b200 ops need contiguous tensors")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+_DTYPE_CODES = {torch.float16: DT_F16, torch.float32: DT_F32, torch.bfloat16: DT_BF16}
 
 
 def dtype_code(dt):
-    code = {torch.float16: DT_F16, torch.float32: DT_F32, torch.bfloat16: DT_BF16}.get(dt)
+    code = _DTYPE_CODES.get(dt)
     if code is None:
         raise PtError(f"unsupported element type {dt}")
     return code
@@ -237,13 +241,13 @@ def glu_rows(gate, up, features):
 
 
 class DenseLinear:
-    """W [n_out, k] of a model whose activations are bfloat16 or float32.  bfloat16: the skinny-matmul kernel up to `skinny_rows` rows
-    and the tcgen05 GEMM beyond (one tiling of the weights each), k padded to `K_PAD` with zero columns, so inputs have `ld` columns.
-    float32: true 32-bit products, no padding.  Outputs may have more columns than n_out (`out_ld`)."""
+    """W [n_out, k] of a model whose activations are bfloat16 or float32.  bfloat16: the tcgen05 GEMM, or for a short k the skinny-matmul
+    kernel up to `skinny_rows` rows, k padded to `K_PAD` with zero columns, so inputs have `ld` columns.  float32: true 32-bit products, no padding.  Outputs may have more columns than n_out (`out_ld`)."""
     K_PAD = 64
-    # Measured on B200 over 2048 x 4096 .. 32000 x 4096: at 8 rows the GEMM is level (2048-wide) to 20 % faster, at 32 rows 10 % to 3x.
-    # Up to a million weights (128 x 2048, 2048 x 128, 1024 x 1024) the skinny kernel takes 0.6 - 0.75 of the GEMM's time at 8 and 16 rows.
-    SKINNY_ROWS, SMALL_ROWS, SMALL_SIZE = 7, 16, 1 << 20
+    # Measured on B200, 1024 x 1024 .. 32000 x 2048: the GEMM is faster from one row on (1 row 4.8 .. 24 us against 5.9 .. 27, 7 rows 4.9 .. 25
+    # against 7.0 .. 30).  2048 x 128: 3.3 us against 2.8 at one row, 4.3 against 3.5 at 8, 4.8 against 5.3 at 16.
+    # (Both tilings are kept of matrices of up to a million weights, where the second costs nothing.)
+    SHORT_K, SHORT_K_ROWS, SMALL_SIZE = 256, 8, 1 << 20
 
     def __init__(self, w, dtype, pad_rows=0, keep=False, bias=None, split=None, limit=0.0, glu=GLU_CLAMPED, xielu=None):
         """pad_rows: zero rows are appended up to this many outputs (an output that is the padded input of the next linear).
@@ -262,9 +266,9 @@ class DenseLinear:
             self.bias = torch.zeros(self.n_out, dtype=torch.float32, device=w.device)
             self.bias[:len(bias)] = bias
         w = w.to(dtype).contiguous()
-        self.skinny_rows = self.SMALL_ROWS if self.n_out * self.ld <= self.SMALL_SIZE else self.SKINNY_ROWS
+        self.skinny_rows = self.SHORT_K_ROWS if self.ld <= self.SHORT_K and self.n_out * self.ld <= self.SMALL_SIZE else 0
         if dtype == torch.bfloat16:
-            self.skinny, self.gemm = PackedLinear(W_BF16, w), GemmWeight(W_BF16, w)
+            self.skinny, self.gemm = PackedLinear(W_BF16, w) if self.n_out * self.ld <= self.SMALL_SIZE else None, GemmWeight(W_BF16, w)
             self.w = w if keep else None
         elif dtype == torch.float32:
             self.w = w
@@ -313,7 +317,8 @@ class GroupedLinear:
     """Matrices [n_out, k] of one shape (experts), one after the other in a buffer: every tile of activation rows is multiplied with
     the matrix that `group_of` names for it.  bfloat16: tiles of one row on the skinny-matmul kernel, tiles of 16 .. 256 rows on the
     tcgen05 GEMM; float32: tiles of 64 rows."""
-    skinny_rows = DenseLinear.SKINNY_ROWS
+    SKINNY_ROWS = 7     # tokens up to which every row is a tile of its own
+    skinny_rows = SKINNY_ROWS
 
     def __init__(self, ws, dtype, pad_rows=0, limit=0.0, glu=GLU_CLAMPED):
         self.dtype, self.groups, self.k_in, self.limit, self.glu = dtype, len(ws), ws[0].shape[1], float(limit), glu

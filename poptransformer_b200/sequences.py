@@ -108,12 +108,9 @@ class SequenceDecoder(DecodeLoop):
     def _linear_workspaces(self, r, rows, linears):
         r.lin_ws = r.gemm_ws = None
         if self.dtype == torch.bfloat16:
-            L = ops._lib.lib()
-            n = max(L.pt_linear_workspace_bytes(min(rows, x.skinny_rows), x.n_out, max(16, x.ld // 256)) for x in linears)     # at least 256 k per slice
-            r.lin_ws = torch.zeros(n, dtype=torch.uint8, device=self.device)
-            if rows > ops.DenseLinear.SKINNY_ROWS:   # k-slices only while there are fewer tiles than SMs: 40 MB hold every such product's
-                n = min(max(L.pt_gemm_workspace_bytes(rows, x.n_out, 8) for x in linears), (40 << 20) + 65536)
-                r.gemm_ws = torch.zeros(n, dtype=torch.uint8, device=self.device)
+            skinny = [ops._lib.lib().pt_linear_workspace_bytes(min(rows, x.skinny_rows), x.n_out, 16) for x in linears if x.skinny_rows]
+            if skinny:
+                r.lin_ws = torch.zeros(max(skinny), dtype=torch.uint8, device=self.device)
 
     def _attn_workspace(self, shapes):
         """shapes: (heads, value width, window, kept first tokens) of the attention layers."""
