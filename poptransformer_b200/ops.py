@@ -176,7 +176,7 @@ class GemmWeight:
 
 
 # fp16 weights: rows from which the tcgen05 GEMM is the faster kernel.
-GEMM_FP16_ROWS = 4
+GEMM_FP16_ROWS = 1
 
 
 def fp16_linear(w, rows, interleave_gate_up=False):
