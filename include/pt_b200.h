@@ -66,7 +66,7 @@ uint64_t pt_launch_count(void);
 #define PT_EPI_BIAS 3         /* y = fp16(fp16(acc) + bias)          layers/linear.py:42-46 */
 #define PT_EPI_BIAS_GELU 4    /* y = gelu(fp16(fp16(acc) + bias))    layers/mlp.py:34-41   */
 #define PT_EPI_BIAS_RESIDUAL 5/* y = fp16(res + fp16(fp16(acc) + bias))                  */
-#define PT_EPI_RELU2 6        /* y = max(acc, 0)^2, squared in fp32 (PT_W_BF16 and pt_gemm_f32) */
+#define PT_EPI_RELU2 6        /* y = max(acc, 0)^2, squared in fp32 (PT_W_BF16 and pt_gemm_f32); pt_gemm, PT_W_FP16: of fp16(acc), in fp16 */
 #define PT_EPI_GLU 7          /* gated unit of row pairs (PT_W_BF16 and pt_gemm_f32, see pt_dense_ext) */
 #define PT_EPI_GELU_MUL 8     /* gelu_tanh(acc) * mul[mul_ids[row]]  (PT_W_BF16 and pt_gemm_f32, see pt_dense_ext) */
 #define PT_EPI_SOFTCAP 9      /* limit * tanh(acc / limit)  (PT_W_BF16 and pt_gemm_f32, see pt_dense_ext) */
@@ -451,6 +451,15 @@ int pt_fp8_matmul(const void *a, const void *b, float scale_a, float scale_b, in
  * num/den/max fp32 [b, c] updated in place; out fp16 [b, c] = fp16(wkv). */
 int pt_wkv(const void *k, const void *v, const float *time_first, const float *time_decay, float *num,
            float *den, float *max_state, int b, int c, void *out, void *stream);
+/* pt_wkv whose output is gated: out = sigmoid(recept) * wkv (attention.py:76,103), each rounded to fp16. */
+int pt_wkv_gated(const void *k, const void *v, const void *recept, const float *time_first, const float *time_decay, float *num,
+                 float *den, float *max_state, int b, int c, void *out, void *stream);
+/* pt_norm_ce, then pt_rwkv_mix of the normalised rows (which are not written themselves): the same roundings in one launch.  dim a multiple of
+ * 8, all pointers 16-byte aligned. */
+int pt_norm_ce_mix(const void *x, const void *gamma, const void *beta, int rows, int dim, float eps, void *state, const void *mix_a,
+                   const void *mix_b, const void *mix_c, void *out_a, void *out_b, void *out_c, void *stream);
+/* End of a feed-forward of RWKV (ffn.py:57-59, rwkv/model.py:112-116): x = x + sigmoid(recept) * value, then x / 2 if `halve`.  fp16 [n]. */
+int pt_rwkv_ffn_out(void *x, const void *recept, const void *value, int halve, int64_t n, void *stream);
 /* Token-shift gates of RWKV (`gate`, rwkv/attention.py:59-64 and ffn.py:40-45): out_x = h * mix_x + (1 - mix_x) * state for up to
  * three fp16 mixing vectors [dim] (out_b / out_c optional), fp16 rounding after every op; then state <- hidden.
  * hidden, state, out_x fp16 [rows, dim]. */

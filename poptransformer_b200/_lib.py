@@ -216,6 +216,9 @@ SIGNATURES = {
     "pt_fp8_matmul": (c_int, [c_void_p, c_void_p, c_float, c_float, c_int, c_int, c_int, c_void_p, c_void_p]),
     "pt_rwkv_mix": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "pt_rwkv_act": (c_int, [c_int, c_void_p, c_void_p, c_void_p, ctypes.c_int64, c_void_p]),
+    "pt_wkv_gated": (c_int, [c_void_p] * 8 + [c_int, c_int, c_void_p, c_void_p]),
+    "pt_norm_ce_mix": (c_int, [c_void_p] * 3 + [c_int, c_int, c_float] + [c_void_p] * 8),
+    "pt_rwkv_ffn_out": (c_int, [c_void_p] * 3 + [c_int, ctypes.c_int64, c_void_p]),
     "pt_wkv": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "pt_embedding": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
     "pt_step_containers": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p]),

@@ -200,10 +200,15 @@ __device__ __forceinline__ bool wait_fast(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return __all_sync(0xffffffffu, wait_fast(bar, parity, abort_flag)); }
 
 // One finished sum of the FP8 / INT4 kernels (fp16 output) or of the BF16 kernel.  (SWIGLU, whose sums come in pairs: store_swiglu.)
+__device__ __forceinline__ __half relu2_h(__half y) {
+  const __half r = __hgt(y, __float2half_rn(0.f)) ? y : __float2half_rn(0.f);
+  return h_mul(r, r);
+}
 __device__ __forceinline__ __half fp16_out(const GemmParams &p, float acc, int m, int n) {
   __half y = __float2half_rn(acc * p.out_scale);
   if (p.epilogue == PT_EPI_RESIDUAL) return h_add(__ldcg(p.residual + (size_t)m * p.N + n), y);
   if (p.epilogue == PT_EPI_BIAS) return h_add(y, p.bias[n]);
+  if (p.epilogue == PT_EPI_RELU2) return relu2_h(y);
   if (p.epilogue == PT_EPI_BIAS_GELU) return gelu_h(h_add(y, p.bias[n]));
   if (p.epilogue == PT_EPI_BIAS_RESIDUAL) return h_add(__ldcg(p.residual + (size_t)m * p.N + n), h_add(y, p.bias[n]));
   return y;
@@ -243,6 +248,7 @@ template <int EPI> __device__ __forceinline__ void fp16_rows16(const GemmParams 
       const float t = __shfl_xor_sync(0xffffffffu, odd ? sum[j] : sum[j + 1], 1);   // even lane: row j of n + 1; odd lane: row j + 1 of n - 1
       __half2 y = odd ? __floats2half2_rn(t * p.out_scale, sum[j + 1] * p.out_scale) : __floats2half2_rn(sum[j] * p.out_scale, t * p.out_scale);
       if constexpr (BIAS) y = __hadd2_rn(y, bias);
+      if constexpr (EPI == PT_EPI_RELU2) y = __halves2half2(relu2_h(__low2half(y)), relu2_h(__high2half(y)));
       if constexpr (EPI == PT_EPI_BIAS_GELU) y = __halves2half2(gelu_h(__low2half(y)), gelu_h(__high2half(y)));
       if constexpr (RES) y = __hadd2_rn(res[j / 2], y);
       *o = y;
@@ -267,6 +273,7 @@ __device__ __forceinline__ void epilogue_fp16(const GemmParams &p, uint32_t tmem
       else if (p.epilogue == PT_EPI_RESIDUAL) fp16_rows16<PT_EPI_RESIDUAL>(p, sum, m, n, lane);
       else if (p.epilogue == PT_EPI_BIAS) fp16_rows16<PT_EPI_BIAS>(p, sum, m, n, lane);
       else if (p.epilogue == PT_EPI_BIAS_GELU) fp16_rows16<PT_EPI_BIAS_GELU>(p, sum, m, n, lane);
+      else if (p.epilogue == PT_EPI_RELU2) fp16_rows16<PT_EPI_RELU2>(p, sum, m, n, lane);
       else if (p.epilogue == PT_EPI_BIAS_RESIDUAL) fp16_rows16<PT_EPI_BIAS_RESIDUAL>(p, sum, m, n, lane);
       else fp16_rows16<PT_EPI_STORE>(p, sum, m, n, lane);
       continue;
@@ -969,8 +976,8 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     PT_REQUIRE(a->out_dtype == PT_DT_BF16 || a->out_dtype == PT_DT_F32, "pt_gemm: BF16 weights write bf16 or fp32, got type %d", a->out_dtype);
   } else {
     PT_REQUIRE(a->epilogue == PT_EPI_STORE || a->epilogue == PT_EPI_RESIDUAL || a->epilogue == PT_EPI_BIAS || ((int4 || fp16) && a->epilogue == PT_EPI_SWIGLU) ||
-                   (fp16 && (a->epilogue == PT_EPI_BIAS_GELU || a->epilogue == PT_EPI_BIAS_RESIDUAL)),
-               "pt_gemm: epilogue %d (store, residual or bias; INT4 and FP16: swiglu; FP16: bias with gelu or residual)", a->epilogue);
+                   (fp16 && (a->epilogue == PT_EPI_BIAS_GELU || a->epilogue == PT_EPI_BIAS_RESIDUAL || a->epilogue == PT_EPI_RELU2)),
+               "pt_gemm: epilogue %d (store, residual or bias; INT4 and FP16: swiglu; FP16: relu2, bias with gelu or residual)", a->epilogue);
     PT_REQUIRE(a->epilogue != PT_EPI_SWIGLU || a->n_out % 16 == 0, "pt_gemm: SwiGLU epilogue needs n_out %% 16 == 0, got %d", a->n_out);
   }
   const bool wants_bias = a->epilogue == PT_EPI_BIAS || a->epilogue == PT_EPI_BIAS_GELU || a->epilogue == PT_EPI_BIAS_RESIDUAL;

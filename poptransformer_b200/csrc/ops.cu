@@ -82,8 +82,11 @@ __global__ void norm_ce_kernel(const __half *__restrict__ x, const __half *__res
 // norm_ce_kernel with the row kept in registers between the statistics and the normalisation: one pass over memory with 16-byte
 // accesses (dim a multiple of 8, below 8192 as the op requires).  Same arithmetic, statistics summed per thread over 8-element
 // units instead of single elements.
+// MIX: instead of the normalised row its RWKV token-shift mixes leave (rwkv_mix_kernel), and the state takes the row.
+struct MixArgs { __half *state; const __half *w[3]; __half *out[3]; };
+template <bool MIX>
 __global__ void norm_ce_vec_kernel(const __half *__restrict__ x, const __half *__restrict__ gamma, const __half *__restrict__ beta,
-                                   int dim, float eps, int single_row, __half *__restrict__ out) {
+                                   int dim, float eps, int single_row, __half *__restrict__ out, const MixArgs mix) {
   early_start();
   __shared__ float red[32];
   const size_t base = (size_t)blockIdx.x * dim;
@@ -130,7 +133,26 @@ __global__ void norm_ce_vec_kernel(const __half *__restrict__ x, const __half *_
       const __half *gh = reinterpret_cast<const __half *>(&gv), *bh = reinterpret_cast<const __half *>(&bv);
 #pragma unroll
       for (int j = 0; j < 8; ++j) h[j] = h_add(h_mul(h_mul(h_sub(h[j], m), r), gh[j]), bh[j]);
-      reinterpret_cast<uint4 *>(out + base)[u] = v[q];
+      if constexpr (MIX) {
+        uint4 *st = reinterpret_cast<uint4 *>(mix.state + base) + u;
+        const uint4 sv = *st;
+        const __half *sh = reinterpret_cast<const __half *>(&sv);
+        const __half one = __float2half_rn(1.0f);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if (!mix.out[k]) continue;
+          const uint4 wv = __ldg(reinterpret_cast<const uint4 *>(mix.w[k]) + u);
+          const __half *wh = reinterpret_cast<const __half *>(&wv);
+          uint4 ov;
+          __half *oh = reinterpret_cast<__half *>(&ov);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) oh[j] = h_add(h_mul(h[j], wh[j]), h_mul(h_sub(one, wh[j]), sh[j]));
+          reinterpret_cast<uint4 *>(mix.out[k] + base)[u] = ov;
+        }
+        *st = v[q];
+      } else {
+        reinterpret_cast<uint4 *>(out + base)[u] = v[q];
+      }
     }
   }
 }
@@ -577,9 +599,12 @@ __global__ void fp8_matmul_kernel(const uint8_t *__restrict__ a, const uint8_t *
 }
 
 // ------------------------------------------------------------------------------------------ RWKV WKV
+__device__ __forceinline__ __half receptance_h(__half r, __half v) { return h_mul(__float2half_rn(1.0f / (1.0f + expf(-__half2float(r)))), v); }
+
+// recept (optional): the output is gated with it, as rwkv_act_kernel's mode 0 would.
 __global__ void wkv_kernel(const __half *__restrict__ k, const __half *__restrict__ v, const float *__restrict__ tf,
                            const float *__restrict__ td, float *__restrict__ num, float *__restrict__ den, float *__restrict__ mx,
-                           int b, int c, __half *__restrict__ out) {
+                           int b, int c, const __half *__restrict__ recept, __half *__restrict__ out) {
   early_start();
   const size_t total = (size_t)b * c;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -589,7 +614,8 @@ __global__ void wkv_kernel(const __half *__restrict__ k, const __half *__restric
     const float ww = kk + tf[ch];
     const float p = fmaxf(m0, ww);
     float e1 = expf(m0 - p), e2 = expf(ww - p);
-    out[i] = __float2half_rn((e1 * n0 + e2 * vv) / (e1 * d0 + e2));
+    const __half o = __float2half_rn((e1 * n0 + e2 * vv) / (e1 * d0 + e2));
+    out[i] = recept ? receptance_h(recept[i], o) : o;
     const float ww2 = m0 - expf(td[ch]);
     const float p2 = fmaxf(ww2, kk);
     e1 = expf(ww2 - p2);
@@ -625,14 +651,22 @@ __global__ void rwkv_act_kernel(int mode, const __half *__restrict__ a, const __
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const __half x = a[i];
     if (mode == 0) {
-      const __half sg = __float2half_rn(1.0f / (1.0f + expf(-__half2float(x))));
-      out[i] = h_mul(sg, b[i]);
+      out[i] = receptance_h(x, b[i]);
     } else if (mode == 1) {
       const __half r = __hgt(x, __float2half_rn(0.f)) ? x : __float2half_rn(0.f);
       out[i] = h_mul(r, r);
     } else {
       out[i] = h_mul(x, __float2half_rn(0.5f));
     }
+  }
+}
+
+// End of a feed-forward: x = fp16(x + fp16(sigmoid(r) * v)), and half of that where the model rescales.
+__global__ void rwkv_ffn_out_kernel(__half *__restrict__ x, const __half *__restrict__ r, const __half *__restrict__ v, int halve, size_t n) {
+  early_start();
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const __half y = h_add(x[i], receptance_h(r[i], v[i]));
+    x[i] = halve ? h_mul(y, __float2half_rn(0.5f)) : y;
   }
 }
 
@@ -775,8 +809,8 @@ extern "C" int pt_norm_ce(const void *x, const void *gamma, const void *beta, in
   PT_REQUIRE((dim & 3) == 0, "our normCEOp require 4x a last dim, and current is: %d", dim);
   PT_REQUIRE(dim < 8192, "normalize_ce, last_dim_size should be <= 8192, and current is: %d", dim);
   if (dim % 8 == 0 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0)
-    launch_early(norm_ce_vec_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
-                                                           rows == 1 ? 1 : 0, (__half *)out);
+    launch_early(norm_ce_vec_kernel<false>, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
+                 rows == 1 ? 1 : 0, (__half *)out, MixArgs{});
   else
     launch_early(norm_ce_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
                                                        rows == 1 ? 1 : 0, (__half *)out);
@@ -955,13 +989,43 @@ extern "C" int pt_fp8_matmul(const void *a, const void *b, float scale_a, float 
   return PT_OK;
 }
 
+static int run_wkv(const void *k, const void *v, const float *time_first, const float *time_decay, float *num, float *den, float *max_state, int b, int c,
+                   const void *recept, void *out, void *stream, const char *name) {
+  PT_REQUIRE(k && v && time_first && time_decay && num && den && max_state && out, "%s: null pointer argument", name);
+  PT_REQUIRE(b > 0 && c > 0, "%s: bad shape [%d, %d]", name, b, c);
+  launch_early(wkv_kernel, grid_for((size_t)b * c), 256, 0, as_stream(stream), (const __half *)k, (const __half *)v, time_first, time_decay, num, den, max_state, b, c,
+               (const __half *)recept, (__half *)out);
+  PT_LAUNCH_CHECK(name);
+  return PT_OK;
+}
 extern "C" int pt_wkv(const void *k, const void *v, const float *time_first, const float *time_decay, float *num, float *den,
                       float *max_state, int b, int c, void *out, void *stream) {
-  PT_REQUIRE(k && v && time_first && time_decay && num && den && max_state && out, "pt_wkv: null pointer argument");
-  PT_REQUIRE(b > 0 && c > 0, "pt_wkv: bad shape [%d, %d]", b, c);
-  launch_early(wkv_kernel, grid_for((size_t)b * c), 256, 0, as_stream(stream), (const __half *)k, (const __half *)v, time_first, time_decay, num, den,
-                                                                     max_state, b, c, (__half *)out);
-  PT_LAUNCH_CHECK("pt_wkv");
+  return run_wkv(k, v, time_first, time_decay, num, den, max_state, b, c, nullptr, out, stream, "pt_wkv");
+}
+extern "C" int pt_wkv_gated(const void *k, const void *v, const void *recept, const float *time_first, const float *time_decay, float *num, float *den,
+                            float *max_state, int b, int c, void *out, void *stream) {
+  PT_REQUIRE(recept, "pt_wkv_gated: null pointer argument");
+  return run_wkv(k, v, time_first, time_decay, num, den, max_state, b, c, recept, out, stream, "pt_wkv_gated");
+}
+
+extern "C" int pt_norm_ce_mix(const void *x, const void *gamma, const void *beta, int rows, int dim, float eps, void *state, const void *mix_a, const void *mix_b,
+                              const void *mix_c, void *out_a, void *out_b, void *out_c, void *stream) {
+  PT_REQUIRE(x && gamma && beta && state && mix_a && out_a && (!out_b || mix_b) && (!out_c || mix_c), "pt_norm_ce_mix: null pointer argument");
+  PT_REQUIRE(rows > 0 && dim > 0 && dim % 8 == 0 && dim < 8192, "pt_norm_ce_mix: bad shape [%d, %d] (a multiple of 8 below 8192)", rows, dim);
+  const uintptr_t all = (uintptr_t)x | (uintptr_t)gamma | (uintptr_t)beta | (uintptr_t)state | (uintptr_t)mix_a | (uintptr_t)mix_b | (uintptr_t)mix_c |
+                        (uintptr_t)out_a | (uintptr_t)out_b | (uintptr_t)out_c;
+  PT_REQUIRE((all & 15) == 0, "pt_norm_ce_mix: all pointers must be 16-byte aligned");
+  const MixArgs m{(__half *)state, {(const __half *)mix_a, (const __half *)mix_b, (const __half *)mix_c}, {(__half *)out_a, (__half *)out_b, (__half *)out_c}};
+  launch_early(norm_ce_vec_kernel<true>, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps, rows == 1 ? 1 : 0,
+               (__half *)nullptr, m);
+  PT_LAUNCH_CHECK("pt_norm_ce_mix");
+  return PT_OK;
+}
+
+extern "C" int pt_rwkv_ffn_out(void *x, const void *recept, const void *value, int halve, int64_t n, void *stream) {
+  PT_REQUIRE(x && recept && value && n > 0, "pt_rwkv_ffn_out: bad arguments");
+  launch_early(rwkv_ffn_out_kernel, grid_for((size_t)n), 256, 0, as_stream(stream), (__half *)x, (const __half *)recept, (const __half *)value, halve, (size_t)n);
+  PT_LAUNCH_CHECK("pt_rwkv_ffn_out");
   return PT_OK;
 }
 

@@ -74,7 +74,7 @@ class RWKVDecoder(DecodeLoop):
         self.ids = torch.full((B, c.max_len), self.pad_id, dtype=torch.int32, device=dev)
         self.step_t = torch.zeros(1, dtype=torch.int32, device=dev)
         self.stop_mask = torch.zeros(B, dtype=torch.int32, device=dev)
-        self.x, self.t, self.k, self.v, self.r, self.vv, self.rr, self.w = (torch.empty((B, d), **f16) for _ in range(8))
+        self.x, self.t, self.k, self.v, self.r, self.vv, self.rr = (torch.empty((B, d), **f16) for _ in range(7))
         self.kk, self.vl, self.rl, self.wl = (torch.empty((B, dl), **f16) for _ in range(4))     # this rank's channels
         self.fk, self.fk2 = torch.empty((B, fl), **f16), torch.empty((B, fl), **f16)
         self.logits = torch.empty((B, self.vocab_loc), **f16)
@@ -103,8 +103,9 @@ class RWKVDecoder(DecodeLoop):
 
     def _linear(self, x, pl, out, epilogue=ops.EPI_STORE, residual=None, side=None):
         """side = None: on the current stream; side = i: on side stream i (between _fork and _join), with that stream's workspace."""
+        # (early start: the GEMM only, and only behind a kernel of the same stream)
         kw = dict(epilogue=epilogue, residual=residual, workspace=self.lin_ws if side is None else self.side_ws[side], error_flag=self.error_flag,
-                  pdl=self.pdl_linear)
+                  pdl=1 if side is None and isinstance(pl, ops.GemmWeight) else self.pdl_linear)
         if side is None:
             ops.linear_fp16(x, pl, out, **kw)
         else:
@@ -131,6 +132,12 @@ class RWKVDecoder(DecodeLoop):
         if self.tp > 1:
             torch.distributed.all_reduce(out, group=self.group)
 
+    def _norm_mix(self, gb, state, mixes, outs):
+        """LayerNorm of x, then its token-shift mixes; `state` takes the normalised rows."""
+        P, L_ = ops._ptr, ops._lib.lib()
+        w, o = ([P(t) for t in ts] + [None] * (3 - len(ts)) for ts in (mixes, outs))
+        ops.check(L_.pt_norm_ce_mix(P(self.x), P(gb[0]), P(gb[1]), self.batch, self.cfg.d_model, self.cfg.eps, P(state), *w, *o, ops._stream()), "pt_norm_ce_mix")
+
     def enqueue_step(self):
         c, L_, P, S = self.cfg, ops._lib.lib(), ops._ptr, ops._stream
         B, d, dl, fl = self.batch, c.d_model, self.d_loc, self.f_loc
@@ -138,9 +145,7 @@ class RWKVDecoder(DecodeLoop):
         for i, L in enumerate(self.layers):
             if L["pre_ln"] is not None:
                 self._norm(self.x, L["pre_ln"], self.x)
-            self._norm(self.x, L["ln1"], self.t)
-            mk, mv, mr = L["a_mix"]
-            ops.check(L_.pt_rwkv_mix(P(self.t), P(self.st_att[i]), P(mk), P(mv), P(mr), P(self.k), P(self.v), P(self.r), B, d, S()), "pt_rwkv_mix")
+            self._norm_mix(L["ln1"], self.st_att[i], L["a_mix"], (self.k, self.v, self.r))
             par = bool(self.side)
             if par:
                 self._fork()
@@ -149,21 +154,21 @@ class RWKVDecoder(DecodeLoop):
             self._linear(self.r, L["a_recept"], self.rl, side=1 if par else None)
             if par:
                 self._join()
-            ops.check(L_.pt_wkv(P(self.kk), P(self.vl), P(L["time_first"]), P(L["time_decay"]), P(self.st_num[i]), P(self.st_den[i]),
-                                P(self.st_max[i]), B, dl, P(self.wl), S()), "pt_wkv")
-            ops.check(L_.pt_rwkv_act(0, P(self.rl), P(self.wl), P(self.wl), B * dl, S()), "pt_rwkv_act")
+            ops.check(L_.pt_wkv_gated(P(self.kk), P(self.vl), P(self.rl), P(L["time_first"]), P(L["time_decay"]), P(self.st_num[i]), P(self.st_den[i]),
+                                      P(self.st_max[i]), B, dl, P(self.wl), S()), "pt_wkv_gated")
             if self.tp == 1:
                 self._linear(self.wl, L["a_out"], self.x, ops.EPI_RESIDUAL, residual=self.x)
             else:
                 self._end(self.wl, L["a_out"], self.vv)
                 ops.check(L_.pt_add_f16(P(self.x), P(self.vv), B * d, P(self.x), S()), "pt_add_f16")
-            self._norm(self.x, L["ln2"], self.t)
-            fk, fr = L["f_mix"]
-            ops.check(L_.pt_rwkv_mix(P(self.t), P(self.st_ffn[i]), P(fk), P(fr), None, P(self.k), P(self.r), None, B, d, S()), "pt_rwkv_mix")
+            self._norm_mix(L["ln2"], self.st_ffn[i], L["f_mix"], (self.k, self.r))
             if par:
                 self._fork()
-            self._linear(self.k, L["f_key"], self.fk)
-            ops.check(L_.pt_rwkv_act(1, P(self.fk), None, P(self.fk2), B * fl, S()), "pt_rwkv_act")
+            if isinstance(L["f_key"], ops.GemmWeight):
+                self._linear(self.k, L["f_key"], self.fk2, ops.EPI_RELU2)
+            else:
+                self._linear(self.k, L["f_key"], self.fk)
+                ops.check(L_.pt_rwkv_act(1, P(self.fk), None, P(self.fk2), B * fl, S()), "pt_rwkv_act")
             self._end(self.fk2, L["f_value"], self.vv)
             if self.tp == 1:
                 self._linear(self.r, L["f_recept"], self.rr, side=0 if par else None)
@@ -173,10 +178,8 @@ class RWKVDecoder(DecodeLoop):
                 self._linear(self.r, L["f_recept"], self.rl)
                 torch.distributed.all_gather_into_tensor(self.gather_r, self.rl, group=self.group)
                 self.rr.view(B, self.tp, dl).copy_(self.gather_r.permute(1, 0, 2))
-            ops.check(L_.pt_rwkv_act(0, P(self.rr), P(self.vv), P(self.w), B * d, S()), "pt_rwkv_act")
-            ops.check(L_.pt_add_f16(P(self.x), P(self.w), B * d, P(self.x), S()), "pt_add_f16")
-            if c.rescale_every > 0 and (i + 1) % c.rescale_every == 0:
-                ops.check(L_.pt_rwkv_act(2, P(self.x), None, P(self.x), B * d, S()), "pt_rwkv_act")
+            halve = c.rescale_every > 0 and (i + 1) % c.rescale_every == 0
+            ops.check(L_.pt_rwkv_ffn_out(P(self.x), P(self.rr), P(self.vv), int(halve), B * d, S()), "pt_rwkv_ffn_out")
         self._norm(self.x, self.ln_out, self.t)
         self._linear(self.t, self.head, self.logits)
         if self.tp == 1:
