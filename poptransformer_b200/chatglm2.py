@@ -85,7 +85,7 @@ class ChatGLM2Decoder(DecodeLoop):
                 return pl
             w = torch.cat(ws, 0).to(torch.float16).contiguous()
             if tp == 1:
-                return ops.fp16_linear(w, batch, interleave_gate_up=interleave)
+                return ops.fp16_linear(w, interleave_gate_up=interleave)
             return ops.PackedLinear(ops.W_FP16, w, interleave_gate_up=interleave)
 
         self.emb = t("transformer.embedding.word_embeddings.weight").to(torch.float16).contiguous()

@@ -61,7 +61,7 @@ class GPT2Decoder(DecodeLoop):
         self.d_loc, self.h_loc = d // tp, c.n_head // tp
         cols = lambda w, k: w[:, r * (k // tp):(r + 1) * (k // tp)].contiguous()        # 'end': rank r's input features
         end_bias = lambda b: b if tp == 1 else b.repeat(B, 1).contiguous()           # added once, after the all-reduce
-        lin = (lambda w: ops.fp16_linear(w, B)) if tp == 1 else (lambda w: ops.PackedLinear(ops.W_FP16, w))
+        lin = (lambda w: ops.fp16_linear(w)) if tp == 1 else (lambda w: ops.PackedLinear(ops.W_FP16, w))
         self.layers = []
         for i in range(c.n_layer):
             p = f"transformer.h.{i}."

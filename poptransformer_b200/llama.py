@@ -99,7 +99,7 @@ class LlamaDecoder(DecodeLoop):
 
         def fp16(w, interleave=False):
             if tp_size == 1 and persistent is None:
-                return ops.fp16_linear(w, batch, interleave_gate_up=interleave)
+                return ops.fp16_linear(w, interleave_gate_up=interleave)
             return ops.PackedLinear(ops.W_FP16, w, interleave_gate_up=interleave)
 
         def row_parallel(key, k_total):

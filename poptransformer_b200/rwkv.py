@@ -48,7 +48,7 @@ class RWKVDecoder(DecodeLoop):
         h = lambda k: state_dict[k].to(dev).to(torch.float16).reshape(-1).contiguous()
         f = lambda k: state_dict[k].to(dev).to(torch.float32).reshape(-1)[r * dl:(r + 1) * dl].contiguous()   # sharded with the channels
         w16 = lambda k: state_dict[k].to(dev).to(torch.float16)
-        pack = (lambda w: ops.fp16_linear(w, batch)) if tp == 1 else (lambda w: ops.PackedLinear(ops.W_FP16, w))
+        pack = (lambda w: ops.fp16_linear(w)) if tp == 1 else (lambda w: ops.PackedLinear(ops.W_FP16, w))
         start = lambda k: pack(rows(w16(k), r, tp).contiguous())
         end = lambda k, kl: pack(w16(k)[:, r * kl:(r + 1) * kl].contiguous())
         ln = lambda p: (h(p + ".weight"), h(p + ".bias"))
