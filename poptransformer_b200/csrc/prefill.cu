@@ -66,6 +66,7 @@ template <bool VEC> __device__ __forceinline__ void store8(__half *x, const uint
   }
 }
 template <bool VEC> __global__ void __launch_bounds__(ROPE_THREADS) prefill_rope_kv_kernel(const Params p) {
+  early_start();
   const int row = blockIdx.x, b = row / p.P, t = row - b * p.P, pos = p.start + t;
   const int dq = p.n_head * H;
   const int phys = p.page_table[(size_t)b * p.max_pages + pos / PAGE], slot = pos % PAGE;
