@@ -38,7 +38,7 @@ namespace tc {
 
 constexpr int BM = 128;            // weight rows per CTA
 constexpr int BKB = 128;           // bytes of k per stage and operand row (one 128-byte swizzle atom)
-constexpr int THREADS_F8 = 192;    // warp 0: producer, warp 1: MMA + tensor-memory allocation, warps 2-5: epilogue
+__host__ __device__ constexpr int dense_threads(int na) { return 64 + 128 * na; }   // warp 0: producer, warp 1: MMA + tensor-memory allocation, then four epilogue warps per accumulator
 constexpr int MAX_CLUSTER = 8;     // k-slices of a tile (one cluster)
 constexpr int A_TILE = BM * BKB;   // 16 KB: 128 rows x 128 bytes of k, 128-byte swizzle
 constexpr int RAW_TILE = BM * 32;  // 4 KB: 128 rows x 64 k of packed nibbles
@@ -497,7 +497,7 @@ template <bool EXT> __device__ __forceinline__ void epilogue_bf16(const GemmPara
 // Dynamic shared memory: [stage][NA A tiles of 16 KB | B tile mb * 128 B], every tile 1024-byte aligned.  NA = 2: a CTA takes 256 weight
 // rows (two accumulators), which fetches a third less per product than NA = 1; without k-slices.
 template <int FMT, int NA, bool EXT>
-__global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+__global__ void __launch_bounds__(dense_threads(NA), 1) gemm_dense_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                                    const GemmParams p) {
   constexpr bool BF16 = FMT == PT_W_BF16, F8 = FMT == PT_W_FP8;
   constexpr int KX = F8 ? BKB : BKB / 2;     // elements of k per stage
@@ -625,7 +625,8 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
       if (NA == 1 && p.ksplit > 1) {
         leave_sums(p, tmem, warp & 3, lane, 0, 1, reinterpret_cast<float *>(smem));
       } else if constexpr (BF16) {
-        for (int a = 0; a < na; ++a) epilogue_bf16<EXT>(p, tmem + a * acc_cols, warp & 3, lane, n0 + a * BM, m0, m_end);
+        const int a = (warp - 2) >> 2;    // (each accumulator has four warps: nothing else runs on the SM while a tile of 256 x 256 leaves)
+        if (a < na) epilogue_bf16<EXT>(p, tmem + a * acc_cols, warp & 3, lane, n0 + a * BM, m0, m_end);
       } else {
         epilogue_fp16(p, tmem, warp & 3, lane, 0, 1, n0, m0);
       }
@@ -635,7 +636,7 @@ __global__ void __launch_bounds__(THREADS_F8, 1) gemm_dense_kernel(const __grid_
   if (NA == 1 && p.ksplit > 1) {
     if (p.pdl) wait_for_prerequisites();
     __syncwarp();
-    sum_cluster<BF16, EXT>(p, ctl, smem_s, ks, n0, m0, m_end, THREADS_F8);
+    sum_cluster<BF16, EXT>(p, ctl, smem_s, ks, n0, m0, m_end, dense_threads(1));
   }
   __syncthreads();
   fence_after();
@@ -1113,7 +1114,7 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   dim3 grid(ceil_div(n_tiles, na), p.ksplit, m_tiles);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(int4 ? (3 + 4 * int4_groups) * 32 : tc::THREADS_F8);
+  cfg.blockDim = dim3(int4 ? (3 + 4 * int4_groups) * 32 : tc::dense_threads(na));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = as_stream(stream);
   cudaLaunchAttribute attr[2];
