@@ -134,7 +134,6 @@ class ChatGLM2Decoder(DecodeLoop):
         self.attn_ws = ops.attn_workspace(B, self.h_loc, c.head_dim, self.caches[0].max_pages, dev)
         self.lin_ws = ops.linear_workspace(B, max(2 * self.f_loc, self.vocab_loc, self.qkv.shape[1], d), 16, dev)
         if self.use_gemm:
-            self.gemm_ws = ops.gemm_workspace(B, max(2 * self.f_loc, self.vocab_loc, self.qkv.shape[1], d), 8, dev)
             self.x8 = torch.empty((B, max(d, self.f_loc)), dtype=torch.uint8, device=dev)      # the E4M3 input of the running linear
             self.gu_out = torch.empty((B, 2 * self.f_loc), **f16)
         self.graph = None
@@ -176,7 +175,7 @@ class ChatGLM2Decoder(DecodeLoop):
             return self.x8.view(-1)[:B * d].view(B, d)
 
         def gemm(x8, pl, out, **kw):
-            ops.gemm(x8, pl, out=out, x_scale=pl.act_scale, workspace=self.gemm_ws, error_flag=self.error_flag, pdl=1, **kw)
+            ops.gemm(x8, pl, out=out, x_scale=pl.act_scale, error_flag=self.error_flag, pdl=1, **kw)
 
         ops.embedding(self.emb, self.ids, self.step_t, out=self.x)
         for li, L in enumerate(self.layers):

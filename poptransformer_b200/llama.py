@@ -212,8 +212,6 @@ class LlamaDecoder(DecodeLoop):
             self.caches.append(kc)
         self.attn_ws = ops.attn_workspace(B, self.h_loc, c.head_dim, self.caches[0].max_pages, dev)
         self.lin_ws = ops.linear_workspace(B, max(3 * self.d_loc, 2 * self.f_loc, d, self.logits.shape[1]), 16, dev)
-        if self.use_gemm:
-            self.gemm_ws = ops.gemm_workspace(B, max(3 * d, 2 * f), 8, dev)
         self.graph = None
         # The persistent whole-step kernel covers INT4, batch <= 2, on one GPU or tensor-parallel over up to 8 (the all-reduces are
         # then fused into the kernel as peer stores); everything else takes the per-op kernels and NCCL.
@@ -384,14 +382,14 @@ class LlamaDecoder(DecodeLoop):
 
         for li, L in enumerate(self.layers):
             norm(L["ln1"])
-            ops.gemm(self.h, L["qkv"], out=self.qkv, workspace=self.gemm_ws, error_flag=self.error_flag, pdl=1)
+            ops.gemm(self.h, L["qkv"], out=self.qkv, error_flag=self.error_flag, pdl=1)
             a = ops.attn_args(self.qkv, self.step_t, self.caches[li], self.attn, self.h_loc, ops.ROPE_LLAMA, ops.SOFTMAX_F32, self.score_scale,
                               self.sin, self.cos, self.attn_ws, self.error_flag, pdl=1)
             ops.check(L_.pt_kv_append_attn(ctypes.byref(a), ops._stream()), "pt_kv_append_attn")
-            ops.gemm(self.attn, L["o"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, workspace=self.gemm_ws, error_flag=self.error_flag, pdl=1)
+            ops.gemm(self.attn, L["o"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, error_flag=self.error_flag, pdl=1)
             norm(L["ln2"])
-            ops.gemm(self.h, L["gu"], out=self.act, out_ld=self.act.shape[1], epilogue=ops.EPI_SWIGLU, workspace=self.gemm_ws, error_flag=self.error_flag, pdl=1)
-            ops.gemm(self.act, L["down"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, workspace=self.gemm_ws, error_flag=self.error_flag, pdl=1)
+            ops.gemm(self.h, L["gu"], out=self.act, out_ld=self.act.shape[1], epilogue=ops.EPI_SWIGLU, error_flag=self.error_flag, pdl=1)
+            ops.gemm(self.act, L["down"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, error_flag=self.error_flag, pdl=1)
 
     def prefill(self, n_tokens=None, chunk=1024):
         """Ingests the first `n_tokens` positions of every sequence in one pass (the work of the reference's first stage,
@@ -420,7 +418,7 @@ class LlamaDecoder(DecodeLoop):
             if rows not in self._pf_bufs:
                 f16 = dict(dtype=torch.float16, device=self.device)
                 self._pf_bufs = {rows: SimpleNamespace(x=torch.empty((rows, d), **f16), h=torch.empty((rows, d), **f16), qkv=torch.empty((rows, 3 * d), **f16),
-                                                       attn=torch.empty((rows, d), **f16), act=torch.empty((rows, f), **f16), ws=ops.gemm_workspace(rows, max(3 * d, 2 * f), 8, self.device))}
+                                                       attn=torch.empty((rows, d), **f16), act=torch.empty((rows, f), **f16))}
             w = self._pf_bufs[rows]
             ops.check(L_.pt_prefill_embed(ops._ptr(self.emb), ops._ptr(self.ids), c.max_len, B, P, s0, d, c.vocab, self.eos_id, ops._ptr(self.stop_mask),
                                           ops._ptr(w.x), ops._stream()), "pt_prefill_embed")
@@ -430,12 +428,12 @@ class LlamaDecoder(DecodeLoop):
 
             for li, L in enumerate(self.pf_layers):
                 norm(L["ln1"])
-                ops.gemm(w.h, L["qkv"], out=w.qkv, workspace=w.ws, error_flag=self.error_flag, pdl=1)
+                ops.gemm(w.h, L["qkv"], out=w.qkv, error_flag=self.error_flag, pdl=1)
                 ops.prefill_attn(w.qkv, self.caches[li], B, P, s0, c.n_head, self.score_scale, self.sin, self.cos, out=w.attn)
-                ops.gemm(w.attn, L["o"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, workspace=w.ws, error_flag=self.error_flag, pdl=1)
+                ops.gemm(w.attn, L["o"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, error_flag=self.error_flag, pdl=1)
                 norm(L["ln2"])
-                ops.gemm(w.h, L["gu"], out=w.act, epilogue=ops.EPI_SWIGLU, workspace=w.ws, error_flag=self.error_flag, pdl=1)
-                ops.gemm(w.act, L["down"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, workspace=w.ws, error_flag=self.error_flag, pdl=1)
+                ops.gemm(w.h, L["gu"], out=w.act, epilogue=ops.EPI_SWIGLU, error_flag=self.error_flag, pdl=1)
+                ops.gemm(w.act, L["down"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, error_flag=self.error_flag, pdl=1)
         self.step_t.fill_(n)
         return n
 
@@ -471,10 +469,10 @@ class LlamaDecoder(DecodeLoop):
         """Every INT4/FP16 transformer linear of one step, back to back (used to time the dominant kernel alone)."""
         if self.use_gemm:
             for L in self.layers:
-                ops.gemm(self.h, L["qkv"], out=self.qkv, workspace=self.gemm_ws)
-                ops.gemm(self.attn, L["o"], out=self.part, workspace=self.gemm_ws)
-                ops.gemm(self.h, L["gu"], out=self.act, out_ld=self.act.shape[1], epilogue=ops.EPI_SWIGLU, workspace=self.gemm_ws)
-                ops.gemm(self.act, L["down"], out=self.part, workspace=self.gemm_ws)
+                ops.gemm(self.h, L["qkv"], out=self.qkv)
+                ops.gemm(self.attn, L["o"], out=self.part)
+                ops.gemm(self.h, L["gu"], out=self.act, out_ld=self.act.shape[1], epilogue=ops.EPI_SWIGLU)
+                ops.gemm(self.act, L["down"], out=self.part)
             return
         for L in self.layers:
             self._norm_linear(self.x, L["ln1"], L["qkv"], self.qkv)
