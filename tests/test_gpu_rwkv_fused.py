@@ -64,4 +64,4 @@ def test_captured_step_keeps_the_state(cuda):
     dec.capture()
     for _ in range(6):
         dec.step()
-    assert (dec.ids.cpu().numpy() == want["Loop:0"]).all() and int(dec.step_t) == int(want["Loop:1"])
+    assert (dec.ids.cpu().numpy() == want["Loop:0"]).all() and dec.step_t.item() == want["Loop:1"].item()
