@@ -65,7 +65,7 @@ struct GemmParams {
   const int *group_of;    // BF16, grouped: the weight matrix of every tile of mb rows (negative: none)
   const int *group_used;  // ... and how many of its rows are in use (null: all)
   int n_tiles;            // tiles of 128 weight rows
-  int pdl;                // BF16: programmatic dependent launch: weights are fetched before the producer of x has finished
+  int pdl;                // programmatic dependent launch (tiled weights): they are fetched before the producer of x has finished
   size_t group_stride;    // bytes between weight matrices
 };
 
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(dense_threads(NA), 1) gemm_dense_kernel(const 
       const unsigned char *wt = p.w + w_base + ((size_t)blockIdx.x * NA * p.n_kb + kb0) * A_TILE;
       const size_t next_tile = (size_t)p.n_kb * A_TILE;
       const uint32_t tx = na * A_TILE + b_bytes, full0 = sa(&ctl.full[0]), empty0 = sa(&ctl.empty[0]);
-      const bool tiled = p.w_tiled != 0;
+      const bool tiled = p.w_tiled != 0;     // (always, if p.pdl: the early loads below do not move kx on)
       int s = 0, kx = kb0 * KX;
       uint32_t par = 1;   // parity of the `empty` phase that must have completed before slot s is refilled (none in the first round)
       bool first_round = true;
@@ -1056,7 +1056,8 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   const bool pair = PT_TC_PAIR && bf16 && p.ksplit == 1 && p.mb >= 128 && n_tiles >= 2 && (long long)ceil_div(n_tiles, 2) * m_tiles >= sm_count();
   const int na = pair ? 2 : 1;
   p.n_tiles = n_tiles;
-  p.pdl = a->pdl ? 1 : 0;
+  // Row-major weights are an operand of a plain product, which the kernel before may have written: nothing of them is read early.
+  p.pdl = a->pdl && p.w_tiled ? 1 : 0;
   const uint32_t b_bytes = (uint32_t)p.mb * tc::BKB;
   const uint32_t stage_bytes = na * tc::A_TILE + ((b_bytes + 1023u) & ~1023u);
   // Up to 64 activation rows a stage is small, and what limits the kernel is the one thread per CTA that issues the MMAs (about
