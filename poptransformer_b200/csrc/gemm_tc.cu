@@ -21,8 +21,8 @@
 // of raw nibble tiles feeds a few slots of fp16 weights) and run the epilogue (tcgen05.ld, scale, fp16, coalesced stores
 // along n).  k-slices of one tile are summed in slice order (deterministic): INT4 by the blocks of a cluster, FP8 and BF16 in a
 // workspace by the last CTA to arrive.
-// Every wait is bounded: on a time-out the CTA raises the error flag, skips its remaining waits and still frees its tensor
-// memory.
+// Every wait on an mbarrier is bounded: on a time-out the CTA raises the error flag, skips its remaining waits and still frees its tensor
+// memory.  Waits for tensor memory and for the blocks of a cluster have no limit and end by construction (gemm_plan.h).
 #include <cuda.h>
 
 #include <algorithm>
@@ -30,27 +30,20 @@
 #include <cstring>
 
 #include "dense_out.cuh"
+#include "gemm_plan.h"
 #include "mbarrier.cuh"
 #include "tile_math.cuh"
 
 namespace pt {
 namespace tc {
 
-constexpr int BM = 128;            // weight rows per CTA
-constexpr int BKB = 128;           // bytes of k per stage and operand row (one 128-byte swizzle atom)
-__host__ __device__ constexpr int dense_threads(int na) { return 64 + 128 * na; }   // warp 0: producer, warp 1: MMA + tensor-memory allocation, then four epilogue warps per accumulator
-constexpr int MAX_CLUSTER = 8;     // k-slices of a tile (one cluster)
-constexpr int A_TILE = BM * BKB;   // 16 KB: 128 rows x 128 bytes of k, 128-byte swizzle
-constexpr int RAW_TILE = BM * 32;  // 4 KB: 128 rows x 64 k of packed nibbles
-constexpr int RAW_STEP = 2 * RAW_TILE;   // a step of the INT4 kernel: 128 k
-
 struct GemmParams {
   int M, N, K;
   int mb;                 // activation rows per CTA (multiple of 16, at most 256)
-  int int4;               // 1: INT4 weights (A tile produced by the transform warps), 0: FP8
   int group;              // INT4 scale group along k
   int kb_per_split, n_kb; // k blocks (of 128 bytes of operand row) per k-slice / in total
   int ksplit, stages, raw_stages;
+  int tmem_columns;       // tensor memory of a CTA
   int w_tiled;            // weights tiled by pt_gemm_repack (one contiguous tile per stage) instead of row-major
   int epilogue;           // PT_EPI_STORE, PT_EPI_RESIDUAL or PT_EPI_BIAS (BF16: see dense)
   float out_scale;
@@ -497,7 +490,7 @@ template <bool EXT> __device__ __forceinline__ void epilogue_bf16(const GemmPara
 // Dynamic shared memory: [stage][NA A tiles of 16 KB | B tile mb * 128 B], every tile 1024-byte aligned.  NA = 2: a CTA takes 256 weight
 // rows (two accumulators), which fetches a third less per product than NA = 1; without k-slices.
 template <int FMT, int NA, bool EXT>
-__global__ void __launch_bounds__(dense_threads(NA), 1) gemm_dense_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+__global__ void __launch_bounds__(64 + 128 * NA, 1) gemm_dense_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                                    const GemmParams p) {
   constexpr bool BF16 = FMT == PT_W_BF16, F8 = FMT == PT_W_FP8;
   constexpr int KX = F8 ? BKB : BKB / 2;     // elements of k per stage
@@ -525,9 +518,7 @@ __global__ void __launch_bounds__(dense_threads(NA), 1) gemm_dense_kernel(const 
       }
     }
   }
-  uint32_t acc_cols = 32;
-  while ((int)acc_cols < p.mb) acc_cols <<= 1;
-  const uint32_t tmem_cols = NA * acc_cols;
+  const uint32_t tmem_cols = p.tmem_columns, acc_cols = tmem_cols / NA;
 
   if (tid == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -636,7 +627,7 @@ __global__ void __launch_bounds__(dense_threads(NA), 1) gemm_dense_kernel(const 
   if (NA == 1 && p.ksplit > 1) {
     if (p.pdl) wait_for_prerequisites();
     __syncwarp();
-    sum_cluster<BF16, EXT>(p, ctl, smem_s, ks, n0, m0, m_end, dense_threads(1));
+    sum_cluster<BF16, EXT>(p, ctl, smem_s, ks, n0, m0, m_end, 64 + 128);
   }
   __syncthreads();
   fence_after();
@@ -670,7 +661,7 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
   const uint32_t half_bytes = (uint32_t)p.mb * BKB, slot_bytes = 2 * half_bytes;          // (half: a multiple of 2 KB)
   unsigned char *raw_ring = smem + (size_t)S * slot_bytes;
   const uint32_t smem_s = sa(smem);
-  const uint32_t a_col = (uint32_t)(p.mb + 31) & ~31u, tmem_cols = a_col + 64 * S <= 256 ? 256 : 512;
+  const uint32_t a_col = (uint32_t)(p.mb + 31) & ~31u, tmem_cols = p.tmem_columns;
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -902,26 +893,6 @@ static int make_map(CUtensorMap *map, const void *base, CUtensorMapDataType dt, 
   return PT_OK;
 }
 
-// Tiles of the INT4 kernel.  A CTA spends on a step (128 k) the longer of transform and single-thread roles (about 350 cycles) and MMAs (4 mb
-// cycles), then its epilogue, and the CTAs run in rounds over the SMs: of all row counts per tile (steps of 16) and k-slices the pair with
-// the least time by this count is taken.
-struct Int4Plan { int mb, ksplit; };
-static Int4Plan plan_int4(int m, int n_tiles, int n_steps, int ksplit_req) {
-  Int4Plan best{16, 1};
-  double least = 1e30;
-  for (int mb = 16; mb <= 256; mb += 16) {
-    const int m_tiles = ceil_div(m, mb);
-    if (mb > 16 && m_tiles == ceil_div(m, mb - 16)) continue;    // fewer rows per tile do as well
-    for (int ks = 1; ks <= MAX_CLUSTER; ++ks) {
-      if (ksplit_req > 0 ? ks != std::min(std::min(ksplit_req, MAX_CLUSTER), n_steps) : ks > 1 && n_steps / ks < 4) continue;
-      const long long ctas = (long long)n_tiles * m_tiles * ks, rounds = (ctas + sm_count() - 1) / sm_count();
-      const double t = (double)rounds * (ceil_div(n_steps, ks) * (double)std::max(350, 4 * mb) + 1500 + 8 * mb) + (ks > 1 ? 2500 + 6 * mb : 0);
-      if (t < least) { least = t; best = {mb, ks}; }
-    }
-  }
-  return best;
-}
-
 }  // namespace tc
 }  // namespace pt
 
@@ -992,47 +963,23 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
 
   tc::GemmParams p{};
   p.M = a->m; p.N = a->n_out; p.K = a->k_in;
-  p.int4 = int4 ? 1 : 0;
   p.group = int4 ? a->group : 0;
   p.w_tiled = a->w_tiled ? 1 : 0;
   p.w = (const unsigned char *)a->w;
-  p.mb = std::min(256, ceil_div(a->m, 16) * 16);
   const bool grouped = bf16 && a->ext && a->ext->n_groups > 0;
-  const int n_tiles = ceil_div(a->n_out, tc::BM);
-  // BF16: fewer activation rows per tile before k-slices (whose sums take a detour over HBM) when there are not enough tiles
   if (grouped) {
-    p.mb = a->ext->group_rows;
-    PT_REQUIRE(p.mb % 16 == 0 && p.mb >= 16 && p.mb <= 256 && a->m % p.mb == 0 && a->m / p.mb <= 65535, "pt_gemm: groups of %d rows (16 .. 256 in steps of 16) in %d rows",
-               p.mb, a->m);
+    const int rows = a->ext->group_rows;
+    PT_REQUIRE(rows % 16 == 0 && rows >= 16 && rows <= 256 && a->m % rows == 0 && a->m / rows <= 65535, "pt_gemm: groups of %d rows (16 .. 256 in steps of 16) in %d rows",
+               rows, a->m);
     p.group_of = a->ext->group_of;
     p.group_used = a->ext->group_used;
     p.group_stride = pt_gemm_packed_bytes(a->wfmt, a->n_out, a->k_in);
-  } else if (bf16 || fp16)
-    while (p.mb > 64 && n_tiles * ceil_div(a->m, p.mb) * 4 < sm_count() * 3) p.mb = ceil_div(p.mb, 32) * 16;
-  int m_tiles = ceil_div(a->m, p.mb);
-  p.n_kb = bf16 || fp16 ? a->k_in / 64 : a->k_in / 128;
-  // k-slices: fill the GPU when there are few tiles, with at least PT_TC_MIN_KB k-blocks per CTA.  Not to the brim: the slices of a tile
-  // start together in one cluster, and 36 clusters of eight did not fit 148 SMs of two CTAs each at once (4608 x 4096 at 8 rows: 14.7 us
-  // with 8 slices, 11.1 with 7; 12288 x 4096: 26 us with 3 slices, 20 with 2).
-#ifndef PT_TC_MIN_KB
-#define PT_TC_MIN_KB 3
-#endif
-  int ksplit = a->ksplit;
-  if (int4) {
-    const tc::Int4Plan plan = tc::plan_int4(a->m, n_tiles, p.n_kb, a->ksplit);
-    p.mb = plan.mb;
-    ksplit = plan.ksplit;
-  } else if (ksplit <= 0) {
-    ksplit = std::max(1, (p.mb <= 64 ? 2 : 1) * sm_count() * 7 / 8 / (n_tiles * m_tiles));   // two CTAs fit an SM up to 64 activation rows
-    // (with several blocks of activation rows a slice's sums cost more than its share of a short k saves: 128 x 2048 at 512 .. 8192
-    // rows takes 19 - 21 us whole and 27 - 41 us in slices)
-    ksplit = std::max(1, std::min(ksplit, p.n_kb / ((bf16 || fp16) && m_tiles > 1 ? 32 : PT_TC_MIN_KB)));
   }
-  ksplit = std::min(ksplit, tc::MAX_CLUSTER);
-  m_tiles = ceil_div(a->m, p.mb);
-  ksplit = std::max(1, std::min(ksplit, p.n_kb));
-  p.kb_per_split = ceil_div(p.n_kb, ksplit);
-  p.ksplit = ceil_div(p.n_kb, p.kb_per_split);
+  const tc::GemmPlan plan = tc::plan_gemm({int4, bf16, fp16, a->m, a->n_out, a->k_in, a->ksplit, grouped ? a->ext->group_rows : 0, sm_count()});
+  PT_REQUIRE(plan.fits, "pt_gemm: tile does not fit shared memory");
+  p.mb = plan.mb; p.n_kb = plan.n_kb; p.ksplit = plan.ksplit; p.kb_per_split = plan.kb_per_split;
+  p.stages = plan.stages; p.raw_stages = plan.raw_stages; p.tmem_columns = plan.tmem_columns;
+  p.n_tiles = plan.n_tiles;
   p.epilogue = a->epilogue;
   p.out_scale = int4 ? 1.0f : (a->x_scale > 0.f ? a->x_scale : 1.0f) * (a->w_scale > 0.f ? a->w_scale : 1.0f);
   p.scales = (const __half *)a->scales;
@@ -1045,49 +992,11 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   if (a->ksplit > 1 && p.ksplit > 1) {   // slices that the caller asked for
     const size_t need = pt_gemm_workspace_bytes(a->m, a->n_out, p.ksplit);
     PT_REQUIRE(a->workspace && a->workspace_bytes >= need, "pt_gemm: %d k-slices need %zu workspace bytes, got %zu", p.ksplit, need, a->workspace_bytes);
-    PT_REQUIRE((size_t)n_tiles * m_tiles <= kGemmMaxCounters, "pt_gemm: %d x %d tiles exceed the %zu arrival counters of a k-slice workspace", n_tiles,
-               m_tiles, kGemmMaxCounters);
+    PT_REQUIRE((size_t)plan.n_tiles * plan.m_tiles <= kGemmMaxCounters, "pt_gemm: %d x %d tiles exceed the %zu arrival counters of a k-slice workspace", plan.n_tiles,
+               plan.m_tiles, kGemmMaxCounters);
   }
-
-  // BF16 without k-slices: two weight tiles per CTA when half as many CTAs still fill the GPU
-#ifndef PT_TC_PAIR
-#define PT_TC_PAIR 1
-#endif
-  const bool pair = PT_TC_PAIR && bf16 && p.ksplit == 1 && p.mb >= 128 && n_tiles >= 2 && (long long)ceil_div(n_tiles, 2) * m_tiles >= sm_count();
-  const int na = pair ? 2 : 1;
-  p.n_tiles = n_tiles;
   // Row-major weights are an operand of a plain product, which the kernel before may have written: nothing of them is read early.
   p.pdl = a->pdl && p.w_tiled ? 1 : 0;
-  const uint32_t b_bytes = (uint32_t)p.mb * tc::BKB;
-  const uint32_t stage_bytes = na * tc::A_TILE + ((b_bytes + 1023u) & ~1023u);
-  // Up to 64 activation rows a stage is small, and what limits the kernel is the one thread per CTA that issues the MMAs (about
-  // 75 cycles per tcgen05.mma whatever its N): two CTAs per SM (half the shared memory each) issue side by side.  Measured on
-  // B200, FP8 65024 x 4096 at 8 / 32 rows: 63 / 66 us with one CTA per SM, 45 / 47 us with two.
-#ifndef PT_TC_BUDGET_SMALL_KB
-#define PT_TC_BUDGET_SMALL_KB 100
-#endif
-  // BF16 also with large tiles when there are more of them than SMs: the epilogue of one CTA then hides behind the products of the
-  // other (two accumulators of 256 columns fill the tensor memory).
-  // (The sums of a slice take 512 bytes per row of the ring.)
-  const bool small = p.mb <= 64 || ((bf16 || fp16) && !(p.ksplit > 1 && p.mb > 128) && na * p.mb <= 256 && (long long)n_tiles * m_tiles * p.ksplit > sm_count());
-  const uint32_t budget = (small ? PT_TC_BUDGET_SMALL_KB : 200) * 1024u;
-  size_t smem;
-  const bool two_int4 = int4 && p.mb <= 128 && n_tiles * m_tiles * p.ksplit > sm_count();   // two CTAs per SM (each has half the tensor memory)
-  const int int4_groups = !two_int4 && p.mb <= 128 ? 4 : 2;   // above 128 rows a step's MMAs take longer than half a transform
-  if (int4) {
-    // slots: 64 tensor-memory columns beside the accumulator and 256 bytes of shared memory per row each
-    p.stages = two_int4 ? (p.mb <= 64 ? 3 : 2) : (p.mb <= 128 ? 4 : p.mb <= 208 ? 3 : 2);
-    const uint32_t slots = p.stages * 2 * b_bytes, room = (two_int4 ? 104 : 217) * 1024u;
-    p.raw_stages = (int)std::min<uint32_t>(12, (room - slots) / tc::RAW_STEP);
-    smem = slots + (size_t)p.raw_stages * tc::RAW_STEP + 1024;
-    PT_REQUIRE(p.stages >= int4_groups && p.raw_stages >= p.stages + int4_groups, "pt_gemm: tile does not fit shared memory");
-    if (!two_int4) smem = std::max<size_t>(smem, 120 * 1024);   // never more CTAs on an SM than its tensor memory serves
-  } else {
-    p.stages = (int)std::min<uint32_t>(8, budget / stage_bytes);
-    PT_REQUIRE(p.stages >= 2, "pt_gemm: tile does not fit shared memory");
-    smem = (size_t)p.stages * stage_bytes + 1024;
-    if (p.mb > 64) smem = std::max<size_t>(smem, (na * p.mb > 256 ? 120 : 80) * 1024);   // never more CTAs on an SM than its tensor memory holds accumulators for
-  }
 
   CUtensorMap map_w, map_x;
   memset(&map_w, 0, sizeof(map_w));
@@ -1112,11 +1021,11 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     PT_CUDA(cudaFuncSetAttribute(tc::gemm_int4_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     attr_set = true;
   }
-  dim3 grid(ceil_div(n_tiles, na), p.ksplit, m_tiles);
+  dim3 grid(ceil_div(plan.n_tiles, plan.na), p.ksplit, plan.m_tiles);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(int4 ? (3 + 4 * int4_groups) * 32 : tc::dense_threads(na));
-  cfg.dynamicSmemBytes = smem;
+  cfg.blockDim = dim3(plan.threads);
+  cfg.dynamicSmemBytes = plan.smem;
   cfg.stream = as_stream(stream);
   cudaLaunchAttribute attr[2];
   int n_attr = 0;
@@ -1134,12 +1043,12 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   cfg.numAttrs = n_attr;
   cudaError_t e;
   if (int4) {
-    e = cudaLaunchKernelEx(&cfg, int4_groups == 2 ? tc::gemm_int4_kernel<2> : tc::gemm_int4_kernel<4>, map_x, p);
+    e = cudaLaunchKernelEx(&cfg, plan.int4_groups == 2 ? tc::gemm_int4_kernel<2> : tc::gemm_int4_kernel<4>, map_x, p);
   } else {
     const bool ext = bf16 && dense_needs_ext(a->epilogue, a->ext);
     const auto kernel = fp16 ? tc::gemm_dense_kernel<PT_W_FP16, 1, false>
                        : !bf16 ? tc::gemm_dense_kernel<PT_W_FP8, 1, false>
-                       : pair ? (ext ? tc::gemm_dense_kernel<PT_W_BF16, 2, true> : tc::gemm_dense_kernel<PT_W_BF16, 2, false>)
+                       : plan.na == 2 ? (ext ? tc::gemm_dense_kernel<PT_W_BF16, 2, true> : tc::gemm_dense_kernel<PT_W_BF16, 2, false>)
                               : (ext ? tc::gemm_dense_kernel<PT_W_BF16, 1, true> : tc::gemm_dense_kernel<PT_W_BF16, 1, false>);
     e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, p);
   }

@@ -1,0 +1,51 @@
+"""What a block of the tensor-core GEMMs takes of its SM, over the sizes that pt_gemm accepts.  Blocks wait without a limit for tensor memory and for
+the other blocks of their cluster, and launches of several streams meet on an SM: the two waits must not be able to close a circle."""
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(__file__), "..", "poptransformer_b200", "csrc")
+DRIVER = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "gemm_plan.h"
+using namespace pt::tc;
+int main() {
+  for (int fmt = 0; fmt < 4; ++fmt)      // INT4, FP8, BF16, FP16
+    for (int m : {1, 9, 16, 17, 32, 33, 48, 64, 65, 80, 96, 112, 128, 129, 144, 176, 208, 224, 255, 256, 257, 511, 2048, 5000})
+      for (int n : {40, 128, 768, 1600, 4096, 12288, 22016, 50257, 65024})
+        for (int k : {128, 256, 768, 2048, 4096, 11008, 16384})
+          for (int ks : {0, 1, 2, 5, 8, 16})
+            for (int rows : {0, 16, 128, 256}) {
+              if (rows && fmt != 2) continue;
+              const GemmPlan p = plan_gemm({fmt == 0, fmt == 2, fmt == 3, rows ? (m + rows - 1) / rows * rows : m, n, k, ks, rows, 148});
+              printf("%d %d %u %d %d %d %d %d %d\n", fmt, (int)p.fits, p.smem, p.tmem_columns, p.ksplit, p.na, p.mb, p.stages, (int)p.stage_bytes);
+            }
+}
+"""
+SM, RESERVE, COLUMNS, LIMIT = 228 * 1024, 1024, 512, 220 * 1024      # bytes of an SM, of them the system's for each block; columns; bytes a block may ask for
+
+
+@pytest.fixture(scope="module")
+def plans(tmp_path_factory):
+    d = tmp_path_factory.mktemp("plan")
+    (d / "plan.cpp").write_text(DRIVER)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, "-o", str(d / "plan"), str(d / "plan.cpp")], check=True)
+    return sorted({tuple(map(int, line.split())) for line in subprocess.run([str(d / "plan")], check=True, capture_output=True, text=True).stdout.splitlines()})
+
+
+def test_plans_fit(plans):
+    for fmt, fits, smem, columns, ksplit, na, mb, stages, stage_bytes in plans:
+        assert fits and smem <= LIMIT and na * mb <= columns <= COLUMNS and columns & (columns - 1) == 0
+        assert ksplit == 1 or (na == 1 and mb * 512 <= smem - 1024)         # the sums of a slice, in the ring
+        if 2 * (smem + RESERVE) <= SM:
+            assert 2 * columns <= COLUMNS                                   # blocks of one launch never wait for one another's columns
+
+
+def test_waits_close_no_circle(plans):
+    assert 3 * (min(p[2] for p in plans) + RESERVE) > SM                    # at most two blocks on an SM
+    clustered = sorted({(p[2], p[3]) for p in plans if p[4] > 1})
+    for a in clustered:
+        for b in clustered:
+            assert a[0] + b[0] + 2 * RESERVE > SM or a[1] + b[1] <= COLUMNS, (a, b)
