@@ -488,9 +488,11 @@ template <bool EXT> __device__ __forceinline__ void epilogue_bf16(const GemmPara
 
 // ------------------------------------------------------------------------------------------ FP8 and BF16
 // Dynamic shared memory: [stage][NA A tiles of 16 KB | B tile mb * 128 B], every tile 1024-byte aligned.  NA = 2: a CTA takes 256 weight
-// rows (two accumulators), which fetches a third less per product than NA = 1; without k-slices.
+// rows (two accumulators), which fetches a third less per product than NA = 1; without k-slices.  With up to 128 activation rows two such CTAs share an
+// SM, so their registers have to allow it (96 a thread): a Pivavik of width 2048 takes four prompts of 2048 tokens, whose experts have tiles of 128
+// rows, in 20.4 ms so and in 24.5 with the 168 registers that one CTA of 320 threads per SM may have (measured on B200).
 template <int FMT, int NA, bool EXT>
-__global__ void __launch_bounds__(64 + 128 * NA, 1) gemm_dense_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+__global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                                    const GemmParams p) {
   constexpr bool BF16 = FMT == PT_W_BF16, F8 = FMT == PT_W_FP8;
   constexpr int KX = F8 ? BKB : BKB / 2;     // elements of k per stage

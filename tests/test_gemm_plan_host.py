@@ -1,6 +1,7 @@
 """What a block of the tensor-core GEMMs takes of its SM, over the sizes that pt_gemm accepts.  Blocks wait without a limit for tensor memory and for
 the other blocks of their cluster, and launches of several streams meet on an SM: the two waits must not be able to close a circle."""
 import os
+import re
 import subprocess
 
 import pytest
@@ -49,3 +50,13 @@ def test_waits_close_no_circle(plans):
     for a in clustered:
         for b in clustered:
             assert a[0] + b[0] + 2 * RESERVE > SM or a[1] + b[1] <= COLUMNS, (a, b)
+
+
+def test_blocks_that_share_an_sm_are_compiled_to(plans):
+    """Where the plan lets two blocks of a launch share an SM, the kernel is bound to registers that allow it (launch bounds)."""
+    text = open(os.path.join(CSRC, "gemm_tc.cu")).read()
+    dense, int4 = (re.search(r"__launch_bounds__\((.*), ([^,]*)\) %s\(" % k, text).groups() for k in ("gemm_dense_kernel", "gemm_int4_kernel"))
+    assert dense == ("64 + 128 * NA", "2") and int4 == ("(3 + 4 * NG) * 32", "NG == 2 ? 2 : 1")
+    for fmt, fits, smem, columns, ksplit, na, mb, stages, stage_bytes in plans:
+        if fmt == 0 and 2 * (smem + RESERVE) <= SM:
+            assert columns == 256                                           # what the plan gives to the kernel of two groups alone
