@@ -123,7 +123,9 @@ __device__ __forceinline__ float4 load_cluster4(uint32_t a) {
   asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
   return v;
 }
+// (The aligned form wants whole warps: lanes that leave a loop at different times are brought together first.)
 __device__ __forceinline__ void cluster_meet() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // The mbarrier gets one arrival once every MMA issued so far by this thread has completed.
@@ -628,7 +630,6 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
   }
   if (NA == 1 && p.ksplit > 1) {
     if (p.pdl) wait_for_prerequisites();
-    __syncwarp();
     sum_cluster<BF16, EXT>(p, ctl, smem_s, ks, n0, m0, m_end, 64 + 128);
   }
   __syncthreads();
@@ -819,7 +820,6 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
   }
   if (p.ksplit > 1) {
     if (p.pdl) wait_for_prerequisites();
-    __syncwarp();
     sum_cluster<false, false>(p, ctl, smem_s, ks, n0, m0, p.M, THREADS);
   }
   __syncthreads();

@@ -467,8 +467,8 @@ __global__ void __cluster_dims__(TOP1_BLOCKS, 1, 1) __launch_bounds__(TOP1_THREA
       asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(av), "f"(bv) : "memory");
       asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(ai), "r"(bi) : "memory");
     }
-    __syncwarp();
   }
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (rank == 0 && warp == 0) {
     bv = lane < TOP1_BLOCKS ? best_v[lane] : -INFINITY;
