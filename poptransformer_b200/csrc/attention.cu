@@ -15,7 +15,7 @@
 namespace pt {
 
 struct AttnParams {
-  int ppb;         // pages per block
+  int runs;        // blocks that share the pages of a (sequence, kv head, part)
   int B, n_head, n_kv, qpk, qsplit, H, page, max_pages, max_len, rope_mode, softmax_mode, rot_half, out_ld, pdl;
   __half scale_h;
   int use_scale;
@@ -77,10 +77,10 @@ __device__ __forceinline__ uint32_t pack_f2h2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// One block = `ppb` consecutive pages of one (sequence, kv head, part of the group's q heads), one page after the other: while a page's
+// One block = a run of consecutive pages of one (sequence, kv head, part of the group's q heads), one page after the other: while a page's
 // weights are formed and multiplied, the K rows of the next are on their way to registers and its V tile to the other of two buffers.
-// The host takes as many pages per block as still leave about four blocks per SM: with one page per block the fixed cost of a block
-// (table look-up, rotation, partial results through L2, arrival) was most of the kernel.  (Measured on B200: see pages_per_block.)
+// The host fixes the number of runs (see runs_of_pages), and the pages in use, which only the device knows, are dealt out evenly: however
+// much room the table has behind the history, the same blocks share the work.
 // Both products run on the tensor cores
 // (mma.sync m16n8k16, fp32 accumulation of exact fp16 products):
 //   scores^T [keys x heads] = K [keys x H] . q^T: warp w takes keys 16 w .. 16 w + 15 of each 64-key pass.  Its K rows go from
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(kAttnThreads, 4) kv_append_attn_kernel(const A
   constexpr int QLD = H + 32;                              // q rows: two heads read in one shared-memory phase sit 16 banks apart
   const int PAGE = p.page, KP = (PAGE + 15) & ~15;         // keys padded to whole 16-key steps
   const int PSLD = KP + 8;                                 // row stride of the score / weight rows
-  __half *Vs0 = reinterpret_cast<__half *>(smem);          // [two of them if a block takes more than one page][KP][VLD]
-  __half *qs = Vs0 + (size_t)(p.ppb > 1 ? 2 : 1) * KP * VLD;                      // [NQ_MAX][QLD], rows >= nq are zero
+  __half *Vs0 = reinterpret_cast<__half *>(smem);          // [two of them if a block can have more than one page][KP][VLD]
+  __half *qs = Vs0 + (size_t)(p.runs < p.max_pages ? 2 : 1) * KP * VLD;           // [NQ_MAX][QLD], rows >= nq are zero
   __half *newk = qs + (size_t)NQ_MAX * QLD;                // [H]: the new token's rotated key (owner block)
   float *ps = reinterpret_cast<float *>(newk + H);         // [NQ_MAX][PSLD]
   float *ml = ps + (size_t)NQ_MAX * PSLD;                  // [NQ_MAX][2]
@@ -109,19 +109,23 @@ __global__ void __launch_bounds__(kAttnThreads, 4) kv_append_attn_kernel(const A
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
   // With many q heads per kv head (multi-query attention) the heads of a group are shared out over `qsplit` blocks: each
   // re-reads the group's K/V page (through L2) and handles nq of the group's heads.
-  const int pg0 = blockIdx.x * p.ppb, kvh = blockIdx.y / p.qsplit, qpart = blockIdx.y - kvh * p.qsplit, b = blockIdx.z;
+  const int run = blockIdx.x, kvh = blockIdx.y / p.qsplit, qpart = blockIdx.y - kvh * p.qsplit, b = blockIdx.z;
   const int nq = p.qpk / p.qsplit, q_lo = qpart * nq;   // this block's heads of the group: q_lo .. q_lo + nq - 1
   early_start();   // (the next kernel may fetch its weights meanwhile; everything this one reads was produced upstream)
-  // the page-table entry does not depend on the step: both loads go out together (one round trip less before the K / V loads)
-  int phys = p.page_table[(size_t)b * p.max_pages + pg0];
+  // The step decides which page is the first.  The table's first 32 entries are asked for together with it, one per lane, so that the K / V loads are
+  // still one round trip away.
+  const int *table = p.page_table + (size_t)b * p.max_pages;
+  const int my_entry = table[min(lane, p.max_pages - 1)];
   const int step = *p.step;
   if (step < 0 || step >= p.max_len) {  // no page / no RoPE row for this position: report it and leave the counters untouched
     if (tid == 0 && p.error_flag) atomicExch(p.error_flag, 12);
     return;
   }
-  const int n_pages = step / PAGE + 1;
+  const int n_pages = step / PAGE + 1, ppb = (n_pages + p.runs - 1) / p.runs, pg0 = run * ppb;
   if (pg0 >= n_pages) return;
-  const int pg1 = min(n_pages, pg0 + p.ppb), n_active = (n_pages + p.ppb - 1) / p.ppb;   // (blocks of this (sequence, kv head) that have pages)
+  const int pg1 = min(n_pages, pg0 + ppb), n_active = (n_pages + ppb - 1) / ppb;   // (blocks of this (sequence, kv head) that have pages)
+  auto entry = [&](int pg) { return pg < 32 ? __shfl_sync(0xffffffffu, my_entry, pg) : table[pg]; };   // (pg is the same in every thread)
+  int phys = entry(pg0);
   const bool has_last = pg1 == n_pages;
   const int slot = step - (n_pages - 1) * PAGE;      // where the new token goes in the last page
   const int row_elems = (p.n_head + 2 * p.n_kv) * H;
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(kAttnThreads, 4) kv_append_attn_kernel(const A
         gV[(size_t)slot * H + j] = Vs[(size_t)slot * VLD + j];
       }
     }
-    if (pg + 1 < pg1) phys = p.page_table[(size_t)b * p.max_pages + pg + 1];
+    if (pg + 1 < pg1) phys = entry(pg + 1);
 
     // ---- scores: keys 16 warp .. + 15 of every 64-key pass against the block's heads
     for (int kbase = warp * 16; kbase < n_valid; kbase += 64) {
@@ -289,7 +293,6 @@ __global__ void __launch_bounds__(kAttnThreads, 4) kv_append_attn_kernel(const A
       }
     }
   }
-  const int run = blockIdx.x;
   if (n_active == 1) {   // the whole history: the output
     if (g < nq) {
       const size_t col = ((size_t)kvh * p.qpk + q_lo + g) * H + warp * (H / 4) + 2 * tig;
@@ -472,11 +475,16 @@ extern "C" size_t pt_attn_workspace_bytes(int batch, int n_head, int head_dim, i
   return align256(heads * sizeof(int)) + align256(heads * max_pages * sizeof(float2)) + heads * max_pages * head_dim * sizeof(float);
 }
 
-// Pages of one block: as many as leave four blocks per SM if the whole table is in use (what the shared memory and registers of a block of
-// two V buffers admit at a time).  Measured on B200 as whole steps, one page per block and this: Llama 7B, 512 (row, kv head) pairs of 8 pages 3.58
-// and 3.38 ms, 1024 of 4 pages 3.73 and 3.52, GPT-2 XL, 400 of 4 pages 2.63 and 2.52, ChatGLM2, 64 of 18 pages level at 3.47.
-static int pages_per_block(int units, int max_pages) {
-  return std::max(1, std::min(max_pages, (int)((long long)units * max_pages / (4 * sm_count()))));
+// Blocks that share the pages of one of `units` (sequence, kv head, part): about four blocks per SM in all (what the registers and two V buffers
+// of a block admit at a time), and no more than the table has pages.  Rounded to the nearest: measured on B200, 32 heads of 128, context 511,
+// 9 / 16 rows 19.9 / 29.0 us, 25.2 / 34.8 with one more run each (a second, nearly empty wave of blocks).
+// The room behind the history costs nothing (a table of 11, 64 or 512 pages at context 511, 4 rows: 12.6 us each); one page per block took
+// 14.3, 17.1 and 72.8 us, runs of a length that fills the SMs when the whole table is in use 13.0, 24.0 and 23.6.
+// A table that is at most a quarter longer than that gives every page its own block, which then needs one V buffer: half the shared memory, and the
+// blocks of the product behind it find room earlier (ChatGLM2 at 8 rows, 32 units and 21 pages, whole steps: 2.79 ms against 2.82).
+static int runs_of_pages(int units, int max_pages) {
+  const int slots = 4 * sm_count();
+  return (long long)units * max_pages * 4 <= slots * 5LL ? max_pages : std::min(max_pages, std::max(1, (slots + units / 2) / units));
 }
 
 extern "C" int pt_kv_append_attn(const pt_attn_args *a, void *stream) {
@@ -524,13 +532,13 @@ extern "C" int pt_kv_append_attn(const pt_attn_args *a, void *stream) {
              a->max_len, a->page_size * a->max_pages);
   p.max_len = a->max_len > 0 ? a->max_len : a->page_size * a->max_pages;
 
-  p.ppb = pages_per_block(a->batch * a->n_kv * p.qsplit, a->max_pages);
+  p.runs = runs_of_pages(a->batch * a->n_kv * p.qsplit, a->max_pages);
   const int kp = (p.page + 15) & ~15;
-  const size_t smem = ((size_t)(p.ppb > 1 ? 2 : 1) * kp * (p.H + 8) + (size_t)NQ_MAX * (p.H + 32) + p.H) * sizeof(__half) +
+  const size_t smem = ((size_t)(p.runs < a->max_pages ? 2 : 1) * kp * (p.H + 8) + (size_t)NQ_MAX * (p.H + 32) + p.H) * sizeof(__half) +
                       ((size_t)NQ_MAX * (kp + 8) + (size_t)NQ_MAX * 2) * sizeof(float);
   PT_REQUIRE(smem <= 200 * 1024, "pt_kv_append_attn: tile needs %zu bytes of shared memory", smem);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ceil_div(a->max_pages, p.ppb), a->n_kv * p.qsplit, a->batch);
+  cfg.gridDim = dim3(p.runs, a->n_kv * p.qsplit, a->batch);
   cfg.blockDim = dim3(kAttnThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = as_stream(stream);
