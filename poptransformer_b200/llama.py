@@ -476,9 +476,9 @@ class LlamaDecoder(DecodeLoop):
             return
         for L in self.layers:
             self._norm_linear(self.x, L["ln1"], L["qkv"], self.qkv)
-            ops.linear(self.attn, L["o"], self.part, workspace=self.lin_ws)
+            ops.linear_fp16(self.attn, L["o"], self.part, workspace=self.lin_ws)
             self._norm_linear_raw(self.x, L["ln2"], L["gu"], self.act.data_ptr(), self.act.shape[1])
-            ops.linear(self.act, L["down"], self.part, workspace=self.lin_ws)
+            ops.linear_fp16(self.act, L["down"], self.part, workspace=self.lin_ws)
 
     def reset(self, input_ids):
         """input_ids int32 [batch, max_len] (host or device), right-padded with pad_id; step <- 0."""
