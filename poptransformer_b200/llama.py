@@ -339,7 +339,7 @@ class LlamaDecoder(DecodeLoop):
     def _row_parallel(self, x_in, pl):
         """x <- fp16(x + all_reduce(fp16(x_in . W_r^T)))  (Linear 'end' + ops.add, llama2/model.py:42,45)."""
         if self.tp == 1:
-            ops.linear_fp16(x_in, pl, self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, workspace=self.lin_ws, pdl=self.pdl)
+            ops.linear_fp16(x_in, pl, self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, workspace=self.lin_ws, error_flag=self.error_flag, pdl=self.pdl)
         else:
             ops.linear(x_in, pl, self.part, workspace=self.lin_ws, pdl=self.pdl)
             self._all_reduce(self.part)

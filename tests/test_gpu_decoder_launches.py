@@ -29,3 +29,65 @@ def test_linears_alone(cuda, batch, group):
         w = torch.stack([w >> 4, (w << 4) >> 4], 2).reshape(w.shape[0], -1).double() * sd[key + "_scale"].reshape(w.shape[0], -1).double().repeat_interleave(group, 1)
     want = dec.act.double() @ w.to(cuda).double().T
     assert float((dec.part.double() - want).norm() / want.norm()) < 2e-3      # fp16 rounding of the result and, on the GEMM, of nibble times scale
+
+
+class _Calls:
+    """Records what is passed to ops.gemm, ops.linear, ops.linear_args and ops.attn_args."""
+
+    def __init__(self, monkeypatch):
+        from poptransformer_b200 import ops
+        self.gemm, self.linear, self.attn = [], [], []
+        gemm, linear_args, attn_args = ops.gemm, ops.linear_args, ops.attn_args
+
+        def seen_gemm(*a, **kw):
+            self.gemm.append(kw)
+            return gemm(*a, **kw)
+
+        def seen_linear(*a, **kw):
+            self.linear.append(kw)
+            return linear_args(*a, **kw)
+
+        def seen_attn(*a, **kw):
+            self.attn.append(kw)
+            return attn_args(*a, **kw)
+
+        monkeypatch.setattr(ops, "gemm", seen_gemm)
+        monkeypatch.setattr(ops, "linear_args", seen_linear)
+        monkeypatch.setattr(ops, "attn_args", seen_attn)
+
+
+def _decoders(cuda, only=None, **kw):
+    """name -> a decoder with its linears on the GEMM (kw: constructor arguments that all take, pdl / pdl_linear / pdl_attn as each has them)."""
+    from poptransformer_b200 import chatglm2, gpt2, rwkv, synth
+    off = kw.pop("off", False)
+    both = dict(pdl_linear=0, pdl_attn=0) if off else {}
+    g2 = dict(n_layer=2, d_model=256, n_head=4, vocab=500, n_positions=64)
+    glm = dict(n_layer=2, d_model=512, n_head=4, n_group=2, ffn=768, vocab=1000)
+    rw = dict(n_layer=2, d_model=256, ffn=512, vocab=500)
+    make = {
+        "llama fp16": lambda: _llama(cuda, 4, 0, **(dict(pdl=False) if off else {})),
+        "llama int4": lambda: _llama(cuda, 12, 128, prefill=True, **(dict(pdl=False) if off else {})),
+        "gpt2": lambda: gpt2.GPT2Decoder(gpt2.GPT2Config(**g2, max_len=64), synth.gpt2_state_dict(**g2, seed=1), 3, device=cuda, **both),
+        "chatglm2 fp16": lambda: chatglm2.ChatGLM2Decoder(chatglm2.ChatGLM2Config(**glm, max_len=64), synth.chatglm2_state_dict(**glm, seed=1), 3, device=cuda, **both),
+        "chatglm2 fp8": lambda: chatglm2.ChatGLM2Decoder(chatglm2.ChatGLM2Config(**glm, max_len=64, precision="fp8"), synth.chatglm2_state_dict(**glm, seed=1, precision="fp8"), 8,
+                                                         device=cuda, **both),
+        "rwkv": lambda: rwkv.RWKVDecoder(rwkv.RWKVConfig(**rw, max_len=64), synth.rwkv_state_dict(**rw, seed=1), 3, device=cuda, **({"pdl_linear": 0} if off else {})),
+    }
+    return {k: f() for k, f in make.items()}
+
+
+def _ids(dec):
+    from poptransformer_b200 import synth
+    return synth.prompt_ids(dec.batch, 6, dec.cfg.max_len, dec.cfg.vocab, dec.pad_id, seed=5)
+
+
+def test_products_can_report(cuda, monkeypatch):
+    """A product whose waits run out leaves its output as it was: the decoder's error flag is the only sign of it."""
+    for name, dec in _decoders(cuda).items():
+        seen = _Calls(monkeypatch)
+        dec.reset(_ids(dec))
+        if name == "llama int4":
+            dec.prefill()
+        dec.step()
+        assert seen.gemm and all(kw.get("error_flag") is dec.error_flag for kw in seen.gemm), name
+        monkeypatch.undo()
