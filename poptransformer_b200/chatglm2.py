@@ -21,7 +21,7 @@ from .loop import DecodeLoop
 from .tp import multi_query_head_index, rows, vocab_rows
 
 
-# Programmatic dependent launch of the (linear, attention) kernels; off by default: measured neutral to 4 % slower at 8 rows on B200.
+# Programmatic dependent launch of the (skinny-matmul linear, attention) kernels; off by default: measured neutral to 4 % slower at 8 rows on B200.
 PDL_DEFAULT = (0, 0)
 
 
@@ -51,7 +51,8 @@ class ChatGLM2Decoder(DecodeLoop):
         Default: from 8 rows on one GPU (measured on B200 at 8 rows, 65024 x 4096: 45 us against 70 us for the skinny-matmul
         kernel), when every k is a multiple of 128."""
         c = cfg
-        self.pdl_linear, self.pdl_attn = PDL_DEFAULT[0] if pdl_linear is None else int(pdl_linear), PDL_DEFAULT[1] if pdl_attn is None else int(pdl_attn)
+        # (linears on the GEMM, and the attention in front of one, start early unless that is switched off)
+        self.pdl_linear, self.pdl_gemm = (PDL_DEFAULT[0], 1) if pdl_linear is None else (int(pdl_linear), int(pdl_linear))
         self.tp, self.rank, self.group = tp_size, tp_rank, group
         tp, r = tp_size, tp_rank
         if (c.n_head // c.n_group) % tp or c.ffn % tp:
@@ -103,6 +104,7 @@ class ChatGLM2Decoder(DecodeLoop):
                 "gu": packed([p + "mlp.dense_h_to_4h_1.weight", p + "mlp.dense_h_to_4h_2.weight"], "norm", interleave=True, pick=[start, start]),
                 "down": packed([p + "mlp.dense_4h_to_h.weight"], "mlp", pick=[lambda w: w[:, r * self.f_loc:(r + 1) * self.f_loc]]),
             })
+        self.pdl_attn = int(PDL_DEFAULT[1] or isinstance(self.layers[0]["dense"], ops.GemmWeight)) if pdl_attn is None else int(pdl_attn)
         self.norm = t("transformer.encoder.final_layernorm.weight").contiguous()
         self.vocab_loc = -(-c.vocab // tp) if tp > 1 else c.vocab
         self.head = packed(["transformer.output_layer.weight"], "norm", pick=[(lambda w: vocab_rows(w, r, tp)[0]) if tp > 1 else None])
@@ -145,7 +147,7 @@ class ChatGLM2Decoder(DecodeLoop):
                 ops.check(ops._lib.lib().pt_rms_norm(ops._ptr(x), None, ops._ptr(gamma), self.batch, self.cfg.d_model, self.cfg.eps, ops._ptr(self.h), None,
                                                      ops._stream()), "pt_rms_norm")
                 x = self.h
-            ops.gemm(x, pl, out=out, epilogue=epilogue, bias=bias, residual=residual, error_flag=self.error_flag, pdl=1)
+            ops.gemm(x, pl, out=out, epilogue=epilogue, bias=bias, residual=residual, error_flag=self.error_flag, pdl=self.pdl_gemm)
             return
         fp8 = pl.wfmt == ops.W_FP8
         pro = (ops.PRO_RMSNORM_CAST_FP8 if fp8 else ops.PRO_RMSNORM) if gamma is not None else (ops.PRO_CAST_FP8 if fp8 else ops.PRO_NONE)
@@ -175,14 +177,14 @@ class ChatGLM2Decoder(DecodeLoop):
             return self.x8.view(-1)[:B * d].view(B, d)
 
         def gemm(x8, pl, out, **kw):
-            ops.gemm(x8, pl, out=out, x_scale=pl.act_scale, error_flag=self.error_flag, pdl=1, **kw)
+            ops.gemm(x8, pl, out=out, x_scale=pl.act_scale, error_flag=self.error_flag, pdl=self.pdl_gemm, **kw)
 
         ops.embedding(self.emb, self.ids, self.step_t, out=self.x)
         for li, L in enumerate(self.layers):
             gemm(norm_cast(L["ln1"], L["qkv"]), L["qkv"], self.qkv, epilogue=ops.EPI_BIAS, bias=L["b_qkv"])
             a8 = self.x8.view(-1)[:B * self.d_loc].view(B, self.d_loc)      # the attention kernel writes dense's E4M3 input itself
             a = ops.attn_args(self.qkv, self.step_t, self.caches[li], self.attn, self.h_loc, ops.ROPE_CHATGLM2, ops.SOFTMAX_F16, self.score_scale,
-                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=self.pdl_attn or isinstance(L["dense"], ops.GemmWeight), out_fp8=a8, out_fp8_scale=L["dense"].act_scale)
+                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=self.pdl_attn, out_fp8=a8, out_fp8_scale=L["dense"].act_scale)
             ops.check(L_.pt_kv_append_attn(ctypes.byref(a), st()), "pt_kv_append_attn")
             gemm(a8, L["dense"], self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x)
             gemm(norm_cast(L["ln2"], L["gu"]), L["gu"], self.gu_out)
@@ -201,7 +203,7 @@ class ChatGLM2Decoder(DecodeLoop):
         for li, L in enumerate(self.layers):
             self._linear(self.x, L["qkv"], self.qkv, "norm", gamma=L["ln1"], epilogue=ops.EPI_BIAS, bias=L["b_qkv"])
             a = ops.attn_args(self.qkv, self.step_t, self.caches[li], self.attn, self.h_loc, ops.ROPE_CHATGLM2, ops.SOFTMAX_F16, self.score_scale,
-                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=self.pdl_attn or isinstance(L["dense"], ops.GemmWeight))
+                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=self.pdl_attn)
             ops.check(L_.pt_kv_append_attn(ctypes.byref(a), ops._stream()), "pt_kv_append_attn")
             self._row_parallel(self.attn, L["dense"], "attn")
             self._linear(self.x, L["gu"], self.act, "norm", gamma=L["ln2"], epilogue=ops.EPI_SWIGLU)

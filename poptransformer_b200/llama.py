@@ -57,6 +57,7 @@ class LlamaDecoder(DecodeLoop):
         """tp_buffers: for tp_size > 1, the exchange buffers of all ranks as this process sees them (a list of tp_size int32 CUDA
         tensors of pt_llama_tp_buffer_bytes each, entry tp_rank being local memory, the others peer mappings the caller set up).
         Default: the buffers are allocated as symmetric memory over `group` (torch.distributed).
+        pdl: the linears and the decode attention are launched early (pt_linear_args.pdl).
         prefill: also keep the weights in the tcgen05 GEMM's tiling so that `prefill()` can ingest a prompt in one pass.
         wait_limit: trip limit of the persistent kernel's polling loops (0 = the library default, about two seconds)."""
         self.cfg, self.batch, self.device = cfg, batch, device
@@ -316,7 +317,7 @@ class LlamaDecoder(DecodeLoop):
         if isinstance(pl, ops.GemmWeight):
             ops.check(ops._lib.lib().pt_rms_norm(ops._ptr(x), None, ops._ptr(gamma), x.shape[0], x.shape[1], self.cfg.eps, ops._ptr(self.h), None,
                                                  ops._stream()), "pt_rms_norm")
-            ops.gemm(self.h, pl, out=out, epilogue=epilogue, out_ld=out_ld, error_flag=self.error_flag, pdl=1)
+            ops.gemm(self.h, pl, out=out, epilogue=epilogue, out_ld=out_ld, error_flag=self.error_flag, pdl=self.pdl)
             return
         if x.shape[0] > 32:
             # beyond the skinny-matmul kernels' 32 rows (the fp16 LM head of a large batch, whose transformer linears run on the
@@ -382,14 +383,14 @@ class LlamaDecoder(DecodeLoop):
 
         for li, L in enumerate(self.layers):
             norm(L["ln1"])
-            ops.gemm(self.h, L["qkv"], out=self.qkv, error_flag=self.error_flag, pdl=1)
+            ops.gemm(self.h, L["qkv"], out=self.qkv, error_flag=self.error_flag, pdl=self.pdl)
             a = ops.attn_args(self.qkv, self.step_t, self.caches[li], self.attn, self.h_loc, ops.ROPE_LLAMA, ops.SOFTMAX_F32, self.score_scale,
-                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=1)
+                              self.sin, self.cos, self.attn_ws, self.error_flag, pdl=self.pdl)
             ops.check(L_.pt_kv_append_attn(ctypes.byref(a), ops._stream()), "pt_kv_append_attn")
-            ops.gemm(self.attn, L["o"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, error_flag=self.error_flag, pdl=1)
+            ops.gemm(self.attn, L["o"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, error_flag=self.error_flag, pdl=self.pdl)
             norm(L["ln2"])
-            ops.gemm(self.h, L["gu"], out=self.act, out_ld=self.act.shape[1], epilogue=ops.EPI_SWIGLU, error_flag=self.error_flag, pdl=1)
-            ops.gemm(self.act, L["down"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, error_flag=self.error_flag, pdl=1)
+            ops.gemm(self.h, L["gu"], out=self.act, out_ld=self.act.shape[1], epilogue=ops.EPI_SWIGLU, error_flag=self.error_flag, pdl=self.pdl)
+            ops.gemm(self.act, L["down"], out=self.x, epilogue=ops.EPI_RESIDUAL, residual=self.x, error_flag=self.error_flag, pdl=self.pdl)
 
     def prefill(self, n_tokens=None, chunk=1024):
         """Ingests the first `n_tokens` positions of every sequence in one pass (the work of the reference's first stage,
@@ -428,12 +429,12 @@ class LlamaDecoder(DecodeLoop):
 
             for li, L in enumerate(self.pf_layers):
                 norm(L["ln1"])
-                ops.gemm(w.h, L["qkv"], out=w.qkv, error_flag=self.error_flag, pdl=1)
+                ops.gemm(w.h, L["qkv"], out=w.qkv, error_flag=self.error_flag, pdl=self.pdl)
                 ops.prefill_attn(w.qkv, self.caches[li], B, P, s0, c.n_head, self.score_scale, self.sin, self.cos, out=w.attn)
-                ops.gemm(w.attn, L["o"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, error_flag=self.error_flag, pdl=1)
+                ops.gemm(w.attn, L["o"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, error_flag=self.error_flag, pdl=self.pdl)
                 norm(L["ln2"])
-                ops.gemm(w.h, L["gu"], out=w.act, epilogue=ops.EPI_SWIGLU, error_flag=self.error_flag, pdl=1)
-                ops.gemm(w.act, L["down"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, error_flag=self.error_flag, pdl=1)
+                ops.gemm(w.h, L["gu"], out=w.act, epilogue=ops.EPI_SWIGLU, error_flag=self.error_flag, pdl=self.pdl)
+                ops.gemm(w.act, L["down"], out=w.x, epilogue=ops.EPI_RESIDUAL, residual=w.x, error_flag=self.error_flag, pdl=self.pdl)
         self.step_t.fill_(n)
         return n
 

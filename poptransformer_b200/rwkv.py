@@ -20,7 +20,7 @@ from .loop import DecodeLoop
 from .tp import rows, vocab_rows
 
 
-# Programmatic dependent launch of the linear kernels; off by default: measured 2 % slower at 32 rows on B200.
+# Programmatic dependent launch of the skinny-matmul linears; off by default: measured 2 % slower at 32 rows on B200.
 PDL_DEFAULT = 0
 
 
@@ -33,7 +33,8 @@ class RWKVConfig:
 class RWKVDecoder(DecodeLoop):
     def __init__(self, cfg, state_dict, batch, device="cuda", pad_id=None, eos_id=-1, tp_rank=0, tp_size=1, group=None, pdl_linear=None, early_stop=False):
         c = cfg
-        self.pdl_linear = PDL_DEFAULT if pdl_linear is None else int(pdl_linear)
+        # (linears on the GEMM start early unless that is switched off)
+        self.pdl_linear, self.pdl_gemm = (PDL_DEFAULT, 1) if pdl_linear is None else (int(pdl_linear), int(pdl_linear))
         self.tp, self.rank, self.group = tp_size, tp_rank, group
         tp, r = tp_size, tp_rank
         if c.d_model % (32 * tp) or c.ffn % (32 * tp):
@@ -105,7 +106,7 @@ class RWKVDecoder(DecodeLoop):
         """side = None: on the current stream; side = i: on side stream i (between _fork and _join), with that stream's workspace."""
         # (early start: the GEMM only, and only behind a kernel of the same stream)
         kw = dict(epilogue=epilogue, residual=residual, workspace=self.lin_ws if side is None else self.side_ws[side], error_flag=self.error_flag,
-                  pdl=1 if side is None and isinstance(pl, ops.GemmWeight) else self.pdl_linear)
+                  pdl=self.pdl_gemm if side is None and isinstance(pl, ops.GemmWeight) else self.pdl_linear)
         if side is None:
             ops.linear_fp16(x, pl, out, **kw)
         else:

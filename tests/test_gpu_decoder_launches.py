@@ -91,3 +91,22 @@ def test_products_can_report(cuda, monkeypatch):
         dec.step()
         assert seen.gemm and all(kw.get("error_flag") is dec.error_flag for kw in seen.gemm), name
         monkeypatch.undo()
+
+
+def test_early_starts_can_be_switched_off(cuda, monkeypatch):
+    outs = []
+    for off in (False, True):
+        for name, dec in _decoders(cuda, off=off).items():
+            seen = _Calls(monkeypatch)
+            dec.reset(_ids(dec))
+            if name == "llama int4":
+                dec.prefill()
+            dec.step()
+            early = [int(kw.get("pdl", 0)) for kw in seen.gemm + seen.linear + seen.attn]
+            assert seen.gemm and not any(early) if off else any(early), (name, off)
+            if not off and name != "rwkv":       # (products on side streams have no launch of their stream in front)
+                assert all(early), name
+            outs.append(dec.logits.clone())
+            monkeypatch.undo()
+    n = len(outs) // 2
+    assert all(torch.equal(a, b) for a, b in zip(outs[:n], outs[n:]))
