@@ -143,7 +143,13 @@ def linear(x, pl, out=None, **kw):
     return out
 
 
-# ------------------------------------------------------------------------------------------ tensor-core GEMMs (16+ rows)
+# ------------------------------------------------------------------------------------------ tensor-core GEMMs
+def aligned(t):
+    """t, contiguous and on a 16-byte boundary: a checkpoint's tensors may be views into one buffer."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class GemmWeight:
     """A weight matrix tiled once for pt_gemm (pt_gemm_repack): FP8 bytes [n_out, k], or INT4 rows in the reference's int8
     [n_out, k/2] format plus fp16 scales [n_out, k/group], or float16 or bfloat16 [n_out, k]."""
@@ -166,7 +172,7 @@ class GemmWeight:
         else:
             raise PtError("GemmWeight: INT4, FP8, FP16 or BF16")
         self.w = torch.empty(L.pt_gemm_packed_bytes(wfmt, self.n_out, self.k_in), dtype=torch.uint8, device=w.device)
-        check(L.pt_gemm_repack(wfmt, _ptr(w.contiguous()), self.n_out, self.k_in, _ptr(self.w), _stream()), "pt_gemm_repack")
+        check(L.pt_gemm_repack(wfmt, _ptr(aligned(w)), self.n_out, self.k_in, _ptr(self.w), _stream()), "pt_gemm_repack")
 
     @property
     def nbytes(self):

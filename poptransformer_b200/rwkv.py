@@ -46,7 +46,7 @@ class RWKVDecoder(DecodeLoop):
         self.eos_id = eos_id
         self._init_loop(device, early_stop)
         dev = device
-        h = lambda k: state_dict[k].to(dev).to(torch.float16).reshape(-1).contiguous()
+        h = lambda k: ops.aligned(state_dict[k].to(dev).to(torch.float16).reshape(-1))
         f = lambda k: state_dict[k].to(dev).to(torch.float32).reshape(-1)[r * dl:(r + 1) * dl].contiguous()   # sharded with the channels
         w16 = lambda k: state_dict[k].to(dev).to(torch.float16)
         pack = (lambda w: ops.fp16_linear(w)) if tp == 1 else (lambda w: ops.PackedLinear(ops.W_FP16, w))
