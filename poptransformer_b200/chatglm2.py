@@ -134,7 +134,7 @@ class ChatGLM2Decoder(DecodeLoop):
             page_table = kc.page_table
             self.caches.append(kc)
         self.attn_ws = ops.attn_workspace(B, self.h_loc, c.head_dim, self.caches[0].max_pages, dev)
-        self.lin_ws = ops.linear_workspace(B, max(2 * self.f_loc, self.vocab_loc, self.qkv.shape[1], d), 16, dev)
+        self.lin_ws = ops.packed_workspace([self.head] + [L[k] for L in self.layers for k in ("qkv", "dense", "gu", "down")], B, dev)
         if self.use_gemm:
             self.x8 = torch.empty((B, max(d, self.f_loc)), dtype=torch.uint8, device=dev)      # the E4M3 input of the running linear
             self.gu_out = torch.empty((B, 2 * self.f_loc), **f16)

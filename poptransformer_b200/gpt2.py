@@ -102,7 +102,7 @@ class GPT2Decoder(DecodeLoop):
             page_table = kc.page_table
             self.caches.append(kc)
         self.attn_ws = ops.attn_workspace(B, self.h_loc, c.head_dim, self.caches[0].max_pages, dev)
-        self.lin_ws = ops.linear_workspace(B, max(4 * d, self.vocab_loc), 16, dev)
+        self.lin_ws = ops.packed_workspace([self.head] + [L[k] for L in self.layers for k in ("c_attn", "c_proj", "c_fc", "m_proj")], B, dev)
         self.graph = None
         torch.cuda.synchronize()
 

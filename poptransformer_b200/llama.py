@@ -212,7 +212,7 @@ class LlamaDecoder(DecodeLoop):
             page_table = kc.page_table
             self.caches.append(kc)
         self.attn_ws = ops.attn_workspace(B, self.h_loc, c.head_dim, self.caches[0].max_pages, dev)
-        self.lin_ws = ops.linear_workspace(B, max(3 * self.d_loc, 2 * self.f_loc, d, self.logits.shape[1]), 16, dev)
+        self.lin_ws = ops.packed_workspace([self.head] + [L[k] for L in self.layers for k in ("qkv", "o", "gu", "down")], B, dev)
         self.graph = None
         # The persistent whole-step kernel covers INT4, batch <= 2, on one GPU or tensor-parallel over up to 8 (the all-reduces are
         # then fused into the kernel as peer stores); everything else takes the per-op kernels and NCCL.

@@ -114,6 +114,12 @@ def linear_workspace(batch, n_out_max, max_ksplit=16, device="cuda"):
     return torch.zeros(n, dtype=torch.uint8, device=device)
 
 
+def packed_workspace(linears, batch, device="cuda"):
+    """`linear_workspace` for those of `linears` that the skinny-matmul kernel serves; None if it serves none."""
+    widths = [x.n_out for x in linears if isinstance(x, PackedLinear)]
+    return linear_workspace(batch, max(widths), 16, device) if widths else None
+
+
 def linear_args(x, pl, out, prologue=PRO_NONE, epilogue=EPI_STORE, gamma=None, eps=0.0, act_scale=0.0, bias=None,
                 residual=None, workspace=None, ksplit=0, out_ld=0, pdl=0, error_flag=None, beta=None, alpha=1.0, ext=None):
     a = LinearArgs()

@@ -110,3 +110,11 @@ def test_early_starts_can_be_switched_off(cuda, monkeypatch):
             monkeypatch.undo()
     n = len(outs) // 2
     assert all(torch.equal(a, b) for a, b in zip(outs[:n], outs[n:]))
+
+
+def test_no_workspace_that_nothing_uses(cuda):
+    """Only the skinny-matmul kernels sum k-slices in a workspace (16 slices x rows x outputs in fp32)."""
+    for name, dec in _decoders(cuda).items():
+        assert dec.lin_ws is None and not any(w is not None for w in getattr(dec, "side_ws", [])), name
+    few = _llama(cuda, 1, 0)                                      # fp16 blocks on the GEMM, the output layer on the skinny-matmul kernel
+    assert few.lin_ws is not None and few.lin_ws.numel() < 16 * LLAMA["vocab"] * 4 + (1 << 20)
