@@ -549,12 +549,12 @@ extern "C" int pt_kv_append_attn(const pt_attn_args *a, void *stream) {
   cfg.numAttrs = p.pdl ? 1 : 0;
   cudaError_t le;
   if (p.H == 128) {
-    static bool set128 = false;
-    if (!set128) { PT_CUDA(cudaFuncSetAttribute(kv_append_attn_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); set128 = true; }
+    static std::atomic<uint64_t> allowed{0};
+    PT_CUDA(allow_smem(kv_append_attn_kernel<128>, 200 * 1024, allowed));
     le = cudaLaunchKernelEx(&cfg, kv_append_attn_kernel<128>, p);
   } else {
-    static bool set64 = false;
-    if (!set64) { PT_CUDA(cudaFuncSetAttribute(kv_append_attn_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); set64 = true; }
+    static std::atomic<uint64_t> allowed{0};
+    PT_CUDA(allow_smem(kv_append_attn_kernel<64>, 200 * 1024, allowed));
     le = cudaLaunchKernelEx(&cfg, kv_append_attn_kernel<64>, p);
   }
   if (le != cudaSuccess) return pt::set_error(PT_ERR_CUDA, "pt_kv_append_attn: %s", cudaGetErrorString(le));

@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/pt_b200.h"
 
 namespace pt {
@@ -65,6 +67,17 @@ static inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, dim3 blo
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Raises a kernel's limit of dynamic shared memory, which every device of the process keeps for itself, once on each.  `done`: a static of the caller.
+template <typename K> static inline cudaError_t allow_smem(K *kernel, int bytes, std::atomic<uint64_t> &done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const uint64_t bit = 1ull << (dev & 63);
+  if (e != cudaSuccess || (done.load(std::memory_order_relaxed) & bit)) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
 }
 
 // ---- fp16 arithmetic with the reference's "one rounding per op" semantics -------------

@@ -282,11 +282,8 @@ extern "C" int pt_prefill_attn(const pt_prefill_attn_args *a, void *stream) {
   const bool vec = (((uintptr_t)a->qkv | (uintptr_t)a->rope_sin | (uintptr_t)a->rope_cos | (uintptr_t)a->pool) & 15) == 0;
   launch_early(vec ? pf::prefill_rope_kv_kernel<true> : pf::prefill_rope_kv_kernel<false>, a->batch * a->n_tokens, pf::ROPE_THREADS, 0, as_stream(stream), p);
   PT_LAUNCH_CHECK("pt_prefill_attn");
-  static bool set = false;
-  if (!set) {
-    PT_CUDA(cudaFuncSetAttribute(pf::prefill_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)sizeof(pf::Tile)));
-    set = true;
-  }
+  static std::atomic<uint64_t> allowed{0};
+  PT_CUDA(allow_smem(pf::prefill_attn_kernel, 2 * (int)sizeof(pf::Tile), allowed));
   launch_early(pf::prefill_attn_kernel, dim3(ceil_div(a->n_tokens, pf::BQ), a->n_head, a->batch), pf::THREADS, 2 * sizeof(pf::Tile), as_stream(stream), p);
   PT_LAUNCH_CHECK("pt_prefill_attn");
   return PT_OK;
