@@ -27,21 +27,6 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr int TILE = 64;             // page size of the tensor-core kernel
 constexpr int kMaxSplit = 32;
 
-// A launch that may start before the kernel in front of it has ended; the kernel waits before it reads what that one wrote.
-template <typename... A, typename... B> static cudaError_t launch_early(void (*kernel)(A...), dim3 grid, int threads, size_t smem, cudaStream_t st, B... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // ------------------------------------------------------------------------------------------ norms, rotation, append
 struct PrepParams {
   int q_rank, rank, rot, row_ld, page, max_pages, max_len, ld, cq_ld;
@@ -621,7 +606,7 @@ extern "C" int pt_latent_prep(const pt_latent_prep_args *a, void *stream) {
   const bool v4 = a->q_rank % 4 == 0 && a->rank % 4 == 0 && a->rot_dim % 4 == 0 && a->ld % 4 == 0 && a->cq_ld % 4 == 0 && al(a->q) && al(a->kv) && al(a->cq) && al(a->pool) &&
                   aligned_to(a->q_norm, 16) && aligned_to(a->kv_norm, 16);
   auto kernel = a->dtype == PT_DT_F32 ? (v4 ? lat::prep_kernel<float, 4> : lat::prep_kernel<float, 1>) : (v4 ? lat::prep_kernel<__nv_bfloat16, 4> : lat::prep_kernel<__nv_bfloat16, 1>);
-  PT_CUDA(lat::launch_early(kernel, dim3(b.n_tok), lat::PREP_THREADS, 0, as_stream(stream), p));
+  PT_CUDA(launch_early(kernel, dim3(b.n_tok), lat::PREP_THREADS, 0, as_stream(stream), p));
   count_launch();
   return PT_OK;
 }
@@ -684,14 +669,14 @@ extern "C" int pt_latent_attn(const pt_latent_attn_args *a, void *stream) {
     ws += lat::align256((size_t)b.n_tok * a->n_head * p.n_split * a->rank * sizeof(float));
     p.o_lat = ws;
     const int tokens16 = ceil_div(b.n_tok, 16);
-    PT_CUDA(lat::launch_early(lat::absorb_kernel, dim3(ceil_div(a->rank, 16 * lat::ABSORB_WARPS), a->n_head, tokens16), lat::ABSORB_WARPS * 32, 0, st, p));
+    PT_CUDA(launch_early(lat::absorb_kernel, dim3(ceil_div(a->rank, 16 * lat::ABSORB_WARPS), a->n_head, tokens16), lat::ABSORB_WARPS * 32, 0, st, p));
     count_launch();
     if (int rc = lat::dispatch_decode(p, lat::two_tiles(a->n_head, p.row_ld), st)) return rc;
-    PT_CUDA(lat::launch_early(lat::combine_kernel, dim3(a->n_head, b.n_tok), lat::COMBINE_THREADS, 0, st, p));
+    PT_CUDA(launch_early(lat::combine_kernel, dim3(a->n_head, b.n_tok), lat::COMBINE_THREADS, 0, st, p));
     count_launch();
     p.ng = 2;
     while (p.ng < lat::EXPAND_WARPS && (long long)ceil_div(a->vdim, 16 * p.ng) * a->n_head * tokens16 > 2 * sm_count()) p.ng *= 2;
-    PT_CUDA(lat::launch_early(lat::expand_kernel, dim3(ceil_div(a->vdim, 16 * p.ng), a->n_head, tokens16), lat::EXPAND_WARPS * 32, 0, st, p));
+    PT_CUDA(launch_early(lat::expand_kernel, dim3(ceil_div(a->vdim, 16 * p.ng), a->n_head, tokens16), lat::EXPAND_WARPS * 32, 0, st, p));
     count_launch();
     return PT_OK;
   }
