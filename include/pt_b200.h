@@ -176,11 +176,10 @@ int pt_linear(const pt_linear_args *args, void *stream);
  *   - Nothing is allocated or freed, by this call or on its behalf. */
 int pt_linear_static_scratch(const pt_linear_args *args, void *stream);
 
-/* ---- tensor-core GEMMs for 16 or more activation rows (batched decode, prefill) ---------------------------------
+/* ---- tensor-core GEMMs (decode steps of any number of rows, prompts) ---------------------------------------------
  * The same layers as pt_linear (Linear.__call__ -> ParamHandler.matmul, poptransformer/layers/linear.py:42-46,
- * utils/param_handler/precision_strategy.py:56-81) when the batch no longer fits a matrix-vector kernel: the reference issues
- * one PopLibs matmul per layer whatever the batch (ops/popart.py:55-67); here 16 or more rows go to tcgen05 / tensor-memory
- * GEMMs fed by TMA.
+ * utils/param_handler/precision_strategy.py:56-81) on tcgen05 / tensor-memory GEMMs fed by TMA, for any number of rows: the
+ * reference issues one PopLibs matmul per layer whatever the batch (ops/popart.py:55-67).
  *   PT_W_FP8 : x = E4M3 bytes [m, k_in] (pt_cast_fp8 with x_scale), w = E4M3 bytes [n_out, k_in], out = fp16((x . w^T) * x_scale
  *              * w_scale) - the FP8MatMul op (custom_ops/matmul_fp8.cpp:885-1091).  w is either row-major as the checkpoint
  *              stores it (w_tiled = 0: what FP8MatMul passes; fetched with strided TMA boxes) or tiled once by pt_gemm_repack
@@ -189,16 +188,19 @@ int pt_linear_static_scratch(const pt_linear_args *args, void *stream);
  *              [n_out, k_in/group]; every weight becomes fp16(q) * scale with one rounding (Int4ToHalf,
  *              custom_ops/int4_to_half_codelets.cpp:18-38) on its way to the tensor core.  Also epilogue PT_EPI_SWIGLU: rows in the
  *              interleaved order of pt_linear_repack (eight gate rows, the same eight up rows), out [m, n_out / 2].
+ *   PT_W_FP16: x = fp16 [m, k_in], w = pt_gemm_repack of fp16 [n_out, k_in] (w_tiled = 1), out = fp16.  k_in a multiple of 64.  Also epilogues
+ *              PT_EPI_BIAS_GELU, _BIAS_RESIDUAL, _RELU2 and, with rows interleaved as for INT4, _SWIGLU.
  *   PT_W_BF16: x = bf16 [m, k_in], w = pt_gemm_repack of bf16 [n_out, k_in] (w_tiled = 1); out = bf16 or fp32 (out_dtype),
  *              epilogue PT_EPI_STORE, _RELU2, _GLU or _GELU_MUL on alpha * (x . w^T).  k_in a multiple of 64.
  * FP8 and INT4: k_in must be a multiple of 128.  Accumulation is fp32.  k-slices (ksplit, 0 = chosen by the library) are summed in a fixed
- * order; with more than one slice a workspace is needed (zeroed once by the caller; every launch leaves its counters at zero). */
+ * order in the shared memory of a cluster, at most eight whatever was asked for.  A caller that asks for slices itself (ksplit > 1) still has
+ * to hand over a workspace of pt_gemm_workspace_bytes, which nothing touches. */
 typedef struct pt_gemm_args {
-  int wfmt;               /* PT_W_FP8, PT_W_INT4 or PT_W_BF16                       */
+  int wfmt;               /* PT_W_FP8, PT_W_INT4, PT_W_FP16 or PT_W_BF16            */
   int m, n_out, k_in;
   int group;              /* INT4: scale group along k (a multiple of 128)          */
-  int epilogue;           /* PT_EPI_STORE, PT_EPI_RESIDUAL, PT_EPI_BIAS or (INT4) PT_EPI_SWIGLU */
-  int ksplit;             /* 0 = let the library choose (INT4: at most 8 are made of what is asked for) */
+  int epilogue;           /* PT_EPI_STORE, PT_EPI_RESIDUAL or PT_EPI_BIAS; more by format: see above */
+  int ksplit;             /* 0 = let the library choose; at most 8 are made of what is asked for */
   int w_tiled;            /* 1: w was tiled by pt_gemm_repack; 0: row-major (FP8 only) */
   const void *x, *w;
   const void *scales;     /* INT4: fp16 [n_out, k_in / group]                        */
@@ -206,10 +208,10 @@ typedef struct pt_gemm_args {
   const void *residual;   /* fp16 [m, n_out]; may alias `out`                        */
   void *out;              /* fp16 [m, n_out]                                         */
   int out_ld;             /* row stride of `out` in elements; 0 = dense              */
-  void *workspace;        /* pt_gemm_workspace_bytes                                 */
+  void *workspace;        /* wanted if ksplit > 1, not used                          */
   size_t workspace_bytes;
-  int32_t *error_flag;    /* optional device int, set non-zero (21..24) if a bounded wait gave up */
-  const void *bias;       /* fp16 [n_out] (PT_EPI_BIAS)                              */
+  int32_t *error_flag;    /* optional device int, set non-zero (21..26) if a bounded wait gave up */
+  const void *bias;       /* fp16 [n_out] (PT_EPI_BIAS..)                             */
   int out_dtype;          /* PT_W_BF16: PT_DT_BF16 or PT_DT_F32                      */
   float alpha;            /* PT_W_BF16: factor on the fp32 sum; 0 = 1                */
   const pt_dense_ext *ext; /* PT_W_BF16: further arguments, or NULL                  */

@@ -1,8 +1,10 @@
-// Block-cooperative tensor-core GEMMs for 16 or more activation rows (batched decode, prefill):
+// Block-cooperative tensor-core GEMMs (decode steps, prompts):
 //     Y[m, n] = sum_k X[m, k] * W[n, k]          W row-major with k contiguous, like every weight of the reference
 //
 //   * FP8:  W and X are OCP E4M3 bytes with per-tensor scales (the reference's FP8MatMul, custom_ops/matmul_fp8.cpp:885-1091,
 //           in the E4M3 form): tcgen05.mma kind::f8f6f4, fp32 accumulation in tensor memory, scales applied in the epilogue.
+//   * FP16: W and X fp16, tcgen05.mma kind::f16, with the bias, GELU, residual, squared-ReLU and SwiGLU epilogues: the same kernel
+//           with 64 elements of k per 128-byte operand row.
 //   * BF16: W and X bfloat16, tcgen05.mma kind::f16, bf16 or fp32 output with the epilogues of dense_out.cuh: the same kernel as FP8
 //           with 64 elements of k per 128-byte operand row.  Grouped: every tile of activation rows names its weight matrix.
 //   * INT4: W is packed nibbles with fp16 group scales (utils/param_handler/precision_strategy.py:24-42,56-60).  Transform
@@ -18,9 +20,8 @@
 // the row width, which caps an SM near 25 GB/s; contiguous bulk copies stream at the HBM rate).  The activations (few rows) and
 // the row-major weights of the plain FP8MatMul op come through tiled TMA (cp.async.bulk.tensor; this GPU's memory only, no
 // multicast).  One thread issues the MMAs and hands stages back with tcgen05.commit; the other warps convert (INT4: a deep ring
-// of raw nibble tiles feeds a few slots of fp16 weights) and run the epilogue (tcgen05.ld, scale, fp16, coalesced stores
-// along n).  k-slices of one tile are summed in slice order (deterministic): INT4 by the blocks of a cluster, FP8 and BF16 in a
-// workspace by the last CTA to arrive.
+// of raw nibble tiles feeds a few slots of fp16 weights in tensor memory) and run the epilogue (tcgen05.ld, scale, fp16, coalesced
+// stores along n).  k-slices of one tile are the blocks of a cluster, which sum them in slice order (deterministic).
 // Every wait on an mbarrier is bounded: on a time-out the CTA raises the error flag, skips its remaining waits and still frees its tensor
 // memory.  Waits for tensor memory and for the blocks of a cluster have no limit and end by construction (gemm_plan.h).
 #include <cuda.h>
@@ -45,7 +46,7 @@ struct GemmParams {
   int ksplit, stages, raw_stages;
   int tmem_columns;       // tensor memory of a CTA
   int w_tiled;            // weights tiled by pt_gemm_repack (one contiguous tile per stage) instead of row-major
-  int epilogue;           // PT_EPI_STORE, PT_EPI_RESIDUAL or PT_EPI_BIAS (BF16: see dense)
+  int epilogue;           // (BF16: see dense)
   float out_scale;
   const unsigned char *w; // tiled weights (w_tiled)
   const __half *scales;   // INT4: [N][K / group]
@@ -194,7 +195,7 @@ __device__ __forceinline__ bool wait_fast(uint32_t bar, uint32_t parity, volatil
 // The same for a whole warp: every lane gets the same answer.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return __all_sync(0xffffffffu, wait_fast(bar, parity, abort_flag)); }
 
-// One finished sum of the FP8 / INT4 kernels (fp16 output) or of the BF16 kernel.  (SWIGLU, whose sums come in pairs: store_swiglu.)
+// One finished sum of the kernels with fp16 output (FP8, INT4, FP16) or of the BF16 kernel.  (SWIGLU, whose sums come in pairs: store_swiglu.)
 __device__ __forceinline__ __half relu2_h(__half y) {
   const __half r = __hgt(y, __float2half_rn(0.f)) ? y : __float2half_rn(0.f);
   return h_mul(r, r);
@@ -488,7 +489,7 @@ template <bool EXT> __device__ __forceinline__ void epilogue_bf16(const GemmPara
   if (whole < rows) epilogue_any<EXT>(p, tmem, q, lane, n0, m0, m_end, whole);
 }
 
-// ------------------------------------------------------------------------------------------ FP8 and BF16
+// ------------------------------------------------------------------------------------------ FP8, FP16 and BF16
 // Dynamic shared memory: [stage][NA A tiles of 16 KB | B tile mb * 128 B], every tile 1024-byte aligned.  NA = 2: a CTA takes 256 weight
 // rows (two accumulators), which fetches a third less per product than NA = 1; without k-slices.  With up to 128 activation rows two such CTAs share an
 // SM, so their registers have to allow it (96 a thread): a Pivavik of width 2048 takes four prompts of 2048 tokens, whose experts have tiles of 128
@@ -925,8 +926,8 @@ extern "C" int pt_gemm_repack(int wfmt, const void *w, int n_out, int k_in, void
   return PT_OK;
 }
 
-// What a caller hands over for k-slices that it asks for.  (The kernels sum the slices of a tile in the shared memory of a cluster and use no
-// workspace; the size is as it always was.)
+// What a caller has to hand over for k-slices that it asks for, from when they were summed in global memory.  (Nothing touches it now: the slices
+// of a tile meet in the shared memory of a cluster.  What was refused without it still is.)
 constexpr size_t kGemmCounterBytes = 65536;
 constexpr size_t kGemmMaxCounters = kGemmCounterBytes / sizeof(int);
 
