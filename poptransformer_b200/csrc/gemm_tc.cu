@@ -940,6 +940,8 @@ extern "C" int pt_gemm_repack(int wfmt, const void *w, int n_out, int k_in, void
 constexpr size_t kGemmCounterBytes = 65536;
 constexpr size_t kGemmMaxCounters = kGemmCounterBytes / sizeof(int);
 
+constexpr int kGemmSmem = 220 * 1024;   // dynamic shared memory that a launch may ask for
+
 extern "C" size_t pt_gemm_workspace_bytes(int m, int n_out, int max_ksplit) {
   return kGemmCounterBytes + (size_t)max_ksplit * m * n_out * sizeof(float);
 }
@@ -1021,18 +1023,6 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
       if (int rc = tc::make_map(&map_w, a->w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)a->k_in, (uint64_t)a->n_out, 128, tc::BM, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
     if (int rc = tc::make_map(&map_x, a->x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)a->k_in, (uint64_t)a->m, 128, (uint32_t)p.mb, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
   }
-  static bool attr_set = false;
-  if (!attr_set) {
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_FP8, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_FP16, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_BF16, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_BF16, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_BF16, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_dense_kernel<PT_W_BF16, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_int4_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    PT_CUDA(cudaFuncSetAttribute(tc::gemm_int4_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    attr_set = true;
-  }
   dim3 grid(ceil_div(plan.n_tiles, plan.na), p.ksplit, plan.m_tiles);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -1055,13 +1045,18 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   cfg.numAttrs = n_attr;
   cudaError_t e;
   if (int4) {
-    e = cudaLaunchKernelEx(&cfg, plan.int4_groups == 2 ? tc::gemm_int4_kernel<2> : tc::gemm_int4_kernel<4>, map_x, p);
+    static std::atomic<uint64_t> allowed[2];
+    const auto kernel = plan.int4_groups == 2 ? tc::gemm_int4_kernel<2> : tc::gemm_int4_kernel<4>;
+    PT_CUDA(allow_smem(kernel, kGemmSmem, allowed[plan.int4_groups == 2]));
+    e = cudaLaunchKernelEx(&cfg, kernel, map_x, p);
   } else {
+    static std::atomic<uint64_t> allowed[6];
     const bool ext = bf16 && dense_needs_ext(a->epilogue, a->ext);
     const auto kernel = fp16 ? tc::gemm_dense_kernel<PT_W_FP16, 1, false>
                        : !bf16 ? tc::gemm_dense_kernel<PT_W_FP8, 1, false>
                        : plan.na == 2 ? (ext ? tc::gemm_dense_kernel<PT_W_BF16, 2, true> : tc::gemm_dense_kernel<PT_W_BF16, 2, false>)
                               : (ext ? tc::gemm_dense_kernel<PT_W_BF16, 1, true> : tc::gemm_dense_kernel<PT_W_BF16, 1, false>);
+    PT_CUDA(allow_smem(kernel, kGemmSmem, allowed[fp16 ? 0 : !bf16 ? 1 : 2 + 2 * (plan.na == 2) + ext]));
     e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, p);
   }
   if (e != cudaSuccess) return pt::set_error(PT_ERR_CUDA, "pt_gemm: %s", cudaGetErrorString(e));
