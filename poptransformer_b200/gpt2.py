@@ -172,24 +172,6 @@ class GPT2Decoder(DecodeLoop):
             ops.lm_head_tp_merge(self)
         ops.step_containers(self.ids, self.step_t, self.next_ids, self.pad_id, self.eos_id, self.stop_mask, done_flag=self._loop_done_flag())
 
-    def capture(self):
-        saved = (self.ids.clone(), self.step_t.clone())
-        s = torch.cuda.Stream()
-        s.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(s):
-            self.enqueue_step()
-        torch.cuda.current_stream().wait_stream(s)
-        torch.cuda.synchronize()
-        self.ids.copy_(saved[0])
-        self.step_t.copy_(saved[1])
-        g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g):
-            self.enqueue_step()
-        self.graph = g
-        self.ids.copy_(saved[0])
-        self.step_t.copy_(saved[1])
-        torch.cuda.synchronize()
-
     def reset(self, input_ids):
         self.ids.copy_(torch.as_tensor(input_ids, dtype=torch.int32).to(self.device))
         self.step_t.zero_()

@@ -30,22 +30,22 @@ class DecodeLoop:
         return self.done_flag if self.early_stop else None
 
     def capture(self):
-        """Captures one loop iteration in a CUDA graph (one eager iteration first so lazy initialisation is done)."""
-        saved = (self.ids.clone(), self.step_t.clone())
+        """Captures one loop iteration in a CUDA graph (one eager iteration first so lazy initialisation is done).  The loop's state (ids,
+        step, stop mask, done flag) stays as it is."""
+        state = [t for t in (self.ids, self.step_t, self.stop_mask, self.done_flag) if t is not None]
+        saved = [t.clone() for t in state]
         s = torch.cuda.Stream()
         s.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(s):
             self.enqueue_step()
         torch.cuda.current_stream().wait_stream(s)
         torch.cuda.synchronize()
-        self.ids.copy_(saved[0])
-        self.step_t.copy_(saved[1])
+        for t, kept in zip(state, saved):
+            t.copy_(kept)
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             self.enqueue_step()
         self.graph = g
-        self.ids.copy_(saved[0])
-        self.step_t.copy_(saved[1])
         torch.cuda.synchronize()
 
     def run(self, input_ids, max_loop=None, poll_every=16, prefill=False):
