@@ -279,9 +279,9 @@ int pt_kv_cache_pipeline_fp8(const int32_t *step_dev, const void *kv_new, void *
  * (llama2/attention.py:64-114; gpt2/attention.py:37-85; chatglm2/attention.py:166-312).
  * The cache is paged: pool[page][2][n_kv][page_size][head_dim] fp16, page_table[batch][max_pages].
  * Token t of sequence b lives in page page_table[b][t / page_size], slot t % page_size.
- * One block per (sequence, kv head, page): scores and P.V on the tensor cores (fp32 sums of exact fp16 products, scores rounded
- * to fp16 like the reference's matmul output), softmax statistics in fp32 (or the reference's fp16 exp), the pages of a head
- * combined in page order by the last block to arrive (deterministic). */
+ * One block per run of pages of a (sequence, kv head): scores and P.V on the tensor cores (fp32 sums of exact fp16 products, scores rounded
+ * to fp16 like the reference's matmul output), softmax statistics in fp32 (or the reference's fp16 exp), the runs of a head
+ * combined in order by the last block to arrive (deterministic). */
 #define PT_ROPE_NONE 0
 #define PT_ROPE_LLAMA 1    /* rotate_half, table [max_len, head_dim/2]  (llama2/attention.py:28-56) */
 #define PT_ROPE_CHATGLM2 2 /* interleaved pairs on the first half of each head (chatglm2/attention.py:110-164) */

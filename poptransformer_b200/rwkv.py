@@ -96,7 +96,7 @@ class RWKVDecoder(DecodeLoop):
         self.lin_ws = ops.packed_workspace([self.head] + [x for L in self.layers for x in L.values()], B, dev)
         # The key / value / receptance linears of a block read different mixes of the same hidden state and are independent:
         # on one GPU they run on three streams (fork / join by events, also inside a captured CUDA graph), each with its own
-        # split-k workspace, so three short waves share the SMs instead of running back to back.
+        # split-k workspace if the skinny-matmul kernel serves them, so three short waves share the SMs instead of running back to back.
         self.side = [torch.cuda.Stream(device=dev) for _ in range(2)] if tp == 1 else []
         self.side_ws = [ops.packed_workspace([L[k] for L in self.layers for k in ("a_value", "a_recept", "f_recept")], B, dev) for _ in self.side]
         self.graph = None
