@@ -302,7 +302,8 @@ typedef struct pt_attn_args {
   int out_ld;                        /* row stride of `out` in elements; 0 = dense             */
   void *workspace;                   /* pt_attn_workspace_bytes                               */
   size_t workspace_bytes;
-  int32_t *error_flag;               /* device int, set to 12 if *step_dev is out of range (the kernel has no waits) */
+  int32_t *error_flag;               /* device int, set to 12 if *step_dev is out of range, to 13 if a bounded wait for the
+                                        other blocks of a cluster ran out */
   int pdl;                           /* 1: programmatic dependent launch (see pt_linear_args.pdl) */
   int max_len;                       /* positions available: rows of rope_sin / rope_cos and of the id container; 0 = page_size *
                                         max_pages.  A launch that finds *step_dev outside [0, max_len) sets error_flag to 12 and

@@ -1,21 +1,22 @@
 // Paged KV cache: append of the new token fused with split flash-decode attention.
 //
-// One block handles a run of pages (page_size cached tokens each) of one (sequence, kv-head): a page's K and V tiles are contiguous
-// in the pool.  The block that owns the page holding position `step` writes the new k/v into the pool and takes them from shared
-// memory itself, so the append costs no extra pass over the cache.  Scores and P.V run on the tensor cores (see the kernel),
-// the softmax statistics are warp-shuffle reductions.  A block whose run is the whole history writes the output; otherwise every block
-// leaves (max, sum, partial output) in the workspace and the last block to arrive for a (sequence, kv-head) combines the runs in a
-// fixed order, which keeps the result deterministic.
+// A warp takes chunks of 16 keys (32 of head width 64) of one (sequence, kv head) on its own: K and V rows come into shared memory of its own by
+// asynchronous copies, both products run on the tensor cores, and the softmax keeps a running maximum and sum, so that nothing but the end of the work
+// makes warps meet.  The warps of a block and, where there are few (sequence, kv head) pairs and long tables, the blocks of a cluster share the chunks;
+// what they leave is summed through shared memory in a fixed order, which keeps the result deterministic.
+// The warp that has the position `step` writes the new k/v into the pool and takes them from shared memory itself, so the append costs no
+// extra pass over the cache.
 //
 // HBM-bound: algorithmic bytes = 2 * (step + 1) * head_dim * 2 per (sequence, kv-head), read once.
 #include <algorithm>
 
 #include "common.cuh"
+#include "mbarrier.cuh"
 
 namespace pt {
 
 struct AttnParams {
-  int runs;        // blocks that share the pages of a (sequence, kv head, part)
+  int runs;        // blocks of a cluster, which share the keys of a (sequence, kv head, part)
   int B, n_head, n_kv, qpk, qsplit, H, page, max_pages, max_len, rope_mode, softmax_mode, rot_half, out_ld, pdl;
   __half scale_h;
   int use_scale;
@@ -26,388 +27,375 @@ struct AttnParams {
   __half *out;
   uint8_t *out8;   // optional: the same output cast to E4M3 with inv_out_scale (the input of an FP8 linear), [B, n_head * H]
   float inv_out_scale;
-  float *ws_o;     // [B, n_head, max_pages, H]
-  float2 *ws_ml;   // [B, n_head, max_pages]
-  int *counters;   // [B, n_kv, qsplit]
+  float2 *ws_ml;   // [B, n_head, max_pages]: maximum and sum of the first warps that have keys
   int *error_flag;
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// RoPE on one head vector x[H] (global, fp16) -> dst[H] (fp16), with the reference's fp16 roundings.
+// RoPE on one head vector (fp16), with the reference's fp16 roundings, sixteen channels (unit u) at a time: two runs of eight.
 // Llama (rotate_half): y_j = fp16(fp16(x_j c_j) + fp16(-x_{j+H/2} s_j)), y_{j+H/2} = fp16(fp16(x_{j+H/2} c_j) + fp16(x_j s_j)).
 // ChatGLM2: only the first H/2 channels rotate, as interleaved pairs (2i, 2i+1) with angle i:
 //   y_{2i} = fp16(fp16(x_{2i} c_i) - fp16(x_{2i+1} s_i)), y_{2i+1} = fp16(fp16(x_{2i+1} c_i) + fp16(x_{2i} s_i)).
-__device__ __forceinline__ void rope_pair(const AttnParams &p, const __half *x, const __half *sin_r, const __half *cos_r, int i,
-                                          __half *dst) {
+struct Half8 { __half v[8]; };
+__device__ __forceinline__ Half8 load8(const __half *x) { return *reinterpret_cast<const Half8 *>(__builtin_assume_aligned(x, 16)); }
+__device__ __forceinline__ void store8(__half *x, const Half8 &h) { *reinterpret_cast<uint4 *>(x) = *reinterpret_cast<const uint4 *>(&h); }
+template <int H> __device__ __forceinline__ void rope_runs(int rope_mode, int u, int &first, int &second) {   // channels where the two runs of unit u begin
+  first = rope_mode == PT_ROPE_LLAMA ? 8 * u : 16 * u;
+  second = rope_mode == PT_ROPE_LLAMA ? H / 2 + 8 * u : 16 * u + 8;
+}
+template <int H> __device__ __forceinline__ void rope16(const AttnParams &p, int u, const __half *sin_r, const __half *cos_r, Half8 &a, Half8 &b) {
+  if (p.rope_mode == PT_ROPE_NONE || (p.rope_mode == PT_ROPE_CHATGLM2 && u >= H / 32)) return;
+  Half8 s, c;
+  if ((((uintptr_t)sin_r | (uintptr_t)cos_r) & 15) == 0) {
+    s = load8(sin_r + 8 * u);
+    c = load8(cos_r + 8 * u);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { s.v[i] = sin_r[8 * u + i]; c.v[i] = cos_r[8 * u + i]; }
+  }
   if (p.rope_mode == PT_ROPE_LLAMA) {
-    const int h2 = p.H / 2;
-    const __half a = x[i], b = x[i + h2], s = sin_r[i], c = cos_r[i];
-    dst[i] = h_add(h_mul(a, c), h_mul(__hneg(b), s));
-    dst[i + h2] = h_add(h_mul(b, c), h_mul(a, s));
-  } else if (p.rope_mode == PT_ROPE_CHATGLM2) {
-    const int nrot = p.H / 4;  // rotated pairs
-    if (i < nrot) {
-      const __half a = x[2 * i], b = x[2 * i + 1], s = sin_r[i], c = cos_r[i];
-      dst[2 * i] = h_sub(h_mul(a, c), h_mul(b, s));
-      dst[2 * i + 1] = h_add(h_mul(b, c), h_mul(a, s));
-    } else {
-      dst[2 * i] = x[2 * i];
-      dst[2 * i + 1] = x[2 * i + 1];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const __half x = a.v[i], y = b.v[i];
+      a.v[i] = h_add(h_mul(x, c.v[i]), h_mul(__hneg(y), s.v[i]));
+      b.v[i] = h_add(h_mul(y, c.v[i]), h_mul(x, s.v[i]));
     }
   } else {
-    dst[2 * i] = x[2 * i];
-    dst[2 * i + 1] = x[2 * i + 1];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      Half8 &r = i < 4 ? a : b;
+      const __half x = r.v[2 * (i & 3)], y = r.v[2 * (i & 3) + 1];
+      r.v[2 * (i & 3)] = h_sub(h_mul(x, c.v[i]), h_mul(y, s.v[i]));
+      r.v[2 * (i & 3) + 1] = h_add(h_mul(y, c.v[i]), h_mul(x, s.v[i]));
+    }
   }
 }
 
-constexpr int kAttnThreads = 128;
-constexpr int NQ_MAX = 8;   // q heads of one kv head per block: the n side of an m16n8 tensor-core tile (larger groups take several blocks)
+constexpr int NQ_MAX = 8;      // q heads of one kv head per block: the n side of an m16n8 tensor-core tile (larger groups take several blocks)
+constexpr int MAX_RUNS = 16;   // blocks of a cluster
 
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
+  uint32_t t;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(t) : "r"(v));
+  return t;
+}
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t pack_f2h2(float lo, float hi) {
   const __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<const uint32_t *>(&h);
 }
+// Stores a value at an address of this block's shared memory in block `rank` of its cluster; it arrives there at the barrier `bar`.
+__device__ __forceinline__ void send(const void *local, int rank, float v, uint32_t bar) {
+  uint32_t a, there;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(bar), "r"(rank));
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a), "r"(__float_as_uint(v)), "r"(there) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { __syncwarp(); asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// One block = a run of consecutive pages of one (sequence, kv head, part of the group's q heads), one page after the other: while a page's
-// weights are formed and multiplied, the K rows of the next are on their way to registers and its V tile to the other of two buffers.
-// The host fixes the number of runs (see runs_of_pages), and the pages in use, which only the device knows, are dealt out evenly: however
-// much room the table has behind the history, the same blocks share the work.
-// Both products run on the tensor cores
-// (mma.sync m16n8k16, fp32 accumulation of exact fp16 products):
-//   scores^T [keys x heads] = K [keys x H] . q^T: warp w takes keys 16 w .. 16 w + 15 of each 64-key pass.  Its K rows go from
-//     global memory STRAIGHT into the A fragments: a lane loads 16 bytes = channels 32 pp + 8 tig .. + 7 of its two key rows,
-//     which serve two k-steps whose k order is a permutation of the channels (a dot product does not care, and q, the B operand,
-//     is read from shared memory with the same permutation: the same 16 bytes of the head's row).  No shared-memory tile, no
-//     bank conflicts, no barrier wait for K.
-//   out [heads x H] += P [heads x keys] . V [keys x H]: P comes from the softmax weights in shared memory (rows = heads, padded
-//     to 16 with zeros), V is staged in shared memory with padded rows and read through ldmatrix.trans; warp w owns H / 4 channels.
-// The new token's key / value are staged in shared memory by the block that owns the last page and appended to the pool by one
-// block per kv head.
-template <int H>
-__global__ void __launch_bounds__(kAttnThreads, 4) kv_append_attn_kernel(const AttnParams p) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int VLD = H + 8;                               // V rows padded: ldmatrix reads 8 rows in 8 different bank groups
-  constexpr int QLD = H + 32;                              // q rows: two heads read in one shared-memory phase sit 16 banks apart
-  const int PAGE = p.page, KP = (PAGE + 15) & ~15;         // keys padded to whole 16-key steps
-  const int PSLD = KP + 8;                                 // row stride of the score / weight rows
-  __half *Vs0 = reinterpret_cast<__half *>(smem);          // [two of them if a block can have more than one page][KP][VLD]
-  __half *qs = Vs0 + (size_t)(p.runs < p.max_pages ? 2 : 1) * KP * VLD;           // [NQ_MAX][QLD], rows >= nq are zero
-  __half *newk = qs + (size_t)NQ_MAX * QLD;                // [H]: the new token's rotated key (owner block)
-  float *ps = reinterpret_cast<float *>(newk + H);         // [NQ_MAX][PSLD]
-  float *ml = ps + (size_t)NQ_MAX * PSLD;                  // [NQ_MAX][2]
-  __shared__ int s_last;
+// Shared memory of a block of NW warps: every warp's K and V rows (afterwards its share of the output), the q heads, the new token's key and value
+// row, statistics, and, if the launch has clusters, the outputs that their blocks send to the one that writes them.
+template <int H, int NW> struct AttnSmem {
+  static constexpr int KEYS = 2048 / H;        // keys that a warp takes at a time: 4 KB of K and of V
+  static constexpr int LD = H + 8;             // rows padded by 16 bytes: eight rows of an ldmatrix lie in eight different bank groups
+  static constexpr int OLD = H + 4;            // a head's outputs, in floats
+  __half kv[NW][2][KEYS * LD];
+  __half q[NQ_MAX * LD];
+  __half fresh[2][H];                          // the new token's (rotated) key and its value
+  float2 ml[NW][NQ_MAX];                       // maximum and sum of every warp
+  float2 sent_ml[MAX_RUNS][NQ_MAX];            // maximum and sum of every block of the cluster
+  uint64_t arrived;                            // what the cluster's blocks send has come
+  volatile int abort;
+  float sent[1];                               // [run][share]: the outputs this block writes
+  static_assert(sizeof(__half) * 2 * KEYS * LD >= sizeof(float) * NQ_MAX * OLD, "a warp's outputs take the place of its keys and values");
+};
+// Outputs of a unit that one of R blocks writes: whole warps of one head's channels.
+__host__ __device__ inline int attn_share(int outputs, int R) { return ((outputs + R - 1) / R + 31) & ~31; }
 
+// One block, or the blocks of a cluster, handle one (sequence, kv head, part of the group's q heads); a warp takes every W-th chunk of its keys, W warps in all.
+// Up to a few MB of cache the time is latency: step and page table, then K and V, then the sums.  Above that the HBM rate bounds it.  Hence no barrier of
+// the block between the first key and the last, and 8.5 KB in flight per warp, sixteen warps to an SM.  A warp has one buffer for K and
+// one for V: while it forms the weights and multiplies them the next K rows are on their way, and the V rows during the next scores.  A chunk costs a
+// warp by itself about a microsecond, most of it the way to memory.  Of a short launch's 3.2 us (context 10) half went into branches on rows
+// behind the newest token and into a chain step -> table -> rotation; hence copies that fill with zeros, and everything asked for at once.
+//   scores [keys x heads] = K [16 keys x H] . q^T, K through ldmatrix, q (B operand) from shared memory into registers once.
+//   out^T [H x heads] += V^T [H x 16 keys] . P^T [keys x heads]: V through ldmatrix.trans, the weights of a lane turned by movmatrix.
+template <int H, int NW>
+__global__ void __launch_bounds__(NW * 32, 16 / NW) kv_append_attn_kernel(const AttnParams p) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  using Smem = AttnSmem<H, NW>;
+  Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+  constexpr int KEYS = Smem::KEYS, T = KEYS / 16, LD = Smem::LD, THREADS = NW * 32;
+  constexpr int U = H / 8, KS = H / 16;       // 16-byte units of a row; k-steps of the scores = m-tiles of the output
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
-  // With many q heads per kv head (multi-query attention) the heads of a group are shared out over `qsplit` blocks: each
-  // re-reads the group's K/V page (through L2) and handles nq of the group's heads.
-  const int run = blockIdx.x, kvh = blockIdx.y / p.qsplit, qpart = blockIdx.y - kvh * p.qsplit, b = blockIdx.z;
+  const int PAGE = p.page, R = p.runs, rank = blockIdx.x, W = R * NW;
+  const int kvh = blockIdx.y / p.qsplit, qpart = blockIdx.y - kvh * p.qsplit, b = blockIdx.z;
   const int nq = p.qpk / p.qsplit, q_lo = qpart * nq;   // this block's heads of the group: q_lo .. q_lo + nq - 1
+  const int share = attn_share(nq * H, R);              // outputs that this block writes if it is one of several
+  if (R > 1) {
+    if (tid == 0) {
+      sm.abort = 0;
+      mbar_init(smem_u32(&sm.arrived), 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      const int mine = max(0, min(nq * H - rank * share, share));
+      mbar_expect_tx(smem_u32(&sm.arrived), R * (mine * sizeof(float) + nq * sizeof(float2)));
+    }
+    cluster_arrive();     // once all have come by here, a block may send
+  }
   early_start();   // (the next kernel may fetch its weights meanwhile; everything this one reads was produced upstream)
-  // The step decides which page is the first.  The table's first 32 entries are asked for together with it, one per lane, so that the K / V loads are
-  // still one round trip away.
-  const int *table = p.page_table + (size_t)b * p.max_pages;
-  const int my_entry = table[min(lane, p.max_pages - 1)];
   const int step = *p.step;
-  if (step < 0 || step >= p.max_len) {  // no page / no RoPE row for this position: report it and leave the counters untouched
+  // The q heads, the new token's key and its value, sixteen channels a thread, asked for together with the step.
+  constexpr int UNITS = H / 16, MOST = ((NQ_MAX + 2) * UNITS + THREADS - 1) / THREADS;
+  const __half *qrow = p.qkv + (size_t)b * (p.n_head + 2 * p.n_kv) * H;
+  Half8 raw[MOST][2];
+#pragma unroll
+  for (int m = 0; m < MOST; ++m) {
+    const int i = m * THREADS + tid, h = i / UNITS, u = i % UNITS;
+    if (h >= nq + 2) continue;
+    const int head = h < nq ? kvh * p.qpk + q_lo + h : p.n_head + (h - nq) * p.n_kv + kvh;
+    int c0, c1;
+    rope_runs<H>(h > nq ? PT_ROPE_NONE : p.rope_mode, u, c0, c1);
+    raw[m][0] = load8(qrow + (size_t)head * H + c0);
+    raw[m][1] = load8(qrow + (size_t)head * H + c1);
+  }
+  // Where this lane's eight rows of chunk c begin (lane mod KEYS / 8; they lie in one page, whose size is a multiple of eight), in the pool's K.
+  const int *table = p.page_table + (size_t)b * p.max_pages;
+  auto rows_of = [&](int c) {
+    const int key = c * KEYS + 8 * (lane & (KEYS / 8 - 1)), pg = min(key / PAGE, p.max_pages - 1);
+    return (((long long)table[pg] * 2 * p.n_kv + kvh) * PAGE + (key - pg * PAGE)) * H;
+  };
+  const int c_first = warp * R + rank;
+  long long rows = rows_of(c_first);                    // (asked for together with the step)
+  if (step < 0 || step >= p.max_len) {  // no page / no RoPE row for this position: report it
     if (tid == 0 && p.error_flag) atomicExch(p.error_flag, 12);
+    if (R > 1) cluster_wait();
     return;
   }
-  const int n_pages = step / PAGE + 1, ppb = (n_pages + p.runs - 1) / p.runs, pg0 = run * ppb;
-  if (pg0 >= n_pages) return;
-  const int pg1 = min(n_pages, pg0 + ppb), n_active = (n_pages + ppb - 1) / ppb;   // (blocks of this (sequence, kv head) that have pages)
-  auto entry = [&](int pg) { return pg < 32 ? __shfl_sync(0xffffffffu, my_entry, pg) : table[pg]; };   // (pg is the same in every thread)
-  int phys = entry(pg0);
-  const bool has_last = pg1 == n_pages;
-  const int slot = step - (n_pages - 1) * PAGE;      // where the new token goes in the last page
-  const int row_elems = (p.n_head + 2 * p.n_kv) * H;
-  const __half *qrow = p.qkv + (size_t)b * row_elems;
-  const __half *vnew = qrow + (size_t)(p.n_head + p.n_kv + kvh) * H;
+  const int n_chunks = step / KEYS + 1, c_last = n_chunks - 1;
 
-  __half *gK, *gV;            // the tiles of the page that is being requested
-  int n_load;                 // its rows in the pool (the newest token is not there yet)
-  auto page_at = [&](int pg) {
-    gK = p.pool + (((size_t)phys * 2 + 0) * p.n_kv + kvh) * PAGE * H;
-    gV = p.pool + (((size_t)phys * 2 + 1) * p.n_kv + kvh) * PAGE * H;
-    n_load = pg == n_pages - 1 ? slot : PAGE;
-  };
-  uint4 kf[2][H / 32];
-  auto load_k = [&](int kbase) {   // this warp's K rows of a 64-key pass: keys kbase + g and + 8
+  __half *sK = sm.kv[warp][0], *sV = sm.kv[warp][1];
+  // The rows of chunk c of K (which = 0) or V.  The newest token's and what lies behind it are zeros; the newest one's is written later.
+  const long long v_rows = (long long)p.n_kv * PAGE * H;
+  const int lane_row = lane / U, lane_unit = lane % U;       // (a step of the warp takes 32 / U rows)
+  auto load = [&](int which, int c) {
+    const uint32_t dst = smem_u32(which ? sV : sK) + (lane_row * LD + lane_unit * 8) * 2;
+    const __half *src = p.pool + (which ? v_rows : 0) + lane_row * H + lane_unit * 8;
+    const int left = step - c * KEYS - lane_row;
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int key = kbase + g + 8 * r;
+    for (int e = 0; e < KEYS / 8; ++e) {
+      const __half *from = src + __shfl_sync(0xffffffffu, rows, e);
 #pragma unroll
-      for (int pp = 0; pp < H / 32; ++pp)
-        kf[r][pp] = key < n_load ? __ldcg(reinterpret_cast<const uint4 *>(gK + (size_t)key * H + pp * 32 + tig * 8)) : make_uint4(0, 0, 0, 0);
-    }
-  };
-  // V page -> shared memory as asynchronous 16-byte copies (no registers, in flight together with the K loads)
-  auto load_v = [&](__half *Vs, bool last) {
-    for (int e = tid; e < KP * (H / 8); e += kAttnThreads) {
-      const int r = e / (H / 8), c8 = e - r * (H / 8);
-      __half *dst = Vs + (size_t)r * VLD + c8 * 8;
-      if (r < n_load) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(gV + (size_t)r * H + c8 * 8) : "memory");
-      } else {   // rows beyond the valid tokens multiply weights of zero: keep them finite; the new token's row comes from qkv
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (last && r == slot) v = *reinterpret_cast<const uint4 *>(vnew + c8 * 8);
-        *reinterpret_cast<uint4 *>(dst) = v;
+      for (int i = 0; i < U / 4; ++i) {
+        const int r = i * (32 / U);      // (a row that is not read is filled with zeros; its address is not used)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (8 * e + r) * LD * 2), "l"(8 * e + r < left ? from + r * H : p.pool), "r"(8 * e + r < left ? 16 : 0) : "memory");
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  page_at(pg0);
-  load_k(warp * 16);   // the first page's loads go out before anything else
-  load_v(Vs0, pg0 == n_pages - 1);
+  if (c_first < n_chunks) {   // the first rows go out before anything else
+    load(0, c_first);
+    load(1, c_first);
+  }
 
-  // ---- RoPE on the block's q heads (and on the new k)
-  const __half *sin_r = p.sin_t + (size_t)step * p.rot_half;
-  const __half *cos_r = p.cos_t + (size_t)step * p.rot_half;
-  for (int i = tid; i < (NQ_MAX - nq) * (H / 2); i += kAttnThreads) {   // unused head rows of the B operand: zeros
-    const int qh = nq + i / (H / 2), j = i - (qh - nq) * (H / 2);
-    reinterpret_cast<uint32_t *>(qs + (size_t)qh * QLD)[j] = 0u;
-  }
-  for (int i = tid; i < nq * (H / 2); i += kAttnThreads) {
-    const int qh = i / (H / 2), j = i - qh * (H / 2);
-    rope_pair(p, qrow + (size_t)(kvh * p.qpk + q_lo + qh) * H, sin_r, cos_r, j, qs + (size_t)qh * QLD);
-  }
-  if (has_last) {
-    const __half *knew = qrow + (size_t)(p.n_head + kvh) * H;
-    for (int j = tid; j < H / 2; j += kAttnThreads) rope_pair(p, knew, sin_r, cos_r, j, newk);
-  }
-  for (int i = tid; i < NQ_MAX * PSLD; i += kAttnThreads) ps[i] = 0.f;   // weights of padded keys and unused heads
-
-  const size_t head0 = (size_t)b * p.n_head + (size_t)kvh * p.qpk + q_lo;
-  constexpr int NT = H / 32;                   // 8-channel tiles per warp: warp w owns channels [w H/4, (w + 1) H/4)
-  float O[NT][2], M = -INFINITY, L = 0.f;      // head g of the block: outputs of this warp's channels, running maximum and sum
+  // ---- RoPE on the block's q heads and on the new key
+  const __half *sin_r = p.sin_t + (size_t)step * p.rot_half, *cos_r = p.cos_t + (size_t)step * p.rot_half;
+  for (int i = tid; i < (NQ_MAX - nq) * U; i += THREADS)   // unused head rows of the B operand: zeros
+    *reinterpret_cast<uint4 *>(sm.q + (nq + i / U) * LD + i % U * 8) = make_uint4(0, 0, 0, 0);
 #pragma unroll
-  for (int j = 0; j < NT; ++j) O[j][0] = O[j][1] = 0.f;
-  for (int pg = pg0; pg < pg1; ++pg) {
-    __half *Vs = Vs0 + (size_t)((pg - pg0) & 1) * KP * VLD;
-    const bool owner = pg == n_pages - 1;
-    const int n_valid = owner ? slot + 1 : PAGE;
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();             // V and (first page) q are there; the weights of the page before have been used
-    if (owner && qpart == 0) {   // one block of the group appends to the pool
-      for (int j = tid; j < H; j += kAttnThreads) {
-        gK[(size_t)slot * H + j] = newk[j];
-        gV[(size_t)slot * H + j] = Vs[(size_t)slot * VLD + j];
-      }
+  for (int m = 0; m < MOST; ++m) {
+    const int i = m * THREADS + tid, h = i / UNITS, u = i % UNITS;
+    if (h >= nq + 2) continue;
+    int c0, c1;
+    rope_runs<H>(h > nq ? PT_ROPE_NONE : p.rope_mode, u, c0, c1);
+    if (h <= nq) rope16<H>(p, u, sin_r, cos_r, raw[m][0], raw[m][1]);
+    __half *to = h < nq ? sm.q + h * LD : sm.fresh[h - nq];
+    store8(to + c0, raw[m][0]);
+    store8(to + c1, raw[m][1]);
+  }
+  __syncthreads();
+  uint32_t qf[KS][2];          // q as B operand: lane (g, tig) holds channels 2 tig, + 1, + 8, + 9 of every 16 of head g
+#pragma unroll
+  for (int k = 0; k < KS; ++k) {
+    qf[k][0] = *reinterpret_cast<const uint32_t *>(sm.q + g * LD + k * 16 + 2 * tig);
+    qf[k][1] = *reinterpret_cast<const uint32_t *>(sm.q + g * LD + k * 16 + 8 + 2 * tig);
+  }
+
+  float O[KS][4], M[2] = {-INFINITY, -INFINITY}, L[2] = {0.f, 0.f};   // lane (g, tig): channels 16 j + g and + 8 of heads 2 tig and 2 tig + 1
+#pragma unroll
+  for (int j = 0; j < KS; ++j) O[j][0] = O[j][1] = O[j][2] = O[j][3] = 0.f;
+  const bool f32 = p.softmax_mode == PT_SOFTMAX_F32;
+  if (!f32) M[0] = M[1] = 0.f;         // the reference exponentiates fp16 scores without subtracting the maximum
+  const uint32_t k_lane = smem_u32(sK + (lane & 15) * LD + (lane >> 4) * 8);                            // matrices: keys 0-7 / 8-15, then channels + 8
+  const uint32_t v_lane = smem_u32(sV + ((lane >> 4) * 8 + (lane & 7)) * LD + ((lane >> 3) & 1) * 8);   // ... channels 0-7 / 8-15, then keys + 8
+  for (int c = c_first; c < n_chunks; c += W) {
+    const bool more = c + W < n_chunks;
+    const bool newest = c == c_last;               // this chunk ends with the new token
+    const int slot = step - c * KEYS;
+    if (newest && qpart == 0) {                    // one block of the group appends to the pool
+      __half *at = p.pool + __shfl_sync(0xffffffffu, rows, slot >> 3) + (slot & 7) * H;
+      for (int j = lane; j < 2 * U; j += 32) store8(at + (j < U ? 0 : v_rows) + j % U * 8, load8(sm.fresh[j / U] + j % U * 8));
     }
-    if (pg + 1 < pg1) phys = entry(pg + 1);
-
-    // ---- scores: keys 16 warp .. + 15 of every 64-key pass against the block's heads
-    for (int kbase = warp * 16; kbase < n_valid; kbase += 64) {
-      if (kbase != warp * 16) load_k(kbase);
-      if (owner) {   // the new token's key row comes from shared memory
+    if (more) rows = rows_of(c + W);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (newest && lane < U) store8(sK + slot * LD + lane * 8, load8(sm.fresh[0] + lane * 8));
+    __syncwarp();              // K is there
+    float sc[T][2][4] = {};    // (two chains each)
 #pragma unroll
-        for (int r = 0; r < 2; ++r)
-          if (kbase + g + 8 * r == slot) {
+    for (int k = 0; k < KS; ++k)
 #pragma unroll
-            for (int pp = 0; pp < H / 32; ++pp) kf[r][pp] = *reinterpret_cast<const uint4 *>(newk + pp * 32 + tig * 8);
-          }
+      for (int t = 0; t < T; ++t) {
+        uint32_t a[4];
+        ldmatrix_x4(k_lane + (t * 16 * LD + k * 16) * 2, a);
+        mma_f16(sc[t][k & 1], a, qf[k][0], qf[k][1]);
       }
-      float sc[4] = {0.f, 0.f, 0.f, 0.f};
+    __syncwarp();              // K has been used
+    if (more) load(0, c + W);
+    else asm volatile("cp.async.commit_group;" ::: "memory");      // (the groups are counted)
+    // lane (g, tig): keys 16 t + g (e = 0, 1) and + 8 (2, 3) against heads 2 tig and 2 tig + 1
+    float w[T][4];
+    bool in[T][2];
 #pragma unroll
-      for (int pp = 0; pp < H / 32; ++pp) {
-        const uint4 qv = *reinterpret_cast<const uint4 *>(qs + (size_t)g * QLD + pp * 32 + tig * 8);
-        mma_f16(sc, kf[0][pp].x, kf[1][pp].x, kf[0][pp].y, kf[1][pp].y, qv.x, qv.y);
-        mma_f16(sc, kf[0][pp].z, kf[1][pp].z, kf[0][pp].w, kf[1][pp].w, qv.z, qv.w);
-      }
-      // lane (g, tig): keys kbase + g (sc[0], sc[1]) and kbase + g + 8 (sc[2], sc[3]) against heads 2 tig and 2 tig + 1
+    for (int t = 0; t < T; ++t) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int key = kbase + g + 8 * (e >> 1), qh = 2 * tig + (e & 1);
-        if (key < KP && qh < nq) {
-          __half s16 = __float2half_rn(sc[e]);           // fp16 matmul output
-          if (p.use_scale) s16 = h_mul(s16, p.scale_h);  // ops.mul by fp16(1/sqrt(H))
-          ps[(size_t)qh * PSLD + key] = key < n_valid ? __half2float(s16) : 0.f;   // (no weight behind the newest key)
+        __half s16 = __float2half_rn(sc[t][0][e] + sc[t][1][e]);   // fp16 matmul output
+        if (p.use_scale) s16 = h_mul(s16, p.scale_h);              // ops.mul by fp16(1/sqrt(H))
+        w[t][e] = __half2float(s16);
+      }
+      in[t][0] = c * KEYS + 16 * t + g <= step;
+      in[t][1] = c * KEYS + 16 * t + 8 + g <= step;
+    }
+    if (f32) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float m = -INFINITY;
+#pragma unroll
+        for (int t = 0; t < T; ++t) m = fmaxf(m, fmaxf(in[t][0] ? w[t][h] : -INFINITY, in[t][1] ? w[t][h + 2] : -INFINITY));
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const float top = fmaxf(M[h], m), was = M[h] == top ? 1.f : expf(M[h] - top), ref = top == -INFINITY ? 0.f : top;
+        M[h] = top;
+        L[h] *= was;
+        if (__any_sync(0xffffffffu, was != 1.f)) {
+#pragma unroll
+          for (int j = 0; j < KS; ++j) { O[j][h] *= was; O[j][h + 2] *= was; }
+        }
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+          w[t][h] = in[t][0] ? expf(w[t][h] - ref) : 0.f;
+          w[t][h + 2] = in[t][1] ? expf(w[t][h + 2] - ref) : 0.f;
         }
       }
-    }
-    if (pg + 1 < pg1) {   // (the other buffer was last read before the barrier above)
-      page_at(pg + 1);
-      load_k(warp * 16);
-      load_v(Vs0 + (size_t)((pg + 1 - pg0) & 1) * KP * VLD, pg + 1 == n_pages - 1);
-    }
-    __syncthreads();
-
-    // ---- per-head softmax statistics of the page (one warp per q head, warp-shuffle reductions)
-    for (int qh = warp; qh < nq; qh += kAttnThreads / 32) {
-      float *pr = ps + (size_t)qh * PSLD;
-      float m = -INFINITY;
-      if (p.softmax_mode == PT_SOFTMAX_F32) {
-        for (int t = lane; t < n_valid; t += 32) m = fmaxf(m, pr[t]);
-        m = warp_max(m);
-      } else {
-        m = 0.f;  // the reference exponentiates fp16 scores without subtracting the maximum
-      }
-      float l = 0.f;
-      for (int t = lane; t < n_valid; t += 32) {
-        float e = expf(pr[t] - m);
-        if (p.softmax_mode == PT_SOFTMAX_F16) e = __half2float(__float2half_rn(e));
-        pr[t] = e;
-        l += e;
-      }
-      l = warp_sum(l);
-      if (lane == 0) { ml[2 * qh] = m; ml[2 * qh + 1] = l; }
-    }
-    __syncthreads();
-
-    // ---- P.V: rows of the A operand = heads (8 .. 15 are zero)
-    float o[NT][4];
+    } else {
 #pragma unroll
-    for (int j = 0; j < NT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-    const float *pr = ps + (size_t)g * PSLD + 2 * tig;      // g < NQ_MAX: rows of unused heads are zero
-    const uint32_t v_lane = smem_u32(Vs + (size_t)(lane & 15) * VLD + warp * (H / 4) + (lane >> 4) * 8);
-    for (int k2 = 0; k2 * 16 < n_valid; ++k2) {
+      for (int t = 0; t < T; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[t][e] = in[t][e >> 1] ? __half2float(__float2half_rn(expf(w[t][e]))) : 0.f;
+    }
+    uint32_t pf[T][2];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      L[0] += w[t][0] + w[t][2];
+      L[1] += w[t][1] + w[t][3];
       // The weights are rounded to fp16 for the tensor core; they are at most 1 (max-subtracted mode) or fp16 values already
       // (the reference's fp16 softmax mode), so this costs at most 2^-11 relative per weight.
-      const float2 p0 = *reinterpret_cast<const float2 *>(pr + k2 * 16), p1 = *reinterpret_cast<const float2 *>(pr + k2 * 16 + 8);
-      const uint32_t a0 = pack_f2h2(p0.x, p0.y), a2 = pack_f2h2(p1.x, p1.y);
+      pf[t][0] = transpose8x8(pack_f2h2(w[t][0], w[t][1]));
+      pf[t][1] = transpose8x8(pack_f2h2(w[t][2], w[t][3]));
+    }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (newest && lane < U) store8(sV + slot * LD + lane * 8, load8(sm.fresh[1] + lane * 8));
+    __syncwarp();              // V is there
 #pragma unroll
-      for (int j = 0; j < NT; j += 2) {
-        uint32_t b0, b1, b2, b3;
-        ldmatrix_x4_trans(v_lane + (uint32_t)(k2 * 16 * VLD + j * 8) * 2u, b0, b1, b2, b3);
-        mma_f16(o[j], a0, 0u, a2, 0u, b0, b1);
-        if (j + 1 < NT) mma_f16(o[j + 1], a0, 0u, a2, 0u, b2, b3);
+    for (int t = 0; t < T; ++t)
+#pragma unroll
+      for (int j = 0; j < KS; ++j) {
+        uint32_t a[4];
+        ldmatrix_x4_trans(v_lane + (t * 16 * LD + j * 16) * 2, a);
+        mma_f16(O[j], a, pf[t][0], pf[t][1]);
       }
-    }
-    // ---- the page joins the run
-    if (g < nq) {
-      const float m = ml[2 * g], top = fmaxf(M, m), was = M == top ? 1.f : expf(M - top), is = m == top ? 1.f : expf(m - top);
-      M = top;
-      L = L * was + ml[2 * g + 1] * is;
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        O[j][0] = O[j][0] * was + o[j][0] * is;
-        O[j][1] = O[j][1] * was + o[j][1] * is;
-      }
-    }
-  }
-  if (n_active == 1) {   // the whole history: the output
-    if (g < nq) {
-      const size_t col = ((size_t)kvh * p.qpk + q_lo + g) * H + warp * (H / 4) + 2 * tig;
-      __half *dst = p.out + (size_t)b * p.out_ld + col;
-      uint8_t *dst8 = p.out8 ? p.out8 + (size_t)b * p.n_head * H + col : nullptr;
-#pragma unroll
-      for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const __half y = __float2half_rn(O[j][e] / L);
-          dst[j * 8 + e] = y;
-          if (dst8) dst8[j * 8 + e] = (uint8_t)__nv_cvt_float_to_fp8(__half2float(y) * p.inv_out_scale, __NV_SATFINITE, __NV_E4M3);
-        }
-    }
-    return;
-  }
-  if (g < nq) {
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-      *reinterpret_cast<float2 *>(&p.ws_o[((head0 + g) * p.max_pages + run) * H + warp * (H / 4) + j * 8 + 2 * tig]) = make_float2(O[j][0], O[j][1]);
-    if (warp == 0 && tig == 0) p.ws_ml[(head0 + g) * p.max_pages + run] = make_float2(M, L);
+    __syncwarp();              // V has been used
+    if (more) load(1, c + W);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
   }
 
-  // ---- last block to arrive for this (sequence, kv-head) combines the runs in order
-  __threadfence();
-  __syncthreads();
-  int *ctr = p.counters + ((size_t)b * p.n_kv + kvh) * p.qsplit + qpart;
-  if (tid == 0) s_last = (atomicAdd(ctr, 1) == n_active - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  if (tid == 0) *ctr = 0;
-  // The V tile is no longer needed: its shared memory takes the pages' (max, sum) pairs, then their weights.  All loads of a
-  // stage are issued before the first is used, so the combine costs a handful of L2 round trips whatever the number of pages
-  // and heads (a loop of dependent-looking loads per head and page made it the longest part of the kernel at 17 pages).
-  float *cw = reinterpret_cast<float *>(Vs0);          // [nq][n_active] weights exp(m_i - M)
-  float *cl = cw + (size_t)nq * n_active;              // [nq][n_active] page sums, then cl[qh * n_active] = L of the head
-  // (worth its two extra barriers from about sixteen (head, page) pairs on: measured 1 % slower than the plain loop at 1 head x 6 pages)
-  const bool staged = nq * n_active >= 16 && (size_t)2 * nq * n_active * sizeof(float) <= (size_t)KP * VLD * sizeof(__half);
-  if (staged) {
-    for (int idx = tid; idx < nq * n_active; idx += kAttnThreads) {
-      const int qh = idx / n_active, i = idx - qh * n_active;
-      const float2 v = __ldcg(&p.ws_ml[(head0 + qh) * p.max_pages + i]);
-      cw[idx] = v.x;
-      cl[idx] = v.y;
+  // ---- the warps of the block that have keys
+  const int n_warps = min(NW, (n_chunks - rank + R - 1) / R);      // (none: a block of a cluster that has no keys)
+  float *own = reinterpret_cast<float *>(sm.kv[warp]);             // [head][channel]
+  float2 *left = p.ws_ml + ((size_t)b * p.n_head + (size_t)kvh * p.qpk + q_lo) * p.max_pages + c_first;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) L[h] += __shfl_xor_sync(0xffffffffu, L[h], o);
+    const int qh = 2 * tig + h;
+    if (g == 0) sm.ml[warp][qh] = make_float2(M[h], L[h]);
+    if (qh >= nq || warp >= n_warps) continue;
+    if (g == 0 && c_first < p.max_pages) left[(size_t)qh * p.max_pages] = make_float2(M[h], L[h]);     // (how the keys were shared out can be read there)
+#pragma unroll
+    for (int j = 0; j < KS; ++j) {
+      own[qh * Smem::OLD + 16 * j + g] = O[j][h];
+      own[qh * Smem::OLD + 16 * j + g + 8] = O[j][h + 2];
     }
-    __syncthreads();
-    for (int qh = warp; qh < nq; qh += kAttnThreads / 32) {
-      float *w = cw + (size_t)qh * n_active, *l = cl + (size_t)qh * n_active;
-      float M = -INFINITY;
-      for (int i = lane; i < n_active; i += 32) M = fmaxf(M, w[i]);
-      M = warp_max(M);
-      for (int i = lane; i < n_active; i += 32) w[i] = expf(w[i] - M);
-      __syncwarp();
-      if (lane == 0) {   // the head's sum in page order, like the outputs below
-        float L = 0.f;
-        for (int i = 0; i < n_active; ++i) L += l[i] * w[i];
-        l[0] = L;
+  }
+  __syncthreads();
+  // n parts of a head, lane i holding the maximum and sum of part i: the parts' weights and the sum.
+  auto weigh = [&](float2 ml, float &m, float &l) {
+    m = warp_max(ml.x);
+    const float f = ml.x == m ? 1.f : expf(ml.x - m);
+    l = warp_sum(ml.y * f);
+    return f;
+  };
+  auto write = [&](int qh, int ch, float o) {
+    const __half y = __float2half_rn(o);
+    const size_t col = ((size_t)kvh * p.qpk + q_lo + qh) * H + ch;
+    p.out[(size_t)b * p.out_ld + col] = y;
+    if (p.out8) p.out8[(size_t)b * p.n_head * H + col] = (uint8_t)__nv_cvt_float_to_fp8(__half2float(y) * p.inv_out_scale, __NV_SATFINITE, __NV_E4M3);
+  };
+  const uint32_t arrived = smem_u32(&sm.arrived);
+  if (R > 1) cluster_wait();
+  for (int e0 = warp * 32; e0 < nq * H; e0 += THREADS) {           // 32 channels of one head
+    const int qh = e0 / H, ch = e0 % H + lane;
+    float m, l, o = 0.f;
+    const float f = weigh(lane < n_warps ? sm.ml[lane][qh] : make_float2(-INFINITY, 0.f), m, l);
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+      const float v = i < n_warps ? reinterpret_cast<const float *>(sm.kv[i])[qh * Smem::OLD + ch] : 0.f;
+      o += v * __shfl_sync(0xffffffffu, f, i);
+    }
+    if (R == 1) {
+      write(qh, ch, o / l);
+    } else {   // the blocks of the cluster: block r gets outputs [r share, (r + 1) share) of the nq heads from all, and everybody's statistics
+      const int to = e0 / share;
+      send(&sm.sent[rank * share + e0 + lane - to * share], to, o, arrived);
+      if (e0 % H == 0 && lane < R) {
+        send(&sm.sent_ml[rank][qh].x, lane, m, arrived);
+        send(&sm.sent_ml[rank][qh].y, lane, l, arrived);
       }
     }
-    __syncthreads();
-    if (tid < H) {
-      constexpr int PB = 8;   // pages in flight per head; two heads at a time
-      for (int q0 = 0; q0 < nq; q0 += 2) {
-        const bool two = q0 + 1 < nq;
-        float o0 = 0.f, o1 = 0.f;
-        const float *w0 = cw + (size_t)q0 * n_active, *w1 = cw + (size_t)(two ? q0 + 1 : q0) * n_active;
-        const float *src0 = p.ws_o + ((head0 + q0) * p.max_pages) * H + tid, *src1 = src0 + (two ? (size_t)p.max_pages * H : 0);
-        for (int i0 = 0; i0 < n_active; i0 += PB) {
-          float v0[PB], v1[PB];
-#pragma unroll
-          for (int j = 0; j < PB; ++j) {
-            const bool in = i0 + j < n_active;
-            v0[j] = in ? __ldcg(src0 + (size_t)(i0 + j) * H) : 0.f;
-            v1[j] = (in && two) ? __ldcg(src1 + (size_t)(i0 + j) * H) : 0.f;
-          }
-#pragma unroll
-          for (int j = 0; j < PB; ++j)
-            if (i0 + j < n_active) {
-              o0 += v0[j] * w0[i0 + j];
-              o1 += v1[j] * w1[i0 + j];
-            }
-        }
-        __half *dst = p.out + (size_t)b * p.out_ld + ((size_t)kvh * p.qpk + q_lo + q0) * H + tid;
-        const __half y0 = __float2half_rn(o0 / cl[(size_t)q0 * n_active]);
-        dst[0] = y0;
-        uint8_t *dst8 = p.out8 ? p.out8 + (size_t)b * p.n_head * H + ((size_t)kvh * p.qpk + q_lo + q0) * H + tid : nullptr;
-        if (dst8) dst8[0] = (uint8_t)__nv_cvt_float_to_fp8(__half2float(y0) * p.inv_out_scale, __NV_SATFINITE, __NV_E4M3);
-        if (two) {
-          const __half y1 = __float2half_rn(o1 / cl[(size_t)(q0 + 1) * n_active]);
-          dst[H] = y1;
-          if (dst8) dst8[H] = (uint8_t)__nv_cvt_float_to_fp8(__half2float(y1) * p.inv_out_scale, __NV_SATFINITE, __NV_E4M3);
-        }
-      }
-    }
+  }
+  if (R == 1) return;
+  if (!mbar_wait(arrived, 0, &sm.abort)) {
+    if (p.error_flag) atomicCAS(p.error_flag, 0, 13);
+    sm.abort = 1;
     return;
   }
-  if (tid < H) {   // few pages and heads: the plain loop
-    for (int qh = 0; qh < nq; ++qh) {
-      const size_t hd = head0 + qh;
-      float M = -INFINITY;
-      for (int i = 0; i < n_active; ++i) M = fmaxf(M, __ldcg(&p.ws_ml[hd * p.max_pages + i]).x);
-      float L = 0.f, o = 0.f;
-      for (int i = 0; i < n_active; ++i) {
-        const float2 v = __ldcg(&p.ws_ml[hd * p.max_pages + i]);
-        const float w = expf(v.x - M);
-        L += v.y * w;
-        o += __ldcg(&p.ws_o[(hd * p.max_pages + i) * H + tid]) * w;
-      }
-      const __half y = __float2half_rn(o / L);
-      p.out[(size_t)b * p.out_ld + ((size_t)kvh * p.qpk + q_lo + qh) * H + tid] = y;
-      if (p.out8)
-        p.out8[(size_t)b * p.n_head * H + ((size_t)kvh * p.qpk + q_lo + qh) * H + tid] =
-            (uint8_t)__nv_cvt_float_to_fp8(__half2float(y) * p.inv_out_scale, __NV_SATFINITE, __NV_E4M3);
-    }
+  for (int e0 = warp * 32; e0 < share && rank * share + e0 < nq * H; e0 += THREADS) {
+    const int e = rank * share + e0 + lane, qh = e / H;
+    float m, l, o = 0.f;
+    const float f = weigh(lane < R ? sm.sent_ml[lane][qh] : make_float2(-INFINITY, 0.f), m, l);
+    for (int i = 0; i < R; ++i) o += sm.sent[i * share + e0 + lane] * __shfl_sync(0xffffffffu, f, i);
+    write(qh, e % H, o / l);
   }
 }
 
@@ -472,19 +460,56 @@ static size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 extern "C" size_t pt_attn_workspace_bytes(int batch, int n_head, int head_dim, int max_pages) {
   const size_t heads = (size_t)batch * n_head;
-  return align256(heads * sizeof(int)) + align256(heads * max_pages * sizeof(float2)) + heads * max_pages * head_dim * sizeof(float);
+  (void)head_dim;
+  return align256(heads * sizeof(int)) + align256(heads * max_pages * sizeof(float2));
 }
 
-// Blocks that share the pages of one of `units` (sequence, kv head, part): about four blocks per SM in all (what the registers and two V buffers
-// of a block admit at a time), and no more than the table has pages.  Rounded to the nearest: measured on B200, 32 heads of 128, context 511,
-// 9 / 16 rows 19.9 / 29.0 us, 25.2 / 34.8 with one more run each (a second, nearly empty wave of blocks).
-// The room behind the history costs nothing (a table of 11, 64 or 512 pages at context 511, 4 rows: 12.6 us each); one page per block took
-// 14.3, 17.1 and 72.8 us, runs of a length that fills the SMs when the whole table is in use 13.0, 24.0 and 23.6.
-// A table that is at most a quarter longer than that gives every page its own block, which then needs one V buffer: half the shared memory, and the
-// blocks of the product behind it find room earlier (ChatGLM2 at 8 rows, 32 units and 21 pages, whole steps: 2.79 ms against 2.82).
-static int runs_of_pages(int units, int max_pages) {
-  const int slots = 4 * sm_count();
-  return (long long)units * max_pages * 4 <= slots * 5LL ? max_pages : std::min(max_pages, std::max(1, (slots + units / 2) / units));
+// Warps per block and blocks per cluster that share the keys of one of `units` (sequence, kv head, part).  Sixteen warps fit an SM whatever the block, so
+// blocks get as many as keep all units on the SMs at once.  A cluster's meeting costs 0.5 to 1 us: it is worth it where a unit's table has a chunk
+// for each of its warps, and as long as every block has an SM (clusters of sixteen: of a GPC).  Measured on B200, us a launch in a row of
+// launches, of (rows, q heads, kv heads, head width, context, room) the kernel before / as warps x blocks:
+//   (1, 12, 12, 64, 159, 352)     6.4 / 8x1 3.6, 16x1 3.8, 4x1 4.6, 16x2 4.2         (16, 25, 25, 64, 255, 448)    11.8 / 4x1 8.1, 8x1 9.3, 4x2 11.2
+//   (1, 32, 32, 128, 511, 704)    8.0 / 16x4 5.2, 16x2 6.1, 16x1 7.8, 8x4 5.8        (4, 32, 32, 128, 511, 704)    12.7 / 16x1 8.3, 8x2 9.2, 16x2 13.3
+//   (9, 32, 32, 128, 511, 704)   20.2 / 8x1 15.3, 4x1 16.0, 16x1 17.4                (16, 32, 32, 128, 511, 704)   29.6 / 4x1 25.8 (bytes alone 20.5)
+//   (8, 32, 2, 128, 1151, 1344)  16.6 / 16x4 8.4, 16x2 11.2, 16x8 18.9               (1, 32, 2, 128, 1151, 1344)   14.0 / 16x8 6.2, 16x4 8.1
+//   (1, 32, 2, 128, 30000, 32768) 54 / 16x16 21, 16x8 34                             (1, 8, 8, 128, 30000, 32768)  34.6 / 16x8 33.4, 16x16 47
+struct AttnSplit { int warps, runs; };
+static AttnSplit split_keys(int units, int max_pages, int page, int head_dim) {
+  const int chunks = (int)std::min<long long>((long long)max_pages * page * head_dim / 2048 + 1, 1 << 20);
+  const int sms = sm_count(), warps = units > 2 * sms ? 4 : units > sms || chunks < 16 ? 8 : 16;
+  int runs = 1;
+  while (warps == 16 && runs < (units <= 4 ? 16 : 8) && 2 * units * runs <= sms && chunks >= 16 * runs) runs *= 2;
+  return {warps, runs};
+}
+template <int H, int NW> static cudaError_t launch_attn(const AttnParams &p, cudaStream_t stream) {
+  static std::atomic<uint64_t> allowed{0}, wide{0};
+  const auto kernel = kv_append_attn_kernel<H, NW>;
+  const int nq = p.qpk / p.qsplit;
+  const size_t smem = sizeof(AttnSmem<H, NW>) + (p.runs > 1 ? (size_t)p.runs * attn_share(nq * H, p.runs) * sizeof(float) : 0);
+  cudaError_t e = allow_smem(kernel, 200 * 1024, allowed);
+  if (e == cudaSuccess) e = allow_wide_clusters(kernel, wide);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.runs, p.n_kv * p.qsplit, p.B);
+  cfg.blockDim = dim3(NW * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  if (p.runs > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = p.runs;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  if (p.pdl) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+template <int H> static cudaError_t launch_attn(const AttnParams &p, int warps, cudaStream_t stream) {
+  return warps == 16 ? launch_attn<H, 16>(p, stream) : warps == 8 ? launch_attn<H, 8>(p, stream) : launch_attn<H, 4>(p, stream);
 }
 
 extern "C" int pt_kv_append_attn(const pt_attn_args *a, void *stream) {
@@ -523,40 +548,16 @@ extern "C" int pt_kv_append_attn(const pt_attn_args *a, void *stream) {
   p.inv_out_scale = a->out_fp8 ? 1.0f / a->out_fp8_scale : 0.f;
   const size_t heads = (size_t)a->batch * a->n_head;
   char *ws = (char *)a->workspace;
-  p.counters = (int *)ws; ws += align256(heads * sizeof(int));
-  p.ws_ml = (float2 *)ws; ws += align256(heads * a->max_pages * sizeof(float2));
-  p.ws_o = (float *)ws;
+  p.ws_ml = (float2 *)(ws + align256(heads * sizeof(int)));
   p.error_flag = a->error_flag;
   p.pdl = a->pdl ? 1 : 0;
   PT_REQUIRE(a->max_len >= 0 && a->max_len <= a->page_size * a->max_pages, "pt_kv_append_attn: max_len=%d exceeds the %d positions of the page table",
              a->max_len, a->page_size * a->max_pages);
   p.max_len = a->max_len > 0 ? a->max_len : a->page_size * a->max_pages;
 
-  p.runs = runs_of_pages(a->batch * a->n_kv * p.qsplit, a->max_pages);
-  const int kp = (p.page + 15) & ~15;
-  const size_t smem = ((size_t)(p.runs < a->max_pages ? 2 : 1) * kp * (p.H + 8) + (size_t)NQ_MAX * (p.H + 32) + p.H) * sizeof(__half) +
-                      ((size_t)NQ_MAX * (kp + 8) + (size_t)NQ_MAX * 2) * sizeof(float);
-  PT_REQUIRE(smem <= 200 * 1024, "pt_kv_append_attn: tile needs %zu bytes of shared memory", smem);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.runs, a->n_kv * p.qsplit, a->batch);
-  cfg.blockDim = dim3(kAttnThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = as_stream(stream);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = p.pdl ? 1 : 0;
-  cudaError_t le;
-  if (p.H == 128) {
-    static std::atomic<uint64_t> allowed{0};
-    PT_CUDA(allow_smem(kv_append_attn_kernel<128>, 200 * 1024, allowed));
-    le = cudaLaunchKernelEx(&cfg, kv_append_attn_kernel<128>, p);
-  } else {
-    static std::atomic<uint64_t> allowed{0};
-    PT_CUDA(allow_smem(kv_append_attn_kernel<64>, 200 * 1024, allowed));
-    le = cudaLaunchKernelEx(&cfg, kv_append_attn_kernel<64>, p);
-  }
+  const AttnSplit split = split_keys(a->batch * a->n_kv * p.qsplit, a->max_pages, a->page_size, a->head_dim);
+  p.runs = split.runs;
+  const cudaError_t le = p.H == 128 ? launch_attn<128>(p, split.warps, as_stream(stream)) : launch_attn<64>(p, split.warps, as_stream(stream));
   if (le != cudaSuccess) return pt::set_error(PT_ERR_CUDA, "pt_kv_append_attn: %s", cudaGetErrorString(le));
   PT_LAUNCH_CHECK("pt_kv_append_attn");
   return PT_OK;

@@ -80,6 +80,17 @@ template <typename K> static inline cudaError_t allow_smem(K *kernel, int bytes,
   return e;
 }
 
+// Lets a kernel be launched with clusters of up to sixteen blocks, once on each device.
+template <typename K> static inline cudaError_t allow_wide_clusters(K *kernel, std::atomic<uint64_t> &done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const uint64_t bit = 1ull << (dev & 63);
+  if (e != cudaSuccess || (done.load(std::memory_order_relaxed) & bit)) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
+}
+
 // ---- fp16 arithmetic with the reference's "one rounding per op" semantics -------------
 __device__ __forceinline__ __half h_mul(__half a, __half b) { return __hmul_rn(a, b); }
 __device__ __forceinline__ __half h_add(__half a, __half b) { return __hadd_rn(a, b); }
