@@ -54,18 +54,33 @@ __device__ __forceinline__ void early_start() {
   launch_dependents();
   wait_for_prerequisites();
 }
+// The blocks of such a launch: clusters of `cluster` blocks along y; early = false: it begins when the kernel before has ended.
+struct Grid {
+  dim3 blocks;
+  int cluster;
+  bool early;
+  Grid(dim3 b, int c = 1, bool e = true) : blocks(b), cluster(c), early(e) {}
+  Grid(int b) : Grid(dim3(b)) {}
+};
 template <typename... P, typename... A>
-static inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+static inline cudaError_t launch_early(void (*kernel)(P...), Grid grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
+  cfg.gridDim = grid.blocks;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  if (grid.cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = 1;
+    attr[cfg.numAttrs].val.clusterDim.y = grid.cluster;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  if (grid.early) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 

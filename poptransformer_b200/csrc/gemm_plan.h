@@ -41,6 +41,8 @@ struct GemmPlan {
   int int4_groups;                 // groups of transform warps
   int stages, raw_stages, threads;
   int tmem_columns;
+  bool x_warps;                    // warps fetch the activations, not TMA
+  uint32_t sum_offset;             // where the slices' sums arrive behind the operands (0: in their place)
   uint32_t stage_bytes, smem;
 };
 
@@ -82,6 +84,11 @@ static inline int slices_that_pay(int most, int n_kb, int mb, bool slow_whole) {
   return best;
 }
 
+// Shared memory for the sums of the slices: a block's share of the groups of four rows, from every slice.  Behind the operands where that takes at most
+// SUM_SMEM, so that a block can send before the one that sums has finished its products.
+constexpr uint32_t SUM_SMEM = 32 * 1024;
+static inline uint32_t sum_bytes(int mb, int ksplit) { return ksplit > 1 ? (uint32_t)gemm_ceil(mb / 4, ksplit) * ksplit * BM * 16 : 0; }
+
 static inline GemmPlan plan_gemm(const GemmAsk &a) {
   GemmPlan p{};
   const bool wide = a.bf16 || a.fp16;
@@ -122,7 +129,8 @@ static inline GemmPlan plan_gemm(const GemmAsk &a) {
 #define PT_TC_PAIR 1
 #endif
   p.na = PT_TC_PAIR && a.bf16 && p.ksplit == 1 && p.mb >= 128 && p.n_tiles >= 2 && (long long)gemm_ceil(p.n_tiles, 2) * p.m_tiles >= a.sms ? 2 : 1;
-  const uint32_t b_bytes = (uint32_t)p.mb * BKB;
+  const uint32_t b_bytes = (uint32_t)p.mb * BKB, sums = sum_bytes(p.mb, p.ksplit);
+  uint32_t behind = sums <= SUM_SMEM ? sums : 0;
   if (a.int4) {
     const bool two = p.mb <= 128 && p.n_tiles * p.m_tiles * p.ksplit > a.sms;     // two CTAs per SM (each has half the tensor memory)
     p.int4_groups = !two && p.mb <= 128 ? 4 : 2;                                  // above 128 rows a step's MMAs take longer than half a transform
@@ -130,10 +138,12 @@ static inline GemmPlan plan_gemm(const GemmAsk &a) {
     // slots: 64 tensor-memory columns beside the accumulator and 256 bytes of shared memory per row each
     p.stages = two ? (p.mb <= 64 ? 3 : 2) : (p.mb <= 128 ? 4 : p.mb <= 208 ? 3 : 2);
     p.stage_bytes = 2 * b_bytes;
-    const uint32_t slots = p.stages * p.stage_bytes, room = (two ? 104 : 217) * 1024u;
-    p.raw_stages = (int)std::min<uint32_t>(12, (room - slots) / RAW_STEP);
-    p.smem = slots + p.raw_stages * RAW_STEP + 1024;
-    p.fits = p.stages >= p.int4_groups && p.raw_stages >= p.stages + p.int4_groups;
+    const uint32_t slots = p.stages * p.stage_bytes, room = (two ? 110 : 217) * 1024u;
+    if (room < slots + behind + (p.stages + p.int4_groups) * RAW_STEP) behind = 0;
+    p.raw_stages = (int)std::min<uint32_t>(12, (room - slots - behind) / RAW_STEP);
+    p.sum_offset = behind ? slots + p.raw_stages * RAW_STEP : 0;
+    p.smem = slots + p.raw_stages * RAW_STEP + behind + 1024;
+    p.fits = p.stages >= p.int4_groups && p.raw_stages >= p.stages + p.int4_groups && sums <= p.smem - 1024;
     p.tmem_columns = ((p.mb + 31) & ~31) + 64 * p.stages <= 256 ? 256 : 512;
     if (p.tmem_columns == SM_COLUMNS) p.smem = std::max(p.smem, ALONE_SMEM);
   } else {
@@ -149,9 +159,11 @@ static inline GemmPlan plan_gemm(const GemmAsk &a) {
     // the other (two accumulators of 256 columns fill the tensor memory).
     // (The sums of a slice take 512 bytes per row of the ring.)
     const bool small = p.mb <= 64 || (wide && !(p.ksplit > 1 && p.mb > 128) && p.na * p.mb <= 256 && (long long)p.n_tiles * p.m_tiles * p.ksplit > a.sms);
-    p.stages = (int)std::min<uint32_t>(8, (small ? PT_TC_BUDGET_SMALL_KB : 200) * 1024u / p.stage_bytes);
-    p.fits = p.stages >= 2;
-    p.smem = p.stages * p.stage_bytes + 1024;
+    p.stages = (int)std::min<uint32_t>(8, ((small ? PT_TC_BUDGET_SMALL_KB : 200) * 1024u + std::min(behind, (small ? 110 - PT_TC_BUDGET_SMALL_KB : 16) * 1024u) - behind) / p.stage_bytes);
+    p.sum_offset = behind ? p.stages * p.stage_bytes : 0;
+    p.smem = p.stages * p.stage_bytes + behind + 1024;
+    p.x_warps = p.na == 1 && p.mb <= 32 && p.stages >= 4;
+    p.fits = p.stages >= 2 && sums <= p.smem - 1024;
     int columns = 32;
     while (columns < p.mb) columns <<= 1;
     p.tmem_columns = p.na * columns;

@@ -36,6 +36,10 @@
 #include "tile_math.cuh"
 
 namespace pt {
+namespace few {   // gemm_few.cu: small products of few activation rows
+bool takes(const pt_gemm_args &a);
+cudaError_t run(const pt_gemm_args &a, int out_ld, cudaStream_t st);
+}  // namespace few
 namespace tc {
 
 struct GemmParams {
@@ -49,6 +53,10 @@ struct GemmParams {
   int epilogue;           // (BF16: see dense)
   float out_scale;
   const unsigned char *w; // tiled weights (w_tiled)
+  const unsigned char *x; // activations, rows of x_pitch bytes
+  size_t x_pitch;
+  int x_warps;            // few activation rows: warps fetch them, not TMA
+  int sum_offset;         // where in a block's shared memory the slices of its share of a tile arrive (0: in place of the operands)
   const __half *scales;   // INT4: [N][K / group]
   const __half *residual;
   const __half *bias;
@@ -113,22 +121,21 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
                : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// Distributed shared memory of a cluster: a local address in block `rank`, and all threads of all its blocks meeting.
+// Distributed shared memory of a cluster: a local address in block `rank`, a store there that arrives at that block's barrier, and all threads of all
+// its blocks meeting.
 __device__ __forceinline__ uint32_t in_block(uint32_t local, uint32_t rank) {
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
   return a;
 }
-__device__ __forceinline__ float4 load_cluster4(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
+__device__ __forceinline__ void send4(uint32_t at, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];" ::"r"(at), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
 }
-// (The aligned form wants whole warps: lanes that leave a loop at different times are brought together first.)
-__device__ __forceinline__ void cluster_meet() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+// (The aligned forms want whole warps: lanes that leave a loop at different times are brought together first.)
+__device__ __forceinline__ void cluster_arrive() { __syncwarp(); asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { __syncwarp(); asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Ordinary stores to shared memory come before what the tensor core and TMA read and write there.
+__device__ __forceinline__ void fence_operands() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // The mbarrier gets one arrival once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -177,7 +184,7 @@ __host__ __device__ inline uint32_t instr_desc(bool bf16, int n) {
 }
 
 struct SharedCtl {
-  uint64_t full[8], ready[8], empty[8], accum;
+  uint64_t full[8], empty[8], accum, sums;
   uint64_t raw_full[24], raw_empty[24];
   uint32_t tmem_base;
   volatile int abort;
@@ -189,8 +196,13 @@ __device__ __forceinline__ void give_up(SharedCtl &ctl, int *error_flag, int cod
   ctl.abort = 1;
 }
 
-// A wait inside a hot loop: the first look is inline, the rest a call.
-__device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return mbar_wait(bar, parity, abort_flag); }
+// A wait inside a hot loop: the first look is inline, the rest a call.  It looks some more before it lets itself be suspended: from that it would wake
+// 250 cycles late (measured on B200).
+__device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+  for (int i = 0; i < 64; ++i)
+    if (mbar_test(bar, parity)) return true;
+  return mbar_wait(bar, parity, abort_flag);
+}
 __device__ __forceinline__ bool wait_fast(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return mbar_test(bar, parity) || wait_on(bar, parity, abort_flag); }
 // The same for a whole warp: every lane gets the same answer.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return __all_sync(0xffffffffu, wait_fast(bar, parity, abort_flag)); }
@@ -217,16 +229,17 @@ template <bool BF16, bool EXT> __device__ __forceinline__ void store_out(const G
 __device__ __forceinline__ __half swiglu_h(const GemmParams &p, float gate, float up) {
   return h_mul(__float2half_rn(up * p.out_scale), swish_h(__float2half_rn(gate * p.out_scale)));
 }
-// The first `rows` of sixteen rows m .. m + 15 of a warp's 32 weight rows (lane = n), fp16.
+// The first `rows` of R rows m .. m + R - 1 of a warp's 32 weight rows (lane = n), fp16.
 // PAIRS: all n are inside the output and neighbours on 4-byte boundaries: neighbouring lanes trade values so that a lane writes two
 // consecutive n.  SWIGLU trades between lanes n and n + 8, and each computes every other row of the pair's feature.
-template <int EPI, bool PAIRS> __device__ __forceinline__ void fp16_rows16(const GemmParams &p, const float (&sum)[16], int m, int rows, int n, int lane) {
+struct Residual2 { __half2 v[2]; };     // of the four rows of a pair of outputs: every other row of a lane's
+template <int EPI, bool PAIRS, int R> __device__ __forceinline__ void fp16_rows(const GemmParams &p, const float (&sum)[R], int m, int rows, int n, int lane, const Residual2 *got = nullptr) {
   constexpr bool RES = EPI == PT_EPI_RESIDUAL || EPI == PT_EPI_BIAS_RESIDUAL, BIAS = EPI == PT_EPI_BIAS || EPI == PT_EPI_BIAS_GELU || EPI == PT_EPI_BIAS_RESIDUAL;
   if constexpr (EPI == PT_EPI_SWIGLU) {
     const bool up = lane & 8, in = PAIRS || n < p.N;
     __half *o = p.out + (size_t)(m + (up ? 1 : 0)) * p.out_ld + n / 16 * 8 + n % 8;
 #pragma unroll
-    for (int j = 0; j < 16; j += 2) {
+    for (int j = 0; j < R; j += 2) {
       const float t = __shfl_xor_sync(0xffffffffu, up ? sum[j] : sum[j + 1], 8);
       if (in && j + (up ? 1 : 0) < rows) *o = up ? swiglu_h(p, t, sum[j + 1]) : swiglu_h(p, sum[j], t);
       o += 2 * (size_t)p.out_ld;
@@ -234,15 +247,16 @@ template <int EPI, bool PAIRS> __device__ __forceinline__ void fp16_rows16(const
   } else if constexpr (PAIRS) {
     const int odd = lane & 1;
     __half2 *o = reinterpret_cast<__half2 *>(p.out + (size_t)(m + odd) * p.out_ld + (n - odd));
-    __half2 res[RES ? 8 : 1], bias = __half2half2(__half(0));
+    __half2 res[RES ? R / 2 : 1], bias = __half2half2(__half(0));
     if constexpr (RES) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (2 * j + odd < rows) res[j] = __ldcg(reinterpret_cast<const __half2 *>(p.residual + (size_t)(m + odd + 2 * j) * p.N + (n - odd)));
+      for (int j = 0; j < R / 2; ++j)
+        if (R == 4 && got) res[j] = got->v[j & 1];
+        else if (2 * j + odd < rows) res[j] = __ldcg(reinterpret_cast<const __half2 *>(p.residual + (size_t)(m + odd + 2 * j) * p.N + (n - odd)));
     }
     if constexpr (BIAS) bias = *reinterpret_cast<const __half2 *>(p.bias + (n - odd));
 #pragma unroll
-    for (int j = 0; j < 16; j += 2) {
+    for (int j = 0; j < R; j += 2) {
       const float t = __shfl_xor_sync(0xffffffffu, odd ? sum[j] : sum[j + 1], 1);   // even lane: row j of n + 1; odd lane: row j + 1 of n - 1
       __half2 y = odd ? __floats2half2_rn(t * p.out_scale, sum[j + 1] * p.out_scale) : __floats2half2_rn(sum[j] * p.out_scale, t * p.out_scale);
       if constexpr (BIAS) y = __hadd2_rn(y, bias);
@@ -256,7 +270,7 @@ template <int EPI, bool PAIRS> __device__ __forceinline__ void fp16_rows16(const
     __half *o = p.out + (size_t)m * p.out_ld + n;
     const __half bias = BIAS ? p.bias[n] : __half(0);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < R; ++j) {
       if (j >= rows) break;
       __half y = __float2half_rn(sum[j] * p.out_scale);
       if constexpr (BIAS) y = h_add(y, bias);
@@ -268,14 +282,19 @@ template <int EPI, bool PAIRS> __device__ __forceinline__ void fp16_rows16(const
     }
   }
 }
-template <bool PAIRS> __device__ __forceinline__ void fp16_rows16(const GemmParams &p, const float (&sum)[16], int m, int rows, int n, int lane) {
-  if (p.epilogue == PT_EPI_SWIGLU) fp16_rows16<PT_EPI_SWIGLU, PAIRS>(p, sum, m, rows, n, lane);
-  else if (p.epilogue == PT_EPI_RESIDUAL) fp16_rows16<PT_EPI_RESIDUAL, PAIRS>(p, sum, m, rows, n, lane);
-  else if (p.epilogue == PT_EPI_BIAS) fp16_rows16<PT_EPI_BIAS, PAIRS>(p, sum, m, rows, n, lane);
-  else if (p.epilogue == PT_EPI_BIAS_GELU) fp16_rows16<PT_EPI_BIAS_GELU, PAIRS>(p, sum, m, rows, n, lane);
-  else if (p.epilogue == PT_EPI_RELU2) fp16_rows16<PT_EPI_RELU2, PAIRS>(p, sum, m, rows, n, lane);
-  else if (p.epilogue == PT_EPI_BIAS_RESIDUAL) fp16_rows16<PT_EPI_BIAS_RESIDUAL, PAIRS>(p, sum, m, rows, n, lane);
-  else fp16_rows16<PT_EPI_STORE, PAIRS>(p, sum, m, rows, n, lane);
+template <bool PAIRS, int R> __device__ __forceinline__ void fp16_rows(const GemmParams &p, const float (&sum)[R], int m, int rows, int n, int lane, const Residual2 *got = nullptr) {
+  if (p.epilogue == PT_EPI_STORE) fp16_rows<PT_EPI_STORE, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (p.epilogue == PT_EPI_SWIGLU) fp16_rows<PT_EPI_SWIGLU, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (p.epilogue == PT_EPI_RESIDUAL) fp16_rows<PT_EPI_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (p.epilogue == PT_EPI_BIAS) fp16_rows<PT_EPI_BIAS, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (p.epilogue == PT_EPI_BIAS_GELU) fp16_rows<PT_EPI_BIAS_GELU, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (p.epilogue == PT_EPI_RELU2) fp16_rows<PT_EPI_RELU2, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else fp16_rows<PT_EPI_BIAS_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
+}
+// Whether the rows of the 32 weight rows from nq on can leave in pairs.
+__device__ __forceinline__ bool fp16_pairs(const GemmParams &p, int nq) {
+  return nq + 32 <= p.N && p.out_ld % 2 == 0 && ((uintptr_t)p.out & 3) == 0 && (!p.residual || (p.N % 2 == 0 && ((uintptr_t)p.residual & 3) == 0)) &&
+         (!p.bias || ((uintptr_t)p.bias & 3) == 0);
 }
 // The epilogue of a tile without k-slices, fp16 outputs: `part` of `parts` warps share a quarter of the rows and take alternate 16 columns.
 // (Measured on B200, FP8 10304 x 2048, whose last tile is half empty, at 256 rows: 12.9 us; element by element over all branches, empty
@@ -283,16 +302,15 @@ template <bool PAIRS> __device__ __forceinline__ void fp16_rows16(const GemmPara
 __device__ __forceinline__ void epilogue_fp16(const GemmParams &p, uint32_t tmem, int q, int lane, int part, int parts, int n0, int m0) {
   const int nq = n0 + q * 32, n = nq + lane, rows = min(p.mb, p.M - m0);
   if (nq >= p.N) return;          // (uniform over the warp, as is `pairs`)
-  const bool pairs = nq + 32 <= p.N && p.out_ld % 2 == 0 && ((uintptr_t)p.out & 3) == 0 && (!p.residual || (p.N % 2 == 0 && ((uintptr_t)p.residual & 3) == 0)) &&
-                     (!p.bias || ((uintptr_t)p.bias & 3) == 0);
+  const bool pairs = fp16_pairs(p, nq);
   for (int c0 = part * 16; c0 < rows; c0 += 16 * parts) {
     uint32_t v[16];
     float sum[16];
     tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
     for (int j = 0; j < 16; ++j) sum[j] = __uint_as_float(v[j]);
-    if (pairs) fp16_rows16<true>(p, sum, m0 + c0, rows - c0, n, lane);
-    else fp16_rows16<false>(p, sum, m0 + c0, rows - c0, n, lane);
+    if (pairs) fp16_rows<true>(p, sum, m0 + c0, rows - c0, n, lane);
+    else fp16_rows<false>(p, sum, m0 + c0, rows - c0, n, lane);
   }
 }
 // Four consecutive fp16 outputs n .. n + 3 < N (n a multiple of four).
@@ -309,72 +327,14 @@ __device__ __forceinline__ void fp16_store4(const GemmParams &p, int m, int n, c
   }
 }
 
-// k-slices of a tile: the blocks of a cluster, slice = rank.  Every block leaves its sums in its own shared memory as [mb][128] floats
-// (`part`: the operand ring, which nobody reads any more), the blocks meet, each sums its share of the tile over all of them in slice
-// order (deterministic) and writes it, and they meet again before their shared memory goes.  On B200 this replaces sums that went
-// through global memory to the last block to arrive, which then summed the whole tile alone.
-__device__ __forceinline__ void leave_sums(const GemmParams &p, uint32_t tmem, int q, int lane, int part, int parts, float *dst) {
-  for (int c0 = part * 16; c0 < p.mb; c0 += 16 * parts) {
-    uint32_t v[16];
-    tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) dst[(c0 + j) * BM + q * 32 + lane] = __uint_as_float(v[j]);
-  }
-}
-template <bool BF16, bool EXT>
-__device__ __forceinline__ void sum_cluster(const GemmParams &p, const SharedCtl &ctl, uint32_t part, int rank, int n0, int m0, int m_end, int threads) {
-  cluster_meet();
-  if (!ctl.abort) {
-    const int units = min(p.mb, m_end - m0) * (BM / 4), share = (units + p.ksplit - 1) / p.ksplit, last = min(units, (rank + 1) * share);
-    for (int i = rank * share + (int)threadIdx.x; i < last; i += threads) {
-      const int m = m0 + i / (BM / 4), n = n0 + (i % (BM / 4)) * 4;
-      if (n >= p.N) continue;
-      auto sum4 = [&](int unit) {
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-        for (int s0 = 0; s0 < p.ksplit; s0 += 4) {   // four loads in flight
-          float4 v[4];
-#pragma unroll
-          for (int s = 0; s < 4; ++s) v[s] = s0 + s < p.ksplit ? load_cluster4(in_block(part + unit * 16, s0 + s)) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-          for (int s = 0; s < 4; ++s) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
-        }
-        return acc;
-      };
-      const bool glu = BF16 ? p.dense.epilogue == PT_EPI_GLU && n < p.dense.split_n : p.epilogue == PT_EPI_SWIGLU;
-      if (glu) {   // gate rows n % 16 < 8, their up rows eight further
-        if (n & 8) continue;
-        const float4 g = sum4(i), u = sum4(i + 2);
-        if constexpr (BF16) {
-          dense_store_glu4<EXT>(p.dense, m, n, g, u);
-        } else {
-          __half *o = p.out + (size_t)m * p.out_ld + n / 16 * 8 + n % 8;
-          o[0] = swiglu_h(p, g.x, u.x); o[1] = swiglu_h(p, g.y, u.y); o[2] = swiglu_h(p, g.z, u.z); o[3] = swiglu_h(p, g.w, u.w);
-        }
-        continue;
-      }
-      const float4 acc = sum4(i);
-      if (n + 4 <= p.N) {
-        if constexpr (BF16) dense_store4<EXT>(p.dense, m, n, acc);
-        else fp16_store4(p, m, n, acc);
-      } else {
-        store_out<BF16, EXT>(p, acc.x, m, n);
-        if (n + 1 < p.N) store_out<BF16, EXT>(p, acc.y, m, n + 1);
-        if (n + 2 < p.N) store_out<BF16, EXT>(p, acc.z, m, n + 2);
-      }
-    }
-  }
-  cluster_meet();
-}
-
-// Sixteen rows of one weight row per lane, gated: lanes n and n + 8 hold a feature's two sums.
-template <int GLU, bool EXT> __device__ __forceinline__ void glu_rows16(const GemmParams &p, const float (&sum)[16], int m, int m_end, int n, int lane) {
+// R rows of one weight row per lane, gated: lanes n and n + 8 hold a feature's two sums.
+template <int GLU, bool EXT, int R> __device__ __forceinline__ void glu_rows(const GemmParams &p, const float (&sum)[R], int m, int m_end, int n, int lane) {
   const DenseOut &d = p.dense;
   const bool store = n < p.N && (lane & 8) == 0;
   const float bg = store && d.bias ? __ldg(d.bias + n) : 0.f, bu = store && d.bias ? __ldg(d.bias + n + 8) : 0.f;
   const int f = n / 16 * 8 + n % 8;
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
+  for (int j = 0; j < R; ++j) {
     const float up = __shfl_xor_sync(0xffffffffu, sum[j], 8);
     if (!store || m + j >= m_end) continue;
     const float s = dense_factor<EXT>(d, m + j);
@@ -382,29 +342,31 @@ template <int GLU, bool EXT> __device__ __forceinline__ void glu_rows16(const Ge
   }
 }
 
-// The BF16 kernel's general epilogue: any sizes and alignment, 16 columns a step.
+// Rows m .. m + R - 1 of the BF16 kernel's 32 weight rows from nq on: any sizes and alignment.
+template <bool EXT, int R> __device__ __forceinline__ void bf16_rows(const GemmParams &p, const float (&sum)[R], int m, int m_end, int nq, int lane) {
+  const int n = nq + lane;
+  if (p.dense.epilogue == PT_EPI_GLU && nq < p.dense.split_n) {   // (uniform over the warp)
+    if (EXT && p.dense.glu == PT_GLU_SILU) glu_rows<PT_GLU_SILU, EXT>(p, sum, m, m_end, n, lane);
+    else if (EXT && p.dense.glu == PT_GLU_GELU) glu_rows<PT_GLU_GELU, EXT>(p, sum, m, m_end, n, lane);
+    else glu_rows<PT_GLU_CLAMPED, EXT>(p, sum, m, m_end, n, lane);
+  } else if (n < p.N) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      if (m + j >= m_end) break;
+      dense_store<EXT>(p.dense, m + j, n, sum[j]);
+    }
+  }
+}
+// The BF16 kernel's general epilogue: 16 columns a step.
 template <bool EXT>
 __device__ __forceinline__ void epilogue_any(const GemmParams &p, uint32_t tmem, int q, int lane, int n0, int m0, int m_end, int c_first) {
-  const int n = n0 + q * 32 + lane;
   for (int c0 = c_first; c0 < min(p.mb, m_end - m0); c0 += 16) {
     uint32_t v[16];
     float sum[16];
     tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
     for (int j = 0; j < 16; ++j) sum[j] = __uint_as_float(v[j]);
-    if (p.dense.epilogue == PT_EPI_GLU && n0 + q * 32 < p.dense.split_n) {   // (uniform over the warp)
-      if (EXT && p.dense.glu == PT_GLU_SILU) glu_rows16<PT_GLU_SILU, EXT>(p, sum, m0 + c0, m_end, n, lane);
-      else if (EXT && p.dense.glu == PT_GLU_GELU) glu_rows16<PT_GLU_GELU, EXT>(p, sum, m0 + c0, m_end, n, lane);
-      else glu_rows16<PT_GLU_CLAMPED, EXT>(p, sum, m0 + c0, m_end, n, lane);
-      continue;
-    }
-    if (n < p.N) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        if (m0 + c0 + j >= m_end) break;
-        dense_store<EXT>(p.dense, m0 + c0 + j, n, sum[j]);
-      }
-    }
+    bf16_rows<EXT>(p, sum, m0 + c0, m_end, n0 + q * 32, lane);
   }
 }
 
@@ -498,6 +460,110 @@ template <bool EXT> __device__ __forceinline__ void epilogue_bf16(const GemmPara
   if (whole < rows) epilogue_any<EXT>(p, tmem, q, lane, n0, m0, m_end, whole);
 }
 
+// k-slices of a tile: the blocks of a cluster, slice = rank.  The tile's activation rows in groups of four are dealt out to the blocks; every block sends each
+// group to the block that writes it, as [group][slice][weight row][4], by stores that arrive at a barrier there, and that block sums the slices in
+// order (deterministic).  (Blocks that left their sums at home, met, fetched what they needed and met again before their shared memory
+// went took longer: 1600 x 1600 at 16 rows in seven slices 4.8 us a launch in a row of launches, so 3.9; 1600 x 6400 7.7 and 7.0; 2048 x 2048 at 32 rows 5.3 and
+// 4.7; B200.)
+__device__ __forceinline__ int own_groups(int groups, int ksplit, int rank) { return rank < groups ? (groups - rank + ksplit - 1) / ksplit : 0; }
+__device__ __forceinline__ int row_groups(const GemmParams &p, int m0, int m_end) { return (min(p.mb, m_end - m0) + 3) >> 2; }
+__device__ __forceinline__ void expect_sums(const GemmParams &p, SharedCtl &ctl, int rank, int m0, int m_end) {
+  mbar_init(sa(&ctl.sums), 1);
+  const int own = own_groups(row_groups(p, m0, m_end), p.ksplit, rank);
+  if (own) mbar_expect_tx(sa(&ctl.sums), own * p.ksplit * BM * 16);
+}
+// The warps that sum have asked for what they need before their products are there: the residual of the first group of rows a warp writes, and
+// (the parameters of a launch are in no cache at first) the fields that the outputs go by.
+struct SumAhead { Residual2 res; bool pairs, got; };
+template <bool BF16> __device__ __forceinline__ SumAhead sums_ahead(const GemmParams &p, int rank, int part, int n0, int m0, int m_end, int q, int lane) {
+  SumAhead a;
+  a.pairs = !BF16 && fp16_pairs(p, n0 + q * 32);
+  a.got = a.pairs && (p.epilogue == PT_EPI_RESIDUAL || p.epilogue == PT_EPI_BIAS_RESIDUAL);
+  if constexpr (BF16) asm volatile("" ::"r"(p.dense.epilogue), "r"(p.dense.out_ld), "f"(p.dense.limit), "r"(p.dense.glu), "l"(p.dense.out), "l"(p.dense.bias));
+  else asm volatile("" ::"r"(p.epilogue), "r"(p.out_ld), "f"(p.out_scale), "l"(p.out), "l"(p.bias));
+  if (a.got) {
+    const int odd = lane & 1, m = m0 + 4 * (part * p.ksplit + rank);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      a.res.v[j] = m + odd + 2 * j < m_end ? __ldcg(reinterpret_cast<const __half2 *>(p.residual + (size_t)(m + odd + 2 * j) * p.N + (n0 + q * 32 + lane - odd))) : __half2half2(__half(0));
+  }
+  return a;
+}
+// The warps that have a tile's quarters q (`parts` times four of them, each part every parts-th step of 16 rows); the other threads of the block call it too.
+template <bool BF16, bool EXT>
+__device__ __forceinline__ void sum_cluster(const GemmParams &p, SharedCtl &ctl, uint32_t tmem, unsigned char *smem, int rank, int n0, int m0, int m_end, int part, int parts, int q, int lane, const SumAhead &ahead) {
+  if (p.sum_offset == 0) {    // where the sums take the place of the operands, nobody reads these any more
+    cluster_arrive();
+    cluster_wait();
+  }
+  if (part < 0) return;
+  const int groups = row_groups(p, m0, m_end), ks = p.ksplit;
+  const uint32_t mine = sa(smem + p.sum_offset) + (q * 32 + lane) * 16, bar = sa(&ctl.sums);
+  // (After a failure what there is goes out all the same: the others' waits end, and the error flag is up.)
+  int to = part * 4 % ks, slot = part * 4 / ks * ks + rank;
+  for (int g0 = part * 4; g0 < groups; g0 += 4 * parts) {
+    uint32_t v[16];
+    tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(4 * g0), v);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      if (g0 + t < groups) send4(in_block(mine + slot * (BM * 16), to), v[4 * t], v[4 * t + 1], v[4 * t + 2], v[4 * t + 3], in_block(bar, to));
+      if (++to == ks) { to = 0; slot += ks; }
+    }
+    for (int skip = 4 * (parts - 1); skip > 0; --skip)
+      if (++to == ks) { to = 0; slot += ks; }
+  }
+  const int own = own_groups(groups, ks, rank);
+  if (!own) return;
+  if (!warp_wait(bar, 0, &ctl.abort)) give_up(ctl, p.error_flag, 27);
+  if (ctl.abort) return;
+  const int nq = n0 + q * 32, n = nq + lane;
+  if (nq >= p.N) return;
+  for (int i = part; i < own; i += parts) {
+    float4 v[MAX_CLUSTER];
+#pragma unroll
+    for (int s = 0; s < MAX_CLUSTER; ++s)
+      v[s] = s < ks ? *reinterpret_cast<const float4 *>(smem + p.sum_offset + ((size_t)(i * ks + s) * BM + q * 32 + lane) * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int s = 0; s < MAX_CLUSTER; ++s) { sum[0] += v[s].x; sum[1] += v[s].y; sum[2] += v[s].z; sum[3] += v[s].w; }
+    const int m = m0 + 4 * (i * ks + rank);
+    if constexpr (BF16) bf16_rows<EXT>(p, sum, m, m_end, nq, lane);
+    else if (ahead.pairs) fp16_rows<true>(p, sum, m, m_end - m, n, lane, ahead.got && i == part ? &ahead.res : nullptr);
+    else fp16_rows<false>(p, sum, m, m_end - m, n, lane);
+  }
+}
+
+// Up to 32 activation rows: four warps fetch a k block in turn, a lane 16 bytes of every fourth row, the next block's loads under way while one is stored
+// in the image that TMA would have written.  (One thread gets a TMA box of 128 bytes a row on its way every 280 cycles, whatever the rows: of four boxes the
+// last arrived 1700 cycles after the kernel in front had ended, B200.)  A wait tells only odd from even uses of a slot, so at least four slots.
+__device__ __forceinline__ void fetch_rows(const GemmParams &p, SharedCtl &ctl, unsigned char *b0, uint32_t stage_bytes, int kb0, int n_it, int m0, int rows, int w, int lane) {
+  const int r0 = lane >> 3, c = lane & 7;
+  const unsigned char *src = p.x + (size_t)(m0 + r0) * p.x_pitch + (size_t)kb0 * BKB + c * 16;
+  const uint32_t full0 = sa(&ctl.full[0]), empty0 = sa(&ctl.empty[0]);
+  uint4 v[8];
+  auto get = [&](int it) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (4 * i + r0 < rows) v[i] = __ldcg(reinterpret_cast<const uint4 *>(src + (size_t)(4 * i) * p.x_pitch + (size_t)it * BKB));
+  };
+  int s = w;
+  uint32_t par = 1;
+  if (w < n_it) get(w);
+  for (int it = w; it < n_it; it += 4) {
+    if (it >= p.stages && !warp_wait(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 25); break; }
+    unsigned char *to = b0 + (size_t)s * stage_bytes + r0 * BKB;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (4 * i + r0 < rows) *reinterpret_cast<uint4 *>(to + 4 * i * BKB + ((c ^ (((i & 1) << 2) + r0)) << 4)) = v[i];
+    if (it + 4 < n_it) get(it + 4);
+    fence_operands();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(full0 + s * 8);
+    s += 4;
+    while (s >= p.stages) { s -= p.stages; par ^= 1u; }
+  }
+}
+
 // ------------------------------------------------------------------------------------------ FP8, FP16 and BF16
 // Dynamic shared memory: [stage][NA A tiles of 16 KB | B tile mb * 128 B], every tile 1024-byte aligned.  NA = 2: a CTA takes 256 weight
 // rows (two accumulators), which fetches a third less per product than NA = 1; without k-slices.  With up to 128 activation rows two such CTAs share an
@@ -536,13 +602,15 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
 
   if (tid == 0) {
     for (int s = 0; s < p.stages; ++s) {
-      mbar_init(sa(&ctl.full[s]), 1);
+      mbar_init(sa(&ctl.full[s]), p.x_warps ? 2 : 1);
       mbar_init(sa(&ctl.empty[s]), 1);
     }
     mbar_init(sa(&ctl.accum), 1);
+    if (NA == 1 && p.ksplit > 1) expect_sums(p, ctl, ks, m0, m_end);
     ctl.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (NA == 1 && p.ksplit > 1) cluster_arrive();
   if (warp == 1) tmem_alloc(sa(&ctl.tmem_base), tmem_cols);
   fence_before();
   __syncthreads();
@@ -550,13 +618,14 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
   const uint32_t tmem = ctl.tmem_base;
   // Not before: a CTA of the next GEMM that found the tensor memory free would keep it while it waits for this kernel to end.
   if (p.pdl) launch_dependents();
+  SumAhead ahead{};
 
   if (warp == 0) {
     if (elect_one()) {
       // (ring positions and parities are carried as counters: this thread's instruction count per stage is what limits a CTA)
       const unsigned char *wt = p.w + w_base + ((size_t)blockIdx.x * NA * p.n_kb + kb0) * A_TILE;
       const size_t next_tile = (size_t)p.n_kb * A_TILE;
-      const uint32_t tx = na * A_TILE + b_bytes, full0 = sa(&ctl.full[0]), empty0 = sa(&ctl.empty[0]);
+      const uint32_t tx = na * A_TILE + (p.x_warps ? 0 : b_bytes), full0 = sa(&ctl.full[0]), empty0 = sa(&ctl.empty[0]);
       const bool tiled = p.w_tiled != 0;     // (always, if p.pdl: the early loads below do not move kx on)
       int s = 0, kx = kb0 * KX;
       uint32_t par = 1;   // parity of the `empty` phase that must have completed before slot s is refilled (none in the first round)
@@ -585,7 +654,7 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
           mbar_expect_tx(fb, tx);
           load_w(st, fb);
         }
-        tma_load_2d(st + NA * A_TILE, &map_x, kx, m0, fb);
+        if (!p.x_warps) tma_load_2d(st + NA * A_TILE, &map_x, kx, m0, fb);
         kx += KX;
         if (++s == p.stages) { s = 0; par ^= 1u; first_round = false; }
       }
@@ -622,26 +691,34 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
       umma_commit(sa(&ctl.accum));   // fires when every MMA above has completed
     }
   } else {
+    if (NA == 1 && p.x_warps) {
+      if (p.pdl) wait_for_prerequisites();
+      fetch_rows(p, ctl, smem + A_TILE, stage_bytes, kb0, n_it, m0, m_end - m0, warp - 2, lane);
+    }
+    if (NA == 1 && p.ksplit > 1) {
+      if (p.pdl) wait_for_prerequisites();
+      ahead = sums_ahead<BF16>(p, ks, 0, n0, m0, m_end, warp & 3, lane);
+      cluster_wait();             // everybody's barrier is there
+    }
     if (p.pdl) wait_for_prerequisites();                // the residual and the output are others' until here
     const bool done = warp_wait(sa(&ctl.accum), 0, &ctl.abort);
     if (!done) give_up(ctl, p.error_flag, 24);
     fence_after();
-    if (done && n_it > 0) {
-      if (NA == 1 && p.ksplit > 1) {
-        leave_sums(p, tmem, warp & 3, lane, 0, 1, reinterpret_cast<float *>(smem));
-      } else if constexpr (BF16) {
+    if (done && (NA > 1 || p.ksplit == 1)) {
+      if constexpr (BF16) {
         const int a = (warp - 2) >> 2;    // (each accumulator has four warps: nothing else runs on the SM while a tile of 256 x 256 leaves)
         if (a < na) epilogue_bf16<EXT>(p, tmem + a * acc_cols, warp & 3, lane, n0 + a * BM, m0, m_end);
       } else {
         epilogue_fp16(p, tmem, warp & 3, lane, 0, 1, n0, m0);
       }
     }
-    fence_before();
   }
   if (NA == 1 && p.ksplit > 1) {
+    if (warp < 2) cluster_wait();
     if (p.pdl) wait_for_prerequisites();
-    sum_cluster<BF16, EXT>(p, ctl, smem_s, ks, n0, m0, m_end, 64 + 128);
+    sum_cluster<BF16, EXT>(p, ctl, tmem, smem, ks, n0, m0, m_end, warp < 2 ? -1 : 0, 1, warp & 3, lane, ahead);
   }
+  fence_before();
   __syncthreads();
   fence_after();
   if (warp == 1) tmem_dealloc(tmem, tmem_cols);
@@ -663,7 +740,7 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
 // Dynamic shared memory: [slot][activations: two halves of 64 k, mb * 128 B each][raw stage][8 KB of packed nibbles].
 template <int NG>
 __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
-  constexpr int THREADS = (3 + 4 * NG) * 32;   // warp 0: raw tiles, warp 1: MMA, then 4 NG transform + epilogue, last: activations
+  // warp 0: raw tiles, warp 1: MMA, then 4 NG transform + epilogue, last: activations
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ SharedCtl ctl;
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -686,14 +763,17 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       mbar_init(sa(&ctl.raw_empty[r]), 4);
     }
     mbar_init(sa(&ctl.accum), 1);
+    if (p.ksplit > 1) expect_sums(p, ctl, ks, m0, p.M);
     ctl.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (p.ksplit > 1) cluster_arrive();
   if (warp == 1) tmem_alloc(sa(&ctl.tmem_base), tmem_cols);
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = ctl.tmem_base;
+  SumAhead ahead{};
   if (p.pdl) launch_dependents();   // not before the tensor memory is ours: a block of the next GEMM would keep it while it waits for this kernel
 
   if (warp == 0) {
@@ -818,20 +898,24 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       s += NG;
       while (s >= S) { s -= S; spar ^= 1u; }
     }
+    if (p.ksplit > 1) {
+      if (p.pdl) wait_for_prerequisites();
+      ahead = sums_ahead<false>(p, ks, group, n0, m0, p.M, q, lane);
+      cluster_wait();             // everybody's barrier is there
+    }
     if (p.pdl) wait_for_prerequisites();                // the residual and the output are others' until here
     const bool done = warp_wait(sa(&ctl.accum), 0, &ctl.abort);
     if (!done) give_up(ctl, p.error_flag, 24);
     fence_after();
-    if (done) {
-      if (p.ksplit > 1) leave_sums(p, tmem, q, lane, group, NG, reinterpret_cast<float *>(smem));
-      else epilogue_fp16(p, tmem, q, lane, group, NG, n0, m0);
-    }
-    fence_before();
+    if (done && p.ksplit == 1) epilogue_fp16(p, tmem, q, lane, group, NG, n0, m0);
   }
   if (p.ksplit > 1) {
+    const bool idle = warp < 2 || warp == 2 + 4 * NG;
+    if (idle) cluster_wait();
     if (p.pdl) wait_for_prerequisites();
-    sum_cluster<false, false>(p, ctl, smem_s, ks, n0, m0, p.M, THREADS);
+    sum_cluster<false, false>(p, ctl, tmem, smem, ks, n0, m0, p.M, idle ? -1 : (warp - 2) >> 2, NG, warp & 3, lane, ahead);
   }
+  fence_before();
   __syncthreads();
   fence_after();
   if (warp == 1) tmem_dealloc(tmem, tmem_cols);
@@ -975,6 +1059,13 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     PT_REQUIRE(a->scales && a->group >= 128 && a->group % 128 == 0 && a->k_in % a->group == 0,
                "pt_gemm: INT4 needs scales and a group (%d) that is a multiple of 128 dividing k_in=%d", a->group, a->k_in);
 
+  const int out_ld = a->out_ld > 0 ? a->out_ld : (a->epilogue == PT_EPI_SWIGLU ? a->n_out / 2 : a->n_out);
+  if (few::takes(*a)) {
+    const cudaError_t e = few::run(*a, out_ld, as_stream(stream));
+    if (e != cudaSuccess) return pt::set_error(PT_ERR_CUDA, "pt_gemm: %s", cudaGetErrorString(e));
+    PT_LAUNCH_CHECK("pt_gemm");
+    return PT_OK;
+  }
   tc::GemmParams p{};
   p.M = a->m; p.N = a->n_out; p.K = a->k_in;
   p.group = int4 ? a->group : 0;
@@ -994,13 +1085,17 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   p.mb = plan.mb; p.n_kb = plan.n_kb; p.ksplit = plan.ksplit; p.kb_per_split = plan.kb_per_split;
   p.stages = plan.stages; p.raw_stages = plan.raw_stages; p.tmem_columns = plan.tmem_columns;
   p.n_tiles = plan.n_tiles;
+  p.x = (const unsigned char *)a->x;
+  p.x_pitch = (size_t)a->k_in * (bf16 || fp16 || int4 ? 2 : 1);
+  p.x_warps = plan.x_warps;
+  p.sum_offset = plan.sum_offset;
   p.epilogue = a->epilogue;
   p.out_scale = int4 ? 1.0f : (a->x_scale > 0.f ? a->x_scale : 1.0f) * (a->w_scale > 0.f ? a->w_scale : 1.0f);
   p.scales = (const __half *)a->scales;
   p.residual = wants_residual ? (const __half *)a->residual : nullptr;
   p.bias = wants_bias ? (const __half *)a->bias : nullptr;
   p.out = (__half *)a->out;
-  p.out_ld = a->out_ld > 0 ? a->out_ld : (a->epilogue == PT_EPI_SWIGLU ? a->n_out / 2 : a->n_out);
+  p.out_ld = out_ld;
   if (bf16) p.dense = make_dense_out(a->out, p.out_ld, a->out_dtype, a->epilogue, a->alpha, a->ext);
   p.error_flag = a->error_flag;
   if (a->ksplit > 1 && p.ksplit > 1) {   // slices that the caller asked for

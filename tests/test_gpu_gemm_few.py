@@ -1,0 +1,50 @@
+"""Small products of up to eight activation rows at the edges of their split, against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# (n, k): whole blocks and ragged ends of weight rows, one k block, warps that share k with a remainder, clusters, many rounds of blocks; the
+# last two are not theirs (too large a matrix)
+@pytest.mark.parametrize("n,k", [(16, 64), (40, 64), (24, 1600), (768, 768), (2056, 512), (768, 3072), (1000, 4096), (50257, 192), (1031, 4096), (2064, 2048)])
+@pytest.mark.parametrize("m", [1, 3, 8])
+@pytest.mark.parametrize("fmt", ["fp16", "bf16"])
+def test_sizes(cuda, n, k, m, fmt):
+    from poptransformer_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(n + k + m)
+    dt = torch.float16 if fmt == "fp16" else torch.bfloat16
+    w, x = (torch.randn((n, k), generator=g, device=cuda) * 0.05).to(dt), torch.randn((m, k), generator=g, device=cuda).to(dt)
+    err = torch.zeros(1, dtype=torch.int32, device=cuda)
+    out = torch.empty((m, n), dtype=dt, device=cuda)
+    ops.gemm(x, ops.GemmWeight(ops.W_FP16 if fmt == "fp16" else ops.W_BF16, w), out=out, error_flag=err)
+    exp, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    # one rounding of the result, and k sums of which each step may lose 2^-23 of what has gathered
+    bound = exp.abs() * 2.0 ** (-11 if fmt == "fp16" else -8) + size * k * 2.0 ** -23 + 1e-6
+    assert bool(((out.double() - exp).abs() <= bound).all()) and int(err.item()) == 0
+
+
+@pytest.mark.parametrize("epilogue", ["residual", "bias", "bias_residual", "bias_gelu", "relu2", "swiglu"])
+@pytest.mark.parametrize("n,k", [(768, 768), (768, 3072), (80, 128), (1000, 64)])
+def test_fp16_epilogues(cuda, n, k, epilogue):
+    """As many roundings as the same steps in fp16; the residual is the output itself, as the decoders have it."""
+    from poptransformer_b200 import ops
+    if epilogue == "swiglu" and n % 16:
+        pytest.skip("gates and ups come in blocks of eight")
+    g = torch.Generator(device=cuda).manual_seed(n + k)
+    m = 5
+    w, x = (torch.randn((n, k), generator=g, device=cuda) * 0.05).half(), torch.randn((m, k), generator=g, device=cuda).half()
+    bias, res = torch.randn(n, generator=g, device=cuda).half(), torch.randn((m, n), generator=g, device=cuda).half()
+    y = (x.double() @ w.double().T)
+    b = bias.double()
+    exp = {"residual": res.double() + y, "bias": y + b, "bias_residual": res.double() + y + b, "bias_gelu": torch.nn.functional.gelu(y + b), "relu2": torch.relu(y) ** 2,
+           "swiglu": None}[epilogue]
+    if epilogue == "swiglu":
+        y = y.view(m, -1, 2, 8)
+        exp = (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(m, -1)
+    out = res.clone() if "residual" in epilogue else torch.empty((m, n // 2 if epilogue == "swiglu" else n), dtype=torch.float16, device=cuda)
+    ops.gemm(x, ops.GemmWeight(ops.W_FP16, w), out=out, epilogue=getattr(ops, "EPI_" + epilogue.upper()), bias=bias if "bias" in epilogue else None,
+             residual=out if "residual" in epilogue else None)
+    # three or four roundings of values of the size of the result and of the sums that went into it
+    bound = 4 * 2.0 ** -11 * (exp.abs() + 4) * (1 + exp.abs().sqrt())
+    assert bool(((out.double() - exp).abs() <= bound).all())
