@@ -71,6 +71,7 @@ uint64_t pt_launch_count(void);
 #define PT_EPI_GELU_MUL 8     /* gelu_tanh(acc) * mul[mul_ids[row]]  (PT_W_BF16 and pt_gemm_f32, see pt_dense_ext) */
 #define PT_EPI_SOFTCAP 9      /* limit * tanh(acc / limit)  (PT_W_BF16 and pt_gemm_f32, see pt_dense_ext) */
 #define PT_EPI_XIELU 10       /* quadratic / exponential unit (PT_W_BF16 and pt_gemm_f32, see pt_dense_ext) */
+#define PT_EPI_GATED_RESIDUAL 11 /* y = fp16(res + fp16(sigmoid(gate) * fp16(acc))), and half of that if asked (pt_gemm, PT_W_FP16) */
 #define PT_GLU_CLAMPED 0      /* kinds of gated units */
 #define PT_GLU_SILU 1
 #define PT_GLU_GELU 2
@@ -189,12 +190,17 @@ int pt_linear_static_scratch(const pt_linear_args *args, void *stream);
  *              custom_ops/int4_to_half_codelets.cpp:18-38) on its way to the tensor core.  Also epilogue PT_EPI_SWIGLU: rows in the
  *              interleaved order of pt_linear_repack (eight gate rows, the same eight up rows), out [m, n_out / 2].
  *   PT_W_FP16: x = fp16 [m, k_in], w = pt_gemm_repack of fp16 [n_out, k_in] (w_tiled = 1), out = fp16.  k_in a multiple of 64.  Also epilogues
- *              PT_EPI_BIAS_GELU, _BIAS_RESIDUAL, _RELU2 and, with rows interleaved as for INT4, _SWIGLU.
+ *              PT_EPI_BIAS_GELU, _BIAS_RESIDUAL, _RELU2, _GATED_RESIDUAL and, with rows interleaved as for INT4, _SWIGLU.
  *   PT_W_BF16: x = bf16 [m, k_in], w = pt_gemm_repack of bf16 [n_out, k_in] (w_tiled = 1); out = bf16 or fp32 (out_dtype),
  *              epilogue PT_EPI_STORE, _RELU2, _GLU or _GELU_MUL on alpha * (x . w^T).  k_in a multiple of 64.
  * FP8 and INT4: k_in must be a multiple of 128.  Accumulation is fp32.  k-slices (ksplit, 0 = chosen by the library) are summed in a fixed
  * order in the shared memory of a cluster, at most eight whatever was asked for.  A caller that asks for slices itself (ksplit > 1) still has
  * to hand over a workspace of pt_gemm_workspace_bytes, which nothing touches. */
+typedef struct pt_gemm_part {
+  int n_out;              /* a multiple of 128, but in the last part                 */
+  int epilogue;           /* PT_EPI_STORE or PT_EPI_RELU2                            */
+  void *out;              /* fp16 [m, n_out]                                         */
+} pt_gemm_part;
 typedef struct pt_gemm_args {
   int wfmt;               /* PT_W_FP8, PT_W_INT4, PT_W_FP16 or PT_W_BF16            */
   int m, n_out, k_in;
@@ -210,12 +216,17 @@ typedef struct pt_gemm_args {
   int out_ld;             /* row stride of `out` in elements; 0 = dense              */
   void *workspace;        /* wanted if ksplit > 1, not used                          */
   size_t workspace_bytes;
-  int32_t *error_flag;    /* optional device int, set non-zero (21..26) if a bounded wait gave up */
+  int32_t *error_flag;    /* optional device int, set non-zero (21..27) if a bounded wait gave up */
   const void *bias;       /* fp16 [n_out] (PT_EPI_BIAS..)                             */
   int out_dtype;          /* PT_W_BF16: PT_DT_BF16 or PT_DT_F32                      */
   float alpha;            /* PT_W_BF16: factor on the fp32 sum; 0 = 1                */
   const pt_dense_ext *ext; /* PT_W_BF16: further arguments, or NULL                  */
   int pdl;                /* 1: programmatic dependent launch (see pt_linear_args.pdl); without effect if w_tiled = 0 */
+  const void *gate;       /* fp16 [m, n_out] (PT_EPI_GATED_RESIDUAL)                 */
+  int halve;              /* PT_EPI_GATED_RESIDUAL: half of the result               */
+  const pt_gemm_part *parts; /* PT_W_FP16: products that share a launch.  Their weight rows follow one another in w (n_out: all of them, epilogue
+                             PT_EPI_STORE), and x has m rows for each: fp16 [n_parts * m, k_in].  `out` and `out_ld` are not used */
+  int n_parts;            /* at most 3; 0: one product                               */
 } pt_gemm_args;
 size_t pt_gemm_workspace_bytes(int m, int n_out, int max_ksplit);
 int pt_gemm(const pt_gemm_args *args, void *stream);

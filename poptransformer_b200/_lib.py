@@ -46,13 +46,17 @@ class AttnArgs(ctypes.Structure):
     ]
 
 
+class GemmPart(ctypes.Structure):
+    _fields_ = [("n_out", c_int), ("epilogue", c_int), ("out", c_void_p)]
+
+
 class GemmArgs(ctypes.Structure):
     _fields_ = [
         ("wfmt", c_int), ("m", c_int), ("n_out", c_int), ("k_in", c_int), ("group", c_int), ("epilogue", c_int), ("ksplit", c_int),
         ("w_tiled", c_int), ("x", c_void_p), ("w", c_void_p), ("scales", c_void_p), ("x_scale", c_float), ("w_scale", c_float),
         ("residual", c_void_p), ("out", c_void_p), ("out_ld", c_int), ("workspace", c_void_p), ("workspace_bytes", c_size_t),
         ("error_flag", c_void_p), ("bias", c_void_p), ("out_dtype", c_int), ("alpha", c_float), ("ext", ctypes.POINTER(DenseExt)),
-        ("pdl", c_int),
+        ("pdl", c_int), ("gate", c_void_p), ("halve", c_int), ("parts", ctypes.POINTER(GemmPart)), ("n_parts", c_int),
     ]
 
 

@@ -478,7 +478,7 @@ static AttnSplit split_keys(int units, int max_pages, int page, int head_dim) {
   const int chunks = (int)std::min<long long>((long long)max_pages * page * head_dim / 2048 + 1, 1 << 20);
   const int sms = sm_count(), warps = units > 2 * sms ? 4 : units > sms || chunks < 16 ? 8 : 16;
   int runs = 1;
-  while (warps == 16 && runs < (units <= 4 ? 16 : 8) && 2 * units * runs <= sms && chunks >= 16 * runs) runs *= 2;
+  while (warps == 16 && runs < (units <= 4 ? 16 : 8) && 2 * units * runs <= sms && chunks >= 20 * runs) runs *= 2;
   return {warps, runs};
 }
 template <int H, int NW> static cudaError_t launch_attn(const AttnParams &p, cudaStream_t stream) {

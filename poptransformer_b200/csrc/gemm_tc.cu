@@ -42,6 +42,15 @@ cudaError_t run(const pt_gemm_args &a, int out_ld, cudaStream_t st);
 }  // namespace few
 namespace tc {
 
+// What becomes of a finished sum of the kernels with fp16 output (FP8, INT4, FP16).
+struct Fp16Out {
+  __half *out;
+  const __half *residual, *bias, *gate;
+  int out_ld, N, epilogue, halve;
+  float scale;
+};
+constexpr int MAX_PARTS = 3;
+
 struct GemmParams {
   int M, N, K;
   int mb;                 // activation rows per CTA (multiple of 16, at most 256)
@@ -50,20 +59,16 @@ struct GemmParams {
   int ksplit, stages, raw_stages;
   int tmem_columns;       // tensor memory of a CTA
   int w_tiled;            // weights tiled by pt_gemm_repack (one contiguous tile per stage) instead of row-major
-  int epilogue;           // (BF16: see dense)
-  float out_scale;
   const unsigned char *w; // tiled weights (w_tiled)
   const unsigned char *x; // activations, rows of x_pitch bytes
   size_t x_pitch;
   int x_warps;            // few activation rows: warps fetch them, not TMA
   int sum_offset;         // where in a block's shared memory the slices of its share of a tile arrive (0: in place of the operands)
   const __half *scales;   // INT4: [N][K / group]
-  const __half *residual;
-  const __half *bias;
-  __half *out;
-  int out_ld;
   int *error_flag;
   DenseOut dense;         // BF16: what becomes of a finished sum
+  Fp16Out o[MAX_PARTS];   // the others.  FP16: outputs of several products that share a launch, part s from tile part_tile[s] on with activation rows s M ..
+  int n_parts, part_tile[MAX_PARTS];
   const int *group_of;    // BF16, grouped: the weight matrix of every tile of mb rows (negative: none)
   const int *group_used;  // ... and how many of its rows are in use (null: all)
   int n_tiles;            // tiles of 128 weight rows
@@ -207,126 +212,110 @@ __device__ __forceinline__ bool wait_fast(uint32_t bar, uint32_t parity, volatil
 // The same for a whole warp: every lane gets the same answer.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return __all_sync(0xffffffffu, wait_fast(bar, parity, abort_flag)); }
 
-// One finished sum of the kernels with fp16 output (FP8, INT4, FP16) or of the BF16 kernel.  (SWIGLU, whose sums come in pairs: store_swiglu.)
 __device__ __forceinline__ __half relu2_h(__half y) {
   const __half r = __hgt(y, __float2half_rn(0.f)) ? y : __float2half_rn(0.f);
   return h_mul(r, r);
 }
-__device__ __forceinline__ __half fp16_out(const GemmParams &p, float acc, int m, int n) {
-  __half y = __float2half_rn(acc * p.out_scale);
-  if (p.epilogue == PT_EPI_RESIDUAL) return h_add(__ldcg(p.residual + (size_t)m * p.N + n), y);
-  if (p.epilogue == PT_EPI_BIAS) return h_add(y, p.bias[n]);
-  if (p.epilogue == PT_EPI_RELU2) return relu2_h(y);
-  if (p.epilogue == PT_EPI_BIAS_GELU) return gelu_h(h_add(y, p.bias[n]));
-  if (p.epilogue == PT_EPI_BIAS_RESIDUAL) return h_add(__ldcg(p.residual + (size_t)m * p.N + n), h_add(y, p.bias[n]));
-  return y;
-}
-template <bool BF16, bool EXT> __device__ __forceinline__ void store_out(const GemmParams &p, float acc, int m, int n) {
-  if constexpr (BF16) dense_store<EXT>(p.dense, m, n, acc);
-  else p.out[(size_t)m * p.out_ld + n] = fp16_out(p, acc, m, n);
-}
 // Sums of the gate row n (n % 16 < 8) and of the up row n + 8.
-__device__ __forceinline__ __half swiglu_h(const GemmParams &p, float gate, float up) {
-  return h_mul(__float2half_rn(up * p.out_scale), swish_h(__float2half_rn(gate * p.out_scale)));
+__device__ __forceinline__ __half swiglu_h(const Fp16Out &p, float gate, float up) {
+  return h_mul(__float2half_rn(up * p.scale), swish_h(__float2half_rn(gate * p.scale)));
 }
 // The first `rows` of R rows m .. m + R - 1 of a warp's 32 weight rows (lane = n), fp16.
 // PAIRS: all n are inside the output and neighbours on 4-byte boundaries: neighbouring lanes trade values so that a lane writes two
 // consecutive n.  SWIGLU trades between lanes n and n + 8, and each computes every other row of the pair's feature.
-struct Residual2 { __half2 v[2]; };     // of the four rows of a pair of outputs: every other row of a lane's
-template <int EPI, bool PAIRS, int R> __device__ __forceinline__ void fp16_rows(const GemmParams &p, const float (&sum)[R], int m, int rows, int n, int lane, const Residual2 *got = nullptr) {
-  constexpr bool RES = EPI == PT_EPI_RESIDUAL || EPI == PT_EPI_BIAS_RESIDUAL, BIAS = EPI == PT_EPI_BIAS || EPI == PT_EPI_BIAS_GELU || EPI == PT_EPI_BIAS_RESIDUAL;
+struct Ahead2 { __half2 res[2], gate[2]; };     // residual and gate of four rows of a pair of outputs: every other row is a lane's
+template <int EPI, bool PAIRS, int R> __device__ __forceinline__ void fp16_rows(const Fp16Out &p, const float (&sum)[R], int m, int rows, int n, int lane, const Ahead2 *got = nullptr) {
+  constexpr bool GATED = EPI == PT_EPI_GATED_RESIDUAL, RES = EPI == PT_EPI_RESIDUAL || EPI == PT_EPI_BIAS_RESIDUAL || GATED, BIAS = EPI == PT_EPI_BIAS || EPI == PT_EPI_BIAS_GELU || EPI == PT_EPI_BIAS_RESIDUAL;
   if constexpr (EPI == PT_EPI_SWIGLU) {
     const bool up = lane & 8, in = PAIRS || n < p.N;
-    __half *o = p.out + (size_t)(m + (up ? 1 : 0)) * p.out_ld + n / 16 * 8 + n % 8;
+    __half *to = p.out + (size_t)(m + (up ? 1 : 0)) * p.out_ld + n / 16 * 8 + n % 8;
 #pragma unroll
     for (int j = 0; j < R; j += 2) {
       const float t = __shfl_xor_sync(0xffffffffu, up ? sum[j] : sum[j + 1], 8);
-      if (in && j + (up ? 1 : 0) < rows) *o = up ? swiglu_h(p, t, sum[j + 1]) : swiglu_h(p, sum[j], t);
-      o += 2 * (size_t)p.out_ld;
+      if (in && j + (up ? 1 : 0) < rows) *to = up ? swiglu_h(p, t, sum[j + 1]) : swiglu_h(p, sum[j], t);
+      to += 2 * (size_t)p.out_ld;
     }
   } else if constexpr (PAIRS) {
     const int odd = lane & 1;
-    __half2 *o = reinterpret_cast<__half2 *>(p.out + (size_t)(m + odd) * p.out_ld + (n - odd));
-    __half2 res[RES ? R / 2 : 1], bias = __half2half2(__half(0));
+    __half2 *to = reinterpret_cast<__half2 *>(p.out + (size_t)(m + odd) * p.out_ld + (n - odd));
+    __half2 res[RES ? R / 2 : 1], gate[GATED ? R / 2 : 1], bias = __half2half2(__half(0));
     if constexpr (RES) {
 #pragma unroll
-      for (int j = 0; j < R / 2; ++j)
-        if (R == 4 && got) res[j] = got->v[j & 1];
-        else if (2 * j + odd < rows) res[j] = __ldcg(reinterpret_cast<const __half2 *>(p.residual + (size_t)(m + odd + 2 * j) * p.N + (n - odd)));
+      for (int j = 0; j < R / 2; ++j) {
+        const size_t at = (size_t)(m + odd + 2 * j) * p.N + (n - odd);
+        if (R == 4 && got) {
+          res[j] = got->res[j & 1];
+          if constexpr (GATED) gate[j] = got->gate[j & 1];
+        } else if (2 * j + odd < rows) {
+          res[j] = __ldcg(reinterpret_cast<const __half2 *>(p.residual + at));
+          if constexpr (GATED) gate[j] = __ldcg(reinterpret_cast<const __half2 *>(p.gate + at));
+        }
+      }
     }
     if constexpr (BIAS) bias = *reinterpret_cast<const __half2 *>(p.bias + (n - odd));
 #pragma unroll
     for (int j = 0; j < R; j += 2) {
       const float t = __shfl_xor_sync(0xffffffffu, odd ? sum[j] : sum[j + 1], 1);   // even lane: row j of n + 1; odd lane: row j + 1 of n - 1
-      __half2 y = odd ? __floats2half2_rn(t * p.out_scale, sum[j + 1] * p.out_scale) : __floats2half2_rn(sum[j] * p.out_scale, t * p.out_scale);
+      __half2 y = odd ? __floats2half2_rn(t * p.scale, sum[j + 1] * p.scale) : __floats2half2_rn(sum[j] * p.scale, t * p.scale);
       if constexpr (BIAS) y = __hadd2_rn(y, bias);
       if constexpr (EPI == PT_EPI_RELU2) y = __halves2half2(relu2_h(__low2half(y)), relu2_h(__high2half(y)));
       if constexpr (EPI == PT_EPI_BIAS_GELU) y = __halves2half2(gelu_h(__low2half(y)), gelu_h(__high2half(y)));
+      if constexpr (GATED) y = __halves2half2(h_mul(sigmoid_h(__low2half(gate[j / 2])), __low2half(y)), h_mul(sigmoid_h(__high2half(gate[j / 2])), __high2half(y)));
       if constexpr (RES) y = __hadd2_rn(res[j / 2], y);
-      if (j + odd < rows) *o = y;
-      o += p.out_ld;   // (two rows, in units of two)
+      if constexpr (GATED) { if (p.halve) y = __hmul2_rn(y, __float2half2_rn(0.5f)); }
+      if (j + odd < rows) *to = y;
+      to += p.out_ld;   // (two rows, in units of two)
     }
   } else if (n < p.N) {
-    __half *o = p.out + (size_t)m * p.out_ld + n;
+    __half *to = p.out + (size_t)m * p.out_ld + n;
     const __half bias = BIAS ? p.bias[n] : __half(0);
 #pragma unroll
     for (int j = 0; j < R; ++j) {
       if (j >= rows) break;
-      __half y = __float2half_rn(sum[j] * p.out_scale);
+      __half y = __float2half_rn(sum[j] * p.scale);
       if constexpr (BIAS) y = h_add(y, bias);
       if constexpr (EPI == PT_EPI_RELU2) y = relu2_h(y);
       if constexpr (EPI == PT_EPI_BIAS_GELU) y = gelu_h(y);
+      if constexpr (GATED) y = h_mul(sigmoid_h(__ldcg(p.gate + (size_t)(m + j) * p.N + n)), y);
       if constexpr (RES) y = h_add(__ldcg(p.residual + (size_t)(m + j) * p.N + n), y);
-      *o = y;
-      o += p.out_ld;
+      if constexpr (GATED) { if (p.halve) y = h_mul(y, __float2half_rn(0.5f)); }
+      *to = y;
+      to += p.out_ld;
     }
   }
 }
-template <bool PAIRS, int R> __device__ __forceinline__ void fp16_rows(const GemmParams &p, const float (&sum)[R], int m, int rows, int n, int lane, const Residual2 *got = nullptr) {
+template <bool PAIRS, int R> __device__ __forceinline__ void fp16_rows(const Fp16Out &p, const float (&sum)[R], int m, int rows, int n, int lane, const Ahead2 *got = nullptr) {
   if (p.epilogue == PT_EPI_STORE) fp16_rows<PT_EPI_STORE, PAIRS, R>(p, sum, m, rows, n, lane, got);
   else if (p.epilogue == PT_EPI_SWIGLU) fp16_rows<PT_EPI_SWIGLU, PAIRS, R>(p, sum, m, rows, n, lane, got);
   else if (p.epilogue == PT_EPI_RESIDUAL) fp16_rows<PT_EPI_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
   else if (p.epilogue == PT_EPI_BIAS) fp16_rows<PT_EPI_BIAS, PAIRS, R>(p, sum, m, rows, n, lane, got);
   else if (p.epilogue == PT_EPI_BIAS_GELU) fp16_rows<PT_EPI_BIAS_GELU, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (p.epilogue == PT_EPI_GATED_RESIDUAL) fp16_rows<PT_EPI_GATED_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
   else if (p.epilogue == PT_EPI_RELU2) fp16_rows<PT_EPI_RELU2, PAIRS, R>(p, sum, m, rows, n, lane, got);
   else fp16_rows<PT_EPI_BIAS_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
 }
 // Whether the rows of the 32 weight rows from nq on can leave in pairs.
-__device__ __forceinline__ bool fp16_pairs(const GemmParams &p, int nq) {
+__device__ __forceinline__ bool fp16_pairs(const Fp16Out &p, int nq) {
   return nq + 32 <= p.N && p.out_ld % 2 == 0 && ((uintptr_t)p.out & 3) == 0 && (!p.residual || (p.N % 2 == 0 && ((uintptr_t)p.residual & 3) == 0)) &&
-         (!p.bias || ((uintptr_t)p.bias & 3) == 0);
+         (!p.bias || ((uintptr_t)p.bias & 3) == 0) && (!p.gate || ((uintptr_t)p.gate & 3) == 0);
 }
 // The epilogue of a tile without k-slices, fp16 outputs: `part` of `parts` warps share a quarter of the rows and take alternate 16 columns.
 // (Measured on B200, FP8 10304 x 2048, whose last tile is half empty, at 256 rows: 12.9 us; element by element over all branches, empty
 // quarters included, 18.9.  2048 x 128 at 12 rows, a step of 16 in part: 3.1 and 4.7.)
-__device__ __forceinline__ void epilogue_fp16(const GemmParams &p, uint32_t tmem, int q, int lane, int part, int parts, int n0, int m0) {
+__device__ __forceinline__ void epilogue_fp16(const GemmParams &p, const Fp16Out &o, uint32_t tmem, int q, int lane, int part, int parts, int n0, int m0) {
   const int nq = n0 + q * 32, n = nq + lane, rows = min(p.mb, p.M - m0);
-  if (nq >= p.N) return;          // (uniform over the warp, as is `pairs`)
-  const bool pairs = fp16_pairs(p, nq);
+  if (nq >= o.N) return;          // (uniform over the warp, as is `pairs`)
+  const bool pairs = fp16_pairs(o, nq);
   for (int c0 = part * 16; c0 < rows; c0 += 16 * parts) {
     uint32_t v[16];
     float sum[16];
     tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
     for (int j = 0; j < 16; ++j) sum[j] = __uint_as_float(v[j]);
-    if (pairs) fp16_rows<true>(p, sum, m0 + c0, rows - c0, n, lane);
-    else fp16_rows<false>(p, sum, m0 + c0, rows - c0, n, lane);
+    if (pairs) fp16_rows<true>(o, sum, m0 + c0, rows - c0, n, lane);
+    else fp16_rows<false>(o, sum, m0 + c0, rows - c0, n, lane);
   }
 }
-// Four consecutive fp16 outputs n .. n + 3 < N (n a multiple of four).
-__device__ __forceinline__ void fp16_store4(const GemmParams &p, int m, int n, const float4 &acc) {
-  const float a[4] = {acc.x, acc.y, acc.z, acc.w};
-  __half y[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) y[j] = fp16_out(p, a[j], m, n + j);
-  __half *o = p.out + (size_t)m * p.out_ld + n;
-  if (((uintptr_t)o & 7) == 0) *reinterpret_cast<uint2 *>(o) = *reinterpret_cast<const uint2 *>(y);
-  else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) o[j] = y[j];
-  }
-}
-
 // R rows of one weight row per lane, gated: lanes n and n + 8 hold a feature's two sums.
 template <int GLU, bool EXT, int R> __device__ __forceinline__ void glu_rows(const GemmParams &p, const float (&sum)[R], int m, int m_end, int n, int lane) {
   const DenseOut &d = p.dense;
@@ -472,26 +461,29 @@ __device__ __forceinline__ void expect_sums(const GemmParams &p, SharedCtl &ctl,
   const int own = own_groups(row_groups(p, m0, m_end), p.ksplit, rank);
   if (own) mbar_expect_tx(sa(&ctl.sums), own * p.ksplit * BM * 16);
 }
-// The warps that sum have asked for what they need before their products are there: the residual of the first group of rows a warp writes, and
+// The warps that sum have asked for what they need before their products are there: residual and gate of the first group of rows a warp writes, and
 // (the parameters of a launch are in no cache at first) the fields that the outputs go by.
-struct SumAhead { Residual2 res; bool pairs, got; };
-template <bool BF16> __device__ __forceinline__ SumAhead sums_ahead(const GemmParams &p, int rank, int part, int n0, int m0, int m_end, int q, int lane) {
+struct SumAhead { Ahead2 v; bool pairs, got; };
+template <bool BF16> __device__ __forceinline__ SumAhead sums_ahead(const GemmParams &p, const Fp16Out &o, int rank, int part, int n0, int m0, int m_end, int q, int lane) {
   SumAhead a;
-  a.pairs = !BF16 && fp16_pairs(p, n0 + q * 32);
-  a.got = a.pairs && (p.epilogue == PT_EPI_RESIDUAL || p.epilogue == PT_EPI_BIAS_RESIDUAL);
+  a.pairs = !BF16 && fp16_pairs(o, n0 + q * 32);
+  a.got = a.pairs && o.residual;
   if constexpr (BF16) asm volatile("" ::"r"(p.dense.epilogue), "r"(p.dense.out_ld), "f"(p.dense.limit), "r"(p.dense.glu), "l"(p.dense.out), "l"(p.dense.bias));
-  else asm volatile("" ::"r"(p.epilogue), "r"(p.out_ld), "f"(p.out_scale), "l"(p.out), "l"(p.bias));
   if (a.got) {
     const int odd = lane & 1, m = m0 + 4 * (part * p.ksplit + rank);
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
-      a.res.v[j] = m + odd + 2 * j < m_end ? __ldcg(reinterpret_cast<const __half2 *>(p.residual + (size_t)(m + odd + 2 * j) * p.N + (n0 + q * 32 + lane - odd))) : __half2half2(__half(0));
+    for (int j = 0; j < 2; ++j) {
+      const size_t at = (size_t)(m + odd + 2 * j) * o.N + (n0 + q * 32 + lane - odd);
+      const bool in = m + odd + 2 * j < m_end;
+      a.v.res[j] = in ? __ldcg(reinterpret_cast<const __half2 *>(o.residual + at)) : __half2half2(__half(0));
+      a.v.gate[j] = in && o.gate ? __ldcg(reinterpret_cast<const __half2 *>(o.gate + at)) : __half2half2(__half(0));
+    }
   }
   return a;
 }
 // The warps that have a tile's quarters q (`parts` times four of them, each part every parts-th step of 16 rows); the other threads of the block call it too.
 template <bool BF16, bool EXT>
-__device__ __forceinline__ void sum_cluster(const GemmParams &p, SharedCtl &ctl, uint32_t tmem, unsigned char *smem, int rank, int n0, int m0, int m_end, int part, int parts, int q, int lane, const SumAhead &ahead) {
+__device__ __forceinline__ void sum_cluster(const GemmParams &p, const Fp16Out &o, SharedCtl &ctl, uint32_t tmem, unsigned char *smem, int rank, int n0, int m0, int m_end, int part, int parts, int q, int lane, const SumAhead &ahead) {
   if (p.sum_offset == 0) {    // where the sums take the place of the operands, nobody reads these any more
     cluster_arrive();
     cluster_wait();
@@ -517,7 +509,7 @@ __device__ __forceinline__ void sum_cluster(const GemmParams &p, SharedCtl &ctl,
   if (!warp_wait(bar, 0, &ctl.abort)) give_up(ctl, p.error_flag, 27);
   if (ctl.abort) return;
   const int nq = n0 + q * 32, n = nq + lane;
-  if (nq >= p.N) return;
+  if (nq >= (BF16 ? p.N : o.N)) return;
   for (int i = part; i < own; i += parts) {
     float4 v[MAX_CLUSTER];
 #pragma unroll
@@ -528,8 +520,8 @@ __device__ __forceinline__ void sum_cluster(const GemmParams &p, SharedCtl &ctl,
     for (int s = 0; s < MAX_CLUSTER; ++s) { sum[0] += v[s].x; sum[1] += v[s].y; sum[2] += v[s].z; sum[3] += v[s].w; }
     const int m = m0 + 4 * (i * ks + rank);
     if constexpr (BF16) bf16_rows<EXT>(p, sum, m, m_end, nq, lane);
-    else if (ahead.pairs) fp16_rows<true>(p, sum, m, m_end - m, n, lane, ahead.got && i == part ? &ahead.res : nullptr);
-    else fp16_rows<false>(p, sum, m, m_end - m, n, lane);
+    else if (ahead.pairs) fp16_rows<true>(o, sum, m, m_end - m, n, lane, ahead.got && i == part ? &ahead.v : nullptr);
+    else fp16_rows<false>(o, sum, m, m_end - m, n, lane);
   }
 }
 
@@ -578,7 +570,11 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
   __shared__ SharedCtl ctl;
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const int n0 = blockIdx.x * (BM * NA), m0 = blockIdx.z * p.mb, ks = blockIdx.y;
+  int part = 0;
+  if (FMT == PT_W_FP16)
+    while (part + 1 < p.n_parts && (int)blockIdx.x >= p.part_tile[part + 1]) ++part;
+  const Fp16Out o = p.o[BF16 ? 0 : part];
+  const int n0 = (blockIdx.x - (FMT == PT_W_FP16 ? p.part_tile[part] : 0)) * (BM * NA), m0 = blockIdx.z * p.mb, x0 = part * p.M + m0, ks = blockIdx.y;     // (x0: the first activation row)
   const int kb0 = ks * p.kb_per_split, kb1 = min(p.n_kb, kb0 + p.kb_per_split);
   const int n_it = kb1 - kb0, na = NA == 1 ? 1 : min(NA, p.n_tiles - (int)blockIdx.x * NA);
   const uint32_t b_bytes = (uint32_t)p.mb * BKB;
@@ -654,7 +650,7 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
           mbar_expect_tx(fb, tx);
           load_w(st, fb);
         }
-        if (!p.x_warps) tma_load_2d(st + NA * A_TILE, &map_x, kx, m0, fb);
+        if (!p.x_warps) tma_load_2d(st + NA * A_TILE, &map_x, kx, x0, fb);
         kx += KX;
         if (++s == p.stages) { s = 0; par ^= 1u; first_round = false; }
       }
@@ -693,11 +689,11 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
   } else {
     if (NA == 1 && p.x_warps) {
       if (p.pdl) wait_for_prerequisites();
-      fetch_rows(p, ctl, smem + A_TILE, stage_bytes, kb0, n_it, m0, m_end - m0, warp - 2, lane);
+      fetch_rows(p, ctl, smem + A_TILE, stage_bytes, kb0, n_it, x0, m_end - m0, warp - 2, lane);
     }
     if (NA == 1 && p.ksplit > 1) {
       if (p.pdl) wait_for_prerequisites();
-      ahead = sums_ahead<BF16>(p, ks, 0, n0, m0, m_end, warp & 3, lane);
+      ahead = sums_ahead<BF16>(p, o, ks, 0, n0, m0, m_end, warp & 3, lane);
       cluster_wait();             // everybody's barrier is there
     }
     if (p.pdl) wait_for_prerequisites();                // the residual and the output are others' until here
@@ -709,14 +705,14 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
         const int a = (warp - 2) >> 2;    // (each accumulator has four warps: nothing else runs on the SM while a tile of 256 x 256 leaves)
         if (a < na) epilogue_bf16<EXT>(p, tmem + a * acc_cols, warp & 3, lane, n0 + a * BM, m0, m_end);
       } else {
-        epilogue_fp16(p, tmem, warp & 3, lane, 0, 1, n0, m0);
+        epilogue_fp16(p, o, tmem, warp & 3, lane, 0, 1, n0, m0);
       }
     }
   }
   if (NA == 1 && p.ksplit > 1) {
     if (warp < 2) cluster_wait();
     if (p.pdl) wait_for_prerequisites();
-    sum_cluster<BF16, EXT>(p, ctl, tmem, smem, ks, n0, m0, m_end, warp < 2 ? -1 : 0, 1, warp & 3, lane, ahead);
+    sum_cluster<BF16, EXT>(p, o, ctl, tmem, smem, ks, n0, m0, m_end, warp < 2 ? -1 : 0, 1, warp & 3, lane, ahead);
   }
   fence_before();
   __syncthreads();
@@ -900,20 +896,20 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
     }
     if (p.ksplit > 1) {
       if (p.pdl) wait_for_prerequisites();
-      ahead = sums_ahead<false>(p, ks, group, n0, m0, p.M, q, lane);
+      ahead = sums_ahead<false>(p, p.o[0], ks, group, n0, m0, p.M, q, lane);
       cluster_wait();             // everybody's barrier is there
     }
     if (p.pdl) wait_for_prerequisites();                // the residual and the output are others' until here
     const bool done = warp_wait(sa(&ctl.accum), 0, &ctl.abort);
     if (!done) give_up(ctl, p.error_flag, 24);
     fence_after();
-    if (done && p.ksplit == 1) epilogue_fp16(p, tmem, q, lane, group, NG, n0, m0);
+    if (done && p.ksplit == 1) epilogue_fp16(p, p.o[0], tmem, q, lane, group, NG, n0, m0);
   }
   if (p.ksplit > 1) {
     const bool idle = warp < 2 || warp == 2 + 4 * NG;
     if (idle) cluster_wait();
     if (p.pdl) wait_for_prerequisites();
-    sum_cluster<false, false>(p, ctl, tmem, smem, ks, n0, m0, p.M, idle ? -1 : (warp - 2) >> 2, NG, warp & 3, lane, ahead);
+    sum_cluster<false, false>(p, p.o[0], ctl, tmem, smem, ks, n0, m0, p.M, idle ? -1 : (warp - 2) >> 2, NG, warp & 3, lane, ahead);
   }
   fence_before();
   __syncthreads();
@@ -1037,7 +1033,7 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   const int k_step = bf16 || fp16 ? 64 : 128;
   PT_REQUIRE(a->m >= 1 && a->n_out >= 1 && a->k_in >= k_step && a->k_in % k_step == 0, "pt_gemm: bad shape m=%d n_out=%d k_in=%d (k_in a multiple of %d)",
              a->m, a->n_out, a->k_in, k_step);
-  PT_REQUIRE(a->x && a->w && a->out, "pt_gemm: null x / w / out");
+  PT_REQUIRE(a->x && a->w && (a->out || a->n_parts), "pt_gemm: null x / w / out");
   PT_REQUIRE(((uintptr_t)a->x & 15) == 0 && ((uintptr_t)a->w & 15) == 0, "pt_gemm: x and w must be 16-byte aligned");
   if (bf16) {
     PT_REQUIRE(dense_epilogue_known(a->epilogue), "pt_gemm: BF16 epilogue %d (store, relu2, glu, gelu-mul, softcap or xielu)", a->epilogue);
@@ -1046,14 +1042,28 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
     PT_REQUIRE(a->out_dtype == PT_DT_BF16 || a->out_dtype == PT_DT_F32, "pt_gemm: BF16 weights write bf16 or fp32, got type %d", a->out_dtype);
   } else {
     PT_REQUIRE(a->epilogue == PT_EPI_STORE || a->epilogue == PT_EPI_RESIDUAL || a->epilogue == PT_EPI_BIAS || ((int4 || fp16) && a->epilogue == PT_EPI_SWIGLU) ||
-                   (fp16 && (a->epilogue == PT_EPI_BIAS_GELU || a->epilogue == PT_EPI_BIAS_RESIDUAL || a->epilogue == PT_EPI_RELU2)),
-               "pt_gemm: epilogue %d (store, residual or bias; INT4 and FP16: swiglu; FP16: relu2, bias with gelu or residual)", a->epilogue);
+                   (fp16 && (a->epilogue == PT_EPI_BIAS_GELU || a->epilogue == PT_EPI_BIAS_RESIDUAL || a->epilogue == PT_EPI_RELU2 || a->epilogue == PT_EPI_GATED_RESIDUAL)),
+               "pt_gemm: epilogue %d (store, residual or bias; INT4 and FP16: swiglu; FP16: relu2, gated residual, bias with gelu or residual)", a->epilogue);
     PT_REQUIRE(a->epilogue != PT_EPI_SWIGLU || a->n_out % 16 == 0, "pt_gemm: SwiGLU epilogue needs n_out %% 16 == 0, got %d", a->n_out);
   }
   const bool wants_bias = a->epilogue == PT_EPI_BIAS || a->epilogue == PT_EPI_BIAS_GELU || a->epilogue == PT_EPI_BIAS_RESIDUAL;
-  const bool wants_residual = a->epilogue == PT_EPI_RESIDUAL || a->epilogue == PT_EPI_BIAS_RESIDUAL;
+  const bool gated = !bf16 && a->epilogue == PT_EPI_GATED_RESIDUAL;
+  const bool wants_residual = a->epilogue == PT_EPI_RESIDUAL || a->epilogue == PT_EPI_BIAS_RESIDUAL || gated;
   PT_REQUIRE(!wants_residual || a->residual, "pt_gemm: residual epilogue needs residual");
   PT_REQUIRE(!wants_bias || a->bias, "pt_gemm: bias epilogue needs bias");
+  PT_REQUIRE(!gated || a->gate, "pt_gemm: gated residual epilogue needs gate");
+  if (a->n_parts) {
+    PT_REQUIRE(fp16 && a->parts && a->n_parts >= 1 && a->n_parts <= tc::MAX_PARTS && a->epilogue == PT_EPI_STORE, "pt_gemm: 1 to %d parts are for FP16, with epilogues of their own",
+               tc::MAX_PARTS);
+    long long n = 0;
+    for (int i = 0; i < a->n_parts; ++i) {
+      const pt_gemm_part &part = a->parts[i];
+      PT_REQUIRE(part.out && part.n_out >= 1 && (i + 1 == a->n_parts || part.n_out % tc::BM == 0) && (part.epilogue == PT_EPI_STORE || part.epilogue == PT_EPI_RELU2),
+                 "pt_gemm: part %d: n_out=%d (a multiple of %d but in the last), epilogue %d (store or relu2)", i, part.n_out, tc::BM, part.epilogue);
+      n += part.n_out;
+    }
+    PT_REQUIRE(n == a->n_out, "pt_gemm: the parts have %lld rows, n_out=%d", n, a->n_out);
+  }
   PT_REQUIRE(a->wfmt == PT_W_FP8 || a->w_tiled, "pt_gemm: INT4, BF16 and FP16 weights must be tiled with pt_gemm_repack");
   if (int4)
     PT_REQUIRE(a->scales && a->group >= 128 && a->group % 128 == 0 && a->k_in % a->group == 0,
@@ -1089,14 +1099,17 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   p.x_pitch = (size_t)a->k_in * (bf16 || fp16 || int4 ? 2 : 1);
   p.x_warps = plan.x_warps;
   p.sum_offset = plan.sum_offset;
-  p.epilogue = a->epilogue;
-  p.out_scale = int4 ? 1.0f : (a->x_scale > 0.f ? a->x_scale : 1.0f) * (a->w_scale > 0.f ? a->w_scale : 1.0f);
   p.scales = (const __half *)a->scales;
-  p.residual = wants_residual ? (const __half *)a->residual : nullptr;
-  p.bias = wants_bias ? (const __half *)a->bias : nullptr;
-  p.out = (__half *)a->out;
-  p.out_ld = out_ld;
-  if (bf16) p.dense = make_dense_out(a->out, p.out_ld, a->out_dtype, a->epilogue, a->alpha, a->ext);
+  p.o[0] = {(__half *)a->out, wants_residual ? (const __half *)a->residual : nullptr, wants_bias ? (const __half *)a->bias : nullptr, gated ? (const __half *)a->gate : nullptr, out_ld,
+            a->n_out, a->epilogue, a->halve, int4 ? 1.0f : (a->x_scale > 0.f ? a->x_scale : 1.0f) * (a->w_scale > 0.f ? a->w_scale : 1.0f)};
+  p.n_parts = std::max(1, a->n_parts);
+  for (int i = 0, tile = 0; i < a->n_parts; ++i) {
+    const pt_gemm_part &part = a->parts[i];
+    p.part_tile[i] = tile;
+    p.o[i] = {(__half *)part.out, nullptr, nullptr, nullptr, part.n_out, part.n_out, part.epilogue, 0, p.o[0].scale};
+    tile += ceil_div(part.n_out, tc::BM);
+  }
+  if (bf16) p.dense = make_dense_out(a->out, out_ld, a->out_dtype, a->epilogue, a->alpha, a->ext);
   p.error_flag = a->error_flag;
   if (a->ksplit > 1 && p.ksplit > 1) {   // slices that the caller asked for
     const size_t need = pt_gemm_workspace_bytes(a->m, a->n_out, p.ksplit);
@@ -1110,7 +1123,7 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   CUtensorMap map_w, map_x;
   memset(&map_w, 0, sizeof(map_w));
   if (int4 || fp16) {
-    if (int rc = tc::make_map(&map_x, a->x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)a->k_in, (uint64_t)a->m, 64, (uint32_t)p.mb, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+    if (int rc = tc::make_map(&map_x, a->x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)a->k_in, (uint64_t)a->m * p.n_parts, 64, (uint32_t)p.mb, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
   } else if (bf16) {
     if (int rc = tc::make_map(&map_x, a->x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a->k_in, (uint64_t)a->m, 64, (uint32_t)p.mb, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
   } else {

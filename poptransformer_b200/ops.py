@@ -26,7 +26,7 @@ from ._lib import (AttnArgs, BatchView, ContextRows, DenseExt, GemmArgs, HyperAr
 W_INT4, W_FP16, W_FP8, W_BF16 = 0, 1, 2, 3
 DT_F16, DT_F32, DT_BF16 = 0, 1, 2
 PRO_NONE, PRO_RMSNORM, PRO_CAST_FP8, PRO_RMSNORM_CAST_FP8, PRO_NORMCE = 0, 1, 2, 3, 4
-EPI_STORE, EPI_RESIDUAL, EPI_SWIGLU, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESIDUAL, EPI_RELU2, EPI_GLU, EPI_GELU_MUL, EPI_SOFTCAP, EPI_XIELU = range(11)
+EPI_STORE, EPI_RESIDUAL, EPI_SWIGLU, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESIDUAL, EPI_RELU2, EPI_GLU, EPI_GELU_MUL, EPI_SOFTCAP, EPI_XIELU, EPI_GATED_RESIDUAL = range(12)
 GLU_CLAMPED, GLU_SILU, GLU_GELU = 0, 1, 2
 MOE_SOFTMAX, MOE_SIGMOID, MOE_SOFTMAX_ALL = 0, 1, 2
 ROPE_NONE, ROPE_LLAMA, ROPE_CHATGLM2 = 0, 1, 2
@@ -208,13 +208,14 @@ def gemm_workspace(m, n_out_max, max_ksplit=8, device="cuda"):
 
 
 def gemm(x, gw, out=None, x_scale=1.0, epilogue=EPI_STORE, residual=None, workspace=None, ksplit=0, error_flag=None, bias=None,
-         out_ld=0, alpha=1.0, ext=None, pdl=0):
+         out_ld=0, alpha=1.0, ext=None, pdl=0, gate=None, halve=0, parts=None):
     """y = x @ W^T on the tcgen05 GEMM.  INT4: x fp16 [m, k]; FP8: x E4M3 bytes [m, k] quantised with `x_scale`; BF16: x bfloat16,
-    `out` bfloat16 or float32."""
-    m = x.shape[0]
+    `out` bfloat16 or float32.  gate, halve: of EPI_GATED_RESIDUAL.  parts = [(out, epilogue), ..] (FP16): as many products in one launch, whose weight rows
+    follow one another in `gw`; x has as many equal runs of rows, and the outputs are returned as a list."""
+    m = x.shape[0] // (len(parts) if parts else 1)
     if x.shape[1] != gw.k_in:
         raise PtError(f"gemm: x has k={x.shape[1]}, weight has k={gw.k_in}")
-    if out is None:
+    if out is None and not parts:
         out = torch.empty((m, gw.n_out // 2 if epilogue == EPI_SWIGLU else gw.n_out), dtype=torch.float16, device=x.device)
     a = GemmArgs()
     a.wfmt, a.m, a.n_out, a.k_in, a.group, a.epilogue, a.ksplit = gw.wfmt, m, gw.n_out, gw.k_in, gw.group, epilogue, ksplit
@@ -222,14 +223,18 @@ def gemm(x, gw, out=None, x_scale=1.0, epilogue=EPI_STORE, residual=None, worksp
     a.x, a.w, a.scales = _ptr(x), _ptr(gw.w), _ptr(gw.scales)
     a.x_scale, a.w_scale = float(x_scale), gw.w_scale
     a.residual, a.out, a.out_ld = _ptr(residual), _ptr(out), out_ld
-    a.out_dtype, a.alpha = dtype_code(out.dtype), float(alpha)
+    a.out_dtype, a.alpha = dtype_code(torch.float16 if parts else out.dtype), float(alpha)
+    if parts:
+        a.parts = (_lib.GemmPart * len(parts))(*[_lib.GemmPart(o.shape[1], e, _ptr(o)) for o, e in parts])
+        a.n_parts = len(parts)
+    a.gate, a.halve = _ptr(gate), int(halve)
     a.workspace, a.workspace_bytes = _ptr(workspace), (workspace.numel() if workspace is not None else 0)
     a.error_flag, a.bias = _ptr(error_flag), _ptr(bias)
     if ext is not None:
         a.ext = ctypes.pointer(ext)
     a.pdl = pdl
     check(_lib.lib().pt_gemm(ctypes.byref(a), _stream()), "pt_gemm")
-    return out
+    return [o for o, _ in parts] if parts else out
 
 
 # ------------------------------------------------------------------------------------------ linears of bf16 / fp32 models

@@ -48,3 +48,33 @@ def test_fp16_epilogues(cuda, n, k, epilogue):
     # three or four roundings of values of the size of the result and of the sums that went into it
     bound = 4 * 2.0 ** -11 * (exp.abs() + 4) * (1 + exp.abs().sqrt())
     assert bool(((out.double() - exp).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("rows", [1, 7, 16, 32, 40, 300])
+@pytest.mark.parametrize("d,f", [(256, 512), (2048, 8192), (128, 136)])
+def test_products_that_share_a_launch(cuda, rows, d, f):
+    """Parts give the bits of products of their own, and the gated residual those of the launches it stands for."""
+    from poptransformer_b200 import ops
+    L, P, S = ops._lib.lib(), ops._ptr, ops._stream
+    g = torch.Generator(device=cuda).manual_seed(rows + d)
+    w = [(torch.randn((n, d), generator=g, device=cuda) * 0.05).half() for n in (d, d, f)]
+    x = torch.randn((3, rows, d), generator=g, device=cuda).half()
+    outs = [torch.full((rows, n.shape[0]), 7, dtype=torch.float16, device=cuda) for n in w]
+    epi = [ops.EPI_STORE, ops.EPI_RELU2, ops.EPI_RELU2]
+    ops.gemm(x.view(-1, d), ops.GemmWeight(ops.W_FP16, torch.cat(w)), parts=list(zip(outs, epi)))
+    for i in range(3):
+        exp = x[i].double() @ w[i].double().T
+        exp = exp if i == 0 else torch.relu(exp) ** 2
+        # the rounding of the sum (and of its square), and k sums of which each step may lose 2^-23 of what has gathered
+        size = x[i].double().abs() @ w[i].double().abs().T
+        assert bool(((outs[i].double() - exp).abs() <= exp.abs() * 2.0 ** -9 + size * d * 2.0 ** -22 * (1 + 2 * exp.sqrt().nan_to_num()) + 1e-6).all())
+    gw = ops.GemmWeight(ops.W_FP16, w[0])
+    gate, res = torch.randn((rows, d), generator=g, device=cuda).half(), torch.randn((rows, d), generator=g, device=cuda).half()
+    for halve in (0, 1):
+        want, got = res.clone(), res.clone()
+        y = ops.gemm(x[0], gw, ksplit=1)
+        ops.check(L.pt_rwkv_ffn_out(P(want), P(gate), P(y), halve, want.numel(), S()), "out")
+        ops.gemm(x[0], gw, out=got, epilogue=ops.EPI_GATED_RESIDUAL, residual=got, gate=gate, halve=halve, ksplit=1)
+        assert torch.equal(got, want)
+        ops.gemm(x[0], gw, out=got.copy_(res), epilogue=ops.EPI_GATED_RESIDUAL, residual=got, gate=gate, halve=halve)
+        assert float((got.double() - want.double()).abs().max()) <= 2.0 ** -7      # another order of the sums: a rounding or two of values below four
