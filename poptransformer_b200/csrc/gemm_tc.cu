@@ -201,16 +201,21 @@ __device__ __forceinline__ void give_up(SharedCtl &ctl, int *error_flag, int cod
   ctl.abort = 1;
 }
 
-// A wait inside a hot loop: the first look is inline, the rest a call.  It looks some more before it lets itself be suspended: from that it would wake
-// 250 cycles late (measured on B200).
-__device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-  for (int i = 0; i < 64; ++i)
+// A wait inside a hot loop: the first look is inline, the rest a call.  It looks MORE times before it lets itself be suspended: from that it would wake
+// 250 cycles late (measured on B200).  (Not in the INT4 kernel, whose transform wants the issue slots.)
+__device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity, volatile int *abort_flag, int more) {
+  for (int i = 0; i < more; ++i)
     if (mbar_test(bar, parity)) return true;
   return mbar_wait(bar, parity, abort_flag);
 }
-__device__ __forceinline__ bool wait_fast(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return mbar_test(bar, parity) || wait_on(bar, parity, abort_flag); }
+__device__ __noinline__ bool wait_plain(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return mbar_wait(bar, parity, abort_flag); }
+template <int MORE = 64> __device__ __forceinline__ bool wait_fast(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+  return mbar_test(bar, parity) || (MORE ? wait_on(bar, parity, abort_flag, MORE) : wait_plain(bar, parity, abort_flag));
+}
 // The same for a whole warp: every lane gets the same answer.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return __all_sync(0xffffffffu, wait_fast(bar, parity, abort_flag)); }
+template <int MORE = 64> __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+  return __all_sync(0xffffffffu, wait_fast<MORE>(bar, parity, abort_flag));
+}
 
 __device__ __forceinline__ __half relu2_h(__half y) {
   const __half r = __hgt(y, __float2half_rn(0.f)) ? y : __float2half_rn(0.f);
@@ -284,15 +289,16 @@ template <int EPI, bool PAIRS, int R> __device__ __forceinline__ void fp16_rows(
     }
   }
 }
-template <bool PAIRS, int R> __device__ __forceinline__ void fp16_rows(const Fp16Out &p, const float (&sum)[R], int m, int rows, int n, int lane, const Ahead2 *got = nullptr) {
-  if (p.epilogue == PT_EPI_STORE) fp16_rows<PT_EPI_STORE, PAIRS, R>(p, sum, m, rows, n, lane, got);
-  else if (p.epilogue == PT_EPI_SWIGLU) fp16_rows<PT_EPI_SWIGLU, PAIRS, R>(p, sum, m, rows, n, lane, got);
+// ALL: the FP16 kernel's epilogues too (the others' code stays short).
+template <bool ALL, bool PAIRS, int R> __device__ __forceinline__ void fp16_rows_by(const Fp16Out &p, const float (&sum)[R], int m, int rows, int n, int lane, const Ahead2 *got = nullptr) {
+  if (p.epilogue == PT_EPI_SWIGLU) fp16_rows<PT_EPI_SWIGLU, PAIRS, R>(p, sum, m, rows, n, lane, got);
   else if (p.epilogue == PT_EPI_RESIDUAL) fp16_rows<PT_EPI_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
   else if (p.epilogue == PT_EPI_BIAS) fp16_rows<PT_EPI_BIAS, PAIRS, R>(p, sum, m, rows, n, lane, got);
-  else if (p.epilogue == PT_EPI_BIAS_GELU) fp16_rows<PT_EPI_BIAS_GELU, PAIRS, R>(p, sum, m, rows, n, lane, got);
-  else if (p.epilogue == PT_EPI_GATED_RESIDUAL) fp16_rows<PT_EPI_GATED_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
-  else if (p.epilogue == PT_EPI_RELU2) fp16_rows<PT_EPI_RELU2, PAIRS, R>(p, sum, m, rows, n, lane, got);
-  else fp16_rows<PT_EPI_BIAS_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (ALL && p.epilogue == PT_EPI_BIAS_GELU) fp16_rows<PT_EPI_BIAS_GELU, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (ALL && p.epilogue == PT_EPI_GATED_RESIDUAL) fp16_rows<PT_EPI_GATED_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (ALL && p.epilogue == PT_EPI_RELU2) fp16_rows<PT_EPI_RELU2, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else if (ALL && p.epilogue == PT_EPI_BIAS_RESIDUAL) fp16_rows<PT_EPI_BIAS_RESIDUAL, PAIRS, R>(p, sum, m, rows, n, lane, got);
+  else fp16_rows<PT_EPI_STORE, PAIRS, R>(p, sum, m, rows, n, lane, got);
 }
 // Whether the rows of the 32 weight rows from nq on can leave in pairs.
 __device__ __forceinline__ bool fp16_pairs(const Fp16Out &p, int nq) {
@@ -302,7 +308,7 @@ __device__ __forceinline__ bool fp16_pairs(const Fp16Out &p, int nq) {
 // The epilogue of a tile without k-slices, fp16 outputs: `part` of `parts` warps share a quarter of the rows and take alternate 16 columns.
 // (Measured on B200, FP8 10304 x 2048, whose last tile is half empty, at 256 rows: 12.9 us; element by element over all branches, empty
 // quarters included, 18.9.  2048 x 128 at 12 rows, a step of 16 in part: 3.1 and 4.7.)
-__device__ __forceinline__ void epilogue_fp16(const GemmParams &p, const Fp16Out &o, uint32_t tmem, int q, int lane, int part, int parts, int n0, int m0) {
+template <bool ALL> __device__ __forceinline__ void epilogue_fp16(const GemmParams &p, const Fp16Out &o, uint32_t tmem, int q, int lane, int part, int parts, int n0, int m0) {
   const int nq = n0 + q * 32, n = nq + lane, rows = min(p.mb, p.M - m0);
   if (nq >= o.N) return;          // (uniform over the warp, as is `pairs`)
   const bool pairs = fp16_pairs(o, nq);
@@ -312,8 +318,8 @@ __device__ __forceinline__ void epilogue_fp16(const GemmParams &p, const Fp16Out
     tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
     for (int j = 0; j < 16; ++j) sum[j] = __uint_as_float(v[j]);
-    if (pairs) fp16_rows<true>(o, sum, m0 + c0, rows - c0, n, lane);
-    else fp16_rows<false>(o, sum, m0 + c0, rows - c0, n, lane);
+    if (pairs) fp16_rows_by<ALL, true>(o, sum, m0 + c0, rows - c0, n, lane);
+    else fp16_rows_by<ALL, false>(o, sum, m0 + c0, rows - c0, n, lane);
   }
 }
 // R rows of one weight row per lane, gated: lanes n and n + 8 hold a feature's two sums.
@@ -482,7 +488,7 @@ template <bool BF16> __device__ __forceinline__ SumAhead sums_ahead(const GemmPa
   return a;
 }
 // The warps that have a tile's quarters q (`parts` times four of them, each part every parts-th step of 16 rows); the other threads of the block call it too.
-template <bool BF16, bool EXT>
+template <bool BF16, bool EXT, bool ALL = false>
 __device__ __forceinline__ void sum_cluster(const GemmParams &p, const Fp16Out &o, SharedCtl &ctl, uint32_t tmem, unsigned char *smem, int rank, int n0, int m0, int m_end, int part, int parts, int q, int lane, const SumAhead &ahead) {
   if (p.sum_offset == 0) {    // where the sums take the place of the operands, nobody reads these any more
     cluster_arrive();
@@ -520,8 +526,8 @@ __device__ __forceinline__ void sum_cluster(const GemmParams &p, const Fp16Out &
     for (int s = 0; s < MAX_CLUSTER; ++s) { sum[0] += v[s].x; sum[1] += v[s].y; sum[2] += v[s].z; sum[3] += v[s].w; }
     const int m = m0 + 4 * (i * ks + rank);
     if constexpr (BF16) bf16_rows<EXT>(p, sum, m, m_end, nq, lane);
-    else if (ahead.pairs) fp16_rows<true>(o, sum, m, m_end - m, n, lane, ahead.got && i == part ? &ahead.v : nullptr);
-    else fp16_rows<false>(o, sum, m, m_end - m, n, lane);
+    else if (ahead.pairs) fp16_rows_by<ALL, true>(o, sum, m, m_end - m, n, lane, ahead.got && i == part ? &ahead.v : nullptr);
+    else fp16_rows_by<ALL, false>(o, sum, m, m_end - m, n, lane);
   }
 }
 
@@ -705,14 +711,14 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
         const int a = (warp - 2) >> 2;    // (each accumulator has four warps: nothing else runs on the SM while a tile of 256 x 256 leaves)
         if (a < na) epilogue_bf16<EXT>(p, tmem + a * acc_cols, warp & 3, lane, n0 + a * BM, m0, m_end);
       } else {
-        epilogue_fp16(p, o, tmem, warp & 3, lane, 0, 1, n0, m0);
+        epilogue_fp16<FMT == PT_W_FP16>(p, o, tmem, warp & 3, lane, 0, 1, n0, m0);
       }
     }
   }
   if (NA == 1 && p.ksplit > 1) {
     if (warp < 2) cluster_wait();
     if (p.pdl) wait_for_prerequisites();
-    sum_cluster<BF16, EXT>(p, o, ctl, tmem, smem, ks, n0, m0, m_end, warp < 2 ? -1 : 0, 1, warp & 3, lane, ahead);
+    sum_cluster<BF16, EXT, FMT == PT_W_FP16>(p, o, ctl, tmem, smem, ks, n0, m0, m_end, warp < 2 ? -1 : 0, 1, warp & 3, lane, ahead);
   }
   fence_before();
   __syncthreads();
@@ -769,7 +775,7 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
   __syncthreads();
   fence_after();
   const uint32_t tmem = ctl.tmem_base;
-  SumAhead ahead{};
+  const Fp16Out o = p.o[0];         // (in registers: read from the parameters where it is used, 12288 x 4096 at 511 rows took 44.2 us instead of 42.8)
   if (p.pdl) launch_dependents();   // not before the tensor memory is ours: a block of the next GEMM would keep it while it waits for this kernel
 
   if (warp == 0) {
@@ -780,7 +786,7 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       int r = 0;
       uint32_t par = 1;
       for (int it = 0; it < n_it; ++it) {
-        if (it >= R && !wait_fast(empty0 + r * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
+        if (it >= R && !wait_fast<0>(empty0 + r * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
         const uint32_t fb = full0 + r * 8;
         mbar_expect_tx(fb, RAW_STEP);
         bulk_g2s(raw0 + r * RAW_STEP, wt, RAW_STEP, fb);
@@ -796,7 +802,7 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       int s = 0, kx = st0 * 128;
       uint32_t par = 1;
       for (int it = 0; it < n_it; ++it) {
-        if (it >= S && !wait_fast(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 25); break; }
+        if (it >= S && !wait_fast<0>(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 25); break; }
         const uint32_t fb = full0 + s * 8, dst = smem_s + s * slot_bytes;
         mbar_expect_tx(fb, slot_bytes);
         tma_load_2d(dst, &map_x, kx, m0, fb);
@@ -813,7 +819,7 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       int s = 0;
       uint32_t par = 0, acc = 0;
       for (int it = 0; it < n_it; ++it) {
-        if (!wait_fast(full0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 22); break; }
+        if (!wait_fast<0>(full0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 22); break; }
         fence_after();
         const uint64_t b0 = bdesc0 + (uint64_t)(s * slot16), b1 = b0 + half16;
         const uint32_t at = tmem + a_col + s * 64;
@@ -852,12 +858,12 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       gpos += NG;
       while (gpos >= steps_per_group) { gpos -= steps_per_group; ++gidx; }
       if (it + NG < n_it) sc_next = __ldg(srow + gidx);   // the next step's scale: its latency hides behind this step
-      if (!warp_wait(raw_full0 + r * 8, rpar, &ctl.abort)) { give_up(ctl, p.error_flag, 23); break; }
+      if (!warp_wait<0>(raw_full0 + r * 8, rpar, &ctl.abort)) { give_up(ctl, p.error_flag, 23); break; }
       uint32_t words[16];
 #pragma unroll
       for (int h = 0; h < 4; ++h)
         *reinterpret_cast<uint4 *>(&words[4 * h]) = *reinterpret_cast<const uint4 *>(raw_mine + (size_t)r * RAW_STEP + (h >> 1) * RAW_TILE + (h & 1) * 16);
-      if (it >= S && !warp_wait(empty0 + s * 8, spar, &ctl.abort)) { give_up(ctl, p.error_flag, 26); break; }
+      if (it >= S && !warp_wait<0>(empty0 + s * 8, spar, &ctl.abort)) { give_up(ctl, p.error_flag, 26); break; }
       fence_after();
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -896,20 +902,21 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
     }
     if (p.ksplit > 1) {
       if (p.pdl) wait_for_prerequisites();
-      ahead = sums_ahead<false>(p, p.o[0], ks, group, n0, m0, p.M, q, lane);
       cluster_wait();             // everybody's barrier is there
     }
     if (p.pdl) wait_for_prerequisites();                // the residual and the output are others' until here
     const bool done = warp_wait(sa(&ctl.accum), 0, &ctl.abort);
     if (!done) give_up(ctl, p.error_flag, 24);
     fence_after();
-    if (done && p.ksplit == 1) epilogue_fp16(p, p.o[0], tmem, q, lane, group, NG, n0, m0);
+    if (done && p.ksplit == 1) epilogue_fp16<false>(p, o, tmem, q, lane, group, NG, n0, m0);
   }
   if (p.ksplit > 1) {
     const bool idle = warp < 2 || warp == 2 + 4 * NG;
     if (idle) cluster_wait();
+    SumAhead ahead{};
+    ahead.pairs = fp16_pairs(o, n0 + (warp & 3) * 32);
     if (p.pdl) wait_for_prerequisites();
-    sum_cluster<false, false>(p, p.o[0], ctl, tmem, smem, ks, n0, m0, p.M, idle ? -1 : (warp - 2) >> 2, NG, warp & 3, lane, ahead);
+    sum_cluster<false, false>(p, o, ctl, tmem, smem, ks, n0, m0, p.M, idle ? -1 : (warp - 2) >> 2, NG, warp & 3, lane, ahead);
   }
   fence_before();
   __syncthreads();

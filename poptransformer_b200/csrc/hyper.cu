@@ -64,12 +64,10 @@ template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params 
     emb = reinterpret_cast<const T *>(p.table) + (size_t)id * p.table_ld;
     if (threadIdx.x == 0 && p.pos_out) p.pos_out[r] = step;
   }
-  __syncthreads();
   float *xrow = p.xs + (size_t)src * ns * p.width;
   const float *yrow = write ? p.y + (size_t)src * p.y_ld : nullptr;
-  float ss = 0.f;
-  for (int i = threadIdx.x * VEC; i < p.width; i += blockDim.x * VEC) {
-    Vec<VEC> x[SM], y, u, sum;
+  Vec<VEC> x[SM], y, w;
+  auto get = [&](int i) {
     if (start) {
       Vec<VEC> e;
 #pragma unroll
@@ -83,6 +81,18 @@ template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params 
         if (s < ns) x[s] = ld<VEC>(xrow + (size_t)s * p.width + i);
     }
     if (write) y = ld<VEC>(yrow + i);
+  };
+  // A step's few rows are latency: a thread's first elements and norm weights are asked for together with the mixing weights, not behind them.
+  const int i0 = threadIdx.x * VEC;
+  if (i0 < p.width) {
+    get(i0);
+    if (p.h) w = ld<VEC>(p.norm_w + i0);
+  }
+  __syncthreads();
+  float ss = 0.f;
+  for (int i = i0; i < p.width; i += blockDim.x * VEC) {
+    Vec<VEC> u, sum;
+    if (i != i0) get(i);
 #pragma unroll
     for (int j = 0; j < VEC; ++j) u.v[j] = sum.v[j] = 0.f;
 #pragma unroll
@@ -114,8 +124,9 @@ template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params 
   if (!p.h) return;
   const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)p.width + p.eps);
   T *hrow = reinterpret_cast<T *>(p.h) + (size_t)r * p.h_ld;
-  for (int i = threadIdx.x * VEC; i < p.width; i += blockDim.x * VEC) {
-    const Vec<VEC> u = ld<VEC>(u_row + i), w = ld<VEC>(p.norm_w + i);
+  for (int i = i0; i < p.width; i += blockDim.x * VEC) {
+    if (i != i0) w = ld<VEC>(p.norm_w + i);
+    const Vec<VEC> u = ld<VEC>(u_row + i);
     float o[VEC];
 #pragma unroll
     for (int j = 0; j < VEC; ++j) o[j] = u.v[j] * inv * w.v[j];

@@ -79,37 +79,66 @@ __global__ void norm_ce_kernel(const __half *__restrict__ x, const __half *__res
     out[(size_t)blockIdx.x * dim + i] = h_add(h_mul(h_mul(h_sub(xr[i], m), r), gamma[i]), beta[i]);
 }
 
+// What the norms below are bound by, up to some hundred rows, is latency: a launch's start, a row's way to the block and what is read after that.  So a
+// thread has one unit of eight elements (two in rows of more than 8192, and where NormCE's many rows are bytes), everything that a row needs is asked for together - the gains of a norm come
+// from HBM in every step -, and both sums meet at one barrier.  Measured on B200, us a launch in a row of launches, before and after: NormCE of 1 x 768 2.13,
+// 1.24; 16 x 1600 2.22, 1.54; 16 x 4096 2.94, 1.75; with RWKV's mixes 32 x 2048 3.63, 2.39; RMS norm of 8 x 4096 2.77, 1.83; 511 x 4096 3.07, 2.94; 2048 x 4096 8.5, 7.4.
+static int norm_threads(int dim, int units) { return ceil_div(ceil_div(dim / 8, units), 32) * 32; }
+// Sums of a block in a fixed order; all threads get both.  (`red` has not been used before.)
+__device__ __forceinline__ float2 block_sums(float a, float b, float2 *red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  a = warp_sum(a);
+  b = warp_sum(b);
+  if (lane == 0) red[warp] = make_float2(a, b);
+  __syncthreads();
+  float2 t = make_float2(0.f, 0.f);
+#pragma unroll 8
+  for (int i = 0; i < nw; ++i) { t.x += red[i].x; t.y += red[i].y; }
+  return t;
+}
+
 // norm_ce_kernel with the row kept in registers between the statistics and the normalisation: one pass over memory with 16-byte
 // accesses (dim a multiple of 8, below 8192 as the op requires).  Same arithmetic, statistics summed per thread over 8-element
 // units instead of single elements.
 // MIX: instead of the normalised row its RWKV token-shift mixes leave (rwkv_mix_kernel), and the state takes the row.
 struct MixArgs { __half *state; const __half *w[3]; __half *out[3]; };
-template <bool MIX>
-__global__ void norm_ce_vec_kernel(const __half *__restrict__ x, const __half *__restrict__ gamma, const __half *__restrict__ beta,
-                                   int dim, float eps, int single_row, __half *__restrict__ out, const MixArgs mix) {
+template <bool MIX, int Q>
+__global__ void __launch_bounds__(1024 / Q) norm_ce_vec_kernel(const __half *__restrict__ x, const __half *__restrict__ gamma, const __half *__restrict__ beta,
+                                                               int dim, float eps, int single_row, __half *__restrict__ out, const MixArgs mix) {
   early_start();
-  __shared__ float red[32];
+  __shared__ float2 red[32];
   const size_t base = (size_t)blockIdx.x * dim;
   const int units = dim / 8;
-  constexpr int MAXQ = 4;
-  uint4 v[MAXQ];
-  float s = 0.f, sq = 0.f;
+  uint4 v[Q], gv[Q], bv[Q], sv[Q], wv[Q][3];
 #pragma unroll
-  for (int q = 0; q < MAXQ; ++q) {
+  for (int q = 0; q < Q; ++q) {
     const int u = threadIdx.x + q * blockDim.x;
-    if (u < units) {
-      v[q] = __ldcg(reinterpret_cast<const uint4 *>(x + base) + u);
-      const __half2 *h2 = reinterpret_cast<const __half2 *>(&v[q]);
+    v[q] = make_uint4(0, 0, 0, 0);
+    if (u >= units) continue;
+    v[q] = __ldcg(reinterpret_cast<const uint4 *>(x + base) + u);
+    gv[q] = __ldg(reinterpret_cast<const uint4 *>(gamma) + u);
+    bv[q] = __ldg(reinterpret_cast<const uint4 *>(beta) + u);
+    if constexpr (MIX) {
+      sv[q] = reinterpret_cast<const uint4 *>(mix.state + base)[u];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = __half22float2(h2[j]);
-        s += f.x + f.y;
-        sq += f.x * f.x + f.y * f.y;
-      }
+      for (int k = 0; k < 3; ++k)
+        if (mix.out[k]) wv[q][k] = __ldg(reinterpret_cast<const uint4 *>(mix.w[k]) + u);
     }
   }
-  s = block_sum(s, red);
-  sq = block_sum(sq, red);
+  float s = 0.f, sq = 0.f;
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const __half2 *h2 = reinterpret_cast<const __half2 *>(&v[q]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(h2[j]);
+      s += f.x + f.y;
+      sq += f.x * f.x + f.y * f.y;
+    }
+  }
+  const float2 sums = block_sums(s, sq, red);
+  s = sums.x;
+  sq = sums.y;
   const float inv_n = 1.0f / (float)dim;
   __half m, r;
   if (single_row) {
@@ -125,54 +154,56 @@ __global__ void norm_ce_vec_kernel(const __half *__restrict__ x, const __half *_
     r = __float2half_rn(1.0f / sqrtf(var));
   }
 #pragma unroll
-  for (int q = 0; q < MAXQ; ++q) {
+  for (int q = 0; q < Q; ++q) {
     const int u = threadIdx.x + q * blockDim.x;
-    if (u < units) {
-      const uint4 gv = __ldg(reinterpret_cast<const uint4 *>(gamma) + u), bv = __ldg(reinterpret_cast<const uint4 *>(beta) + u);
-      __half *h = reinterpret_cast<__half *>(&v[q]);
-      const __half *gh = reinterpret_cast<const __half *>(&gv), *bh = reinterpret_cast<const __half *>(&bv);
+    if (u >= units) continue;
+    __half *h = reinterpret_cast<__half *>(&v[q]);
+    const __half *gh = reinterpret_cast<const __half *>(&gv[q]), *bh = reinterpret_cast<const __half *>(&bv[q]);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) h[j] = h_add(h_mul(h_mul(h_sub(h[j], m), r), gh[j]), bh[j]);
-      if constexpr (MIX) {
-        uint4 *st = reinterpret_cast<uint4 *>(mix.state + base) + u;
-        const uint4 sv = *st;
-        const __half *sh = reinterpret_cast<const __half *>(&sv);
-        const __half one = __float2half_rn(1.0f);
+    for (int j = 0; j < 8; ++j) h[j] = h_add(h_mul(h_mul(h_sub(h[j], m), r), gh[j]), bh[j]);
+    if constexpr (MIX) {
+      const __half *sh = reinterpret_cast<const __half *>(&sv[q]);
+      const __half one = __float2half_rn(1.0f);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          if (!mix.out[k]) continue;
-          const uint4 wv = __ldg(reinterpret_cast<const uint4 *>(mix.w[k]) + u);
-          const __half *wh = reinterpret_cast<const __half *>(&wv);
-          uint4 ov;
-          __half *oh = reinterpret_cast<__half *>(&ov);
+      for (int k = 0; k < 3; ++k) {
+        if (!mix.out[k]) continue;
+        const __half *wh = reinterpret_cast<const __half *>(&wv[q][k]);
+        uint4 ov;
+        __half *oh = reinterpret_cast<__half *>(&ov);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) oh[j] = h_add(h_mul(h[j], wh[j]), h_mul(h_sub(one, wh[j]), sh[j]));
-          reinterpret_cast<uint4 *>(mix.out[k] + base)[u] = ov;
-        }
-        *st = v[q];
-      } else {
-        reinterpret_cast<uint4 *>(out + base)[u] = v[q];
+        for (int j = 0; j < 8; ++j) oh[j] = h_add(h_mul(h[j], wh[j]), h_mul(h_sub(one, wh[j]), sh[j]));
+        reinterpret_cast<uint4 *>(mix.out[k] + base)[u] = ov;
       }
+      reinterpret_cast<uint4 *>(mix.state + base)[u] = v[q];
+    } else {
+      reinterpret_cast<uint4 *>(out + base)[u] = v[q];
     }
   }
 }
 
 // The row stays in registers between the statistics and the scaling: one pass over memory, 16-byte accesses (dim a multiple of 8,
-// at most 8 * 8 * 256).  The scalar two-pass kernel below took 15 us for 16 rows of 4096, all of it load latency.
-__global__ void rms_norm_vec_kernel(const __half *__restrict__ x, const __half *__restrict__ residual, const __half *__restrict__ gamma,
-                                    int dim, float eps, __half *__restrict__ out, __half *__restrict__ sum_out) {
+// at most 8 * 1024 * Q).
+template <int Q>
+__global__ void __launch_bounds__(1024) rms_norm_vec_kernel(const __half *__restrict__ x, const __half *__restrict__ residual, const __half *__restrict__ gamma,
+                                                            int dim, float eps, __half *__restrict__ out, __half *__restrict__ sum_out) {
   early_start();
-  __shared__ float red[32];
+  __shared__ float2 red[32];
   const size_t base = (size_t)blockIdx.x * dim;
   const int units = dim / 8;
-  constexpr int MAXQ = 8;
-  uint4 v[MAXQ];
+  uint4 v[Q], gv[Q];
   float sq = 0.f;
 #pragma unroll
-  for (int q = 0; q < MAXQ; ++q) {
+  for (int q = 0; q < Q; ++q) {
     const int u = threadIdx.x + q * blockDim.x;
     if (u < units) {
       v[q] = __ldcg(reinterpret_cast<const uint4 *>(x + base) + u);
+      gv[q] = __ldg(reinterpret_cast<const uint4 *>(gamma) + u);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int u = threadIdx.x + q * blockDim.x;
+    if (u < units) {
       if (residual) {
         const uint4 rv = __ldcg(reinterpret_cast<const uint4 *>(residual + base) + u);
         __half *h = reinterpret_cast<__half *>(&v[q]);
@@ -189,15 +220,14 @@ __global__ void rms_norm_vec_kernel(const __half *__restrict__ x, const __half *
       }
     }
   }
-  sq = block_sum(sq, red);
+  sq = block_sums(sq, 0.f, red).x;
   const __half r = __float2half_rn(1.0f / sqrtf(sq / (float)dim + eps));
 #pragma unroll
-  for (int q = 0; q < MAXQ; ++q) {
+  for (int q = 0; q < Q; ++q) {
     const int u = threadIdx.x + q * blockDim.x;
     if (u < units) {
-      const uint4 gv = __ldg(reinterpret_cast<const uint4 *>(gamma) + u);
       __half *h = reinterpret_cast<__half *>(&v[q]);
-      const __half *gh = reinterpret_cast<const __half *>(&gv);
+      const __half *gh = reinterpret_cast<const __half *>(&gv[q]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) h[j] = h_mul(h_mul(h[j], r), gh[j]);
       reinterpret_cast<uint4 *>(out + base)[u] = v[q];
@@ -808,8 +838,10 @@ extern "C" int pt_norm_ce(const void *x, const void *gamma, const void *beta, in
   PT_REQUIRE(rows > 0 && dim > 0, "pt_norm_ce: bad shape [%d, %d]", rows, dim);
   PT_REQUIRE((dim & 3) == 0, "our normCEOp require 4x a last dim, and current is: %d", dim);
   PT_REQUIRE(dim < 8192, "normalize_ce, last_dim_size should be <= 8192, and current is: %d", dim);
+  const bool many = rows > 4 * sm_count();
+  const auto kernel = many ? norm_ce_vec_kernel<false, 2> : norm_ce_vec_kernel<false, 1>;
   if (dim % 8 == 0 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0)
-    launch_early(norm_ce_vec_kernel<false>, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
+    launch_early(kernel, rows, norm_threads(dim, many ? 2 : 1), 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
                  rows == 1 ? 1 : 0, (__half *)out, MixArgs{});
   else
     launch_early(norm_ce_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
@@ -824,8 +856,9 @@ extern "C" int pt_rms_norm(const void *x, const void *residual, const void *gamm
   PT_REQUIRE(rows > 0 && dim > 0, "pt_rms_norm: bad shape [%d, %d]", rows, dim);
   PT_REQUIRE(!residual || sum_out, "pt_rms_norm: residual given without sum_out");
   const bool vec = dim % 8 == 0 && dim <= 8 * 8 * 256 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)residual | (uintptr_t)sum_out) & 15) == 0;
+  const auto kernel = dim <= 8192 ? rms_norm_vec_kernel<1> : rms_norm_vec_kernel<2>;
   if (vec)
-    launch_early(rms_norm_vec_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
+    launch_early(kernel, rows, norm_threads(dim, dim <= 8192 ? 1 : 2), 0, as_stream(stream), (const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
                                                             (__half *)out, (__half *)sum_out);
   else
     launch_early(rms_norm_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
@@ -1016,7 +1049,7 @@ extern "C" int pt_norm_ce_mix(const void *x, const void *gamma, const void *beta
                         (uintptr_t)out_a | (uintptr_t)out_b | (uintptr_t)out_c;
   PT_REQUIRE((all & 15) == 0, "pt_norm_ce_mix: all pointers must be 16-byte aligned");
   const MixArgs m{(__half *)state, {(const __half *)mix_a, (const __half *)mix_b, (const __half *)mix_c}, {(__half *)out_a, (__half *)out_b, (__half *)out_c}};
-  launch_early(norm_ce_vec_kernel<true>, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps, rows == 1 ? 1 : 0,
+  launch_early(norm_ce_vec_kernel<true, 1>, rows, norm_threads(dim, 1), 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps, rows == 1 ? 1 : 0,
                (__half *)nullptr, m);
   PT_LAUNCH_CHECK("pt_norm_ce_mix");
   return PT_OK;
