@@ -513,8 +513,10 @@ template <int NP, int CP> __global__ void __launch_bounds__(CHUNK_THREADS) ssm_c
 // ------------------------------------------------------------------------------------------ one token per sequence
 constexpr int STEP_THREADS = 256;
 // Block: one sequence and one head.  Thread (n group, column quad) walks state rows n group, + n groups, ...; every state element is
-// read and written once, coalesced along the columns.
-template <typename T, int VEC> __global__ void __launch_bounds__(STEP_THREADS) ssm_step_kernel(const Params p) {
+// read and written once, coalesced along the columns.  8 sequences of 64 heads, state 64 x 128: 34 MB, 5.1 us at the copy rate.  What the kernel takes
+// beyond that is the chain index -> convolution inputs -> state update; with the taps asked for together instead of one behind the other 11.3 us (12.4
+// before).  Four blocks an SM hold those 512 blocks in one wave: two channels a trip need 79 registers, three blocks an SM, 16.0 us; held to 64 they spill.
+template <typename T, int VEC> __global__ void __launch_bounds__(STEP_THREADS, 4) ssm_step_kernel(const Params p) {
   early_start();
   extern __shared__ __align__(16) float sm[];
   const int s = blockIdx.y, h = blockIdx.x, tid = threadIdx.x, g = h / (p.heads / p.groups);
@@ -541,19 +543,29 @@ template <typename T, int VEC> __global__ void __launch_bounds__(STEP_THREADS) s
     }
   };
   if (ngrp < ng && q < pq) load_rows(ngrp, q);   // on their way while the convolution is computed
-  for (int i = tid; i < p.P + 2 * p.N; i += STEP_THREADS) {
-    const int c = i < p.P ? h * p.P + i : (i < p.P + p.N ? p.inner + g * p.N + i - p.P : p.inner + (p.groups + g) * p.N + i - p.P - p.N);
+  const float dt_in = to_f(zx[p.inner + p.C + h]), dt_bias = p.dt_bias[h], A_log = p.A_log[h], D = p.D[h];
+  const int at = pos % p.taps;
+  for (int i0 = tid; i0 < p.P + 2 * p.N; i0 += STEP_THREADS) {     // four taps at a time, all of them asked for before one is used
+    const int c = i0 < p.P ? h * p.P + i0 : (i0 < p.P + p.N ? p.inner + g * p.N + i0 - p.P : p.inner + (p.groups + g) * p.N + i0 - p.P - p.N);
     float a = p.conv_b[c];
-    for (int k = 0; k < p.taps; ++k) {
-      const int back = p.taps - 1 - k;
-      float v = 0.f;
-      if (back == 0) v = to_f(zx[p.inner + c]);
-      else if (back <= pos) v = to_f(ring[(size_t)((pos - back) % p.taps) * p.C + c]);
-      a = fmaf(p.conv_w[(size_t)c * p.taps + k], v, a);
+    for (int k0 = 0; k0 < p.taps; k0 += 4) {
+      float f[4], w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int back = p.taps - 1 - k0 - k;
+        f[k] = w[k] = 0.f;
+        if (back < 0) continue;
+        w[k] = p.conv_w[(size_t)c * p.taps + k0 + k];
+        if (back == 0) f[k] = to_f(zx[p.inner + c]);
+        else if (back <= pos) f[k] = to_f(ring[(size_t)(at >= back ? at - back : at - back + p.taps) * p.C + c]);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k0 + k < p.taps) a = fmaf(w[k], f[k], a);
     }
-    sm[i] = silu_f(a);
+    sm[i0] = silu_f(a);
   }
-  const float dt = softplus_f(to_f(zx[p.inner + p.C + h]) + p.dt_bias[h]), decay = expf(-expf(p.A_log[h]) * dt);
+  const float dt = softplus_f(dt_in + dt_bias), decay = expf(-expf(A_log) * dt);
   __syncthreads();
   for (int q0 = q; q0 < pq; q0 += STEP_THREADS) {     // (one trip unless a row of the state is wider than the block)
     if (ngrp >= ng) break;
@@ -578,7 +590,6 @@ template <typename T, int VEC> __global__ void __launch_bounds__(STEP_THREADS) s
     store_vec<VEC>(part + (size_t)ngrp * p.P + q0 * VEC, y);
   }
   __syncthreads();
-  const float D = p.D[h];
   for (int i = tid; i < p.P; i += STEP_THREADS) {
     float a = D * x[i];
     for (int k = 0; k < ng; ++k) a += part[(size_t)k * p.P + i];
@@ -587,22 +598,34 @@ template <typename T, int VEC> __global__ void __launch_bounds__(STEP_THREADS) s
 }
 
 // ------------------------------------------------------------------------------------------ gate + group norm + ring
+// A step's rows are one chain of latencies: a thread's first elements and norm weights are asked for before the sequence's place is known, and each
+// thread ends its group's sum itself, which saves a barrier.  8 rows of 4096: 4.2 us a launch behind ssm_step_kernel, 5.4 before.
 template <typename T, int VEC> __global__ void ssm_norm_kernel(const Params p) {
   early_start();
   extern __shared__ __align__(16) float sm[];
   float *gbuf = sm, *sums = sm + (p.inner + 3) / 4 * 4;     // gated row, then [norm_groups][warps per group]
   const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  const int s = p.tok_seq[t], t0 = p.cu[s], t1 = p.cu[s + 1], pos = p.start[s] + t - t0;
+  const int s = p.tok_seq[t];
   const T *zx = reinterpret_cast<const T *>(p.zx) + (size_t)t * p.zx_ld;
   const float *y = p.y + (size_t)t * p.inner;
   const int len = p.inner / p.norm_groups, wpg = p.norm_groups >= nw ? 1 : nw / p.norm_groups, gstep = nw / wpg;
-  for (int g = warp / wpg; g < p.norm_groups; g += gstep) {
+  const int g0 = warp / wpg, i0 = ((warp % wpg) * 32 + lane) * VEC;
+  const bool works = warp < wpg * gstep && g0 < p.norm_groups && i0 < len;
+  float v[VEC], z[VEC], w[VEC];
+  if (works) {
+    load_vec<VEC>(y + g0 * len + i0, v);
+    load_vec<VEC>(zx + g0 * len + i0, z);
+  }
+  if (tid * VEC < p.inner) load_vec<VEC>(p.norm_w + tid * VEC, w);
+  const int t0 = p.cu[s], t1 = p.cu[s + 1], start = p.start[s], slot = p.slot[s];
+  for (int g = g0; g < p.norm_groups; g += gstep) {
     if (warp >= wpg * gstep) break;
     float ss = 0.f;
-    for (int i = ((warp % wpg) * 32 + lane) * VEC; i < len; i += wpg * 32 * VEC) {
-      float v[VEC], z[VEC];
-      load_vec<VEC>(y + g * len + i, v);
-      load_vec<VEC>(zx + g * len + i, z);
+    for (int i = i0; i < len; i += wpg * 32 * VEC) {
+      if (g != g0 || i != i0) {
+        load_vec<VEC>(y + g * len + i, v);
+        load_vec<VEC>(zx + g * len + i, z);
+      }
 #pragma unroll
       for (int j = 0; j < VEC; ++j) {
         v[j] *= silu_f(z[j]);
@@ -613,34 +636,35 @@ template <typename T, int VEC> __global__ void ssm_norm_kernel(const Params p) {
     ss = warp_sum(ss);
     if (lane == 0) sums[g * wpg + warp % wpg] = ss;
   }
-  if (t >= t1 - p.taps) {   // the last `taps` raw convolution inputs of the sequence stay in its ring
-    T *ring = reinterpret_cast<T *>(p.ring) + ((size_t)p.slot[s] * p.taps + pos % p.taps) * p.C;
-    if constexpr (VEC == 4) {
-      typedef typename std::conditional<sizeof(T) == 4, uint4, uint2>::type V;
-#pragma unroll 4
-      for (int c = tid; c < p.C / 4; c += blockDim.x) reinterpret_cast<V *>(ring)[c] = reinterpret_cast<const V *>(zx + p.inner)[c];
-    } else {
-      for (int c = tid; c < p.C; c += blockDim.x) ring[c] = zx[p.inner + c];
-    }
-  }
-  __syncthreads();
-  for (int g = tid; g < p.norm_groups; g += blockDim.x) {
-    float a = 0.f;
-    for (int k = 0; k < wpg; ++k) a += sums[g * wpg + k];
-    sums[g * wpg] = 1.0f / sqrtf(a / (float)len + p.eps);
-  }
+  // the last `taps` raw convolution inputs of the sequence stay in its ring: asked for in front of the barrier, written at the end
+  typedef typename std::conditional<VEC == 1, T, typename std::conditional<sizeof(T) == 4, uint4, uint2>::type>::type V;
+  const bool keep = t >= t1 - p.taps;
+  const V *raw = reinterpret_cast<const V *>(zx + p.inner);
+  V *ring = reinterpret_cast<V *>(reinterpret_cast<T *>(p.ring) + ((size_t)slot * p.taps + (start + t - t0) % p.taps) * p.C);
+  V kept[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    if (keep && tid + u * (int)blockDim.x < p.C / VEC) kept[u] = raw[tid + u * blockDim.x];
   __syncthreads();
   T *out = reinterpret_cast<T *>(p.out) + (size_t)t * p.out_ld;
   for (int i = tid * VEC; i < p.inner; i += blockDim.x * VEC) {
-    const float inv = sums[i / len * wpg];
-    float v[VEC], w[VEC];
+    const int g = i / len;
+    float a = 0.f;
+    for (int k = 0; k < wpg; ++k) a += sums[g * wpg + k];
+    const float inv = 1.0f / sqrtf(a / (float)len + p.eps);
     load_vec<VEC>(gbuf + i, v);
-    load_vec<VEC>(p.norm_w + i, w);
+    if (i != tid * VEC) load_vec<VEC>(p.norm_w + i, w);
 #pragma unroll
     for (int j = 0; j < VEC; ++j) v[j] *= inv * w[j];
     store_vec<VEC>(out + i, v);
   }
   for (int i = p.inner + tid; i < p.out_ld; i += blockDim.x) out[i] = from_f<T>(0.f);   // k padding of the output product
+  if (keep) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (tid + u * (int)blockDim.x < p.C / VEC) ring[tid + u * blockDim.x] = kept[u];
+    for (int c = tid + 2 * blockDim.x; c < p.C / VEC; c += blockDim.x) ring[c] = raw[c];
+  }
 }
 
 template <int NP, int CP> static int launch_chunks(const Params &p, cudaStream_t st) {
