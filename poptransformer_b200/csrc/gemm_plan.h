@@ -72,6 +72,8 @@ static inline Int4Plan plan_int4(int m, int n_tiles, int n_steps, int ksplit_req
 // rows, where the MMAs are the longer part) against half a microsecond and (8 + 44 / slices) ns per row of the tile for the meetings of the
 // cluster.  Fitted on B200 to 768 x 384 .. 8192 and 4096 x 384 .. 8192 in FP8 at 8 .. 512 rows, us whole and in 2 and 4 slices: 768 x 768 at 16 rows 4.3, 4.7, 4.3;
 // at 256 rows 7.8, 14.9, 12.2; 768 x 4096 at 16 rows 9.8, 7.6, 5.6; at 256 rows 15.3, 18.8, 12.7 (8 slices 11.1).
+// (With the sums sent to the block that writes them instead of fetched by it slices cost less at few rows and the line still holds: 768 x 768 at
+// 16 rows whole, 2 and 4 slices 3.2, 3.5, 3.4; at 256 rows 7.2, 16.5, 13.3; 768 x 4096 at 16 rows 8.6, 6.4, 4.4, 8 slices 3.8; at 256 rows 14.4, 20.2, 13.4, 10.6.)
 // A BF16 tile whose rows are no multiple of 32 leaves element by element when it is whole: a microsecond more.
 static inline int slices_that_pay(int most, int n_kb, int mb, bool slow_whole) {
   const double block = 200.0 + (mb > 128 ? 1.1 * (mb - 128) : 0.0);

