@@ -43,7 +43,16 @@ template <int VEC> __device__ __forceinline__ void st(float *p, const Vec<VEC> &
 }
 
 // S > 0: that many streams, unrolled.  S == 0: p.streams (at most kMaxStreams).
-template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params p) {
+//
+// FEW rows (a step's) are latency: a thread's first elements and norm weights are asked for together with the mixing weights, not behind them, and a
+// block has as many threads as the registers that this takes allow.  us a launch in a chain of launches on B200, bf16, nothing asked for early / 512 threads /
+// 768 threads with everything asked for early: 8 rows of 3 x 4096 4.01 / 3.60 / 3.85, of 4 x 4096 4.33 / 4.00 / 4.24, of 4 x 2048 3.08 / 2.83 / 2.83; of 1 x 4096
+// and 2 x 2048 in blocks of 1024 threads 3.01 / 2.67 and 2.57 / 2.37.  (With 1024 threads three streams do not fit the registers of an SM.)
+// Many rows are bytes, and what counts is how many blocks of 256 threads an SM holds: 600 rows of 2 x 2048 take 5.8 us with 48 registers, five blocks,
+// and 7.2 with 56.  Three streams fit 64 only if nothing is asked for early (2048 rows of 3 x 4096 43.6 us, 45.1 else); four spill there (58.1; 53.7 with 79 registers).
+constexpr int most_threads(int S, bool few) { return S == 0 || !few ? 256 : S > 2 ? 512 : 1024; }
+constexpr int least_blocks(int S, bool few) { return S == 0 || few ? 1 : S <= 2 ? 5 : S == 3 ? 4 : 3; }
+template <typename T, int S, int VEC, bool FEW> __global__ void __launch_bounds__(most_threads(S, FEW), least_blocks(S, FEW)) hyper_kernel(const Params p) {
   early_start();
   constexpr int SM = S > 0 ? S : kMaxStreams;
   extern __shared__ __align__(16) float u_row[];   // [width]
@@ -82,10 +91,9 @@ template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params 
     }
     if (write) y = ld<VEC>(yrow + i);
   };
-  // A step's few rows are latency: a thread's first elements and norm weights are asked for together with the mixing weights, not behind them.
-  // (8 rows of 2 x 2048 in a chain of launches: 3.3 us, 4.1 before.)
   const int i0 = threadIdx.x * VEC;
-  if (i0 < p.width) {
+  constexpr bool AHEAD = FEW || (S != 0 && S != 3);
+  if (AHEAD && i0 < p.width) {
     get(i0);
     if (p.h) w = ld<VEC>(p.norm_w + i0);
   }
@@ -93,7 +101,7 @@ template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params 
   float ss = 0.f;
   for (int i = i0; i < p.width; i += blockDim.x * VEC) {
     Vec<VEC> u, sum;
-    if (i != i0) get(i);
+    if (!AHEAD || i != i0) get(i);
 #pragma unroll
     for (int j = 0; j < VEC; ++j) u.v[j] = sum.v[j] = 0.f;
 #pragma unroll
@@ -126,7 +134,7 @@ template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params 
   const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)p.width + p.eps);
   T *hrow = reinterpret_cast<T *>(p.h) + (size_t)r * p.h_ld;
   for (int i = i0; i < p.width; i += blockDim.x * VEC) {
-    if (i != i0) w = ld<VEC>(p.norm_w + i);
+    if (!AHEAD || i != i0) w = ld<VEC>(p.norm_w + i);
     const Vec<VEC> u = ld<VEC>(u_row + i);
     float o[VEC];
 #pragma unroll
@@ -136,27 +144,27 @@ template <typename T, int S, int VEC> __global__ void hyper_kernel(const Params 
   for (int i = p.width + threadIdx.x; i < p.h_ld; i += blockDim.x) hrow[i] = from_f<T>(0.f);   // k padding of the next product
 }
 
-template <typename T, int S, int VEC> static int launch(const Params &p, cudaStream_t st) {
+template <typename T, int S, int VEC, bool FEW> static int launch(const Params &p, cudaStream_t st) {
   const size_t smem = (size_t)p.width * sizeof(float);
   if (smem > 48 * 1024) {
     static bool set = false;
-    if (!set) { PT_CUDA(cudaFuncSetAttribute(hyper_kernel<T, S, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); set = true; }
+    if (!set) { PT_CUDA(cudaFuncSetAttribute(hyper_kernel<T, S, VEC, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); set = true; }
   }
-  const int want = ceil_div(ceil_div(p.width, VEC), 32) * 32, cap = p.rows <= 2 * sm_count() ? 1024 : 256;
-  const int regs_cap = S == 0 ? 256 : 1024;
-  launch_early(hyper_kernel<T, S, VEC>, p.rows, std::min(std::min(want, cap), regs_cap), smem, st, p);
+  const int want = ceil_div(ceil_div(p.width, VEC), 32) * 32;
+  launch_early(hyper_kernel<T, S, VEC, FEW>, p.rows, std::min(want, most_threads(S, FEW)), smem, st, p);
   PT_LAUNCH_CHECK("pt_hyper");
   return PT_OK;
 }
+template <typename T, int S> static int launch4(const Params &p, cudaStream_t st) { return p.rows <= 2 * sm_count() ? launch<T, S, 4, true>(p, st) : launch<T, S, 4, false>(p, st); }
 template <typename T> static int dispatch(const Params &p, bool vec4, cudaStream_t st) {
   if (vec4) switch (p.streams) {
-      case 1: return launch<T, 1, 4>(p, st);
-      case 2: return launch<T, 2, 4>(p, st);
-      case 3: return launch<T, 3, 4>(p, st);
-      case 4: return launch<T, 4, 4>(p, st);
+      case 1: return launch4<T, 1>(p, st);
+      case 2: return launch4<T, 2>(p, st);
+      case 3: return launch4<T, 3>(p, st);
+      case 4: return launch4<T, 4>(p, st);
       default: break;
     }
-  return launch<T, 0, 1>(p, st);
+  return launch<T, 0, 1, false>(p, st);
 }
 
 }  // namespace hyper

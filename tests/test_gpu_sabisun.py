@@ -54,6 +54,32 @@ def test_hyper_connections(cuda, dtype, streams, width):
     assert rel(h[:2, :width].float().cpu(), ref.rms(M, eps) * nw) < tol and torch.equal(before, xs)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows", [1, 8, 296, 297])
+@pytest.mark.parametrize("streams,width", [(3, 3588), (3, 4096), (4, 4096), (4, 5120), (2, 8192), (5, 4096)])
+def test_wide_hyper_connections(cuda, dtype, streams, width, rows):
+    """Widths whose blocks have as many threads as a kernel's registers allow: the start of a token, a write with the next read, and the end, against float64."""
+    from poptransformer_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(streams * width + rows)
+    rand = lambda *s: torch.randn(s, generator=g, device=cuda)
+    table, ids = rand(7, width).bfloat16().to(dtype), torch.randint(0, 7, (rows,), generator=g, device=cuda, dtype=torch.int32)
+    w_in, w_out, mix, nw, y = rand(streams), rand(streams), rand(streams, streams), rand(width), rand(rows, width)
+    xs, h = torch.empty((rows, streams, width), device=cuda), torch.empty((rows, width), dtype=dtype, device=cuda)
+    norm = lambda u: u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-5) * nw.double()
+    close = lambda got, exp, tol: float((got.double() - exp).norm() / exp.norm()) < tol
+    tol = 1e-5 if dtype == torch.float32 else 6e-3
+    ops.hyper(xs, rows, 1e-5, norm_w=nw, h=h, h_ld=width, w_in=w_in, table=table, ids=ids)
+    X = table[ids.long()].double().unsqueeze(1).expand(rows, streams, width)
+    assert torch.equal(xs.double(), X) and close(h, norm(torch.einsum("s,rsw->rw", w_in.double(), X)), tol)
+    xs = rand(rows, streams, width)
+    N = torch.einsum("st,rsw->rtw", mix.double(), xs.double()) + 0.6 * torch.einsum("t,rw->rtw", w_out.double(), y.double())
+    ops.hyper(xs, rows, 1e-5, norm_w=nw, h=h, h_ld=width, w_in=w_in, y=y, y_ld=width, mix=mix, w_out=w_out, mult=0.6)
+    assert close(xs, N, 1e-6) and close(h, norm(torch.einsum("s,rsw->rw", w_in.double(), N)), tol)
+    E = (torch.einsum("st,rsw->rtw", mix.double(), xs.double()) + 0.6 * torch.einsum("t,rw->rtw", w_out.double(), y.double())).sum(1)
+    ops.hyper(xs, rows, 1e-5, norm_w=nw, h=h, h_ld=width, y=y, y_ld=width, mix=mix, w_out=w_out, mult=0.6)
+    assert close(h, norm(E), tol)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 5, 7), (3, 64, 16), (70, 130, 33), (129, 65, 200)])
 def test_true_fp32_product(cuda, m, n, k):
     from poptransformer_b200 import ops
