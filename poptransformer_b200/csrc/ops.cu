@@ -10,7 +10,7 @@ namespace pt {
 // ------------------------------------------------------------------------------------------ Int4ToHalf
 // axis 1: w int8 [n, m] -> out fp16 [2m, n].  32x32 byte tile through shared memory so that both the byte reads
 // (along m) and the fp16 writes (along n) are coalesced.
-__global__ void int4_to_half_axis1_kernel(const int8_t *__restrict__ w, const __half *__restrict__ scale, int n, int m, int group,
+__global__ void __launch_bounds__(256, 1) int4_to_half_axis1_kernel(const int8_t *__restrict__ w, const __half *__restrict__ scale, int n, int m, int group,
                                           __half *__restrict__ out) {
   __shared__ int8_t tile[32][33];
   const int j0 = blockIdx.x * 32, i0 = blockIdx.y * 32;
@@ -385,7 +385,7 @@ __device__ __forceinline__ bool better(float v, int i, float bv, int bi) { retur
 // zero_sub: exact-zero inputs are read as -10000 (the TP LM head's vocabulary-padding rule); id_offset is added to
 // the reported indices (rank * vocab_per_rank).
 template <typename T>
-__global__ void topk_kernel(const T *__restrict__ x, int dim, int k, T *__restrict__ vals, int *__restrict__ ids, int zero_sub = 0,
+__global__ void __launch_bounds__(1024, 1) topk_kernel(const T *__restrict__ x, int dim, int k, T *__restrict__ vals, int *__restrict__ ids, int zero_sub = 0,
                             int id_offset = 0) {
   __shared__ float sv[32];
   __shared__ int si[32];

@@ -600,7 +600,7 @@ template <typename T, int VEC> __global__ void __launch_bounds__(STEP_THREADS, 4
 // ------------------------------------------------------------------------------------------ gate + group norm + ring
 // A step's rows are one chain of latencies: a thread's first elements and norm weights are asked for before the sequence's place is known, and each
 // thread ends its group's sum itself, which saves a barrier.  8 rows of 4096: 4.2 us a launch behind ssm_step_kernel, 5.4 before.
-template <typename T, int VEC> __global__ void ssm_norm_kernel(const Params p) {
+template <typename T, int VEC> __global__ void __launch_bounds__(1024, 1) ssm_norm_kernel(const Params p) {
   early_start();
   extern __shared__ __align__(16) float sm[];
   float *gbuf = sm, *sums = sm + (p.inner + 3) / 4 * 4;     // gated row, then [norm_groups][warps per group]
