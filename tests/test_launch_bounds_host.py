@@ -7,7 +7,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(__file__), "..", "poptransformer_b200", "csrc")
-CONSTANT = r"[\s\d*+/()A-Z_:a-z]*\b[A-Z_]{3,}\b[\s\d*+/()A-Z_:]*|\d+|k[A-Z]\w*"
+CONSTANT = r"[\s\d*+/()A-Z_:a-z]*\b[A-Z][A-Z\d_]{2,}\b[\s\d*+/()A-Z_:]*|\d+|k[A-Z]\w*"
 
 
 def _arguments(text, i):
