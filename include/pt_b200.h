@@ -210,7 +210,7 @@ typedef struct pt_gemm_args {
   int w_tiled;            /* 1: w was tiled by pt_gemm_repack; 0: row-major (FP8 only) */
   const void *x, *w;
   const void *scales;     /* INT4: fp16 [n_out, k_in / group]                        */
-  float x_scale, w_scale; /* FP8 per-tensor scales                                   */
+  float x_scale, w_scale; /* FP8, FP16: factors of the sums (not positive: 1)          */
   const void *residual;   /* fp16 [m, n_out]; may alias `out`                        */
   void *out;              /* fp16 [m, n_out]                                         */
   int out_ld;             /* row stride of `out` in elements; 0 = dense              */

@@ -26,6 +26,7 @@ struct Params {
   const unsigned char *w, *x;
   int B, n_rt, nchunks, chunks_per_split, xs_stride, pdl;   // activation rows, units, k blocks (in all / of a slice), bytes of an activation row
   int N, epilogue, out_ld;
+  float scale;             // fp16 outputs: factor of a sum
   const __half *residual, *bias;
   __half *out;
   int *error_flag;
@@ -271,9 +272,10 @@ __global__ void __launch_bounds__(64 + 32 * MAX_WARPS, 2) linear_kernel(const Pa
       }
     } else {
       Half4 y;
+      sum.x *= p.scale; sum.y *= p.scale; sum.z *= p.scale; sum.w *= p.scale;
       if (glu) {
         if (lane & 2) continue;
-        const float a[4] = {sum.x, sum.y, sum.z, sum.w}, b[4] = {up.x, up.y, up.z, up.w};
+        const float a[4] = {sum.x, sum.y, sum.z, sum.w}, b[4] = {up.x * p.scale, up.y * p.scale, up.z * p.scale, up.w * p.scale};
 #pragma unroll
         for (int j = 0; j < 4; ++j) y.v[j] = h_mul(__float2half_rn(b[j]), swish_h(__float2half_rn(a[j])));
         const int f = n / 16 * 8 + n % 8;
@@ -314,6 +316,7 @@ cudaError_t run(const pt_gemm_args &a, int out_ld, cudaStream_t st) {
   p.pdl = a.pdl ? 1 : 0;
   p.epilogue = a.epilogue;
   p.out_ld = out_ld;
+  p.scale = (a.x_scale > 0.f ? a.x_scale : 1.0f) * (a.w_scale > 0.f ? a.w_scale : 1.0f);
   p.residual = (const __half *)a.residual;
   p.bias = a.epilogue == PT_EPI_BIAS || a.epilogue == PT_EPI_BIAS_GELU || a.epilogue == PT_EPI_BIAS_RESIDUAL ? (const __half *)a.bias : nullptr;
   p.out = (__half *)a.out;

@@ -50,6 +50,26 @@ def test_fp16_epilogues(cuda, n, k, epilogue):
     assert bool(((out.double() - exp).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("epilogue", ["store", "residual", "swiglu"])
+@pytest.mark.parametrize("n,k", [(768, 768), (768, 3072)])
+@pytest.mark.parametrize("m", [1, 8, 9])
+def test_fp16_scales(cuda, n, k, m, epilogue):
+    """Scales of weights and activations multiply the sums whatever the number of rows (eight is the last that the kernel for few rows takes)."""
+    from poptransformer_b200 import ops
+    g = torch.Generator(device=cuda).manual_seed(n + k + m)
+    w, x = torch.randn((n, k), generator=g, device=cuda).half(), torch.randn((m, k), generator=g, device=cuda).half()
+    res = torch.randn((m, n), generator=g, device=cuda).half()
+    y = x.double() @ w.double().T * (0.25 * 0.1875)
+    exp = res.double() + y if epilogue == "residual" else y
+    if epilogue == "swiglu":
+        y = y.view(m, -1, 2, 8)
+        exp = (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(m, -1)
+    out = torch.empty_like(exp, dtype=torch.float16)
+    ops.gemm(x, ops.GemmWeight(ops.W_FP16, w, w_scale=0.1875), out=out, x_scale=0.25, epilogue=getattr(ops, "EPI_" + epilogue.upper()), residual=res if epilogue == "residual" else None)
+    # as in test_fp16_epilogues: three or four roundings of values of the size of the result and of the sums (below eight) that went into it
+    assert bool(((out.double() - exp).abs() <= 4 * 2.0 ** -11 * (exp.abs() + 8) * (1 + exp.abs().sqrt())).all())
+
+
 @pytest.mark.parametrize("rows", [1, 7, 16, 32, 40, 300])
 @pytest.mark.parametrize("d,f", [(256, 512), (2048, 8192), (128, 136)])
 def test_products_that_share_a_launch(cuda, rows, d, f):
