@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) kv_append_attn_kernel(const 
     }
     if (more) rows = rows_of(c + W);
     asm volatile("cp.async.wait_group 1;" ::: "memory");
-    if (newest && lane < U) store8(sK + slot * LD + lane * 8, load8(sm.fresh[0] + lane * 8));
+    if (newest && lane_row == slot % (32 / U)) store8(sK + slot * LD + lane_unit * 8, load8(sm.fresh[0] + lane_unit * 8));     // (the lanes that copied zeros there: they have waited for them)
     __syncwarp();              // K is there
     float sc[T][2][4] = {};    // (two chains each)
 #pragma unroll
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) kv_append_attn_kernel(const 
       pf[t][1] = transpose8x8(pack_f2h2(w[t][2], w[t][3]));
     }
     asm volatile("cp.async.wait_group 1;" ::: "memory");
-    if (newest && lane < U) store8(sV + slot * LD + lane * 8, load8(sm.fresh[1] + lane * 8));
+    if (newest && lane_row == slot % (32 / U)) store8(sV + slot * LD + lane_unit * 8, load8(sm.fresh[1] + lane_unit * 8));
     __syncwarp();              // V is there
 #pragma unroll
     for (int t = 0; t < T; ++t)
