@@ -385,9 +385,10 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) kv_append_attn_kernel(const 
     }
   }
   if (R == 1) return;
-  if (!mbar_wait(arrived, 0, &sm.abort)) {
+  if (!__all_sync(0xffffffffu, mbar_wait(arrived, 0, &sm.abort))) {
     if (p.error_flag) atomicCAS(p.error_flag, 0, 13);
     sm.abort = 1;
+    stay_for_cluster();     // what was late may still come
     return;
   }
   for (int e0 = warp * 32; e0 < share && rank * share + e0 < nq * H; e0 += THREADS) {

@@ -13,7 +13,8 @@
 // sum meet in one step: every warp sends its 16 x 8 sums to the block that writes them, by stores that arrive at a barrier there, or with one
 // slice through its own shared memory.  They are added in a fixed order.  Warp 0 fetches weights, warp 1 activations (16-byte asynchronous
 // copies into the swizzled image that ldmatrix reads without conflicts).  What was asked of the epilogue (residual) is requested before the products.
-// Every wait is bounded, as in gemm_tc.cu; after a failure the sums go out all the same, so that nobody's wait runs out for another's failure.
+// Every wait is bounded, as in gemm_tc.cu, and the meetings of a cluster wait for threads that come in bounded time or have ended.  After a failure the sums
+// go out all the same, so that nobody's wait runs out for another's failure, and a block that gave up stays until nobody can send to it.
 #include "dense_out.cuh"
 #include "gemm_few.h"
 #include "mbarrier.cuh"
@@ -52,6 +53,10 @@ __device__ __forceinline__ bool wait_fast(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) { return __all_sync(0xffffffffu, wait_fast(bar, parity, abort_flag)); }
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// A warp's way out of the kernel: if its block has given up, not before the others of the cluster.
+__device__ __forceinline__ void leave(const Ctl &ctl, int slices) {
+  if (slices > 1 && __any_sync(0xffffffffu, ctl.abort)) stay_for_cluster();
 }
 __device__ __forceinline__ uint32_t in_block(uint32_t local, uint32_t rank) {
   uint32_t a;
@@ -158,7 +163,8 @@ __global__ void __launch_bounds__(64 + 32 * MAX_WARPS, 2) linear_kernel(const Pa
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == 0) {
     if (lane == 0) {
-      for (int st = 0, s = 0, par = 1; st < n_st; ++st) {
+      int st = 0;
+      for (int s = 0, par = 1; st < n_st; ++st) {
         if (st >= S && !wait_fast(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
         const int kbs = min(KW, n_kb - st * KW);
         mbar_expect_tx(full0 + s * 8, kbs * units * UNIT_BYTES);
@@ -173,10 +179,13 @@ __global__ void __launch_bounds__(64 + 32 * MAX_WARPS, 2) linear_kernel(const Pa
         }
         if (++s == S) { s = 0; par ^= 1; }
       }
+      mbar_wait_ring(full0, st, S);     // (long over when the others end, but for failures)
     }
+    __syncwarp();
   }
   if (warp < 2) {
     if (slices > 1) { __syncwarp(); asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+    leave(ctl, slices);
     return;
   }
 
@@ -228,7 +237,7 @@ __global__ void __launch_bounds__(64 + 32 * MAX_WARPS, 2) linear_kernel(const Pa
       send(at + 32, acc[2], bar);
       send(at + 112, acc[3], bar);
     }
-    if (cw >= own) return;
+    if (cw >= own) { leave(ctl, slices); return; }
     if (!warp_wait(smem_addr(&ctl.sums), 0, &ctl.abort)) give_up(ctl, p.error_flag, 27);
   } else {
     if (active) {
@@ -241,7 +250,7 @@ __global__ void __launch_bounds__(64 + 32 * MAX_WARPS, 2) linear_kernel(const Pa
     if (KW > 1) asm volatile("bar.sync 1, %0;" ::"r"(CW * 32) : "memory");
     else __syncwarp();
   }
-  if (ctl.abort) return;
+  if (__any_sync(0xffffffffu, ctl.abort)) { leave(ctl, slices); return; }
   for (int i = cw; i < own; i += CW) {
     const int m = lane >> 2, n = (u0 + rank + i * slices) * UNIT + (lane & 3) * 4;
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -562,6 +562,15 @@ __device__ __forceinline__ void fetch_rows(const GemmParams &p, SharedCtl &ctl, 
   }
 }
 
+// The end of a block that gave up, all threads: what it has asked for has landed (`full0` and `issued` of the thread that asked), its MMAs are done with
+// shared and tensor memory, and nobody sends it sums any more.
+__device__ __noinline__ void end_after_failure(SharedCtl &ctl, uint32_t full0, int issued, int stages, int warp, int ksplit) {
+  if (issued) mbar_wait_ring(full0, issued, stages);
+  if (warp == 1) mbar_wait_ring(sa(&ctl.accum), 1, 1);
+  if (ksplit > 1) stay_for_cluster();
+  __syncthreads();
+}
+
 // ------------------------------------------------------------------------------------------ FP8, FP16 and BF16
 // Dynamic shared memory: [stage][NA A tiles of 16 KB | B tile mb * 128 B], every tile 1024-byte aligned.  NA = 2: a CTA takes 256 weight
 // rows (two accumulators), which fetches a third less per product than NA = 1; without k-slices.  With up to 128 activation rows two such CTAs share an
@@ -621,6 +630,7 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
   // Not before: a CTA of the next GEMM that found the tensor memory free would keep it while it waits for this kernel to end.
   if (p.pdl) launch_dependents();
   SumAhead ahead{};
+  int issued = 0;     // stages that this thread has asked for
 
   if (warp == 0) {
     if (elect_one()) {
@@ -649,10 +659,10 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
         }
         wait_for_prerequisites();
       }
-      for (int it = 0; it < n_it; ++it) {
+      for (; issued < n_it; ++issued) {
         if (!first_round && !wait_fast(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
         const uint32_t st = smem_s + s * stage_bytes, fb = full0 + s * 8;
-        if (it >= early) {
+        if (issued >= early) {
           mbar_expect_tx(fb, tx);
           load_w(st, fb);
         }
@@ -723,6 +733,7 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
   fence_before();
   __syncthreads();
   fence_after();
+  if (ctl.abort) end_after_failure(ctl, sa(&ctl.full[0]), issued, p.stages, warp, NA == 1 ? p.ksplit : 1);
   if (warp == 1) tmem_dealloc(tmem, tmem_cols);
 }
 
@@ -776,6 +787,7 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
   fence_after();
   const uint32_t tmem = ctl.tmem_base;
   const Fp16Out o = p.o[0];         // (in registers: read from the parameters where it is used, 12288 x 4096 at 511 rows took 44.2 us instead of 42.8)
+  int issued = 0;                   // stages that this thread has asked for
   if (p.pdl) launch_dependents();   // not before the tensor memory is ours: a block of the next GEMM would keep it while it waits for this kernel
 
   if (warp == 0) {
@@ -785,8 +797,8 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       const uint32_t raw0 = sa(raw_ring), full0 = sa(&ctl.raw_full[0]), empty0 = sa(&ctl.raw_empty[0]);
       int r = 0;
       uint32_t par = 1;
-      for (int it = 0; it < n_it; ++it) {
-        if (it >= R && !wait_fast<0>(empty0 + r * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
+      for (; issued < n_it; ++issued) {
+        if (issued >= R && !wait_fast<0>(empty0 + r * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
         const uint32_t fb = full0 + r * 8;
         mbar_expect_tx(fb, RAW_STEP);
         bulk_g2s(raw0 + r * RAW_STEP, wt, RAW_STEP, fb);
@@ -801,8 +813,8 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       const uint32_t full0 = sa(&ctl.full[0]), empty0 = sa(&ctl.empty[0]);
       int s = 0, kx = st0 * 128;
       uint32_t par = 1;
-      for (int it = 0; it < n_it; ++it) {
-        if (it >= S && !wait_fast<0>(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 25); break; }
+      for (; issued < n_it; ++issued) {
+        if (issued >= S && !wait_fast<0>(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 25); break; }
         const uint32_t fb = full0 + s * 8, dst = smem_s + s * slot_bytes;
         mbar_expect_tx(fb, slot_bytes);
         tma_load_2d(dst, &map_x, kx, m0, fb);
@@ -921,6 +933,7 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
   fence_before();
   __syncthreads();
   fence_after();
+  if (ctl.abort) end_after_failure(ctl, warp == 0 ? sa(&ctl.raw_full[0]) : sa(&ctl.full[0]), issued, warp == 0 ? R : S, warp, p.ksplit);
   if (warp == 1) tmem_dealloc(tmem, tmem_cols);
 }
 
