@@ -313,7 +313,7 @@ bool takes(const pt_gemm_args &a) {
 }
 cudaError_t run(const pt_gemm_args &a, int out_ld, cudaStream_t st) {
   const bool bf16 = a.wfmt == PT_W_BF16;
-  const Plan plan = make_plan(a.m, a.n_out, a.k_in, sm_count());
+  const Plan &plan = kept_plan(a.m, a.n_out, a.k_in, sm_count());
   Params p{};
   p.w = (const unsigned char *)a.w;
   p.x = (const unsigned char *)a.x;

@@ -1,0 +1,59 @@
+"""The plan of a small product is searched once for a size that comes again, and is the one that a search gives: for sizes that share a place in the table,
+in any order, and on any number of SMs."""
+import os
+import subprocess
+
+CSRC = os.path.join(os.path.dirname(__file__), "..", "poptransformer_b200", "csrc")
+DRIVER = r"""
+#include <chrono>
+#include <cstdio>
+#include <cstring>
+#include <thread>
+#include "gemm_few.h"
+using namespace pt::few;
+static int differ = 0, seen = 0;
+static void all(int sms) {
+  for (int round = 0; round < 2; ++round)
+    for (int m = 1; m <= 8; ++m)
+      for (int n : {1, 8, 16, 40, 768, 1000, 2048, 2304, 8000, 50257, 262144})
+        for (int k : {64, 128, 768, 1024, 1600, 4096, 65536})
+          for (int again = 0; again < 2; ++again)
+            if (small(m, n, k)) {
+              const Plan a = kept_plan(m, n, k, sms), b = make_plan(m, n, k, sms);
+              differ += std::memcmp(&a, &b, sizeof(Plan)) != 0;
+              ++seen;
+            }
+}
+template <typename F> static double least(F f) {
+  double best = 1e30;
+  for (int t = 0; t < 7; ++t) {
+    const auto a = std::chrono::steady_clock::now();
+    for (int i = 0; i < 500; ++i) f(i);
+    best = std::min(best, std::chrono::duration<double>(std::chrono::steady_clock::now() - a).count());
+  }
+  return best;
+}
+int main() {
+  all(148);
+  all(132);
+  std::thread([] { all(148); }).join();
+  volatile int sum = 0;
+  const int n[4] = {768, 2048, 512, 2304}, k[4] = {3072, 2048, 8192, 1088};      // what a step asks for in turn
+  const double search = least([&](int i) { sum += make_plan(1, n[i & 3], k[i & 3], 148).units; });
+  const double keep = least([&](int i) { sum += kept_plan(1, n[i & 3], k[i & 3], 148).units; });
+  printf("%d %d %.9f %.9f\n", seen, differ, search, keep);
+}
+"""
+
+
+def test_plans_are_kept(tmp_path):
+    (tmp_path / "plan.cpp").write_text(DRIVER)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-pthread", "-I", CSRC, "-o", str(tmp_path / "plan"), str(tmp_path / "plan.cpp")], check=True)
+    seen, differ, search, keep = map(float, subprocess.run([str(tmp_path / "plan")], check=True, capture_output=True, text=True).stdout.split())
+    assert seen > 3000 and differ == 0
+    assert keep < search / 10, (search, keep)
+
+
+def test_calls_take_the_kept_plan():
+    text = open(os.path.join(CSRC, "gemm_few.cu")).read()
+    assert "kept_plan(a.m, a.n_out, a.k_in, sm_count())" in text and "make_plan(a.m" not in text
