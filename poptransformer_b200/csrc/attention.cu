@@ -73,6 +73,10 @@ template <int H> __device__ __forceinline__ void rope16(const AttnParams &p, int
 }
 
 constexpr int NQ_MAX = 8;      // q heads of one kv head per block: the n side of an m16n8 tensor-core tile (larger groups take several blocks)
+// Weight of a warp's largest score, max-subtracted mode (sums carry it too, and the quotient drops it).  Behind a high score the others of a long history are
+// small: as fp16 fractions of 1 they lose bits below 2^-14 and are gone below 2^-25 while the sum still has them, as fractions of 2^15 not before
+// 2^-29 (twenty below the largest score), where 100,000 keys together weigh less than a rounding of the output.
+constexpr float WEIGHT_ONE = 32768.f;
 constexpr int MAX_RUNS = 16;   // blocks of a cluster
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
@@ -294,8 +298,8 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) kv_append_attn_kernel(const 
         }
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-          w[t][h] = in[t][0] ? expf(w[t][h] - ref) : 0.f;
-          w[t][h + 2] = in[t][1] ? expf(w[t][h + 2] - ref) : 0.f;
+          w[t][h] = in[t][0] ? WEIGHT_ONE * expf(w[t][h] - ref) : 0.f;
+          w[t][h + 2] = in[t][1] ? WEIGHT_ONE * expf(w[t][h + 2] - ref) : 0.f;
         }
       }
     } else {
@@ -309,7 +313,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) kv_append_attn_kernel(const 
     for (int t = 0; t < T; ++t) {
       L[0] += w[t][0] + w[t][2];
       L[1] += w[t][1] + w[t][3];
-      // The weights are rounded to fp16 for the tensor core; they are at most 1 (max-subtracted mode) or fp16 values already
+      // The weights are rounded to fp16 for the tensor core; they are at most 2^15 (max-subtracted mode, see WEIGHT_ONE) or fp16 values already
       // (the reference's fp16 softmax mode), so this costs at most 2^-11 relative per weight.
       pf[t][0] = transpose8x8(pack_f2h2(w[t][0], w[t][1]));
       pf[t][1] = transpose8x8(pack_f2h2(w[t][2], w[t][3]));
