@@ -659,10 +659,11 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
         }
         wait_for_prerequisites();
       }
-      for (; issued < n_it; ++issued) {
+      for (int it = 0; it < n_it; ++it) {
         if (!first_round && !wait_fast(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
+        issued = it + 1;
         const uint32_t st = smem_s + s * stage_bytes, fb = full0 + s * 8;
-        if (issued >= early) {
+        if (it >= early) {
           mbar_expect_tx(fb, tx);
           load_w(st, fb);
         }
@@ -797,8 +798,9 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       const uint32_t raw0 = sa(raw_ring), full0 = sa(&ctl.raw_full[0]), empty0 = sa(&ctl.raw_empty[0]);
       int r = 0;
       uint32_t par = 1;
-      for (; issued < n_it; ++issued) {
-        if (issued >= R && !wait_fast<0>(empty0 + r * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
+      for (int it = 0; it < n_it; ++it) {
+        if (it >= R && !wait_fast<0>(empty0 + r * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 21); break; }
+        issued = it + 1;
         const uint32_t fb = full0 + r * 8;
         mbar_expect_tx(fb, RAW_STEP);
         bulk_g2s(raw0 + r * RAW_STEP, wt, RAW_STEP, fb);
@@ -813,8 +815,9 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       const uint32_t full0 = sa(&ctl.full[0]), empty0 = sa(&ctl.empty[0]);
       int s = 0, kx = st0 * 128;
       uint32_t par = 1;
-      for (; issued < n_it; ++issued) {
-        if (issued >= S && !wait_fast<0>(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 25); break; }
+      for (int it = 0; it < n_it; ++it) {
+        if (it >= S && !wait_fast<0>(empty0 + s * 8, par, &ctl.abort)) { give_up(ctl, p.error_flag, 25); break; }
+        issued = it + 1;
         const uint32_t fb = full0 + s * 8, dst = smem_s + s * slot_bytes;
         mbar_expect_tx(fb, slot_bytes);
         tma_load_2d(dst, &map_x, kx, m0, fb);
