@@ -16,6 +16,7 @@
 // Every wait is bounded, as in gemm_tc.cu, and the meetings of a cluster wait for threads that come in bounded time or have ended.  After a failure the sums
 // go out all the same, so that nobody's wait runs out for another's failure, and a block that gave up stays until nobody can send to it.
 #include "dense_out.cuh"
+#include "fp16_out.cuh"
 #include "gemm_few.h"
 #include "mbarrier.cuh"
 #include "tile_math.cuh"
@@ -65,58 +66,6 @@ __device__ __forceinline__ uint32_t in_block(uint32_t local, uint32_t rank) {
 }
 __device__ __forceinline__ void send(uint32_t at, float v, uint32_t bar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(at), "r"(__float_as_uint(v)), "r"(bar) : "memory");
-}
-
-// ---- four finished sums of an fp16 output, n .. n + 3 (n a multiple of four)
-struct alignas(8) Half4 { __half v[4]; };
-__device__ __forceinline__ Half4 load4(const __half *x, int n, int N, bool whole) {
-  Half4 h;
-  if (whole) *reinterpret_cast<uint2 *>(&h) = __ldcg(reinterpret_cast<const uint2 *>(x));
-  else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) h.v[j] = n + j < N ? __ldcg(reinterpret_cast<const __half *>(x + j)) : __half(0);
-  }
-  return h;
-}
-__device__ __forceinline__ void store4(__half *o, const Half4 &h, int n, int N) {
-  if (n + 4 <= N && ((uintptr_t)o & 7) == 0) *reinterpret_cast<uint2 *>(o) = *reinterpret_cast<const uint2 *>(&h);
-  else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (n + j < N) o[j] = h.v[j];
-  }
-}
-
-// (The branches are outside the elements: with them inside, a warp alone took 1100 cycles from the sums to the store.)
-__device__ __forceinline__ Half4 finish4(int epilogue, const float4 &sum, const Half4 &res, const Half4 &bias) {
-  __half2 y0 = __floats2half2_rn(sum.x, sum.y), y1 = __floats2half2_rn(sum.z, sum.w);
-  const __half2 b0 = __halves2half2(bias.v[0], bias.v[1]), b1 = __halves2half2(bias.v[2], bias.v[3]), r0 = __halves2half2(res.v[0], res.v[1]), r1 = __halves2half2(res.v[2], res.v[3]);
-  if (epilogue != PT_EPI_STORE) {
-    if (epilogue == PT_EPI_RESIDUAL) {
-      y0 = __hadd2_rn(r0, y0);
-      y1 = __hadd2_rn(r1, y1);
-    } else if (epilogue == PT_EPI_RELU2) {
-      const __half2 zero = __float2half2_rn(0.f), p0 = __hgt2(y0, zero), p1 = __hgt2(y1, zero);      // (1 or 0; NaN gives 0)
-      y0 = __halves2half2(__low2float(p0) != 0.f ? __low2half(y0) : __half(0), __high2float(p0) != 0.f ? __high2half(y0) : __half(0));
-      y1 = __halves2half2(__low2float(p1) != 0.f ? __low2half(y1) : __half(0), __high2float(p1) != 0.f ? __high2half(y1) : __half(0));
-      y0 = __hmul2_rn(y0, y0);
-      y1 = __hmul2_rn(y1, y1);
-    } else {
-      y0 = __hadd2_rn(y0, b0);
-      y1 = __hadd2_rn(y1, b1);
-      if (epilogue == PT_EPI_BIAS_RESIDUAL) {
-        y0 = __hadd2_rn(r0, y0);
-        y1 = __hadd2_rn(r1, y1);
-      } else if (epilogue == PT_EPI_BIAS_GELU) {
-        y0 = __halves2half2(gelu_h(__low2half(y0)), gelu_h(__high2half(y0)));
-        y1 = __halves2half2(gelu_h(__low2half(y1)), gelu_h(__high2half(y1)));
-      }
-    }
-  }
-  Half4 y;
-  *reinterpret_cast<__half2 *>(&y.v[0]) = y0;
-  *reinterpret_cast<__half2 *>(&y.v[2]) = y1;
-  return y;
 }
 
 template <bool BF16, bool EXT>
@@ -262,6 +211,7 @@ __global__ void __launch_bounds__(64 + 32 * MAX_WARPS, 2) linear_kernel(const Pa
 #pragma unroll
       for (int k = 0; k < 8; ++k) { sum.x += v[k].x; sum.y += v[k].y; sum.z += v[k].z; sum.w += v[k].w; }
     }
+    if constexpr (!BF16) { sum.x *= p.scale; sum.y *= p.scale; sum.z *= p.scale; sum.w *= p.scale; }
     const bool glu = BF16 ? p.dense.epilogue == PT_EPI_GLU && n < p.dense.split_n : p.epilogue == PT_EPI_SWIGLU;      // (the same in the whole warp)
     float4 up;
     if (glu) {   // weight rows 0 .. 7 of the unit are gates, 8 .. 15 their ups
@@ -281,10 +231,9 @@ __global__ void __launch_bounds__(64 + 32 * MAX_WARPS, 2) linear_kernel(const Pa
       }
     } else {
       Half4 y;
-      sum.x *= p.scale; sum.y *= p.scale; sum.z *= p.scale; sum.w *= p.scale;
       if (glu) {
         if (lane & 2) continue;
-        const float a[4] = {sum.x, sum.y, sum.z, sum.w}, b[4] = {up.x * p.scale, up.y * p.scale, up.z * p.scale, up.w * p.scale};
+        const float a[4] = {sum.x, sum.y, sum.z, sum.w}, b[4] = {up.x, up.y, up.z, up.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) y.v[j] = h_mul(__float2half_rn(b[j]), swish_h(__float2half_rn(a[j])));
         const int f = n / 16 * 8 + n % 8;
@@ -294,7 +243,7 @@ __global__ void __launch_bounds__(64 + 32 * MAX_WARPS, 2) linear_kernel(const Pa
       Half4 bias{};
       if (p.bias) bias = load4(p.bias + n, n, p.N, n + 4 <= p.N && ((uintptr_t)p.bias & 7) == 0);
       if (i != cw && residual) res = load4(p.residual + (size_t)m * p.N + n, n, p.N, res_whole);
-      y = finish4(p.epilogue, sum, res, bias);
+      y = finish4<false>(p.epilogue, sum, res, bias);
       store4(p.out + (size_t)m * p.out_ld + n, y, n, p.N);
     }
   }

@@ -42,6 +42,7 @@ struct GemmPlan {
   int stages, raw_stages, threads;
   int tmem_columns;
   bool x_warps;                    // warps fetch the activations, not TMA
+  bool sent, few;                  // the slices send their sums to the block that writes them, otherwise it fetches them; that, or a whole tile of so few rows
   uint32_t sum_offset;             // where the slices' sums arrive behind the operands (0: in their place)
   uint32_t stage_bytes, smem;
 };
@@ -72,8 +73,8 @@ static inline Int4Plan plan_int4(int m, int n_tiles, int n_steps, int ksplit_req
 // rows, where the MMAs are the longer part) against half a microsecond and (8 + 44 / slices) ns per row of the tile for the meetings of the
 // cluster.  Fitted on B200 to 768 x 384 .. 8192 and 4096 x 384 .. 8192 in FP8 at 8 .. 512 rows, us whole and in 2 and 4 slices: 768 x 768 at 16 rows 4.3, 4.7, 4.3;
 // at 256 rows 7.8, 14.9, 12.2; 768 x 4096 at 16 rows 9.8, 7.6, 5.6; at 256 rows 15.3, 18.8, 12.7 (8 slices 11.1).
-// (With the sums sent to the block that writes them instead of fetched by it slices cost less at few rows and the line still holds: 768 x 768 at
-// 16 rows whole, 2 and 4 slices 3.2, 3.5, 3.4; at 256 rows 7.2, 16.5, 13.3; 768 x 4096 at 16 rows 8.6, 6.4, 4.4, 8 slices 3.8; at 256 rows 14.4, 20.2, 13.4, 10.6.)
+// (Sums that are sent, see below, make slices of few rows cheaper, and the line still holds: 768 x 768 at 16 rows whole, 2 and 4 slices 3.2, 3.5, 3.4; 768 x 4096 at
+// 16 rows 8.6, 6.4, 4.4, 8 slices 3.8.)
 // A BF16 tile whose rows are no multiple of 32 leaves element by element when it is whole: a microsecond more.
 static inline int slices_that_pay(int most, int n_kb, int mb, bool slow_whole) {
   const double block = 200.0 + (mb > 128 ? 1.1 * (mb - 128) : 0.0);
@@ -86,7 +87,13 @@ static inline int slices_that_pay(int most, int n_kb, int mb, bool slow_whole) {
   return best;
 }
 
-// Shared memory for the sums of the slices: a block's share of the groups of four rows, from every slice.  Behind the operands where that takes at most
+// Which slices' sums are sent to the block that writes them, and which are fetched by it (gemm_tc.cu).  Sent sums save two meetings of the cluster, but the four warps of a
+// block that sum them take group after group of four rows: worth it up to 32 rows and where a block has at most two groups, with a short k one (three if they leave as fp16).  us sent / fetched / before
+// there was sending, BF16: 2048 x 2048 at 24 rows in 8 slices 4.5 / 5.2 / 5.2, 1600 x 1600 in 7 4.4 / 5.4 / 5.2, 8192 x 1024 in 4 6.2 / 6.7 / 6.4; but 2304 x 768 in 4 4.6 / 4.1 / 4.1,
+// 2048 x 512 in 2 5.0 / 4.5 / 4.3; at 64 rows 10304 x 2048 in 3 13.6 / 11.9 / 12.0, 2048 x 2048 in 8 7.1 / 7.0 / 6.8.  FP8 12288 x 4096 at 9 rows in 2 10.5 / 11.1 / 11.1.
+// INT4, whose eight or sixteen warps sum, up to 64 rows (on average over 11 sizes 24 to 48 rows 4 % less than fetched; 64 rows level).
+constexpr int SENT_ROWS = 32, SENT_ROWS_INT4 = 64;
+// Shared memory for the sums of the slices that are sent: a block's share of the groups of four rows, from every slice.  Behind the operands where that takes at most
 // SUM_SMEM, so that a block can send before the one that sums has finished its products.
 constexpr uint32_t SUM_SMEM = 32 * 1024;
 static inline uint32_t sum_bytes(int mb, int ksplit) { return ksplit > 1 ? (uint32_t)gemm_ceil(mb / 4, ksplit) * ksplit * BM * 16 : 0; }
@@ -131,8 +138,12 @@ static inline GemmPlan plan_gemm(const GemmAsk &a) {
 #define PT_TC_PAIR 1
 #endif
   p.na = PT_TC_PAIR && a.bf16 && p.ksplit == 1 && p.mb >= 128 && p.n_tiles >= 2 && (long long)gemm_ceil(p.n_tiles, 2) * p.m_tiles >= a.sms ? 2 : 1;
-  const uint32_t b_bytes = (uint32_t)p.mb * BKB, sums = sum_bytes(p.mb, p.ksplit);
-  uint32_t behind = sums <= SUM_SMEM ? sums : 0;
+  const int most_sent = a.int4 ? SENT_ROWS_INT4 : SENT_ROWS;
+  p.sent = p.ksplit > 1 && p.mb <= most_sent && (a.int4 || gemm_ceil(p.mb / 4, p.ksplit) <= (p.n_kb < 16 ? 1 : a.bf16 ? 2 : 3));
+  p.few = p.sent || (p.ksplit == 1 && p.mb <= most_sent);
+  // (Sums that are fetched take 512 bytes per row of the ring.)
+  const uint32_t b_bytes = (uint32_t)p.mb * BKB, sums = p.sent ? sum_bytes(p.mb, p.ksplit) : p.ksplit > 1 ? p.mb * BM * 4 : 0;
+  uint32_t behind = p.sent && sums <= SUM_SMEM ? sums : 0;
   if (a.int4) {
     const bool two = p.mb <= 128 && p.n_tiles * p.m_tiles * p.ksplit > a.sms;     // two CTAs per SM (each has half the tensor memory)
     p.int4_groups = !two && p.mb <= 128 ? 4 : 2;                                  // above 128 rows a step's MMAs take longer than half a transform
@@ -140,7 +151,7 @@ static inline GemmPlan plan_gemm(const GemmAsk &a) {
     // slots: 64 tensor-memory columns beside the accumulator and 256 bytes of shared memory per row each
     p.stages = two ? (p.mb <= 64 ? 3 : 2) : (p.mb <= 128 ? 4 : p.mb <= 208 ? 3 : 2);
     p.stage_bytes = 2 * b_bytes;
-    const uint32_t slots = p.stages * p.stage_bytes, room = (two ? 110 : 217) * 1024u;
+    const uint32_t slots = p.stages * p.stage_bytes, room = (two ? (behind ? 110 : 104) : 217) * 1024u;
     if (room < slots + behind + (p.stages + p.int4_groups) * RAW_STEP) behind = 0;
     p.raw_stages = (int)std::min<uint32_t>(12, (room - slots - behind) / RAW_STEP);
     p.sum_offset = behind ? slots + p.raw_stages * RAW_STEP : 0;
@@ -159,12 +170,12 @@ static inline GemmPlan plan_gemm(const GemmAsk &a) {
 #endif
     // 16-bit weights also with large tiles when there are more of them than SMs: the epilogue of one CTA then hides behind the products of
     // the other (two accumulators of 256 columns fill the tensor memory).
-    // (The sums of a slice take 512 bytes per row of the ring.)
     const bool small = p.mb <= 64 || (wide && !(p.ksplit > 1 && p.mb > 128) && p.na * p.mb <= 256 && (long long)p.n_tiles * p.m_tiles * p.ksplit > a.sms);
     p.stages = (int)std::min<uint32_t>(8, ((small ? PT_TC_BUDGET_SMALL_KB : 200) * 1024u + std::min(behind, (small ? 110 - PT_TC_BUDGET_SMALL_KB : 16) * 1024u) - behind) / p.stage_bytes);
     p.sum_offset = behind ? p.stages * p.stage_bytes : 0;
     p.smem = p.stages * p.stage_bytes + behind + 1024;
-    p.x_warps = p.na == 1 && p.mb <= 32 && p.stages >= 4;
+    // (A whole tile of a short k gains nothing from warps that fetch: FP8 768 x 768 at 16 rows 3.4 us so, 3.2 by TMA.)
+    p.x_warps = (p.ksplit > 1 || p.n_kb >= 16) && p.na == 1 && p.mb <= 32 && p.stages >= 4;
     p.fits = p.stages >= 2 && sums <= p.smem - 1024;
     int columns = 32;
     while (columns < p.mb) columns <<= 1;

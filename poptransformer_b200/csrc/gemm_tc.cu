@@ -22,18 +22,19 @@
 // multicast).  One thread issues the MMAs and hands stages back with tcgen05.commit; the other warps convert (INT4: a deep ring
 // of raw nibble tiles feeds a few slots of fp16 weights in tensor memory) and run the epilogue (tcgen05.ld, scale, fp16, coalesced
 // stores along n).  k-slices of one tile are the blocks of a cluster, which sum them in slice order (deterministic).
-// Every wait on an mbarrier is bounded: on a time-out the CTA raises the error flag, skips its remaining waits and still frees its tensor
-// memory.  Waits for tensor memory and for the blocks of a cluster have no limit and end by construction (gemm_plan.h).
+// Every wait on an mbarrier is bounded: on a time-out the CTA raises the error flag, skips its remaining waits, stays until nothing is on its way to its shared
+// memory any more, and frees its tensor memory.  Waits for tensor memory and for the blocks of a cluster have no limit and end by construction (gemm_plan.h).
 #include <cuda.h>
 
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "dense_out.cuh"
+#include "fp16_out.cuh"
 #include "gemm_plan.h"
 #include "mbarrier.cuh"
-#include "tile_math.cuh"
 
 namespace pt {
 namespace few {   // gemm_few.cu: small products of few activation rows
@@ -50,7 +51,11 @@ struct Fp16Out {
   float scale;
 };
 constexpr int MAX_PARTS = 3;
+// How the sums of a tile's k-slices come together, if it has any.  (Instantiations for both, since a kernel with both is slower for either; none for whole tiles: products
+// that follow one another in a step are sliced or not, and found each other's code no longer in the instruction cache, ChatGLM2 at 8 rows 2.45 -> 2.48 ms.)
+enum Sums { SENT, FETCHED };
 
+// (A launch's parameters come from memory: what every block reads first lies together, and the outputs, of which it reads one set, at the end.)
 struct GemmParams {
   int M, N, K;
   int mb;                 // activation rows per CTA (multiple of 16, at most 256)
@@ -59,21 +64,21 @@ struct GemmParams {
   int ksplit, stages, raw_stages;
   int tmem_columns;       // tensor memory of a CTA
   int w_tiled;            // weights tiled by pt_gemm_repack (one contiguous tile per stage) instead of row-major
+  int pdl;                // programmatic dependent launch (tiled weights): they are fetched before the producer of x has finished
+  int x_warps;            // few activation rows: warps fetch them, not TMA
+  int sum_offset;         // where in a block's shared memory the slices of its share of a tile arrive (0: in place of the operands)
+  int n_tiles;            // tiles of 128 weight rows
+  int n_parts, part_tile[MAX_PARTS];   // FP16: products that share a launch, part s from tile part_tile[s] on with activation rows s M ..
   const unsigned char *w; // tiled weights (w_tiled)
   const unsigned char *x; // activations, rows of x_pitch bytes
   size_t x_pitch;
-  int x_warps;            // few activation rows: warps fetch them, not TMA
-  int sum_offset;         // where in a block's shared memory the slices of its share of a tile arrive (0: in place of the operands)
   const __half *scales;   // INT4: [N][K / group]
   int *error_flag;
-  DenseOut dense;         // BF16: what becomes of a finished sum
-  Fp16Out o[MAX_PARTS];   // the others.  FP16: outputs of several products that share a launch, part s from tile part_tile[s] on with activation rows s M ..
-  int n_parts, part_tile[MAX_PARTS];
   const int *group_of;    // BF16, grouped: the weight matrix of every tile of mb rows (negative: none)
   const int *group_used;  // ... and how many of its rows are in use (null: all)
-  int n_tiles;            // tiles of 128 weight rows
-  int pdl;                // programmatic dependent launch (tiled weights): they are fetched before the producer of x has finished
   size_t group_stride;    // bytes between weight matrices
+  DenseOut dense;         // BF16: what becomes of a finished sum
+  Fp16Out o[MAX_PARTS];   // the others: of every part
 };
 
 // ------------------------------------------------------------------------------------------ PTX
@@ -352,6 +357,29 @@ template <bool EXT, int R> __device__ __forceinline__ void bf16_rows(const GemmP
     }
   }
 }
+// Four rows of a warp's 32 weight rows (lane = n): four lanes trade their values, so that each has one row of their four weight rows and leaves them at once.
+// (Element by element: 1600 x 1600 at 24 rows in seven slices 4.65 us, so 4.3.)
+template <bool EXT> __device__ __forceinline__ void bf16_rows4(const GemmParams &p, const float (&sum)[4], int m, int m_end, int nq, int lane) {
+  const bool odd = lane & 1, high = lane & 2;
+  const float a = __shfl_xor_sync(0xffffffffu, odd ? sum[0] : sum[1], 1), b = __shfl_xor_sync(0xffffffffu, odd ? sum[2] : sum[3], 1);
+  // rows odd and odd + 2 of two neighbours, then row (lane & 3) of all four
+  const float r0 = odd ? a : sum[0], r1 = odd ? sum[1] : a, s0 = odd ? b : sum[2], s1 = odd ? sum[3] : b;
+  const float c = __shfl_xor_sync(0xffffffffu, high ? r0 : s0, 2), d = __shfl_xor_sync(0xffffffffu, high ? r1 : s1, 2);
+  const float4 v = high ? make_float4(c, d, s0, s1) : make_float4(r0, r1, c, d);
+  const int row = m + (lane & 3), n = nq + (lane & ~3);
+  if (p.dense.epilogue == PT_EPI_GLU && nq < p.dense.split_n) {   // (uniform over the warp; gate rows n % 16 < 8, their up rows eight further)
+    float4 up;
+    up.x = __shfl_xor_sync(0xffffffffu, v.x, 8); up.y = __shfl_xor_sync(0xffffffffu, v.y, 8);
+    up.z = __shfl_xor_sync(0xffffffffu, v.z, 8); up.w = __shfl_xor_sync(0xffffffffu, v.w, 8);
+    if (row < m_end && n < p.N && !(lane & 8)) dense_store_glu4<EXT>(p.dense, row, n, v, up);
+  } else if (row < m_end && n + 4 <= p.N) {
+    dense_store4<EXT>(p.dense, row, n, v);
+  } else if (row < m_end && n < p.N) {
+    dense_store<EXT>(p.dense, row, n, v.x);
+    if (n + 1 < p.N) dense_store<EXT>(p.dense, row, n + 1, v.y);
+    if (n + 2 < p.N) dense_store<EXT>(p.dense, row, n + 2, v.z);
+  }
+}
 // The BF16 kernel's general epilogue: 16 columns a step.
 template <bool EXT>
 __device__ __forceinline__ void epilogue_any(const GemmParams &p, uint32_t tmem, int q, int lane, int n0, int m0, int m_end, int c_first) {
@@ -457,7 +485,7 @@ template <bool EXT> __device__ __forceinline__ void epilogue_bf16(const GemmPara
 
 // k-slices of a tile: the blocks of a cluster, slice = rank.  The tile's activation rows in groups of four are dealt out to the blocks; every block sends each
 // group to the block that writes it, as [group][slice][weight row][4], by stores that arrive at a barrier there, and that block sums the slices in
-// order (deterministic).  (Blocks that left their sums at home, met, fetched what they needed and met again before their shared memory
+// order (deterministic).  That is for tiles of few rows (gemm_plan.h has the rule).  (Blocks that left their sums at home, met, fetched what they needed and met again before their shared memory
 // went took longer: 1600 x 1600 at 16 rows in seven slices 4.8 us a launch in a row of launches, so 3.9; 1600 x 6400 7.7 and 7.0; 2048 x 2048 at 32 rows 5.3 and
 // 4.7; B200.)
 __device__ __forceinline__ int own_groups(int groups, int ksplit, int rank) { return rank < groups ? (groups - rank + ksplit - 1) / ksplit : 0; }
@@ -486,6 +514,80 @@ template <bool BF16> __device__ __forceinline__ SumAhead sums_ahead(const GemmPa
     }
   }
   return a;
+}
+// Larger tiles leave the sums at home: every block in its own shared memory as [mb][128] floats (the operand ring, which nobody reads any more), the blocks meet,
+// each sums its share of the tile over all of them in slice order, all its threads at once, and they meet again before their shared memory goes.  Sent and summed by four
+// warps, a group of rows after the other, they take longer: us sent / fetched, 4096 x 4096 at 128 rows (two slices of 64-row tiles) fp16 18.3 / 15.3, bf16 19.5 / 15.5;
+// 4608 x 4096 at 256 rows fp8 18.1 / 15.5; 4096 x 4096 at 200 rows int4 13.7 / 12.0.
+__device__ __forceinline__ void leave_sums(const GemmParams &p, uint32_t tmem, int q, int lane, int part, int parts, float *dst) {
+  for (int c0 = part * 16; c0 < p.mb; c0 += 16 * parts) {
+    uint32_t v[16];
+    tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) dst[(c0 + j) * BM + q * 32 + lane] = __uint_as_float(v[j]);
+  }
+}
+__device__ __forceinline__ float4 load_cluster4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+template <bool BF16, bool EXT, bool ALL = false>
+__device__ __forceinline__ void fetch_sums(const GemmParams &p, const Fp16Out &o, const SharedCtl &ctl, uint32_t part, int rank, int n0, int m0, int m_end, int threads) {
+  cluster_arrive();
+  cluster_wait();
+  if (!ctl.abort) {
+    const int N = BF16 ? p.N : o.N, units = min(p.mb, m_end - m0) * (BM / 4), share = (units + p.ksplit - 1) / p.ksplit, last = min(units, (rank + 1) * share);
+    const bool rows_of_4 = !BF16 && N % 4 == 0, res_whole = rows_of_4 && ((uintptr_t)o.residual & 7) == 0, gate_whole = rows_of_4 && ((uintptr_t)o.gate & 7) == 0;
+    for (int i = rank * share + (int)threadIdx.x; i < last; i += threads) {
+      const int m = m0 + i / (BM / 4), n = n0 + (i % (BM / 4)) * 4;
+      if (n >= N) continue;
+      Half4 res{}, gate{}, bias{};
+      if constexpr (!BF16) {
+        if (o.residual) res = load4(o.residual + (size_t)m * N + n, n, N, res_whole);
+        if (ALL && o.gate) gate = load4(o.gate + (size_t)m * N + n, n, N, gate_whole);
+        if (o.bias) bias = load4(o.bias + n, n, N, n + 4 <= N && ((uintptr_t)o.bias & 7) == 0);
+      }
+      auto sum4 = [&](int unit) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int s0 = 0; s0 < p.ksplit; s0 += 4) {   // four loads in flight
+          float4 v[4];
+#pragma unroll
+          for (int s = 0; s < 4; ++s) v[s] = s0 + s < p.ksplit ? load_cluster4(in_block(part + unit * 16, s0 + s)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int s = 0; s < 4; ++s) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
+        }
+        return acc;
+      };
+      const bool glu = BF16 ? p.dense.epilogue == PT_EPI_GLU && n < p.dense.split_n : o.epilogue == PT_EPI_SWIGLU;
+      if (glu) {   // gate rows n % 16 < 8, their up rows eight further
+        if (n & 8) continue;
+        const float4 g = sum4(i), u = sum4(i + 2);
+        if constexpr (BF16) {
+          dense_store_glu4<EXT>(p.dense, m, n, g, u);
+        } else {
+          const int f = n / 16 * 8 + n % 8;
+          const Half4 y = {swiglu_h(o, g.x, u.x), swiglu_h(o, g.y, u.y), swiglu_h(o, g.z, u.z), swiglu_h(o, g.w, u.w)};
+          store4(o.out + (size_t)m * o.out_ld + f, y, f, N / 2);
+        }
+        continue;
+      }
+      float4 acc = sum4(i);
+      if constexpr (!BF16) {
+        acc.x *= o.scale; acc.y *= o.scale; acc.z *= o.scale; acc.w *= o.scale;
+        store4(o.out + (size_t)m * o.out_ld + n, finish4<ALL>(o.epilogue, acc, res, bias, gate, o.halve), n, N);
+      } else if (n + 4 <= N) {
+        dense_store4<EXT>(p.dense, m, n, acc);
+      } else {
+        dense_store<EXT>(p.dense, m, n, acc.x);
+        if (n + 1 < N) dense_store<EXT>(p.dense, m, n + 1, acc.y);
+        if (n + 2 < N) dense_store<EXT>(p.dense, m, n + 2, acc.z);
+      }
+    }
+  }
+  cluster_arrive();
+  cluster_wait();
 }
 // The warps that have a tile's quarters q (`parts` times four of them, each part every parts-th step of 16 rows); the other threads of the block call it too.
 template <bool BF16, bool EXT, bool ALL = false>
@@ -525,7 +627,7 @@ __device__ __forceinline__ void sum_cluster(const GemmParams &p, const Fp16Out &
 #pragma unroll
     for (int s = 0; s < MAX_CLUSTER; ++s) { sum[0] += v[s].x; sum[1] += v[s].y; sum[2] += v[s].z; sum[3] += v[s].w; }
     const int m = m0 + 4 * (i * ks + rank);
-    if constexpr (BF16) bf16_rows<EXT>(p, sum, m, m_end, nq, lane);
+    if constexpr (BF16) bf16_rows4<EXT>(p, sum, m, m_end, nq, lane);
     else if (ahead.pairs) fp16_rows_by<ALL, true>(o, sum, m, m_end - m, n, lane, ahead.got && i == part ? &ahead.v : nullptr);
     else fp16_rows_by<ALL, false>(o, sum, m, m_end - m, n, lane);
   }
@@ -576,7 +678,7 @@ __device__ __noinline__ void end_after_failure(SharedCtl &ctl, uint32_t full0, i
 // rows (two accumulators), which fetches a third less per product than NA = 1; without k-slices.  With up to 128 activation rows two such CTAs share an
 // SM, so their registers have to allow it (96 a thread): a Pivavik of width 2048 takes four prompts of 2048 tokens, whose experts have tiles of 128
 // rows, in 20.4 ms so and in 24.5 with the 168 registers that one CTA of 320 threads per SM may have (measured on B200).
-template <int FMT, int NA, bool EXT>
+template <int FMT, int NA, bool EXT, Sums SUMS>
 __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                                    const GemmParams p) {
   constexpr bool BF16 = FMT == PT_W_BF16, F8 = FMT == PT_W_FP8;
@@ -588,13 +690,15 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
   int part = 0;
   if (FMT == PT_W_FP16)
     while (part + 1 < p.n_parts && (int)blockIdx.x >= p.part_tile[part + 1]) ++part;
-  const Fp16Out o = p.o[BF16 ? 0 : part];
+  // (FP16: a copy.  Which part it is the compiler does not know, and read where it is used 128 x 128 at 128 rows takes 3.7 us instead of 3.0.)
+  const std::conditional_t<FMT == PT_W_FP16, Fp16Out, const Fp16Out &> o = p.o[FMT == PT_W_FP16 ? part : 0];
   const int n0 = (blockIdx.x - (FMT == PT_W_FP16 ? p.part_tile[part] : 0)) * (BM * NA), m0 = blockIdx.z * p.mb, x0 = part * p.M + m0, ks = blockIdx.y;     // (x0: the first activation row)
   const int kb0 = ks * p.kb_per_split, kb1 = min(p.n_kb, kb0 + p.kb_per_split);
   const int n_it = kb1 - kb0, na = NA == 1 ? 1 : min(NA, p.n_tiles - (int)blockIdx.x * NA);
   const uint32_t b_bytes = (uint32_t)p.mb * BKB;
   const uint32_t stage_bytes = NA * A_TILE + ((b_bytes + 1023u) & ~1023u);
   const uint32_t smem_s = sa(smem);
+  const bool sent = SUMS == SENT && NA == 1 && p.ksplit > 1, fetched = SUMS == FETCHED && NA == 1 && p.ksplit > 1;
   int m_end = min(p.M, m0 + p.mb), mma_n = p.mb;
   size_t w_base = 0;
   if constexpr (BF16) {
@@ -617,11 +721,11 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
       mbar_init(sa(&ctl.empty[s]), 1);
     }
     mbar_init(sa(&ctl.accum), 1);
-    if (NA == 1 && p.ksplit > 1) expect_sums(p, ctl, ks, m0, m_end);
+    if (sent) expect_sums(p, ctl, ks, m0, m_end);
     ctl.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (NA == 1 && p.ksplit > 1) cluster_arrive();
+  if (sent) cluster_arrive();
   if (warp == 1) tmem_alloc(sa(&ctl.tmem_base), tmem_cols);
   fence_before();
   __syncthreads();
@@ -708,7 +812,7 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
       if (p.pdl) wait_for_prerequisites();
       fetch_rows(p, ctl, smem + A_TILE, stage_bytes, kb0, n_it, x0, m_end - m0, warp - 2, lane);
     }
-    if (NA == 1 && p.ksplit > 1) {
+    if (sent) {
       if (p.pdl) wait_for_prerequisites();
       ahead = sums_ahead<BF16>(p, o, ks, 0, n0, m0, m_end, warp & 3, lane);
       cluster_wait();             // everybody's barrier is there
@@ -717,7 +821,8 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
     const bool done = warp_wait(sa(&ctl.accum), 0, &ctl.abort);
     if (!done) give_up(ctl, p.error_flag, 24);
     fence_after();
-    if (done && (NA > 1 || p.ksplit == 1)) {
+    if (done && fetched) leave_sums(p, tmem, warp & 3, lane, 0, 1, reinterpret_cast<float *>(smem));
+    if (done && !sent && !fetched) {
       if constexpr (BF16) {
         const int a = (warp - 2) >> 2;    // (each accumulator has four warps: nothing else runs on the SM while a tile of 256 x 256 leaves)
         if (a < na) epilogue_bf16<EXT>(p, tmem + a * acc_cols, warp & 3, lane, n0 + a * BM, m0, m_end);
@@ -726,15 +831,18 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
       }
     }
   }
-  if (NA == 1 && p.ksplit > 1) {
+  if (sent) {
     if (warp < 2) cluster_wait();
     if (p.pdl) wait_for_prerequisites();
     sum_cluster<BF16, EXT, FMT == PT_W_FP16>(p, o, ctl, tmem, smem, ks, n0, m0, m_end, warp < 2 ? -1 : 0, 1, warp & 3, lane, ahead);
+  } else if (fetched) {
+    if (p.pdl) wait_for_prerequisites();
+    fetch_sums<BF16, EXT, FMT == PT_W_FP16>(p, o, ctl, smem_s, ks, n0, m0, m_end, 64 + 128);
   }
   fence_before();
   __syncthreads();
   fence_after();
-  if (ctl.abort) end_after_failure(ctl, sa(&ctl.full[0]), issued, p.stages, warp, NA == 1 ? p.ksplit : 1);
+  if (ctl.abort) end_after_failure(ctl, sa(&ctl.full[0]), issued, p.stages, warp, sent || fetched ? p.ksplit : 1);
   if (warp == 1) tmem_dealloc(tmem, tmem_cols);
 }
 
@@ -752,7 +860,7 @@ __global__ void __launch_bounds__(64 + 128 * NA, 2) gemm_dense_kernel(const __gr
 // slot (i + NG) % S; that the use before it is over follows from step i - S being over (which step i waited for) only if NG <= S.  The
 // same for a raw stage, whose copies may land in any order: R >= NG + S.
 // Dynamic shared memory: [slot][activations: two halves of 64 k, mb * 128 B each][raw stage][8 KB of packed nibbles].
-template <int NG>
+template <int NG, Sums SUMS>
 __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
   // warp 0: raw tiles, warp 1: MMA, then 4 NG transform + epilogue, last: activations
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -765,6 +873,7 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
   const uint32_t half_bytes = (uint32_t)p.mb * BKB, slot_bytes = 2 * half_bytes;          // (half: a multiple of 2 KB)
   unsigned char *raw_ring = smem + (size_t)S * slot_bytes;
   const uint32_t smem_s = sa(smem);
+  const bool sent = SUMS == SENT && p.ksplit > 1, fetched = SUMS == FETCHED && p.ksplit > 1;
   const uint32_t a_col = (uint32_t)(p.mb + 31) & ~31u, tmem_cols = p.tmem_columns;
 
   if (tid == 0) {
@@ -777,17 +886,17 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       mbar_init(sa(&ctl.raw_empty[r]), 4);
     }
     mbar_init(sa(&ctl.accum), 1);
-    if (p.ksplit > 1) expect_sums(p, ctl, ks, m0, p.M);
+    if (sent) expect_sums(p, ctl, ks, m0, p.M);
     ctl.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (p.ksplit > 1) cluster_arrive();
+  if (sent) cluster_arrive();
   if (warp == 1) tmem_alloc(sa(&ctl.tmem_base), tmem_cols);
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = ctl.tmem_base;
-  const Fp16Out o = p.o[0];         // (in registers: read from the parameters where it is used, 12288 x 4096 at 511 rows took 44.2 us instead of 42.8)
+  const Fp16Out &o = p.o[0];
   int issued = 0;                   // stages that this thread has asked for
   if (p.pdl) launch_dependents();   // not before the tensor memory is ours: a block of the next GEMM would keep it while it waits for this kernel
 
@@ -915,7 +1024,7 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
       s += NG;
       while (s >= S) { s -= S; spar ^= 1u; }
     }
-    if (p.ksplit > 1) {
+    if (sent) {
       if (p.pdl) wait_for_prerequisites();
       cluster_wait();             // everybody's barrier is there
     }
@@ -923,20 +1032,24 @@ __global__ void __launch_bounds__((3 + 4 * NG) * 32, NG == 2 ? 2 : 1) gemm_int4_
     const bool done = warp_wait(sa(&ctl.accum), 0, &ctl.abort);
     if (!done) give_up(ctl, p.error_flag, 24);
     fence_after();
-    if (done && p.ksplit == 1) epilogue_fp16<false>(p, o, tmem, q, lane, group, NG, n0, m0);
+    if (done && fetched) leave_sums(p, tmem, q, lane, group, NG, reinterpret_cast<float *>(smem));
+    if (done && !sent && !fetched) epilogue_fp16<false>(p, o, tmem, q, lane, group, NG, n0, m0);
   }
-  if (p.ksplit > 1) {
+  if (sent) {
     const bool idle = warp < 2 || warp == 2 + 4 * NG;
     if (idle) cluster_wait();
     SumAhead ahead{};
     ahead.pairs = fp16_pairs(o, n0 + (warp & 3) * 32);
     if (p.pdl) wait_for_prerequisites();
     sum_cluster<false, false>(p, o, ctl, tmem, smem, ks, n0, m0, p.M, idle ? -1 : (warp - 2) >> 2, NG, warp & 3, lane, ahead);
+  } else if (fetched) {
+    if (p.pdl) wait_for_prerequisites();
+    fetch_sums<false, false>(p, o, ctl, smem_s, ks, n0, m0, p.M, (3 + 4 * NG) * 32);
   }
   fence_before();
   __syncthreads();
   fence_after();
-  if (ctl.abort) end_after_failure(ctl, warp == 0 ? sa(&ctl.raw_full[0]) : sa(&ctl.full[0]), issued, warp == 0 ? R : S, warp, p.ksplit);
+  if (ctl.abort) end_after_failure(ctl, warp == 0 ? sa(&ctl.raw_full[0]) : sa(&ctl.full[0]), issued, warp == 0 ? R : S, warp, sent || fetched ? p.ksplit : 1);
   if (warp == 1) tmem_dealloc(tmem, tmem_cols);
 }
 
@@ -1176,18 +1289,20 @@ extern "C" int pt_gemm(const pt_gemm_args *a, void *stream) {
   cfg.numAttrs = n_attr;
   cudaError_t e;
   if (int4) {
-    static std::atomic<uint64_t> allowed[2];
-    const auto kernel = plan.int4_groups == 2 ? tc::gemm_int4_kernel<2> : tc::gemm_int4_kernel<4>;
-    PT_CUDA(allow_smem(kernel, kGemmSmem, allowed[plan.int4_groups == 2]));
+    static std::atomic<uint64_t> allowed[4];
+    const auto kernel = plan.int4_groups == 2 ? (plan.few ? tc::gemm_int4_kernel<2, tc::SENT> : tc::gemm_int4_kernel<2, tc::FETCHED>)
+                                              : (plan.few ? tc::gemm_int4_kernel<4, tc::SENT> : tc::gemm_int4_kernel<4, tc::FETCHED>);
+    PT_CUDA(allow_smem(kernel, kGemmSmem, allowed[2 * (plan.int4_groups == 2) + plan.few]));
     e = cudaLaunchKernelEx(&cfg, kernel, map_x, p);
   } else {
-    static std::atomic<uint64_t> allowed[6];
     const bool ext = bf16 && dense_needs_ext(a->epilogue, a->ext);
-    const auto kernel = fp16 ? tc::gemm_dense_kernel<PT_W_FP16, 1, false>
-                       : !bf16 ? tc::gemm_dense_kernel<PT_W_FP8, 1, false>
-                       : plan.na == 2 ? (ext ? tc::gemm_dense_kernel<PT_W_BF16, 2, true> : tc::gemm_dense_kernel<PT_W_BF16, 2, false>)
-                              : (ext ? tc::gemm_dense_kernel<PT_W_BF16, 1, true> : tc::gemm_dense_kernel<PT_W_BF16, 1, false>);
-    PT_CUDA(allow_smem(kernel, kGemmSmem, allowed[fp16 ? 0 : !bf16 ? 1 : 2 + 2 * (plan.na == 2) + ext]));
+    static std::atomic<uint64_t> allowed[10];
+    const auto kernel = plan.na == 2 ? (ext ? tc::gemm_dense_kernel<PT_W_BF16, 2, true, tc::FETCHED> : tc::gemm_dense_kernel<PT_W_BF16, 2, false, tc::FETCHED>)
+                        : fp16       ? (plan.few ? tc::gemm_dense_kernel<PT_W_FP16, 1, false, tc::SENT> : tc::gemm_dense_kernel<PT_W_FP16, 1, false, tc::FETCHED>)
+                        : !bf16      ? (plan.few ? tc::gemm_dense_kernel<PT_W_FP8, 1, false, tc::SENT> : tc::gemm_dense_kernel<PT_W_FP8, 1, false, tc::FETCHED>)
+                        : ext        ? (plan.few ? tc::gemm_dense_kernel<PT_W_BF16, 1, true, tc::SENT> : tc::gemm_dense_kernel<PT_W_BF16, 1, true, tc::FETCHED>)
+                                     : (plan.few ? tc::gemm_dense_kernel<PT_W_BF16, 1, false, tc::SENT> : tc::gemm_dense_kernel<PT_W_BF16, 1, false, tc::FETCHED>);
+    PT_CUDA(allow_smem(kernel, kGemmSmem, allowed[plan.na == 2 ? 8 + ext : 2 * (fp16 ? 0 : !bf16 ? 1 : 2 + ext) + plan.few]));
     e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, p);
   }
   if (e != cudaSuccess) return pt::set_error(PT_ERR_CUDA, "pt_gemm: %s", cudaGetErrorString(e));
