@@ -79,10 +79,19 @@ __global__ void norm_ce_kernel(const __half *__restrict__ x, const __half *__res
     out[(size_t)blockIdx.x * dim + i] = h_add(h_mul(h_mul(h_sub(xr[i], m), r), gamma[i]), beta[i]);
 }
 
-// What the norms below are bound by, up to some hundred rows, is latency: a launch's start, a row's way to the block and what is read after that.  So a
-// thread has one unit of eight elements (two in rows of more than 8192, and where NormCE's many rows are bytes), everything that a row needs is asked for together - the gains of a norm come
-// from HBM in every step -, and both sums meet at one barrier.  Measured on B200, us a launch in a row of launches, before and after: NormCE of 1 x 768 2.13,
-// 1.24; 16 x 1600 2.22, 1.54; 16 x 4096 2.94, 1.75; with RWKV's mixes 32 x 2048 3.63, 2.39; RMS norm of 8 x 4096 2.77, 1.83; 511 x 4096 3.07, 2.94; 2048 x 4096 8.5, 7.4.
+// What the norms below are bound by, up to some hundred rows, is latency: a launch's start, a row's way to the block and what is read after that.  So everything that a
+// row needs is asked for together - the gains of a norm come from HBM in every step -, a thread has one or two units of eight elements, and both sums meet
+// at one barrier.  Many rows are bytes: a thread has four units, and the gains of NormCE are asked for behind the sums.  Measured on B200, us a launch in a row of launches, before and
+// after: NormCE of 1 x 768 1.76, 1.16; 16 x 1600 2.22, 1.54; 512 x 4096 4.31, 2.63; 2048 x 8184 9.9, 9.1; 8192 x 4096 27.9, 20.9; with RWKV's mixes 32 x 2048 2.38, 2.00; RMS norm of 1 x 4096 2.12,
+// 1.34; 512 x 4096 2.75, 2.20, with a residual 3.04, 2.77; 2048 x 8184 11.9, 10.0.  (One unit a thread whatever the size: 512 x 8184 6.1, 2048 x 8184 18.7; NormCE 20.9.)
+struct NormShape { int units; bool late; };       // units of a thread; gains behind the sums
+static NormShape norm_ce_shape(int rows, int dim, bool mix) {
+  if ((long long)rows * dim > (mix ? 4000000 : 5000000)) return {4, true};
+  return {dim <= (mix ? 4096 : 2048) ? 1 : 2, false};
+}
+// Launches of one to four blocks an SM ask for so much shared memory that no SM takes five.  Blocks of the next such launch start early, wherever there is room: with
+// room for all of them some SMs got most (512 x 4096 with a residual 3.9 us instead of 2.8, 512 x 1600 2.7 and 1.9, NormCE of 512 x 1600 2.8 and 1.9).
+static size_t norm_smem(int rows, int dim) { return rows > (dim > 2048 ? 1 : 2) * sm_count() && rows <= 4 * sm_count() ? 47 * 1024 : 0; }
 static int norm_threads(int dim, int units) { return ceil_div(ceil_div(dim / 8, units), 32) * 32; }
 // Sums of a block in a fixed order; all threads get both.  (`red` has not been used before.)
 __device__ __forceinline__ float2 block_sums(float a, float b, float2 *red) {
@@ -102,7 +111,7 @@ __device__ __forceinline__ float2 block_sums(float a, float b, float2 *red) {
 // units instead of single elements.
 // MIX: instead of the normalised row its RWKV token-shift mixes leave (rwkv_mix_kernel), and the state takes the row.
 struct MixArgs { __half *state; const __half *w[3]; __half *out[3]; };
-template <bool MIX, int Q>
+template <bool MIX, int Q, bool LATE = false>
 __global__ void __launch_bounds__(1024 / Q) norm_ce_vec_kernel(const __half *__restrict__ x, const __half *__restrict__ gamma, const __half *__restrict__ beta,
                                                                int dim, float eps, int single_row, __half *__restrict__ out, const MixArgs mix) {
   early_start();
@@ -116,8 +125,10 @@ __global__ void __launch_bounds__(1024 / Q) norm_ce_vec_kernel(const __half *__r
     v[q] = make_uint4(0, 0, 0, 0);
     if (u >= units) continue;
     v[q] = __ldcg(reinterpret_cast<const uint4 *>(x + base) + u);
-    gv[q] = __ldg(reinterpret_cast<const uint4 *>(gamma) + u);
-    bv[q] = __ldg(reinterpret_cast<const uint4 *>(beta) + u);
+    if constexpr (!LATE) {
+      gv[q] = __ldg(reinterpret_cast<const uint4 *>(gamma) + u);
+      bv[q] = __ldg(reinterpret_cast<const uint4 *>(beta) + u);
+    }
     if constexpr (MIX) {
       sv[q] = reinterpret_cast<const uint4 *>(mix.state + base)[u];
 #pragma unroll
@@ -157,6 +168,10 @@ __global__ void __launch_bounds__(1024 / Q) norm_ce_vec_kernel(const __half *__r
   for (int q = 0; q < Q; ++q) {
     const int u = threadIdx.x + q * blockDim.x;
     if (u >= units) continue;
+    if constexpr (LATE) {
+      gv[q] = __ldg(reinterpret_cast<const uint4 *>(gamma) + u);
+      bv[q] = __ldg(reinterpret_cast<const uint4 *>(beta) + u);
+    }
     __half *h = reinterpret_cast<__half *>(&v[q]);
     const __half *gh = reinterpret_cast<const __half *>(&gv[q]), *bh = reinterpret_cast<const __half *>(&bv[q]);
 #pragma unroll
@@ -182,42 +197,40 @@ __global__ void __launch_bounds__(1024 / Q) norm_ce_vec_kernel(const __half *__r
 }
 
 // The row stays in registers between the statistics and the scaling: one pass over memory, 16-byte accesses (dim a multiple of 8,
-// at most 8 * 1024 * Q).
-template <int Q>
+// at most 8 * 1024 * 2).
 __global__ void __launch_bounds__(1024) rms_norm_vec_kernel(const __half *__restrict__ x, const __half *__restrict__ residual, const __half *__restrict__ gamma,
                                                             int dim, float eps, __half *__restrict__ out, __half *__restrict__ sum_out) {
   early_start();
   __shared__ float2 red[32];
+  constexpr int Q = 2;
   const size_t base = (size_t)blockIdx.x * dim;
   const int units = dim / 8;
-  uint4 v[Q], gv[Q];
+  uint4 v[Q], rv[Q], gv[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int u = threadIdx.x + q * blockDim.x;
+    v[q] = rv[q] = make_uint4(0, 0, 0, 0);
+    if (u >= units) continue;
+    v[q] = __ldcg(reinterpret_cast<const uint4 *>(x + base) + u);
+    if (residual) rv[q] = __ldcg(reinterpret_cast<const uint4 *>(residual + base) + u);
+    gv[q] = __ldg(reinterpret_cast<const uint4 *>(gamma) + u);
+  }
   float sq = 0.f;
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const int u = threadIdx.x + q * blockDim.x;
-    if (u < units) {
-      v[q] = __ldcg(reinterpret_cast<const uint4 *>(x + base) + u);
-      gv[q] = __ldg(reinterpret_cast<const uint4 *>(gamma) + u);
+    if (residual) {
+      __half *h = reinterpret_cast<__half *>(&v[q]);
+      const __half *rh = reinterpret_cast<const __half *>(&rv[q]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) h[j] = h_add(h[j], rh[j]);
+      if (u < units) reinterpret_cast<uint4 *>(sum_out + base)[u] = v[q];
     }
-  }
+    const __half2 *h2 = reinterpret_cast<const __half2 *>(&v[q]);
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const int u = threadIdx.x + q * blockDim.x;
-    if (u < units) {
-      if (residual) {
-        const uint4 rv = __ldcg(reinterpret_cast<const uint4 *>(residual + base) + u);
-        __half *h = reinterpret_cast<__half *>(&v[q]);
-        const __half *rh = reinterpret_cast<const __half *>(&rv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) h[j] = h_add(h[j], rh[j]);
-        reinterpret_cast<uint4 *>(sum_out + base)[u] = v[q];
-      }
-      const __half2 *h2 = reinterpret_cast<const __half2 *>(&v[q]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = __half22float2(h2[j]);
-        sq += f.x * f.x + f.y * f.y;
-      }
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(h2[j]);
+      sq += f.x * f.x + f.y * f.y;
     }
   }
   sq = block_sums(sq, 0.f, red).x;
@@ -225,13 +238,12 @@ __global__ void __launch_bounds__(1024) rms_norm_vec_kernel(const __half *__rest
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const int u = threadIdx.x + q * blockDim.x;
-    if (u < units) {
-      __half *h = reinterpret_cast<__half *>(&v[q]);
-      const __half *gh = reinterpret_cast<const __half *>(&gv[q]);
+    if (u >= units) continue;
+    __half *h = reinterpret_cast<__half *>(&v[q]);
+    const __half *gh = reinterpret_cast<const __half *>(&gv[q]);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) h[j] = h_mul(h_mul(h[j], r), gh[j]);
-      reinterpret_cast<uint4 *>(out + base)[u] = v[q];
-    }
+    for (int j = 0; j < 8; ++j) h[j] = h_mul(h_mul(h[j], r), gh[j]);
+    reinterpret_cast<uint4 *>(out + base)[u] = v[q];
   }
 }
 
@@ -838,10 +850,10 @@ extern "C" int pt_norm_ce(const void *x, const void *gamma, const void *beta, in
   PT_REQUIRE(rows > 0 && dim > 0, "pt_norm_ce: bad shape [%d, %d]", rows, dim);
   PT_REQUIRE((dim & 3) == 0, "our normCEOp require 4x a last dim, and current is: %d", dim);
   PT_REQUIRE(dim < 8192, "normalize_ce, last_dim_size should be <= 8192, and current is: %d", dim);
-  const bool many = rows > 4 * sm_count();
-  const auto kernel = many ? norm_ce_vec_kernel<false, 2> : norm_ce_vec_kernel<false, 1>;
+  const NormShape shape = norm_ce_shape(rows, dim, false);
+  const auto kernel = shape.late ? norm_ce_vec_kernel<false, 4, true> : shape.units == 2 ? norm_ce_vec_kernel<false, 2> : norm_ce_vec_kernel<false, 1>;
   if (dim % 8 == 0 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0)
-    launch_early(kernel, rows, norm_threads(dim, many ? 2 : 1), 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
+    launch_early(kernel, rows, norm_threads(dim, shape.units), norm_smem(rows, dim), as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
                  rows == 1 ? 1 : 0, (__half *)out, MixArgs{});
   else
     launch_early(norm_ce_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps,
@@ -856,9 +868,8 @@ extern "C" int pt_rms_norm(const void *x, const void *residual, const void *gamm
   PT_REQUIRE(rows > 0 && dim > 0, "pt_rms_norm: bad shape [%d, %d]", rows, dim);
   PT_REQUIRE(!residual || sum_out, "pt_rms_norm: residual given without sum_out");
   const bool vec = dim % 8 == 0 && dim <= 8 * 8 * 256 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)residual | (uintptr_t)sum_out) & 15) == 0;
-  const auto kernel = dim <= 8192 ? rms_norm_vec_kernel<1> : rms_norm_vec_kernel<2>;
   if (vec)
-    launch_early(kernel, rows, norm_threads(dim, dim <= 8192 ? 1 : 2), 0, as_stream(stream), (const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
+    launch_early(rms_norm_vec_kernel, rows, norm_threads(dim, 2), norm_smem(rows, dim), as_stream(stream), (const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
                                                             (__half *)out, (__half *)sum_out);
   else
     launch_early(rms_norm_kernel, rows, 256, 0, as_stream(stream), (const __half *)x, (const __half *)residual, (const __half *)gamma, dim, eps,
@@ -1049,7 +1060,9 @@ extern "C" int pt_norm_ce_mix(const void *x, const void *gamma, const void *beta
                         (uintptr_t)out_a | (uintptr_t)out_b | (uintptr_t)out_c;
   PT_REQUIRE((all & 15) == 0, "pt_norm_ce_mix: all pointers must be 16-byte aligned");
   const MixArgs m{(__half *)state, {(const __half *)mix_a, (const __half *)mix_b, (const __half *)mix_c}, {(__half *)out_a, (__half *)out_b, (__half *)out_c}};
-  launch_early(norm_ce_vec_kernel<true, 1>, rows, norm_threads(dim, 1), 0, as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps, rows == 1 ? 1 : 0,
+  const NormShape shape = norm_ce_shape(rows, dim, true);
+  const auto kernel = shape.late ? norm_ce_vec_kernel<true, 4, true> : shape.units == 2 ? norm_ce_vec_kernel<true, 2> : norm_ce_vec_kernel<true, 1>;
+  launch_early(kernel, rows, norm_threads(dim, shape.units), norm_smem(rows, dim), as_stream(stream), (const __half *)x, (const __half *)gamma, (const __half *)beta, dim, eps, rows == 1 ? 1 : 0,
                (__half *)nullptr, m);
   PT_LAUNCH_CHECK("pt_norm_ce_mix");
   return PT_OK;
