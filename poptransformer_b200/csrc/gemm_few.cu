@@ -258,7 +258,7 @@ template <bool BF16, bool EXT> static cudaError_t launch(const Params &p, const 
 
 // Whether a product of checked arguments (pt_gemm) is one of these kernels'.
 bool takes(const pt_gemm_args &a) {
-  return (a.wfmt == PT_W_FP16 || a.wfmt == PT_W_BF16) && a.ksplit <= 0 && !a.n_parts && a.epilogue != PT_EPI_GATED_RESIDUAL && !(a.ext && a.ext->n_groups > 0) && small(a.m, a.n_out, a.k_in);
+  return (a.wfmt == PT_W_FP16 || a.wfmt == PT_W_BF16) && a.ksplit <= 0 && !a.n_parts && a.epilogue != PT_EPI_GATED_RESIDUAL && !(a.ext && a.ext->n_groups > 0) && small(a.m, a.n_out, a.k_in) && pays(a.n_out, a.k_in, sm_count());
 }
 cudaError_t run(const pt_gemm_args &a, int out_ld, cudaStream_t st) {
   const bool bf16 = a.wfmt == PT_W_BF16;

@@ -22,9 +22,18 @@ struct Plan {
 };
 constexpr int ceil_to(int a, int b) { return (a + b - 1) / b; }
 
-// Which products are faster here than in tensor memory (gemm_few.cu has the times): up to eight rows, of matrices up to 8 MB or of a short k, where a block's
-// tile is over before it has begun (50257 x 768 at 8 rows: 14.6 us and 17.2).
+// Which products may come here: up to eight rows, of matrices up to 8 MB or of a short k, where a block's tile is over before it has begun.
 static inline bool small(int m, int n_out, int k_in) { return m <= ROWS && (k_in <= 1024 || (long long)n_out * k_in <= 1 << 22); }
+
+// ... and which of them are faster here than in tensor memory (gemm_few.cu has the times of small ones).  Not large ones whose tiles of 128 weight rows fill the last round
+// there (two a SM) to four fifths: 32003 x 512 at 1 row 6.2 us there and 6.8 here, 65536 x 768 17.1 and 18.4; where they leave more of it empty it is the other
+// way: 50257 x 768 15.8 and 12.9, 20000 x 1024 9.3 and 8.1, 16384 x 1024 7.2 and 6.8.  Nor large ones of k up to 256, of which one or two stages are all: 16384 x 256 3.1
+// there, 3.4 here; unless the tiles are more than a round (50257 x 256 7.4, 5.8).
+static inline bool pays(int n_out, int k_in, int sms) {
+  const int tiles = ceil_to(n_out, 128), rounds = ceil_to(tiles, 2 * sms);
+  const bool filled = tiles * 5 >= rounds * 2 * sms * 4;
+  return k_in <= 256 ? n_out <= 8192 || (rounds > 1 && !filled) : (long long)n_out * k_in <= 1 << 22 || !filled;
+}
 
 static inline Plan split(int n_units, int n_kb, int units, int warps_k, int slices) {
   Plan p{units, warps_k, slices, 0, 0, 0, 0, 0, 0};
@@ -42,8 +51,14 @@ static inline Plan split(int n_units, int n_kb, int units, int warps_k, int slic
 // The split with the least time by a linear model of what a block does (us: k blocks of a warp, a cluster's meeting, activations and weights to fetch, parts
 // of a sum, warps), fitted on B200 to 24 sizes of 640 x 2048 .. 2048 x 2048 and 8000 x 512 at 1 and 8 rows, some 100 splits of each: what it takes is
 // on average 4 % above the best.  (Up to 1024 k clusters give 0.1 us at most: none.)  More blocks than SMs only if they are small, so that they share the SMs.
+// Matrices of more than twice the size that it was fitted to take rounds of two blocks an SM: us at 8 rows by the model / so, fp16, 12288 x 1024 8.0 / 6.6, 16384 x 768 6.5 / 5.7, 20000 x 1024
+// 9.5 / 8.2, 50257 x 768 14.1 / 13.3, 128256 x 1024 48.6 / 43.4.
 static inline Plan make_plan(int m, int n_out, int k_in, int sms) {
   const int n_units = ceil_to(n_out, UNIT), n_kb = k_in / 64;
+  if ((long long)n_out * k_in > 1 << 23) {     // (k up to 1024) what counts is that the blocks fill every round of two an SM evenly
+    const int rounds = ceil_to(n_units, 2 * sms * MAX_WARPS), units = ceil_to(n_units, 2 * sms * rounds);
+    return split(n_units, n_kb, units, std::min(n_kb, units <= 2 ? 3 : units <= 5 ? 2 : 1), 1);
+  }
   Plan best = split(n_units, n_kb, MAX_WARPS, 1, 1);       // (many rounds of blocks)
   double least = 1e30;
   for (int units = 1; units <= MAX_WARPS; ++units)

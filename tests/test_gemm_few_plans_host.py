@@ -57,3 +57,38 @@ def test_plans_are_kept(tmp_path):
 def test_calls_take_the_kept_plan():
     text = open(os.path.join(CSRC, "gemm_few.cu")).read()
     assert "kept_plan(a.m, a.n_out, a.k_in, sm_count())" in text and "make_plan(a.m" not in text
+
+
+LARGE = r"""
+#include <cstdio>
+#include "gemm_few.h"
+using namespace pt::few;
+int main() {
+  for (int sms : {132, 148})
+    for (int n = 4097; n < 300000; n += 1 + n / 50)
+      for (int k : {64, 256, 320, 512, 768, 1024})
+        if (small(8, n, k) && pays(n, k, sms)) {
+          const Plan p = make_plan(8, n, k, sms);
+          printf("%d %d %d %d %d %d %d %d %u\n", sms, n, k, p.units, p.warps_k, p.slices, p.stages, p.blocks, p.smem);
+        }
+}
+"""
+
+
+def test_large_matrices_fill_their_rounds(tmp_path):
+    """Two blocks fit an SM, and no round of them is left nearly empty; with k up to 256 only where the other kernel's rounds are."""
+    (tmp_path / "plan.cpp").write_text(LARGE)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, "-o", str(tmp_path / "plan"), str(tmp_path / "plan.cpp")], check=True)
+    lines = subprocess.run([str(tmp_path / "plan")], check=True, capture_output=True, text=True).stdout.splitlines()
+    assert len(lines) > 500
+    for line in lines:
+        sms, n, k, units, warps, slices, stages, blocks, smem = map(int, line.split())
+        tiles, places = -(-n // 128), 2 * sms
+        filled = tiles / (-(-tiles // places) * places)
+        if n * k > 1 << 23:
+            assert slices == 1 and units * warps <= 12 and stages >= 2 and 2 * (smem + 2048) <= 228 * 1024, line
+            assert blocks / (-(-blocks // places) * places) >= 0.6, line           # (0.56 and less: 32003 x 512 took half as long again)
+        if n * k > 1 << 22 and k > 256:
+            assert filled < 0.8, line
+        if k <= 256 and n > 8192:
+            assert tiles > places, line
