@@ -471,7 +471,9 @@ extern "C" size_t pt_attn_workspace_bytes(int batch, int n_head, int head_dim, i
 
 // Warps per block and blocks per cluster that share the keys of one of `units` (sequence, kv head, part).  Sixteen warps fit an SM whatever the block, so
 // blocks get as many as keep all units on the SMs at once.  A cluster's meeting costs 0.5 to 1 us: it is worth it where a unit's table has 20
-// chunks for each block (of 16 warps), and as long as every block has an SM (clusters of sixteen: of a GPC).  Measured on B200, us a launch in a row of
+// chunks for each block (of 16 warps), and as long as every block has an SM (clusters of sixteen: of a GPC).  The table's room decides, since the step is not
+// known here: at context 10 in room for 2048 a cluster takes 4.2 us where one block took 3.9 (12 heads of 64), at 100 and more it is ahead (4.3 and 6.5).  Leaving
+// histories of one page to the first block mends the former and costs every other launch of a cluster 0.12 us: not done.  Measured on B200, us a launch in a row of
 // launches, of (rows, q heads, kv heads, head width, context, room) the kernel before / as warps x blocks:
 //   (1, 12, 12, 64, 159, 352)     6.4 / 8x1 3.6, 16x1 3.8, 4x1 4.6, 16x2 4.2         (16, 25, 25, 64, 255, 448)    11.8 / 4x1 8.1, 8x1 9.3, 4x2 11.2
 //   (1, 32, 32, 128, 511, 704)    8.0 / 16x4 5.2, 16x2 6.1, 16x1 7.8, 8x4 5.8        (4, 32, 32, 128, 511, 704)    12.7 / 16x1 8.3, 8x2 9.2, 16x2 13.3

@@ -239,14 +239,14 @@ def gemm(x, gw, out=None, x_scale=1.0, epilogue=EPI_STORE, residual=None, worksp
     m, k = x.shape[0] // (len(parts) if parts else 1), x.shape[1]
     if k != gw.k_in:
         raise PtError(f"gemm: x has k={k}, weight has k={gw.k_in}")
-    if parts and x.shape[0] % len(parts):
-        raise PtError(f"gemm: {len(parts)} parts want as many equal runs of rows, x has {x.shape[0]} rows")
-    for o, _ in parts or ():       # (what the kernel gets of a part is a pointer and its width)
-        if o.dim() != 2 or o.shape[0] != m or o.dtype != torch.float16:
-            raise PtError(f"gemm: the output of a part is float16 [{m}, n], got {o.dtype} {tuple(o.shape)}")
     if out is None and not parts:
         out = torch.empty((m, gw.n_out // 2 if epilogue == EPI_SWIGLU else gw.n_out), dtype=torch.float16, device=x.device)
     if parts:
+        if x.shape[0] != m * len(parts):
+            raise PtError(f"gemm: {len(parts)} parts want as many equal runs of rows, x has {x.shape[0]} rows")
+        for o, _ in parts:       # (what the kernel gets of a part is a pointer and its width)
+            if o.dim() != 2 or o.shape[0] != m or o.dtype != torch.float16:
+                raise PtError(f"gemm: the output of a part is float16 [{m}, n], got {o.dtype} {tuple(o.shape)}")
         table = (_lib.GemmPart * len(parts))(*[_lib.GemmPart(o.shape[1], e, _ptr(o)) for o, e in parts])
     _gemm_launch(_ptr(x), m, gw, _ptr(out), DT_F16 if parts else dtype_code(out.dtype), out_ld, epilogue, float(x_scale), float(alpha), _ptr(residual), workspace, ksplit, error_flag, _ptr(bias), ext, pdl,
                  _ptr(gate), halve, table if parts else None)
